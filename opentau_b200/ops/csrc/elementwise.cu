@@ -57,11 +57,12 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float* v) {
 // ------------------------------------------------------------------------------------------ RMSNorm
 // One block per row.  mode: 0 = no weight, 1 = (1 + w), 2 = w.
 // Adaptive form: y = xhat * (1 + scale) + shift with scale/shift rows taken from `mod`
-// (row stride mod_stride, one mod row per `rows_per_mod` consecutive rows).
+// (row stride mod_stride; row `mod_idx[row]`, or one mod row per `rows_per_mod` consecutive rows).
 template <int MAXV>
 __global__ void rms_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long x_stride,
                                const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ mod,
-                               long long mod_stride, int rows_per_mod, __nv_bfloat16* __restrict__ y,
+                               long long mod_stride, int rows_per_mod, const int* __restrict__ mod_idx,
+                               __nv_bfloat16* __restrict__ y,
                                float* __restrict__ rstd_out, int H, float eps, int mode) {
   __shared__ float red[32];
   pdl_launch_dependents();
@@ -83,7 +84,7 @@ __global__ void rms_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long x_
   ss = block_sum(ss, red);
   const float rstd = rsqrtf(ss / H + eps);
   if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
-  const __nv_bfloat16* mrow = mod ? mod + (row / rows_per_mod) * mod_stride : nullptr;
+  const __nv_bfloat16* mrow = mod ? mod + (mod_idx ? mod_idx[row] : row / rows_per_mod) * mod_stride : nullptr;
 #pragma unroll
   for (int i = 0; i < MAXV; ++i) {
     int idx = threadIdx.x + i * blockDim.x;
@@ -648,7 +649,7 @@ __global__ void time_embed_kernel(const float* __restrict__ t, OutT* __restrict_
 template <typename VT>
 __global__ void euler_step_kernel(float* __restrict__ x, const VT* __restrict__ v, float dt,
                                   const unsigned char* __restrict__ frozen, const float* __restrict__ prefix,
-                                  long long rows, int D) {
+                                  __nv_bfloat16* __restrict__ x16, long long rows, int D) {
   pdl_launch_dependents();
   pdl_wait();
   const long long total = rows * D;
@@ -660,6 +661,7 @@ __global__ void euler_step_kernel(float* __restrict__ x, const VT* __restrict__ 
     float xi = x[i] + dt * vi;
     if (frozen != nullptr && frozen[r]) xi = prefix[i];
     x[i] = xi;
+    if (x16 != nullptr) x16[i] = __float2bfloat16(xi);       // the next step's projection reads bf16
   }
 }
 
@@ -858,7 +860,10 @@ __global__ void resize_pad_kernel(const float* __restrict__ in, float* __restric
 // out = x + y * gate, gate row = gate + (row / rows_per_gate) * gate_stride.
 __global__ void gated_residual_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ y,
                                       const __nv_bfloat16* __restrict__ gate, long long gate_stride,
-                                      int rows_per_gate, __nv_bfloat16* __restrict__ out, long long rows, int H) {
+                                      int rows_per_gate, const int* __restrict__ gate_idx,
+                                      __nv_bfloat16* __restrict__ out, long long rows, int H) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long long nvec = rows * (long long)(H >> 3);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nvec;
        t += (long long)gridDim.x * blockDim.x) {
@@ -867,7 +872,7 @@ __global__ void gated_residual_kernel(const __nv_bfloat16* __restrict__ x, const
     float xv[8], yv[8], gv[8], o[8];
     load8(x + row * (long long)H + c, xv);
     load8(y + row * (long long)H + c, yv);
-    load8(gate + (row / rows_per_gate) * gate_stride + c, gv);
+    load8(gate + (gate_idx ? gate_idx[row] : row / rows_per_gate) * gate_stride + c, gv);
 #pragma unroll
     for (int e = 0; e < 8; ++e) o[e] = xv[e] + yv[e] * gv[e];
     store8(out + row * (long long)H + c, o);
@@ -910,12 +915,12 @@ typedef __nv_bfloat16 bf16;
   } while (0)
 
 extern "C" int otb_rms_fwd(const void* x, long long x_stride, const void* w, const void* mod, long long mod_stride,
-                           int rows_per_mod, void* y, float* rstd, long long rows, int H, float eps, int mode,
+                           int rows_per_mod, const int* mod_idx, void* y, float* rstd, long long rows, int H, float eps, int mode,
                            cudaStream_t stream) {
   if (H % 8 || rows <= 0) return -1;
   dim3 grid((unsigned)rows);
   LAUNCH_BY_H_PDL(rms_fwd_kernel, H, (const bf16*)x, x_stride, (const bf16*)w, (const bf16*)mod, mod_stride,
-                  rows_per_mod < 1 ? 1 : rows_per_mod, (bf16*)y, rstd, H, eps, mode);
+                  rows_per_mod < 1 ? 1 : rows_per_mod, mod_idx, (bf16*)y, rstd, H, eps, mode);
   return (int)cudaGetLastError();
 }
 
@@ -1033,13 +1038,13 @@ extern "C" int otb_time_embed(const float* t, void* out, long long rows, int dim
 }
 
 extern "C" int otb_euler_step(float* x, const void* v, int v_bf16, float dt, const unsigned char* frozen,
-                              const float* prefix, long long rows, int D, cudaStream_t stream) {
+                              const float* prefix, void* x16, long long rows, int D, cudaStream_t stream) {
   if (rows <= 0 || D <= 0 || (frozen != nullptr && prefix == nullptr)) return -1;
   const dim3 grid(grid_for(rows * D, 256));
   cudaError_t e = v_bf16 ? launch_pdl(euler_step_kernel<bf16>, grid, dim3(256), 0, stream, 0u, x, (const bf16*)v, dt,
-                                      frozen, prefix, rows, D)
+                                      frozen, prefix, (bf16*)x16, rows, D)
                          : launch_pdl(euler_step_kernel<float>, grid, dim3(256), 0, stream, 0u, x, (const float*)v, dt,
-                                      frozen, prefix, rows, D);
+                                      frozen, prefix, (bf16*)x16, rows, D);
   return (int)e;
 }
 
@@ -1115,12 +1120,12 @@ extern "C" int otb_resize_pad(const float* in, float* out, int NC, int Hin, int 
 }
 
 extern "C" int otb_gated_residual(const void* x, const void* y, const void* gate, long long gate_stride,
-                                  int rows_per_gate, void* out, long long rows, int H, cudaStream_t stream) {
+                                  int rows_per_gate, const int* gate_idx, void* out, long long rows, int H, cudaStream_t stream) {
   if (H % 8) return -1;
-  gated_residual_kernel<<<grid_for(rows * (H / 8), 256), 256, 0, stream>>>(
-      (const bf16*)x, (const bf16*)y, (const bf16*)gate, gate_stride, rows_per_gate < 1 ? 1 : rows_per_gate,
-      (bf16*)out, rows, H);
-  return (int)cudaGetLastError();
+  cudaError_t e = launch_pdl(gated_residual_kernel, dim3(grid_for(rows * (H / 8), 256)), dim3(256), 0, stream, 0u,
+                             (const bf16*)x, (const bf16*)y, (const bf16*)gate, gate_stride,
+                             rows_per_gate < 1 ? 1 : rows_per_gate, gate_idx, (bf16*)out, rows, H);
+  return (int)e;
 }
 
 // Status word helpers: the library owns one KernelStatus in device memory per device in use.

@@ -1,22 +1,25 @@
-// Weight-streaming bf16 GEMM for few rows (inference: a 51-token action suffix, a ~200-token prefix, a few hundred
-// vision patches) on sm_100a:   out[M,N] = X[M,K] * W[N,K]^T   with M small.
+// Weight-streaming bf16 GEMM for few rows (inference: one decoded token, a 50-token action suffix, a few hundred
+// candidate rows) on sm_100a:   out[M,N] = X[M,K] * W[N,K]^T.
 //
-// The persistent 128 x BN GEMM turns such a product into N/BN tiles: 8..40 CTAs stream the whole weight matrix while
-// a hundred SMs idle, and the weights of an M = 2-tile problem are fetched once per row tile.  Here the operands are
-// swapped and the reduction dimension is split:
+// What bounds it: a 4 - 17 MB weight matrix is 1 - 3 us of HBM time, so a launch of this kernel is a chain of latencies
+// (dependency wait, first load, MMA, cross-CTA reduction, store) and everything below is about keeping that chain short:
 //
-//   * the WEIGHT rows are the 128-row M operand of tcgen05.mma, the tokens are the N operand (64 / 128 / 256 wide),
-//     so every weight element crosses shared memory exactly once per 256 tokens and the accumulator
-//     D^T[128 weight rows, tokens] sits in TMEM with one weight row per lane;
-//   * K is split over the CTAs of a thread-block cluster (1 to 8): grid = (N/128, splits, token chunks), so even
-//     an N = 1024 projection puts 64 CTAs to work.  Each CTA leaves its fp32 partial tile in its own shared memory
-//     (the TMA ring is free by then), the cluster synchronises, and every CTA reduces 1/splits of the tile over
-//     distributed shared memory in fixed rank order (deterministic, no global workspace, no atomics) and applies the
-//     epilogue: bias, GELU, residual, bf16 / fp32 store, or the gated-MLP product on block-interleaved rows.
+//   * operands are swapped: the WEIGHT rows are the 128-row M operand of tcgen05.mma, the tokens are the N operand
+//     (any multiple of 16 up to 256), so every weight element crosses shared memory once per 256 tokens and the
+//     accumulator D^T[128 weight rows, tokens] sits in TMEM with one weight row per lane;
+//   * K is split over the CTAs of a thread-block cluster (1 to 8), grid = (N/128, splits, token chunks).  Tokens are
+//     dealt to the ranks; every CTA drains its fp32 partial tile into its own shared memory and sends each owner its
+//     tokens with ONE bulk copy that completes on the owner's mbarrier, so no cluster barrier stands between the last
+//     MMA and the epilogue and the sum reads local shared memory.  (Element-wise remote stores move about 12 bytes a
+//     clock: 1.5 us for 50 tokens, measured; remote loads between two cluster barriers were slower still.)  The sum
+//     runs in rank order: deterministic, no atomics, no workspace;
+//   * the first ring of weight tiles is requested before the dependency wait (weights do not depend on the preceding
+//     kernel), so under programmatic dependent launch its HBM latency overlaps the predecessor's tail;
+//   * ring depth follows from the shared memory that lets two CTAs share an SM: the next kernel of the chain can then
+//     become resident (and prefetch) while this one drains.
 //
-// Warp roles as in the big GEMM: warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 TMEM readers; all six warps take
-// part in the cluster reduction.  Every wait is bounded; a CTA whose wait gave up still arrives at both cluster
-// barriers, so its peers are never left waiting.
+// Warp roles: warp 0 TMA producer, warp 1 MMA issuer, warps 2..9 TMEM readers and epilogue.  Every
+// wait is bounded; a CTA whose wait gave up still sends its peers their (zero) partials and arrives at the barriers.
 #include "common.cuh"
 
 namespace otb {
@@ -25,6 +28,9 @@ constexpr unsigned KID_SKINNY = 4;
 constexpr int SK_BW = 128;  // weight rows per CTA (UMMA M)
 constexpr int SK_BK = 64;
 constexpr int SK_UMMA_K = 16;
+constexpr int SK_THREADS = 320;
+constexpr int SK_WORKERS = 256;
+constexpr int SK_MAX_STAGES = 12;
 
 enum SkinnyFlags {  // same values as the big GEMM's epilogue flags
   SK_BIAS = 1,
@@ -47,85 +53,64 @@ struct SkinnyParams {
   long long ldr;
   __nv_bfloat16* out2;
   long long ldo2;
-  const __nv_bfloat16* gate;      // rows of N gates; row (m / rows_per_gate), row stride gate_stride
+  const __nv_bfloat16* gate;      // rows of N gates; row (gate_idx ? gate_idx[m] : m / rows_per_gate), stride gate_stride
   long long gate_stride;
   int rows_per_gate;
+  const int* mod_idx;             // per output row: row of `gate` (null: m / rows_per_gate)
   int flags;
   int splits;
+  int stages;
+  int nt;
+  int stage_bytes;
+  int tmem_cols;
+  int buf_offset;                 // byte offset of the peers' partial tiles
+  int bar_offset;
   KernelStatus* status;
 };
 
-template <int NT, int STAGES>
-struct SkinnySmem {
-  static constexpr int W_BYTES = SK_BW * SK_BK * 2;
-  static constexpr int X_BYTES = NT * SK_BK * 2;
-  static constexpr int STAGE_BYTES = W_BYTES + X_BYTES;
-  static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
-  static constexpr int PARTIAL_BYTES = NT * SK_BW * 4;   // fp32 partial tile, overlays the ring after the last MMA
-  static_assert(PARTIAL_BYTES <= BAR_OFFSET, "partial tile does not fit in the ring");
-  static constexpr int TOTAL = BAR_OFFSET + (2 * STAGES + 1) * 8 + 16 + 1024;
-};
-
-__device__ __forceinline__ void cluster_sync_all() {
-  __syncwarp();   // the role branches above diverge inside warps 0 and 1; the aligned barrier wants whole warps
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+// Neither use of the cluster barrier publishes data (the bulk copies carry their own completion): relaxed arrivals.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ float ld_dsmem_f32(uint32_t local_addr, uint32_t rank) {
+__device__ __forceinline__ uint32_t map_rank(uint32_t local_addr, uint32_t rank) {
   uint32_t remote;
-  float v;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
-  return v;
+  return remote;
 }
-
-// sum of one partial-tile element over the S ranks of the cluster, in rank order; the loads are issued together
-__device__ __forceinline__ float reduce_ranks(uint32_t local_addr, int S) {
-  float v[8];
-#pragma unroll
-  for (int s = 0; s < 8; ++s) v[s] = s < S ? ld_dsmem_f32(local_addr, (uint32_t)s) : 0.f;
-  float acc = v[0];
-#pragma unroll
-  for (int s = 1; s < 8; ++s) acc += v[s];
-  return acc;
+// Bulk copy of `bytes` (a multiple of 16) from this CTA's shared memory to a peer's, counted on the peer's mbarrier.
+__device__ __forceinline__ void bulk_to_peer(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "r"(src), "r"(bytes), "r"(bar)
+               : "memory");
 }
+__device__ __forceinline__ void workers_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
-// bias / activation / residual / store of one element
-__device__ __forceinline__ void skinny_store(const SkinnyParams& p, int m, int n, float v) {
-  const int flags = p.flags;
-  if (flags & SK_BIAS) {
-    v += (flags & SK_BIAS_F32) ? __ldg(static_cast<const float*>(p.bias) + n)
-                               : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[n]);
-  }
-  if (flags & SK_ACT_GELU) v = gelu_tanh_f(v);
-  if (flags & SK_RESIDUAL) {
-    if (flags & SK_GATE) v *= __bfloat162float(p.gate[(long long)(m / p.rows_per_gate) * p.gate_stride + n]);
-    v += __bfloat162float(p.residual[(long long)m * p.ldr + n]);
-  }
-  if (flags & SK_OUT_F32) {
-    static_cast<float*>(p.out)[(long long)m * p.ldo + n] = v;
-  } else {
-    static_cast<__nv_bfloat16*>(p.out)[(long long)m * p.ldo + n] = __float2bfloat16(v);
-  }
-}
-
-template <int NT, int STAGES>
-__global__ void __launch_bounds__(192, NT <= 128 ? 2 : 1)
+// MAXT: tokens per CTA at most (64: two CTAs may share an SM; 256: one).
+// EPI >= 0: the epilogue flags are known at compile time (the products of a decoder layer); -1: any flags.
+template <int MAXT, int EPI>
+__global__ void __launch_bounds__(SK_THREADS, MAXT <= 64 ? 2 : 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant__ CUtensorMap tma_x,
                    SkinnyParams p) {
-  using L = SkinnySmem<NT, STAGES>;
+  constexpr int W_BYTES = SK_BW * SK_BK * 2;
+  const int NT = p.nt;                               // tokens per CTA, a multiple of 16
+  const int STAGE_BYTES = p.stage_bytes;             // weight tile + token tile, rounded up to the swizzle atom
+  const int X_LOAD = NT * SK_BK * 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::BAR_OFFSET);
-  uint64_t* empty_bar = full_bar + STAGES;
-  uint64_t* tfull_bar = empty_bar + STAGES;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull_bar + 1);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + p.bar_offset);
+  uint64_t* empty_bar = full_bar + SK_MAX_STAGES;
+  uint64_t* tfull_bar = empty_bar + SK_MAX_STAGES;
+  uint64_t* recv_bar = tfull_bar + 1;                // the peers' partials of my tokens have landed
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(recv_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* partial = reinterpret_cast<float*>(smem);   // [token][128 weight rows], valid after the last MMA retired
+  // partial tiles, [token][128 weight rows]: mine of all tokens goes over the ring (my MMAs have retired by then), the
+  // other ranks' partials of MY tokens into buffers of their own (they may arrive while my MMAs still read the ring)
+  float* own_part = reinterpret_cast<float*>(smem);
+  float* peer_part = reinterpret_cast<float*>(smem + p.buf_offset);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -134,34 +119,33 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
   const int n0 = blockIdx.x * SK_BW;
   const int m_base = blockIdx.z * NT;
   const int m_valid = min(NT, p.M - m_base);
+  const int tpr = (m_valid + S - 1) / S;             // tokens a rank owns
+  const int t0 = split * tpr, own = max(0, min(tpr, m_valid - t0));      // my tokens: [t0, t0 + own)
   const int num_kb = (p.K + SK_BK - 1) / SK_BK;
   const int per = (num_kb + S - 1) / S;
   const int kb0 = split * per;
-  const int kb1 = min(num_kb, kb0 + per);
-  const int nkb = max(kb1 - kb0, 0);
-  const bool glu = (p.flags & (SK_GLU_GELU | SK_GLU_SILU)) != 0;
-  const bool direct = S == 1 && !glu;                // straight from TMEM to global memory
+  const int nkb = max(min(num_kb, kb0 + per) - kb0, 0);
+  const int stages = p.stages;
+  const int early = min(stages, nkb);
 
-  const int early = min(STAGES, nkb);
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
     mbar_init(tfull_bar, 1);
+    mbar_init(recv_bar, 1);
     *abort_flag = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&tma_x);
-    // The weights do not depend on the preceding kernel: the first ring of weight tiles is requested at once, before
-    // the TMEM allocation, the block barrier and the dependency wait, so that their HBM latency overlaps all three
-    // (and, under programmatic dependent launch, the predecessor's tail).  Activations follow after the wait.
     for (int i = 0; i < early; ++i) {
-      mbar_expect_tx(&full_bar[i], L::STAGE_BYTES);
-      tma_load_2d(smem + i * L::STAGE_BYTES, &tma_w, &full_bar[i], (kb0 + i) * SK_BK, n0);
+      mbar_expect_tx(&full_bar[i], W_BYTES + X_LOAD);
+      tma_load_2d(smem + i * STAGE_BYTES, &tma_w, &full_bar[i], (kb0 + i) * SK_BK, n0);
     }
+    tma_prefetch_desc(&tma_x);
+    if (S > 1) mbar_expect_tx(recv_bar, (uint32_t)((S - 1) * own * SK_BW * 4));
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, NT);   // 64 / 128 / 256 columns
+    tmem_alloc(tmem_slot, p.tmem_cols);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -169,27 +153,32 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_launch_dependents();                 // after the TMEM allocation (see common.cuh)
+  if (S > 1) cluster_arrive();             // waited for in front of the first copy to a peer: all have started
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
+    pdl_wait();
     if (elect_one()) {
-      pdl_wait();
       for (int i = 0; i < early; ++i)
-        tma_load_2d(smem + i * L::STAGE_BYTES + L::W_BYTES, &tma_x, &full_bar[i], (kb0 + i) * SK_BK, m_base);
-      int stage = early == STAGES ? 0 : early;
-      uint32_t phase = early == STAGES ? 1 : 0;
-      for (int kb = kb0 + early; kb < kb1; ++kb) {
+        tma_load_2d(smem + i * STAGE_BYTES + W_BYTES, &tma_x, &full_bar[i], (kb0 + i) * SK_BK, m_base);
+      int stage = early == stages ? 0 : early;
+      uint32_t phase = early == stages ? 1 : 0;
+      for (int i = early; i < nkb; ++i) {
         if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, KID_SKINNY, 1, stage)) break;
-        uint8_t* sw = smem + stage * L::STAGE_BYTES;
-        uint8_t* sx = sw + L::W_BYTES;
-        mbar_expect_tx(&full_bar[stage], L::STAGE_BYTES);
-        tma_load_2d(sw, &tma_w, &full_bar[stage], kb * SK_BK, n0);
-        tma_load_2d(sx, &tma_x, &full_bar[stage], kb * SK_BK, m_base);
-        if (++stage == STAGES) {
+        uint8_t* sw = smem + stage * STAGE_BYTES;
+        mbar_expect_tx(&full_bar[stage], W_BYTES + X_LOAD);
+        tma_load_2d(sw, &tma_w, &full_bar[stage], (kb0 + i) * SK_BK, n0);
+        tma_load_2d(sw + W_BYTES, &tma_x, &full_bar[stage], (kb0 + i) * SK_BK, m_base);
+        if (++stage == stages) {
           stage = 0;
           phase ^= 1;
         }
       }
+    }
+    __syncwarp();
+    if (S > 1) {
+      cluster_wait();
+      cluster_arrive();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
@@ -200,8 +189,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
       for (int i = 0; i < nkb; ++i) {
         if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, KID_SKINNY, 2, stage)) break;
         tc_fence_after();
-        const uint32_t sw = smem_u32(smem + stage * L::STAGE_BYTES);
-        const uint32_t sx = sw + L::W_BYTES;
+        const uint32_t sw = smem_u32(smem + stage * STAGE_BYTES);
+        const uint32_t sx = sw + W_BYTES;
 #pragma unroll
         for (int k = 0; k < SK_BK / SK_UMMA_K; ++k) {
           uint64_t wd = make_smem_desc(sw + k * 32u, 16u, 1024);
@@ -209,197 +198,309 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
           umma_ss(tmem_base, wd, xd, idesc, (i | k) != 0 ? 1u : 0u);
         }
         umma_commit(&empty_bar[stage]);
-        if (++stage == STAGES) {
+        if (++stage == stages) {
           stage = 0;
           phase ^= 1;
         }
       }
       umma_commit(tfull_bar);   // fires when every MMA above has retired (at once if there was none)
     }
+    __syncwarp();
+    if (S > 1) {
+      cluster_wait();
+      cluster_arrive();
+    }
   } else {
-    // ------------------------------------------------------------------ TMEM readers (warps 2..5)
-    pdl_wait();                                       // residual / gate / output buffers belong to the predecessor
-    const int quad = warp & 3;                        // TMEM lane quadrant this warp may read
-    const int wrow = quad * 32 + lane;                // weight row inside the tile
-    const int n = n0 + wrow;
-    bool ok = mbar_wait(tfull_bar, 0, abort_flag, p.status, KID_SKINNY, 3, 0);
-    tc_fence_after();
-    const uint32_t taddr = tmem_base + (uint32_t(quad * 32) << 16);
-    const int nchunk = (m_valid + 31) / 32;
-#pragma unroll 1
-    for (int c = 0; c < nchunk; ++c) {
-      uint32_t r[32];
-      if (nkb > 0 && ok) {
-        __syncwarp();
-        tmem_ld_x32(taddr + c * 32, r);
-        tmem_wait_ld();
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) r[j] = 0u;       // this split owns no k-block (or gave up): contributes zeros
+    const int wt = threadIdx.x - 64, ww = warp - 2;
+    pdl_wait();                                       // X, residual, gates and outputs belong to the predecessor
+    // ------------------------------------------------------------------ epilogue operands of my first token
+    const int flags = EPI >= 0 ? EPI : p.flags;
+    const bool glu = (flags & (SK_GLU_GELU | SK_GLU_SILU)) != 0;
+    const int n = n0 + lane * 4;
+    uint2 res_v = make_uint2(0u, 0u), gate_v = make_uint2(0u, 0u);
+    auto fetch_epi = [&](int t) {
+      if (t < own && (flags & SK_RESIDUAL) && n < p.N) {
+        const int m = m_base + t0 + t;
+        if (flags & SK_GATE)
+          gate_v = *reinterpret_cast<const uint2*>(
+              p.gate + (long long)(p.mod_idx ? __ldg(p.mod_idx + m) : m / p.rows_per_gate) * p.gate_stride + n);
+        res_v = *reinterpret_cast<const uint2*>(p.residual + (long long)m * p.ldr + n);
       }
-      if (direct) {
-        if (n < p.N) {
+    };
+    fetch_epi(ww);
+    float bias_v[4] = {0.f, 0.f, 0.f, 0.f};
+    if ((flags & SK_BIAS) && n < p.N) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int m = c * 32 + j;
-            if (m < m_valid) skinny_store(p, m_base + m, n, __uint_as_float(r[j]));
-          }
-        }
-      } else {
+      for (int e = 0; e < 4; ++e)
+        bias_v[e] = (flags & SK_BIAS_F32) ? __ldg(static_cast<const float*>(p.bias) + n + e)
+                                          : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[n + e]);
+    }
+    // ------------------------------------------------------------------ TMEM -> my partial tile -> the tokens' owners
+    const int quad = warp & 3;                        // TMEM lane quadrant this warp may read
+    const bool ok = mbar_wait(tfull_bar, 0, abort_flag, p.status, KID_SKINNY, 3, 0);
+    tc_fence_after();
+    {
+      const uint32_t taddr = tmem_base + (uint32_t(quad * 32) << 16);
+      float* col = own_part + quad * 32 + lane;       // weight row inside the tile
+      constexpr int CHUNK = MAXT > 64 ? 32 : 16;      // a chunk's tail past the last token is never looked at
+      const bool have = nkb > 0 && ok;                // a split without k-blocks (or one that gave up) sends zeros
+#pragma unroll 1
+      for (int c0 = (ww >> 2) * CHUNK; c0 < m_valid; c0 += 2 * CHUNK) {
+        uint32_t r[32];
+        __syncwarp();
+        if (CHUNK == 32) tmem_ld_x32(taddr + c0, r); else tmem_ld_x16(taddr + c0, r);
+        tmem_wait_ld();
+        if (!have) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int m = c * 32 + j;
-          if (m < m_valid) partial[m * SK_BW + wrow] = __uint_as_float(r[j]);
+          for (int j = 0; j < CHUNK; ++j) r[j] = 0u;
         }
+        float* dst = col + c0 * SK_BW;
+#pragma unroll
+        for (int j = 0; j < CHUNK; ++j) dst[j * SK_BW] = __uint_as_float(r[j]);
       }
     }
     tc_fence_before();
-  }
-
-  // ---------------------------------------------------------------------- cluster reduction + epilogue
-  cluster_sync_all();                                 // every CTA's partial tile is complete and visible
-  pdl_wait();                                         // warps 0 / 1 join the reduction: they write outputs too
-  if (!direct && !*abort_flag) {
-    const uint32_t pbase = smem_u32(partial);
-    if (!(p.flags & SK_NO_OUT)) {
-      // plain output: this rank reduces weight rows [r0, r0 + rows) (the last rank takes the remainder)
-      const int rows_per = (SK_BW + S - 1) / S, r0 = split * rows_per;
-      const int rows = max(0, min(rows_per, SK_BW - r0));
-      for (int i = threadIdx.x; i < m_valid * rows; i += blockDim.x) {
-        const int m = i / rows, wr = r0 + i % rows;
-        if (n0 + wr >= p.N) continue;
-        skinny_store(p, m_base + m, n0 + wr, reduce_ranks(pbase + (uint32_t)(m * SK_BW + wr) * 4u, S));
+    if (S > 1) fence_async_smem();                    // the bulk copies read what the workers have just written
+    workers_sync();
+    if (S > 1) {
+      cluster_wait();
+      if (wt < S && wt != split) {
+        const int owner = wt, cnt = min(tpr, m_valid - owner * tpr);
+        if (cnt > 0)
+          bulk_to_peer(map_rank(smem_u32(peer_part) + (uint32_t)(split < owner ? split : split - 1) * (uint32_t)tpr * (SK_BW * 4u),
+                                (uint32_t)owner),
+                       smem_u32(own_part) + (uint32_t)(owner * tpr) * (SK_BW * 4u), (uint32_t)cnt * (SK_BW * 4u),
+                       map_rank(smem_u32(recv_bar), (uint32_t)owner));
+      }
+      if (own > 0) mbar_wait(recv_bar, 0, abort_flag, p.status, KID_SKINNY, 5, 0);
+      __syncwarp();
+      cluster_arrive();                               // my tokens have all arrived; waited for before leaving
+    }
+    // ------------------------------------------------------------------ reduction + epilogue of my tokens
+    if (!*abort_flag) {
+#pragma unroll 1
+      for (int t = ww; t < own; t += SK_WORKERS / 32) {
+        const int m = m_base + t0 + t;
+        const uint2 rv = res_v, gv = gate_v;
+        fetch_epi(t + SK_WORKERS / 32);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int s = 0; s < S; ++s) {
+          const float* part = s == split ? own_part + t0 * SK_BW : peer_part + (s < split ? s : s - 1) * tpr * SK_BW;
+          const float4 u = reinterpret_cast<const float4*>(part + t * SK_BW)[lane];
+          v.x += u.x;
+          v.y += u.y;
+          v.z += u.z;
+          v.w += u.w;
+        }
+        const float f[4] = {v.x, v.y, v.z, v.w};
+        if (!(flags & SK_NO_OUT)) {
+          if (n < p.N) {
+            float o[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] = f[e] + bias_v[e];
+            if (flags & SK_ACT_GELU) {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) o[e] = gelu_tanh_f(o[e]);
+            }
+            if (flags & SK_RESIDUAL) {
+              if (flags & SK_GATE) {
+                const float2 g0 = unpack_bf16(gv.x), g1 = unpack_bf16(gv.y);
+                o[0] *= g0.x; o[1] *= g0.y; o[2] *= g1.x; o[3] *= g1.y;
+              }
+              const float2 q0 = unpack_bf16(rv.x), q1 = unpack_bf16(rv.y);
+              o[0] += q0.x; o[1] += q0.y; o[2] += q1.x; o[3] += q1.y;
+            }
+            if (flags & SK_OUT_F32) {
+              *reinterpret_cast<float4*>(static_cast<float*>(p.out) + (long long)m * p.ldo + n) =
+                  make_float4(o[0], o[1], o[2], o[3]);
+            } else {
+              *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.out) + (long long)m * p.ldo + n) =
+                  make_uint2(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]));
+            }
+          }
+        }
+        if (glu) {
+          // rows come in blocks of 32: [gate | up | gate | up]; a gate lane takes its up values from 8 lanes further
+          float o[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            // match the unfused path: gate / up are rounded to bf16 before the activation
+            const float up = __bfloat162float(__float2bfloat16(__shfl_down_sync(0xffffffffu, f[e], 8)));
+            const float g = __bfloat162float(__float2bfloat16(f[e]));
+            o[e] = ((flags & SK_GLU_GELU) ? gelu_tanh_f(g) : silu_f(g)) * up;
+          }
+          if (!(lane & 8) && n < p.N)
+            *reinterpret_cast<uint2*>(p.out2 + (long long)m * p.ldo2 + (n0 >> 1) + (lane >> 4) * 32 + (lane & 7) * 4) =
+                make_uint2(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]));
+        }
       }
     }
-    if (glu) {
-      // rows come in blocks of 32: [gate | up | gate | up]; 64 output columns per tile, split evenly over the ranks
-      const int units_per = (64 + S - 1) / S, u0 = split * units_per;
-      const int units = max(0, min(units_per, 64 - u0));
-      for (int i = threadIdx.x; i < m_valid * units; i += blockDim.x) {
-        const int m = i / units, u = u0 + i % units;
-        const int gr = (u >> 5) * 64 + (u & 31);      // gate row inside the tile; its up row is 32 further
-        if (n0 + (u >> 5) * 64 >= p.N) continue;
-        float g = reduce_ranks(pbase + (uint32_t)(m * SK_BW + gr) * 4u, S);
-        float up = reduce_ranks(pbase + (uint32_t)(m * SK_BW + gr + 32) * 4u, S);
-        // match the unfused path: gate / up are rounded to bf16 before the activation
-        g = __bfloat162float(__float2bfloat16(g));
-        up = __bfloat162float(__float2bfloat16(up));
-        const float a = (p.flags & SK_GLU_GELU) ? gelu_tanh_f(g) : silu_f(g);
-        p.out2[(long long)(m_base + m) * p.ldo2 + (n0 >> 1) + u] = __float2bfloat16(a * up);
-      }
-    }
   }
-  cluster_sync_all();                                 // nobody leaves while a peer may still read its shared memory
 
   // ---------------------------------------------------------------------- teardown
-  tc_fence_before();
   __syncthreads();
+  if (S > 1) cluster_wait();                         // every copy out of my shared memory has arrived at its owner
   if (warp == 1) {
     if (*abort_flag) {
       for (int i = 0; i < 2000; ++i) __nanosleep(1000);   // let TMA copies / MMAs in flight finish
     }
     __syncwarp();
     tc_fence_after();
-    tmem_dealloc(tmem_base, NT);
+    tmem_dealloc(tmem_base, p.tmem_cols);
   }
 }
 
 static int g_sk_sms = 0;
 
-template <int NT, int STAGES>
-static int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyParams& p, int n_tiles, int chunks,
-                         cudaStream_t stream) {
-  using L = SkinnySmem<NT, STAGES>;
+template <int MAXT, int EPI>
+static int launch_skinny_epi(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyParams& p, int n_tiles, int chunks,
+                         int smem_bytes, cudaStream_t stream) {
   static bool configured = false;
-  auto kern = gemm_skinny_kernel<NT, STAGES>;
+  auto kern = gemm_skinny_kernel<MAXT, EPI>;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  cudaError_t e = launch_pdl(kern, dim3((unsigned)n_tiles, (unsigned)p.splits, (unsigned)chunks), dim3(192, 1, 1),
-                             (size_t)L::TOTAL, stream, (unsigned)p.splits, tw, tx, p);
+  cudaError_t e = launch_pdl(kern, dim3((unsigned)n_tiles, (unsigned)p.splits, (unsigned)chunks),
+                             dim3(SK_THREADS, 1, 1), (size_t)smem_bytes, stream, (unsigned)p.splits, tw, tx, p);
   return (int)e;
+}
+
+// A launch runs its code once, from a cold instruction cache: at about nine cycles an instruction, code that is only
+// branched over costs as much as the loads it hides.  The flag sets of the decoder layers get code of their own.
+template <int MAXT>
+static int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyParams& p, int n_tiles, int chunks,
+                         int smem_bytes, cudaStream_t stream) {
+  switch (p.flags) {
+    case 0: return launch_skinny_epi<MAXT, 0>(tw, tx, p, n_tiles, chunks, smem_bytes, stream);
+    case SK_RESIDUAL: return launch_skinny_epi<MAXT, SK_RESIDUAL>(tw, tx, p, n_tiles, chunks, smem_bytes, stream);
+    case SK_RESIDUAL | SK_GATE:
+      return launch_skinny_epi<MAXT, SK_RESIDUAL | SK_GATE>(tw, tx, p, n_tiles, chunks, smem_bytes, stream);
+    case SK_NO_OUT | SK_GLU_GELU:
+      return launch_skinny_epi<MAXT, SK_NO_OUT | SK_GLU_GELU>(tw, tx, p, n_tiles, chunks, smem_bytes, stream);
+    default: return launch_skinny_epi<MAXT, -1>(tw, tx, p, n_tiles, chunks, smem_bytes, stream);
+  }
 }
 
 }  // namespace otb
 
 using namespace otb;
 
-// out[M,N] = X[M,K] W[N,K]^T (+ epilogue).  Returns 0, a CUDA / driver error code, or a negative argument-check code.
-// `splits_override`: 0 = choose (see the rule at the selection below).
-extern "C" int otb_gemm_skinny_bf16(const void* X, const void* W, void* out, int M, int N, int K, long long ldx,
-                                    long long ldw, long long ldo, const void* bias, const void* residual,
-                                    long long ldr, void* out2, long long ldo2, const void* gate,
-                                    long long gate_stride, int rows_per_gate, int flags, int splits_override,
-                                    void* status, cudaStream_t stream) {
-  if (M <= 0 || N <= 0 || K <= 0) return -2;
-  if ((ldx % 8) || (ldw % 8)) return -3;
-  if ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15) return -4;
+// Arguments of one launch (mirrored field by field by the ctypes structure of the Python launcher).
+struct OtbSkinnyArgs {
+  const void* x;
+  const void* w;
+  void* out;
+  const void* bias;
+  const void* residual;
+  void* out2;
+  const void* gate;
+  const int* mod_idx;
+  void* status;
+  long long ldx, ldw, ldo, ldr, ldo2, gate_stride;
+  int M, N, K;
+  int rows_per_gate, flags, splits;
+};
+
+// out[M,N] = X[M,K] W[N,K]^T (+ epilogue).  Returns 0, a CUDA / driver error code, or a negative argument-check
+// code.  `splits`: 0 = choose (see the rule at the selection below).
+extern "C" int otb_gemm_skinny_bf16(const OtbSkinnyArgs* a, cudaStream_t stream) {
+  const int M = a->M, N = a->N, K = a->K, flags = a->flags;
+  if (M <= 0 || N <= 0 || K <= 0 || (N % 8)) return -2;
+  if ((a->ldx % 8) || (a->ldw % 8)) return -3;
+  if ((reinterpret_cast<uintptr_t>(a->x) | reinterpret_cast<uintptr_t>(a->w)) & 15) return -4;
   if (flags & 4) return -9;                                  // accumulate-into-output is the big GEMM's job
-  if ((flags & SK_GATE) && (!(flags & SK_RESIDUAL) || gate == nullptr || rows_per_gate < 1)) return -10;
+  if ((flags & SK_RESIDUAL) && ((a->ldr % 4) || (reinterpret_cast<uintptr_t>(a->residual) & 7))) return -11;
+  if ((flags & SK_GATE) && (!(flags & SK_RESIDUAL) || a->gate == nullptr || (a->gate_stride % 4) ||
+                            (reinterpret_cast<uintptr_t>(a->gate) & 7)))
+    return -10;
+  if (a->rows_per_gate < 1) return -10;
   const bool glu = (flags & (SK_GLU_GELU | SK_GLU_SILU)) != 0;
-  if (glu && ((N % 64) || out2 == nullptr)) return -6;
-  if (!(flags & SK_NO_OUT) && out == nullptr) return -6;
+  if (glu && ((N % 64) || a->out2 == nullptr || (a->ldo2 % 4) || (reinterpret_cast<uintptr_t>(a->out2) & 7))) return -6;
+  if (!(flags & SK_NO_OUT) &&
+      (a->out == nullptr || (a->ldo % 4) || (reinterpret_cast<uintptr_t>(a->out) & ((flags & SK_OUT_F32) ? 15 : 7))))
+    return -6;
   if (g_sk_sms == 0) {
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_sk_sms, cudaDevAttrMultiProcessorCount, dev);
     if (g_sk_sms <= 0) return -7;
   }
-  const int nt = M <= 64 ? 64 : (M <= 128 ? 128 : 256);
-  const int chunks = (M + nt - 1) / nt;
+  // Tokens per CTA: as few chunks of at most 256 as cover M, all of one size (a multiple of the MMA's 16): 200 rows run
+  // as one 208-token tile, 400 as two, instead of padding to powers of two.
+  int chunks = (M + 255) / 256;
+  int nt = ((M + chunks - 1) / chunks + 15) / 16 * 16;
+  // my partial tile (over the ring) and the peers' partials of my tokens must fit side by side
+  const auto reduction_fits = [](int tokens, int s) {
+    return (((tokens + 31) / 32 * 32) + (tokens + s - 1) / s * (s - 1)) * SK_BW * 4 <= 222 * 1024;
+  };
   const int n_tiles = (N + SK_BW - 1) / SK_BW;
   const int num_kb = (K + SK_BK - 1) / SK_BK;
-  int splits = splits_override;
+  int splits = a->splits;
   if (splits == 0) {
-    // OPENTAU_B200_SKINNY_SLOTS: CTAs the automatic choice may fill, per SM (default 2 for the <= 128-token tiles);
-    // OPENTAU_B200_SKINNY_MAX_SPLITS caps the cluster size.  Tuning knobs for measurements.
-    static int slots_per_sm = -1, max_splits = -1;
-    if (slots_per_sm < 0) {
-      const char* e = getenv("OPENTAU_B200_SKINNY_SLOTS");
-      slots_per_sm = (e != nullptr && atoi(e) > 0) ? atoi(e) : 2;
-      e = getenv("OPENTAU_B200_SKINNY_MAX_SPLITS");
-      max_splits = (e != nullptr && atoi(e) >= 1 && atoi(e) <= 8) ? atoi(e) : 8;
-    }
-    // Largest cluster size whose grid is resident at once and leaves every CTA two k-blocks, with one refinement
-    // measured on the action-expert chains: going beyond ONE CTA per SM only pays while each CTA still streams four
-    // k-blocks; a 256-CTA launch of two-k-block CTAs fills every SM twice and keeps the next kernel of the chain
-    // (programmatic dependent launch) from becoming resident early.
-    const long long slots = (long long)g_sk_sms * (nt <= 128 ? slots_per_sm : 1);
+    // Largest cluster size whose grid is resident at once and leaves every CTA two k-blocks; going beyond ONE CTA per
+    // SM only pays while each CTA still streams four k-blocks (a launch of two-k-block CTAs that fills every SM twice
+    // keeps the next kernel of the chain from becoming resident early).
+    const long long slots = (long long)g_sk_sms * (nt <= 64 ? 2 : 1);
     splits = 1;
-    for (int s = 2; s <= max_splits; ++s) {
+    for (int s = 2; s <= 8; ++s) {
       const long long ctas = (long long)n_tiles * chunks * s;
-      if (ctas <= slots && num_kb / s >= 2 && (ctas <= g_sk_sms || num_kb / s >= 4)) splits = s;
+      if (ctas <= slots && num_kb / s >= 2 && (ctas <= g_sk_sms || num_kb / s >= 4) && reduction_fits(nt, s)) splits = s;
     }
   }
   if (splits < 1 || splits > 8) return -8;
+  if (!reduction_fits(nt, splits)) {                          // a forced split: narrower token tiles
+    chunks = (M + 127) / 128;
+    nt = ((M + chunks - 1) / chunks + 15) / 16 * 16;
+  }
+  // Shared memory: the ring (as deep as the CTA's k-blocks need or the budget gives; my own partial overlays it), the
+  // peers' partials behind it, barriers.  111 KB keeps two CTAs on an SM while there are at most 64 tokens;
+  // wider tiles take the SM alone.
+  const int stage_bytes = (SK_BW * SK_BK * 2 + nt * SK_BK * 2 + 1023) / 1024 * 1024;
+  const int tile_bytes = (nt <= 64 ? nt : (nt + 31) / 32 * 32) * SK_BW * 4;   // my partial tile, over the ring
+  const int buf_bytes = (nt + splits - 1) / splits * SK_BW * 4 * (splits - 1);
+  const int budget = nt > 64 ? 224 * 1024 : 111 * 1024;
+  const int tail = 1024 /* barriers */ + 1024 /* alignment */;
+  const int tile_over = tile_bytes > budget - tail - buf_bytes;
+  const int per = (num_kb + splits - 1) / splits;
+  int stages = (budget - tail - buf_bytes) / stage_bytes;
+  if (stages > per) stages = per;
+  if (stages > SK_MAX_STAGES) stages = SK_MAX_STAGES;
+  if (stages < 1 || tile_over) return -13;
+  const int ring = stages * stage_bytes > tile_bytes ? stages * stage_bytes : tile_bytes;
+  SkinnyParams p;
+  p.buf_offset = ring;
+  p.bar_offset = ring + buf_bytes;
+  const int smem_bytes = p.bar_offset + tail;
   CUtensorMap tw, tx;
   {
     uint64_t dims[2], strides[1];
     uint32_t box[2];
     dims[0] = (uint64_t)K; dims[1] = (uint64_t)N; box[0] = 64; box[1] = SK_BW;
-    strides[0] = (uint64_t)ldw * 2;
-    int r = make_tmap_bf16(&tw, W, 2, dims, strides, box);
+    strides[0] = (uint64_t)a->ldw * 2;
+    int r = make_tmap_bf16(&tw, a->w, 2, dims, strides, box);
     if (r) return 1000 + r;
     dims[0] = (uint64_t)K; dims[1] = (uint64_t)M; box[0] = 64; box[1] = (uint32_t)nt;
-    strides[0] = (uint64_t)ldx * 2;
-    r = make_tmap_bf16(&tx, X, 2, dims, strides, box);
+    strides[0] = (uint64_t)a->ldx * 2;
+    r = make_tmap_bf16(&tx, a->x, 2, dims, strides, box);
     if (r) return 2000 + r;
   }
-  SkinnyParams p;
   p.M = M; p.N = N; p.K = K;
-  p.out = out; p.ldo = ldo;
-  p.bias = bias;
-  p.residual = static_cast<const __nv_bfloat16*>(residual); p.ldr = ldr;
-  p.out2 = static_cast<__nv_bfloat16*>(out2); p.ldo2 = ldo2;
-  p.gate = static_cast<const __nv_bfloat16*>(gate); p.gate_stride = gate_stride; p.rows_per_gate = rows_per_gate;
+  p.out = a->out; p.ldo = a->ldo;
+  p.bias = a->bias;
+  p.residual = static_cast<const __nv_bfloat16*>(a->residual); p.ldr = a->ldr;
+  p.out2 = static_cast<__nv_bfloat16*>(a->out2); p.ldo2 = a->ldo2;
+  p.gate = static_cast<const __nv_bfloat16*>(a->gate); p.gate_stride = a->gate_stride;
+  p.rows_per_gate = a->rows_per_gate;
+  p.mod_idx = a->mod_idx;
   p.flags = flags;
   p.splits = splits;
-  p.status = static_cast<KernelStatus*>(status);
-  switch (nt) {
-    case 64: return launch_skinny<64, 4>(tw, tx, p, n_tiles, chunks, stream);
-    case 128: return launch_skinny<128, 3>(tw, tx, p, n_tiles, chunks, stream);
-    default: return launch_skinny<256, 4>(tw, tx, p, n_tiles, chunks, stream);
-  }
+  p.stages = stages;
+  p.nt = nt;
+  p.stage_bytes = stage_bytes;
+  p.tmem_cols = nt <= 32 ? 32 : (nt <= 64 ? 64 : (nt <= 128 ? 128 : 256));
+  p.status = static_cast<KernelStatus*>(a->status);
+  if (nt <= 64) return launch_skinny<64>(tw, tx, p, n_tiles, chunks, smem_bytes, stream);
+  return launch_skinny<256>(tw, tx, p, n_tiles, chunks, smem_bytes, stream);
 }

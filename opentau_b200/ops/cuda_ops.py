@@ -68,9 +68,34 @@ def use_skinny(layout: str, M: int, N: int, accumulate: bool, bn: int) -> bool:
     """``x @ W^T`` with few rows goes to the weight-streaming split-K kernel."""
     if not SKINNY or layout != "nt" or accumulate or bn:
         return False
-    # measured: up to 128 rows the split-K kernel always wins; a 129..256-row product keeps its advantage only while
-    # the 128 x 256 tiling has too few tiles (N <= 8192); beyond that the persistent kernel is faster
-    return M <= 128 or (M <= 256 and N <= 8192)
+    # measured inside a replayed graph: up to 64 rows the split-K kernel always wins (50 x 8192 x 1024 7.8 us against
+    # 10.2); at 65..256 rows only where the persistent kernel has too few tiles for the chip (200 x 1024 x 4096 14.5 us
+    # against 17.2, but 200 x 2560 x 1024 11.8 against 7.6)
+    return M <= 64 or (M <= 256 and N <= 2048)
+
+
+class _SkinnyArgs(ctypes.Structure):
+    """``OtbSkinnyArgs`` of ``csrc/gemm_skinny_tcgen05.cu``."""
+
+    _fields_ = ([(n, c_void_p) for n in ("x", "w", "out", "bias", "residual", "out2", "gate", "mod_idx", "status")]
+                + [(n, c_longlong) for n in ("ldx", "ldw", "ldo", "ldr", "ldo2", "gate_stride")]
+                + [(n, c_int) for n in ("M", "N", "K", "rows_per_gate", "flags", "splits")])
+
+
+def _ptr(t: Tensor | None) -> int | None:
+    return t.data_ptr() if t is not None else None
+
+
+def _skinny_launch(x: Tensor, w: Tensor, out: Tensor | None, M: int, N: int, K: int, flags: int, *, bias=None,
+                   residual=None, ldr: int = 0, out2=None, ldo2: int = 0, gate=None, gate_stride: int = 0,
+                   rows_per_gate: int = 1, mod_idx=None, splits: int = 0) -> None:
+    global launch_count
+    args = _SkinnyArgs(_ptr(x), _ptr(w), _ptr(out), _ptr(bias), _ptr(residual), _ptr(out2), _ptr(gate), _ptr(mod_idx),
+                       status_pointer(), x.stride(0), w.stride(0), out.stride(0) if out is not None else N, ldr, ldo2,
+                       gate_stride, M, N, K, rows_per_gate, flags, splits)
+    _check(_lib.load("gemm_skinny_tcgen05").otb_gemm_skinny_bf16(ctypes.byref(args), _stream()),
+           f"gemm_skinny[{M}x{N}x{K}]")
+    launch_count += 1
 
 
 def gemm(a: Tensor, b: Tensor, layout: str, bias: Tensor | None = None, residual: Tensor | None = None,
@@ -155,13 +180,14 @@ def gemm(a: Tensor, b: Tensor, layout: str, bias: Tensor | None = None, residual
         flags |= EPI_GATE
         g_stride, g_rows = gate.stride(0), M // gate.shape[0]
     if skinny:
-        rc = _lib.load("gemm_skinny_tcgen05").otb_gemm_skinny_bf16(
-            _p(a), _p(b), _p(out), c_int(M), c_int(N), c_int(K), c_longlong(a.stride(0)), c_longlong(b.stride(0)),
-            c_longlong(out.stride(0) if out is not None else N), _p(bias), _p(residual), c_longlong(ldr), _p(glu_out),
-            c_longlong(ldo2), _p(gate), c_longlong(g_stride), c_int(g_rows), c_int(flags), c_int(splits),
-            c_void_p(status_pointer()), _stream())
-        _check(rc, f"gemm_skinny[{M}x{N}x{K}]")
-        launch_count += 1
+        if residual is not None and (ldr % 4 or residual.data_ptr() % 8):
+            residual = residual.contiguous()
+            ldr = residual.stride(0)
+        if gate is not None and (gate.stride(0) % 4 or gate.data_ptr() % 8):
+            gate = gate.contiguous()
+            g_stride = gate.stride(0)
+        _skinny_launch(a, b, out, M, N, K, flags, bias=bias, residual=residual, ldr=ldr, out2=glu_out, ldo2=ldo2,
+                       gate=gate, gate_stride=g_stride, rows_per_gate=g_rows, splits=splits)
         if glu is not None:
             return glu_out if not store_out else (out, glu_out)
         return out
@@ -174,6 +200,81 @@ def gemm(a: Tensor, b: Tensor, layout: str, bias: Tensor | None = None, residual
     launch_count += 1
     if glu is not None:
         return glu_out if not store_out else (out, glu_out)
+    return out
+
+
+# --------------------------------------------------------------------------------------------- few-row products
+class RowNorm:
+    """The RMS norm in front of a product: ``weight`` (plain norms, ``unit_offset`` adds 1) or ``mod`` rows of
+    ``(scale | shift | gate)`` picked per row by ``idx`` (adaptive norms)."""
+
+    __slots__ = ("eps", "weight", "unit_offset", "mod", "idx")
+
+    def __init__(self, eps: float, weight: Tensor | None = None, unit_offset: bool = True, mod: Tensor | None = None,
+                 idx: Tensor | None = None):
+        self.eps, self.weight, self.unit_offset, self.mod, self.idx = eps, weight, unit_offset, mod, idx
+
+    def apply(self, x2: Tensor) -> Tensor:
+        """The norm as its own launch."""
+        global launch_count
+        R, H = x2.shape
+        y = torch.empty_like(x2)
+        wt = self.weight.to(torch.bfloat16).contiguous() if self.weight is not None else None
+        mode = 0 if wt is None else (1 if self.unit_offset else 2)
+        _check(_lib.load("elementwise").otb_rms_fwd(
+            _p(x2), c_longlong(x2.stride(0)), _p(wt), _p(self.mod),
+            c_longlong(self.mod.stride(0) if self.mod is not None else 0), c_int(1), _p(self.idx), _p(y), c_void_p(0),
+            c_longlong(R), c_int(H), c_float(self.eps), c_int(mode), _stream()), "rms_fwd")
+        launch_count += 1
+        return y
+
+    @property
+    def gate(self) -> Tensor | None:
+        return self.mod[:, 2 * (self.mod.shape[1] // 3):] if self.mod is not None else None
+
+
+def rows_linear(x: Tensor, w: Tensor, bias: Tensor | None = None, *, norm: RowNorm | None = None,
+                residual: Tensor | None = None, gated_by: RowNorm | None = None, glu: str | None = None,
+                out_f32: bool = False) -> Tensor:
+    """``x @ w^T`` for the rows of an inference pass: ``x (R, K)`` dense bf16, optionally normalised first (``norm``),
+    plus ``residual + gate * ...`` with the gate rows of the adaptive norm ``gated_by``, or the gated-MLP product
+    (``glu``).  The norm is a launch of its own: folded into the product's staging warps it measured slower (12.7 us
+    against 2.3 + 6.6 for 50 rows: the code that runs once per launch from a cold instruction cache outweighs the
+    launch)."""
+    global launch_count
+    R, K = x.shape
+    N = w.shape[0]
+    if norm is not None:
+        x = norm.apply(x)
+    gate = gated_by.gate if gated_by is not None else None
+    if not use_skinny("nt", R, N, False, 0):
+        if gate is not None:
+            y = gemm(x, w, "nt", bias=bias)
+            out = torch.empty_like(y)
+            _check(_lib.load("elementwise").otb_gated_residual(
+                _p(residual), _p(y), _p(gate), c_longlong(gate.stride(0)), c_int(1), _p(gated_by.idx), _p(out),
+                c_longlong(R), c_int(N), _stream()), "gated_residual")
+            launch_count += 1
+            return out
+        if glu is not None:
+            return gemm(x, w, "nt", glu=glu, store_out=False)
+        return gemm(x, w, "nt", bias=bias, residual=residual, out_dtype=torch.float32 if out_f32 else None)
+    flags, kw = 0, {}
+    if bias is not None:
+        flags |= EPI_BIAS | (EPI_BIAS_F32 if bias.dtype == torch.float32 else 0)
+    if residual is not None:
+        flags |= EPI_RESIDUAL
+        kw.update(residual=residual, ldr=residual.stride(0))
+    if gate is not None:
+        flags |= EPI_GATE
+        kw.update(gate=gate, gate_stride=gate.stride(0), mod_idx=gated_by.idx)
+    if glu is not None:
+        out = torch.empty(R, N // 2, dtype=torch.bfloat16, device=x.device)
+        flags |= EPI_NO_OUT | (EPI_GLU_GELU if glu == "gelu_tanh" else EPI_GLU_SILU)
+        _skinny_launch(x, w, None, R, N, K, flags, out2=out, ldo2=N // 2, **kw)
+        return out
+    out = torch.empty(R, N, dtype=torch.float32 if out_f32 else torch.bfloat16, device=x.device)
+    _skinny_launch(x, w, out, R, N, K, flags | (EPI_OUT_F32 if out_f32 else 0), bias=bias, **kw)
     return out
 
 
@@ -194,7 +295,7 @@ def rms_fwd(x: Tensor, w: Tensor | None, eps: float, unit_offset: bool):
     mode = 0 if w is None else (1 if unit_offset else 2)
     wt = w.to(torch.bfloat16).contiguous() if w is not None else None
     _check(_lib.load("elementwise").otb_rms_fwd(_p(x2), c_longlong(x2.stride(0)), _p(wt), c_void_p(0), c_longlong(0),
-                                                c_int(1), _p(y), _p(rstd), c_longlong(R), c_int(H), c_float(eps),
+                                                c_int(1), c_void_p(0), _p(y), _p(rstd), c_longlong(R), c_int(H), c_float(eps),
                                                 c_int(mode), _stream()), "rms_fwd")
     launch_count += 1
     return y.view(x.shape), rstd
@@ -250,7 +351,7 @@ def ada_rms_fwd(x: Tensor, mod: Tensor, eps: float):
     y = torch.empty(R, H, dtype=x.dtype, device=x.device)
     rstd = torch.empty(R, dtype=torch.float32, device=x.device)
     _check(_lib.load("elementwise").otb_rms_fwd(_p(x2), c_longlong(x2.stride(0)), c_void_p(0), _p(mod2),
-                                                c_longlong(mod2.stride(0)), c_int(rows_per_mod), _p(y), _p(rstd),
+                                                c_longlong(mod2.stride(0)), c_int(rows_per_mod), c_void_p(0), _p(y), _p(rstd),
                                                 c_longlong(R), c_int(H), c_float(eps), c_int(0), _stream()),
            "ada_rms_fwd")
     launch_count += 1
@@ -508,7 +609,7 @@ def gated_residual(x: Tensor, y: Tensor, gate: Tensor) -> Tensor:
     rows_per_gate = (B * S) // g2.shape[0]
     out = torch.empty_like(x2)
     _check(_lib.load("elementwise").otb_gated_residual(_p(x2), _p(y2), _p(g2), c_longlong(g2.stride(0)),
-                                                       c_int(rows_per_gate), _p(out), c_longlong(B * S), c_int(H),
+                                                       c_int(rows_per_gate), c_void_p(0), _p(out), c_longlong(B * S), c_int(H),
                                                        _stream()), "gated_residual")
     launch_count += 1
     return out.view(x.shape)
@@ -575,8 +676,10 @@ def time_embed(time: Tensor, dim: int, min_period: float, max_period: float, out
     return out
 
 
-def euler_step_(x: Tensor, v: Tensor, dt: float, frozen: Tensor | None = None, prefix: Tensor | None = None) -> Tensor:
-    """In place: ``x += dt * v``; rows with ``frozen`` set take ``prefix`` instead.  ``x`` fp32 contiguous (B,T,D)."""
+def euler_step_(x: Tensor, v: Tensor, dt: float, frozen: Tensor | None = None, prefix: Tensor | None = None,
+                x16: Tensor | None = None) -> Tensor:
+    """In place: ``x += dt * v``; rows with ``frozen`` set take ``prefix`` instead.  ``x`` fp32 contiguous (B,T,D).
+    ``x16``: a contiguous bf16 tensor of the same shape that receives a rounded copy."""
     global launch_count
     assert x.dtype == torch.float32 and x.is_contiguous() and v.shape == x.shape
     v = v.contiguous()
@@ -587,7 +690,8 @@ def euler_step_(x: Tensor, v: Tensor, dt: float, frozen: Tensor | None = None, p
         pf = prefix.float().contiguous()
     D = x.shape[-1]
     _check(_lib.load("elementwise").otb_euler_step(_p(x), _p(v), c_int(int(v.dtype == torch.bfloat16)), c_float(dt),
-                                                   _p(fz), _p(pf), c_longlong(x.numel() // D), c_int(D), _stream()),
+                                                   _p(fz), _p(pf), _p(x16), c_longlong(x.numel() // D), c_int(D),
+                                                   _stream()),
            "euler_step")
     launch_count += 1
     return x
