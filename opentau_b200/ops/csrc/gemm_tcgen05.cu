@@ -623,12 +623,24 @@ extern "C" int otb_gemm_bf16(const void* A, const void* B, void* out, int M, int
       !(a_mn_major && b_mn_major && N <= 2048))
     bn = 512;
   if (bn == 0) {
-    int m_tiles = (M + BM - 1) / BM;
-    if ((long long)m_tiles * ((N + 255) / 256) >= g_num_sms || N >= 4096) bn = 256;
-    else if ((long long)m_tiles * ((N + 127) / 128) >= g_num_sms / 2 || N >= 1024) bn = 128;
-    else bn = 64;
-    if (N <= 64) bn = 64;
-    else if (N <= 128 && bn > 128) bn = 128;
+    // Column tile of the one-CTA kernel: the cheapest of waves x k-blocks x (time per k-block) + drain, with the times
+    // measured on 200 - 968 rows (us per 64-deep k-block 0.20 / 0.21 / 0.35 and drain 1.3 / 2.3 / 4.0 for 64 / 128 / 256
+    // columns: the narrow tiles are bound by the load latency, so their k-blocks cost the same).  200 x 2560 x 1024 runs
+    // 7.6 us on 64 columns against 8.8 / 12.3, 968 x 2048 x 2048 13.6 us on 128 against 18.3 / 20.5.
+    const int cand[3] = {64, 128, 256};
+    const double per_kb[3] = {0.20, 0.21, 0.35}, drain[3] = {1.3, 2.3, 4.0};
+    const long long m_tiles = (M + BM - 1) / BM;
+    const double kbs = (K + BK - 1) / BK;
+    double best = 0;
+    for (int i = 0; i < 3; ++i) {
+      if (i > 0 && cand[i] >= 2 * N) break;                       // a tile at least half empty
+      const long long tiles = m_tiles * ((N + cand[i] - 1) / cand[i]);
+      const double t = (double)((tiles + g_num_sms - 1) / g_num_sms) * kbs * per_kb[i] + drain[i];
+      if (bn == 0 || t < best) {
+        best = t;
+        bn = cand[i];
+      }
+    }
   }
   CUtensorMap ta, tb;
   {
