@@ -235,6 +235,74 @@ class DualStreamDecoder(nn.Module):
                 outs.append(ops.dropout_gated_residual(y, layer.mlp(n), g2, drop.p, True))
         return outs, new_k, new_v
 
+    # -- few-row inference: one tower behind a cached prefix ----------------------------------------
+    def can_run_rows(self, ti: int, x: Tensor) -> bool:
+        """Whether :meth:`rows_pass` covers tower ``ti`` (pre-norm layers whose widths the vector loads take, weights
+        resident and dense); other towers take :meth:`forward`."""
+        cfg = self.towers[ti].cfg
+        w = self.towers[ti].layers[0].self_attn.qkv_proj.weight
+        return (ops.can_fuse_qkv_post(x, cfg.head_dim) and not cfg.sandwich_norms and self.param_gate is None
+                and not self.training and w.dtype == torch.bfloat16 and cfg.hidden_size % 8 == 0
+                and cfg.intermediate_size % 32 == 0 and (cfg.num_attention_heads * cfg.head_dim) % 8 == 0)
+
+    def rows_pass(self, ti: int, x: Tensor, cache: KVCache, q_blk: Tensor, q_valid: Tensor, k_blk: Tensor,
+                  k_valid: Tensor, tables, mods: list[Tensor] | None = None,
+                  mod_idx: Tensor | None = None) -> Tensor:
+        """Runs tower ``ti`` over ``x (B, T, d)``, appending the tokens' keys / values behind ``cache`` in place (the
+        cache's ``length`` is left as it is).
+
+        ``k_blk / k_valid`` cover ``cache.length + T`` keys; ``tables(theta)`` gives the rotary tables; ``mods[j]
+        (n, 3d)`` are the modulation rows of the tower's ``j``-th adaptive norm and ``mod_idx (B*T)`` picks one per
+        token.  Returns the hidden rows ``(B*T, d)`` before the final norm; :meth:`final_norm` names the norm the
+        caller's head applies."""
+        tower = self.towers[ti]
+        cfg = tower.cfg
+        B, T, d = x.shape
+        off, n_k = cache.length, cache.length + T
+        x2 = x.reshape(B * T, d)
+        for li in range(self.num_layers):
+            layer: DecoderLayer = tower.layers[li]
+            attn = layer.self_attn
+            n1 = self._row_norm(layer.input_layernorm, mods, 2 * li, mod_idx)
+            n2 = self._row_norm(layer.post_attention_layernorm, mods, 2 * li + 1, mod_idx)
+            qkv = ops.rows_linear(x2, attn.qkv_proj.weight, attn.qkv_proj.bias, norm=n1)
+            cos, sin = tables(self.towers[0].cfg.layer_theta(li))
+            kb, vb = cache.k[li], cache.v[li]
+            q, _, _ = ops.qkv_post(qkv.view(B, T, -1), cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim,
+                                   attn.q_norm if cfg.qk_norm else None, attn.k_norm if cfg.qk_norm else None, cos, sin,
+                                   kb[:, off:n_k], vb[:, off:n_k])
+            att = ops.block_attention(q, kb[:, :n_k], vb[:, :n_k], q_blk, k_blk, q_valid, k_valid, cfg.attn_scale)
+            x2 = ops.rows_linear(att.view(B * T, -1), attn.o_proj.weight, attn.o_proj.bias, residual=x2,
+                                 gated_by=n1 if mods is not None else None)
+            h = ops.rows_linear(x2, layer.mlp.gate_up_proj.weight, norm=n2, glu=layer.mlp.act)
+            x2 = ops.rows_linear(h, layer.mlp.down_proj.weight, residual=x2,
+                                 gated_by=n2 if mods is not None else None)
+        return x2
+
+    def rope_tables(self, ti: int, position_ids: Tensor, mrope: bool = False):
+        """``theta -> (cos, sin)`` of the given positions for tower ``ti``, computed once per base (Gemma-3 alternates
+        two bases)."""
+        cfg, cache = self.towers[ti].cfg, {}
+        if mrope and position_ids.dim() == 2:
+            position_ids = position_ids[None].expand(3, -1, -1)
+
+        def tables(theta: float) -> tuple[Tensor, Tensor]:
+            if theta not in cache:
+                cache[theta] = (ops.mrope_angles(position_ids, cfg.head_dim, theta, True, cfg.mrope_sections) if mrope
+                                else ops.rope_angles(position_ids, cfg.head_dim, theta))
+            return cache[theta]
+
+        return tables
+
+    def final_norm(self, ti: int, mods: list[Tensor] | None = None, mod_idx: Tensor | None = None):
+        return self._row_norm(self.towers[ti].norm, mods, 2 * self.num_layers, mod_idx)
+
+    @staticmethod
+    def _row_norm(norm, mods, j: int, mod_idx):
+        if mods is not None:
+            return ops.RowNorm(norm.eps, mod=mods[j], idx=mod_idx)
+        return ops.RowNorm(norm.eps, weight=norm.weight, unit_offset=norm.unit_offset)
+
     def forward(self, inputs_embeds: list[Tensor | None], position_ids: Tensor, q_blk: Tensor,
                 q_valid: Tensor, *, adarms_cond: list[Tensor | None] | None = None,
                 past: KVCache | None = None, fill_cache_len: int | None = None,

@@ -105,17 +105,20 @@ def flow_interpolate(actions: Tensor, noise: Tensor, time: Tensor):
 
 
 def euler_step(x_t: Tensor, v_t: Tensor, dt: float, frozen: Tensor | None = None,
-               action_prefix: Tensor | None = None) -> Tensor:
+               action_prefix: Tensor | None = None, x16: Tensor | None = None) -> Tensor:
     """One Euler step of the flow ODE, ``x_t + dt * v_t``, with rows of a committed action prefix (``frozen (B,T)``)
-    held at ``action_prefix``.  On CUDA the fp32 sample is updated in place by one kernel."""
+    held at ``action_prefix``.  On CUDA the fp32 sample is updated in place by one kernel, which also leaves a bf16 copy
+    in ``x16`` when that is given."""
     import torch
     if x_t.is_cuda and not oracle_mode() and x_t.dtype == torch.float32 and x_t.is_contiguous() \
             and not torch.is_grad_enabled():
         from . import cuda_ops
-        return cuda_ops.euler_step_(x_t, v_t, dt, frozen if action_prefix is not None else None, action_prefix)
+        return cuda_ops.euler_step_(x_t, v_t, dt, frozen if action_prefix is not None else None, action_prefix, x16)
     x = x_t + dt * v_t.to(x_t.dtype)
     if action_prefix is not None and frozen is not None:
         x = torch.where(frozen[:, :, None], action_prefix.to(x.dtype), x)
+    if x16 is not None:
+        x16.copy_(x)
     return x
 
 
@@ -183,6 +186,17 @@ def qkv_post(qkv: Tensor, heads: int, kv_heads: int, head_dim: int, q_norm, k_no
 
 def can_fuse_qkv_post(x: Tensor, head_dim: int) -> bool:
     return _native_nograd(x) and head_dim % 8 == 0 and head_dim <= 256
+
+
+def rows_linear(*args, **kw):
+    """Product of an inference pass over few rows with its norm, gate and residual (``cuda_ops.rows_linear``)."""
+    from . import cuda_ops
+    return cuda_ops.rows_linear(*args, **kw)
+
+
+def RowNorm(*args, **kw):
+    from . import cuda_ops
+    return cuda_ops.RowNorm(*args, **kw)
 
 
 def rope(x: Tensor, cos: Tensor, sin: Tensor) -> Tensor:

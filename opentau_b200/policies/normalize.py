@@ -239,6 +239,16 @@ class _StatsModule(nn.Module):
         self._snap_active = active
         return active
 
+    def _all_finite(self, stat: Tensor) -> bool:
+        """Whether no entry of a statistics buffer is infinite, looked at once per value of the buffer: the verdict of
+        every call would be a host synchronisation, and it can only change when the buffer is written or replaced."""
+        seen = self.__dict__.setdefault("_finite_seen", {})
+        key, state = id(stat), (stat.data_ptr(), stat._version)
+        hit = seen.get(key)
+        if hit is None or hit[0] is not stat or hit[1] != state:
+            hit = seen[key] = (stat, state, not bool(torch.isinf(stat).any()))
+        return hit[2]
+
     @property
     def num_heads(self) -> int:
         for p in self.parameters():
@@ -264,7 +274,8 @@ class _StatsModule(nn.Module):
                 idx = torch.zeros(x.shape[0], dtype=torch.long, device=x.device)
             a_name, b_name = stat_names_for_mode(mode)
             a, b = _rows(buf[a_name], idx, x), _rows(buf[b_name], idx, x)
-            if torch.isinf(a).any() or torch.isinf(b).any():
+            if not (self._all_finite(buf[a_name]) and self._all_finite(buf[b_name])) and \
+                    (torch.isinf(a).any() or torch.isinf(b).any()):
                 raise AssertionError(
                     f"`{a_name}`/`{b_name}` of '{key}' is infinity: initialise with per_dataset_stats, "
                     "call policy._inject_stats(...), or load a checkpoint that has the normalization buffers")

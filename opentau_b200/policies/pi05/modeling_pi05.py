@@ -498,30 +498,48 @@ class PI05FlowMatching(nn.Module):
         if bos is None or eos is None or pad is None:
             raise ValueError("response generation needs a tokenizer with bos, eos and pad ids")
         mrope = getattr(self, "_mrope", False)
-        tokens = torch.empty(B, 0, dtype=torch.long, device=device)
-        masks = torch.empty(B, 0, dtype=torch.bool, device=device)
+        L, base, dec = cfg.response_max_length, cache.length, pwe.decoder
+        d = pwe.vlm_cfg.hidden_size
+        probe = cache.k.new_empty(0, 1, d)
+        in_place = cache.writable_room() >= L and dec.can_run_rows(0, probe)
+        blk_all = self._const(("resp_blk", B, base, L, str(device)),
+                              lambda: torch.zeros(B, base + L, dtype=torch.int32, device=device))
+        valid_all = torch.cat([cache.valid[:, :base], torch.zeros(B, L, dtype=torch.bool, device=device)], dim=1)
+        one = torch.ones(B, 1, dtype=torch.bool, device=device)
+        tokens, lives = [], []
         offset = prefix_len.clone()
-        out = None
-        for step in range(cfg.response_max_length):
-            if step == 0:
-                nxt = torch.full((B, 1), bos, dtype=torch.long, device=device)
-            else:
-                nxt = ops.linear(out[:, -1:], pwe.lm_head_weight()).float().argmax(dim=-1)
-            if tokens.shape[1] > 1:
-                done = ((tokens == eos) | (tokens == pad)).any(dim=1, keepdim=True)
-                live = ~done
+        ended = None
+        logits = None
+        for step in range(L):
+            nxt = torch.full((B, 1), bos, dtype=torch.long, device=device) if step == 0 else logits.argmax(dim=-1)
+            live = one
+            if step > 1:
+                live = ~ended
                 nxt = torch.where(live, nxt, torch.full_like(nxt, pad))
-            else:
-                live = torch.ones(B, 1, dtype=torch.bool, device=device)
-            tokens, masks = torch.cat([tokens, nxt], 1), torch.cat([masks, live], 1)
+            tokens.append(nxt), lives.append(live)
+            stop = (nxt == eos) | (nxt == pad)
+            ended = stop if ended is None else ended | stop
             emb = pwe.embed_language_tokens(nxt)
             pos = offset                                            # a finished sample's pad takes no new position
             offset = offset + live.long()
+            if in_place:
+                n_k = base + step + 1
+                valid_all[:, n_k - 1:n_k] = live
+                past = KVCache(cache.k, cache.v, valid_all, base + step)
+                hid = dec.rows_pass(0, emb, past, blk_all[:, :1].contiguous(), live, blk_all[:, :n_k].contiguous(),
+                                    valid_all[:, :n_k].contiguous(), dec.rope_tables(0, pos, mrope))
+                if step + 1 < L:
+                    logits = ops.rows_linear(hid, pwe.lm_head_weight(), norm=dec.final_norm(0))[:, None]
+                continue
             blk, valid = ops.make_block_ids(live, torch.ones(B, 1, dtype=torch.long, device=device))
             (out, _), new = self.wrapper(inputs_embeds=[emb, None], position_ids=pos[None].expand(3, -1, -1) if mrope else pos,
                                          q_blk=blk, q_valid=valid, past=cache, fill_cache_len=1, mrope=mrope)
             cache = self._append_cache(cache, new, live)
-        return cache, offset, tokens, masks
+            if step + 1 < L:
+                logits = ops.linear(out[:, -1:], pwe.lm_head_weight())
+        if in_place:
+            cache = KVCache(cache.k, cache.v, valid_all, base + L)
+        return cache, offset, torch.cat(tokens, 1), torch.cat(lives, 1)
 
     @staticmethod
     def _append_cache(cache: KVCache, new: KVCache, valid: Tensor) -> KVCache:
@@ -602,6 +620,8 @@ class PI05FlowMatching(nn.Module):
         has_prefix = action_prefix is not None
         if has_prefix:               # committed actions enter every step unchanged ...
             x_t = torch.where(frozen[:, :, None], action_prefix.to(x_t.dtype), x_t)
+        if self._can_plan_loop(cache, x_t):
+            return self._planned_loop(cache, prefix_len, x_t, frozen, action_prefix, accel)
         for i in range(n):
             t = 1.0 + i * dt
             time = live * t          # frozen rows run at diffusion time 0
@@ -610,6 +630,63 @@ class PI05FlowMatching(nn.Module):
                 accel.update(v_t)
             # ... and are restored by the same kernel that takes the Euler step
             x_t = ops.euler_step(x_t, v_t, dt, frozen if has_prefix else None, action_prefix)
+        return x_t
+
+    def _can_plan_loop(self, cache: KVCache, x_t: Tensor) -> bool:
+        """Whether :meth:`_planned_loop` covers this policy: the suffix is the action chunk alone, conditioned on time
+        through adaptive norms (a subclass that changes either keeps the step-by-step loop)."""
+        cls, dec = type(self), self.wrapper.decoder
+        if cls.denoise_step is not PI05FlowMatching.denoise_step or cls.embed_suffix is not PI05FlowMatching.embed_suffix:
+            return False
+        ti, T = len(dec.towers) - 1, x_t.shape[1]
+        w_in = self.action_in_proj.weight
+        return (ti == 1 and cache.k.is_cuda and cache.k.shape[2] - cache.length >= T and T == self.config.chunk_size
+                and self.wrapper.expert_cfg.use_adarms and w_in.shape[1] % 8 == 0
+                and dec.can_run_rows(ti, cache.k.new_empty(0, T, w_in.shape[0])))
+
+    @torch.no_grad()
+    def _planned_loop(self, cache: KVCache, prefix_len: Tensor, x_t: Tensor, frozen: Tensor,
+                      action_prefix: Tensor | None, accel) -> Tensor:
+        """The Euler loop with everything that does not change from step to step computed once per chunk: masks,
+        rotary tables, and the time conditions of ALL steps (a token runs at its step's time, or at time 0 when it is
+        frozen, so ``n + 1`` distinct conditions cover the loop; the modulation weights, the largest matrix of the
+        expert, are then read once per chunk instead of once per step, and the rows need no per-token copy: kernels
+        pick them through an index)."""
+        cfg, dec = self.config, self.wrapper.decoder
+        n, ti = cfg.num_steps, len(self.wrapper.decoder.towers) - 1
+        dt = -1.0 / n
+        B, T, A = x_t.shape
+        device, dtype = x_t.device, self.action_in_proj.weight.dtype
+        if cache.writable_room() < T:          # best-of-N: the candidates share an expanded view of the prefix
+            cache = KVCache(cache.k.contiguous(), cache.v.contiguous(), cache.valid, cache.length)
+        times = self._const(("times", n, str(device)),
+                            lambda: torch.tensor([[1.0 + i * dt for i in range(n)] + [0.0]], device=device))
+        emb = ops.sinusoidal_time_embedding(times, self.action_in_proj.out_features, 4e-3, 4.0, out_dtype=dtype)
+        cond = F.silu(self.time_mlp_out(F.silu(self.time_mlp_in(emb))))
+        mods = [m[0] for m in dec._ada_mods(dec.towers[ti], cond)]
+        steps = self._const(("steps", n, str(device)), lambda: torch.arange(n, dtype=torch.int32, device=device)[:, None])
+        idx = torch.where(frozen.reshape(1, B * T), n, steps).to(torch.int32)
+        q_blk = self._const(("suffix_blk", B, T, str(device)),
+                            lambda: torch.ones(B, T, dtype=torch.int32, device=device))
+        q_valid = self._const(("suffix_valid", B, T, str(device)),
+                              lambda: torch.ones(B, T, dtype=torch.bool, device=device))
+        k_blk = self._const(("suffix_keys", B, cache.length, T, str(device)), lambda: torch.cat(
+            [torch.full((B, cache.length), ops.INT_MIN, dtype=torch.int32, device=device), q_blk], dim=1))
+        k_valid = torch.cat([cache.valid[:, :cache.length], q_valid], dim=1)
+        pos = prefix_len + self._const(("suffix_pos", T, str(device)), lambda: torch.arange(T, device=device)[None])
+        tables = dec.rope_tables(ti, pos, getattr(self, "_mrope", False))
+        x_t, x16 = x_t.contiguous(), x_t.to(dtype).contiguous()
+        fz = frozen.contiguous() if action_prefix is not None else None
+        for i in range(n):
+            x = ops.rows_linear(x16.view(B * T, A), self.action_in_proj.weight, self.action_in_proj.bias)
+            if cfg.use_modality_embedding:
+                x = x + self.action_modality_embedding.weight.to(x.dtype)
+            hid = dec.rows_pass(ti, x.view(B, T, -1), cache, q_blk, q_valid, k_blk, k_valid, tables, mods, idx[i])
+            v_t = ops.rows_linear(hid, self.action_out_proj.weight, self.action_out_proj.bias,
+                                  norm=dec.final_norm(ti, mods, idx[i]), out_f32=True).view(B, T, A)
+            if accel is not None:
+                accel.update(v_t)
+            x_t = ops.euler_step(x_t, v_t, dt, fz, action_prefix, x16)
         return x_t
 
     @torch.no_grad()
@@ -822,20 +899,12 @@ class PI05Policy(PreTrainedPolicy):
         ``accel_prefix`` set, ``last_accel`` / ``last_accel_provenance`` are published for the emitted chunk."""
         from ..accel import make_meter, publish
         from ..candidates import expand_candidates, pick, select_candidate, warn_if_no_candidate_scored
-        self.eval()
+        self._ensure_eval()
         cfg = self.config
         raw_state = self._delta_anchor_state(batch)          # before normalize_inputs: the raw state anchors the chunk
         B = batch["state"].shape[0]
         device = batch["state"].device
         idx = self._resolve_dataset_index(batch, B, device)
-        nb = self.normalize_inputs(batch, idx)
-        images, img_masks = self.prepare_images(nb)
-        lang_tokens, lang_masks = self.prepare_language(nb)
-        state = nb["state"]
-        if state.dim() == 3:
-            state = state[:, -1]
-        if action_prefix is not None:
-            action_prefix = self._model_space_prefix(action_prefix, raw_state, idx)
         n = int(n_candidates or getattr(self, "_n_candidates", None) or 1)
         critic = getattr(self, "_critic", None)
         if n > 1 and critic is None:
@@ -847,23 +916,37 @@ class PI05Policy(PreTrainedPolicy):
                                  "candidates.configure_candidates")
         sampler_idx = expand_candidates(idx, n)
         meter = make_meter(self, batch_size=B * n, device=device, dataset_index=sampler_idx)
-        st = state if cfg.state_type == "continuous" else None
+        if action_prefix is not None:
+            action_prefix = self._model_space_prefix(action_prefix, raw_state, idx)
         # the meter keeps host-side step counts, which a replayed graph would not advance: metered calls run eagerly
-        if getattr(self, "_use_graphs", False) and device.type == "cuda" and meter is None and not cfg.predict_response:
-            actions = self._graphed_sample(images, img_masks, lang_tokens, lang_masks, action_prefix, delay, noise,
-                                           st, n)
-        else:
-            actions = self.model.sample_actions(images, img_masks, lang_tokens, lang_masks,
-                                                action_prefix=action_prefix, delay=delay, noise=noise, state=st,
-                                                n_candidates=n, accel=meter,
-                                                prefix_kwargs=self._prefix_kwargs(batch, nb))
-        self.last_response = self._decode_response()
-        if n == 1:
-            # before the un-normalisation: if that raises (non-finite buffers) the score is still there
+        graphs = getattr(self, "_use_graphs", False) and device.type == "cuda" and meter is None
+        if graphs and self._request_fits_graph(batch):
+            actions = self._graphed_request(batch, idx, sampler_idx, action_prefix, delay, noise, n)
+            self.last_response = self._decode_response()
             publish(self, meter, dataset_index=idx)
-        feat = cfg.action_feature
-        real = feat.shape[0] if feat is not None else actions.shape[-1]
-        actions = self.unnormalize_outputs({"actions": actions[:, :, :real]}, sampler_idx)["actions"]
+        else:
+            nb = self.normalize_inputs(batch, idx)
+            images, img_masks = self.prepare_images(nb)
+            lang_tokens, lang_masks = self.prepare_language(nb)
+            state = nb["state"]
+            if state.dim() == 3:
+                state = state[:, -1]
+            st = state if cfg.state_type == "continuous" else None
+            if graphs and not cfg.predict_response:
+                actions = self._graphed_sample(images, img_masks, lang_tokens, lang_masks, action_prefix, delay, noise,
+                                               st, n)
+            else:
+                actions = self.model.sample_actions(images, img_masks, lang_tokens, lang_masks,
+                                                    action_prefix=action_prefix, delay=delay, noise=noise, state=st,
+                                                    n_candidates=n, accel=meter,
+                                                    prefix_kwargs=self._prefix_kwargs(batch, nb))
+            self.last_response = self._decode_response()
+            if n == 1:
+                # before the un-normalisation: if that raises (non-finite buffers) the score is still there
+                publish(self, meter, dataset_index=idx)
+            feat = cfg.action_feature
+            real = feat.shape[0] if feat is not None else actions.shape[-1]
+            actions = self.unnormalize_outputs({"actions": actions[:, :, :real]}, sampler_idx)["actions"]
         if raw_state is not None:
             # the dataset subtracted the chunk-start state from the mapped dims; without the other half the consumer
             # would read displacements as absolute joint targets
@@ -921,7 +1004,68 @@ class PI05Policy(PreTrainedPolicy):
     def enable_cuda_graphs(self, flag: bool = True) -> None:
         """Replay the sampler (prefix pass + Euler loop) from a CUDA graph: one launch per action chunk."""
         self._use_graphs = bool(flag)
-        self._graph_runner = None
+        self._graph_runner = self._sampler_runner = None
+        self._request_signature = None
+
+    def _ensure_eval(self) -> None:
+        """``self.eval()`` when anything the forward pass reads is in training mode (the recursion over every module
+        costs more than the host side of a replayed chunk)."""
+        if self.training or self.model.training or self.model.wrapper.training or self.model.wrapper.decoder.training:
+            self.eval()
+
+    def _request_fits_graph(self, batch) -> bool:
+        """Whether a whole request (normalisation, image preparation, sampler, un-normalisation) can be captured: the
+        prompt arrives tokenised, this policy's own preparation runs, and no zero-variance dim wants its host-side
+        report.  Otherwise only the sampler is replayed, or nothing."""
+        from .. import normalize
+        cls = type(self)
+        return ("lang_tokens" in batch and cls.prepare_images is PI05Policy.prepare_images
+                and cls._prefix_kwargs is PI05Policy._prefix_kwargs
+                and not (normalize.SNAP_WARN_TOL > 0 and self.normalize_inputs._snapping_possible()))
+
+    def _graphed_request(self, batch, idx, sampler_idx, action_prefix, delay, noise, n: int) -> Tensor:
+        """One request as ONE graph launch: input copies, replay, output copies."""
+        from ...runtime.graphs import CudaGraphRunner
+        cfg = self.config
+        B, device = batch["state"].shape[0], batch["state"].device
+        if noise is None:
+            noise = self.model.sample_noise((B * n, cfg.chunk_size, cfg.max_action_dim), device)
+        if action_prefix is None:
+            action_prefix = self.model._const(("no_prefix", B, str(device)), lambda: torch.zeros(
+                B, cfg.chunk_size, cfg.max_action_dim, device=device))
+        frozen = self.model.frozen_mask(delay, B, device)
+        keys = ["state", *sorted(k for k in batch if (k in cfg.image_features or k.startswith("camera"))
+                                 and isinstance(batch[k], Tensor))]
+        if batch.get("img_is_pad") is not None:
+            keys.append("img_is_pad")
+        feat = cfg.action_feature
+
+        def fn(values, idx, sampler_idx, lang_tokens, lang_masks, noise, action_prefix, frozen):
+            b = dict(zip(keys, values))
+            nb = self.normalize_inputs(b, idx)
+            images, img_masks = self.prepare_images(nb)
+            state = nb["state"]
+            state = state[:, -1] if state.dim() == 3 else state
+            actions = self.model.sample_actions(images, img_masks, lang_tokens, lang_masks, action_prefix=action_prefix,
+                                                noise=noise, frozen=frozen, n_candidates=n,
+                                                state=state if cfg.state_type == "continuous" else None)
+            real = feat.shape[0] if feat is not None else actions.shape[-1]
+            actions = self.unnormalize_outputs({"actions": actions[:, :, :real]}, sampler_idx)["actions"]
+            if cfg.predict_response:
+                return actions, self.model.last_response_tokens, self.model.last_response_masks
+            return (actions,)
+
+        # the captured kernels read the statistics by address: replaced buffers (an injection) mean a new capture
+        stats = tuple(p.data_ptr() for m in (self.normalize_inputs, self.unnormalize_outputs) for p in m.parameters())
+        signature = (tuple(keys), n, stats)
+        if getattr(self, "_graph_runner", None) is None or self._request_signature != signature:
+            self._request_signature, self._graph_runner = signature, CudaGraphRunner(fn)
+        out = self._graph_runner(tuple(batch[k] for k in keys), idx, sampler_idx, batch["lang_tokens"].to(device),
+                                 batch["lang_masks"].to(device).bool(), noise.float(), action_prefix.float(), frozen)
+        self.model.last_response_tokens = self.model.last_response_masks = None
+        if cfg.predict_response:
+            self.model.last_response_tokens, self.model.last_response_masks = out[1].clone(), out[2].clone()
+        return out[0].clone()
 
     def _graphed_sample(self, images, img_masks, lang_tokens, lang_masks, action_prefix, delay, noise, state, n):
         from ...runtime.graphs import CudaGraphRunner
@@ -934,14 +1078,14 @@ class PI05Policy(PreTrainedPolicy):
             action_prefix = torch.zeros(B, cfg.chunk_size, cfg.max_action_dim, device=device)
         frozen = self.model.frozen_mask(delay, B, device).contiguous()
         has_state = state is not None
-        if getattr(self, "_graph_runner", None) is None:
+        if getattr(self, "_sampler_runner", None) is None:
             def fn(images, img_masks, lang_tokens, lang_masks, noise, action_prefix, frozen, state):
                 return self.model.sample_actions(list(images), list(img_masks), lang_tokens, lang_masks,
                                                  action_prefix=action_prefix, noise=noise, frozen=frozen,
                                                  state=state if has_state else None, n_candidates=n)
-            self._graph_runner = CudaGraphRunner(fn)
+            self._sampler_runner = CudaGraphRunner(fn)
         st = state if has_state else torch.zeros(1, device=device)
-        out = self._graph_runner(tuple(images), tuple(img_masks), lang_tokens, lang_masks.bool(), noise.float(),
+        out = self._sampler_runner(tuple(images), tuple(img_masks), lang_tokens, lang_masks.bool(), noise.float(),
                                  action_prefix.float(), frozen, st)
         return out.clone()
 

@@ -47,7 +47,7 @@ class CudaGraphRunner:
     then replayed.  Outputs are returned as views of the graph's static output buffers: copy them if they
     must survive the next call."""
 
-    def __init__(self, fn: Callable, warmup: int = 2):
+    def __init__(self, fn: Callable, warmup: int = 1):
         self.fn, self.warmup = fn, warmup
         self._graphs: dict[tuple, tuple] = {}
 
