@@ -172,6 +172,33 @@ def _rows(stat: Tensor, index: Tensor, like: Tensor) -> Tensor:
     return g
 
 
+def _infinite_message(key: str, a_name: str, b_name: str) -> str:
+    return (f"`{a_name}`/`{b_name}` of '{key}' is infinity: initialise with per_dataset_stats, "
+            "call policy._inject_stats(...), or load a checkpoint that has the normalization buffers")
+
+
+def infinite_verdict(*modules: nn.Module):
+    """Asks once, behind the work queued so far, whether any statistic of ``modules`` is infinite; the returned function
+    waits for that answer alone and gives it.  Work queued in between runs meanwhile, so a caller that replays a graph
+    pays no idle GPU for the check."""
+    stats = [p.detach().reshape(-1) for m in modules for p in m.parameters()]
+    if not stats:
+        return lambda: False
+    found = torch.isinf(torch.cat(stats)).any()
+    if found.device.type != "cuda":
+        return lambda: bool(found)
+    flag = torch.empty((), dtype=torch.bool, pin_memory=True)
+    flag.copy_(found, non_blocking=True)
+    done = torch.cuda.Event()
+    done.record()
+
+    def verdict() -> bool:
+        done.synchronize()
+        return bool(flag)
+
+    return verdict
+
+
 class _StatsModule(nn.Module):
     inverse = False
 
@@ -239,15 +266,20 @@ class _StatsModule(nn.Module):
         self._snap_active = active
         return active
 
-    def _all_finite(self, stat: Tensor) -> bool:
-        """Whether no entry of a statistics buffer is infinite, looked at once per value of the buffer: the verdict of
-        every call would be a host synchronisation, and it can only change when the buffer is written or replaced."""
-        seen = self.__dict__.setdefault("_finite_seen", {})
-        key, state = id(stat), (stat.data_ptr(), stat._version)
-        hit = seen.get(key)
-        if hit is None or hit[0] is not stat or hit[1] != state:
-            hit = seen[key] = (stat, state, not bool(torch.isinf(stat).any()))
-        return hit[2]
+    def _stat_names(self, key: str) -> tuple[str, str] | None:
+        """The two statistics that feature ``key`` uses; None where it is passed through."""
+        mode = _mode_of(self.norm_map, self.features[key])
+        return None if mode is NormalizationMode.IDENTITY else stat_names_for_mode(mode)
+
+    def refuse_infinite(self, keys, dataset_index: Tensor) -> None:
+        """Raises if a row of statistics that ``forward`` would use for the features ``keys`` is infinite."""
+        for key in self.features:
+            names = self._stat_names(key) if key in keys else None
+            if names is None:
+                continue
+            buf = getattr(self, "buffer_" + key.replace(".", "_"))
+            if any(torch.isinf(buf[n].index_select(0, dataset_index.to(buf[n].device))).any() for n in names):
+                raise AssertionError(_infinite_message(key, *names))
 
     @property
     def num_heads(self) -> int:
@@ -256,7 +288,10 @@ class _StatsModule(nn.Module):
         return 1
 
     @torch.no_grad()
-    def forward(self, batch: dict[str, Tensor], dataset_index: Tensor | None = None) -> dict[str, Tensor]:
+    def forward(self, batch: dict[str, Tensor], dataset_index: Tensor | None = None,
+                check: bool = True) -> dict[str, Tensor]:
+        """``check=False``: the caller looks for infinite statistics itself (a captured graph cannot read a verdict
+        back; see :func:`infinite_verdict`)."""
         warn_missing_keys(self.features, batch, "unnormalization" if self.inverse else "normalization")
         batch = dict(batch)
         for key, ft in self.features.items():
@@ -274,11 +309,8 @@ class _StatsModule(nn.Module):
                 idx = torch.zeros(x.shape[0], dtype=torch.long, device=x.device)
             a_name, b_name = stat_names_for_mode(mode)
             a, b = _rows(buf[a_name], idx, x), _rows(buf[b_name], idx, x)
-            if not (self._all_finite(buf[a_name]) and self._all_finite(buf[b_name])) and \
-                    (torch.isinf(a).any() or torch.isinf(b).any()):
-                raise AssertionError(
-                    f"`{a_name}`/`{b_name}` of '{key}' is infinity: initialise with per_dataset_stats, "
-                    "call policy._inject_stats(...), or load a checkpoint that has the normalization buffers")
+            if check and (torch.isinf(a).any() or torch.isinf(b).any()):
+                raise AssertionError(_infinite_message(key, a_name, b_name))
             xf = x.to(torch.float32)
             watch = (not self.inverse and SNAP_WARN_TOL > 0 and not torch.compiler.is_compiling()
                      and not torch.onnx.is_in_onnx_export() and self._snapping_possible())

@@ -501,7 +501,8 @@ class PI05FlowMatching(nn.Module):
         L, base, dec = cfg.response_max_length, cache.length, pwe.decoder
         d = pwe.vlm_cfg.hidden_size
         probe = cache.k.new_empty(0, 1, d)
-        in_place = cache.writable_room() >= L and dec.can_run_rows(0, probe)
+        in_place = (cache.writable_room() >= L and dec.can_run_rows(0, probe)
+                    and pwe.lm_head_weight().shape[0] % 8 == 0)       # the few-row product stores eight logits at a time
         blk_all = self._const(("resp_blk", B, base, L, str(device)),
                               lambda: torch.zeros(B, base + L, dtype=torch.int32, device=device))
         valid_all = torch.cat([cache.valid[:, :base], torch.zeros(B, L, dtype=torch.bool, device=device)], dim=1)
@@ -1005,7 +1006,7 @@ class PI05Policy(PreTrainedPolicy):
         """Replay the sampler (prefix pass + Euler loop) from a CUDA graph: one launch per action chunk."""
         self._use_graphs = bool(flag)
         self._graph_runner = self._sampler_runner = None
-        self._request_signature = None
+        self._request_runners, self._request_stats = {}, None
 
     def _ensure_eval(self) -> None:
         """``self.eval()`` when anything the forward pass reads is in training mode (the recursion over every module
@@ -1023,8 +1024,11 @@ class PI05Policy(PreTrainedPolicy):
                 and cls._prefix_kwargs is PI05Policy._prefix_kwargs
                 and not (normalize.SNAP_WARN_TOL > 0 and self.normalize_inputs._snapping_possible()))
 
+    MAX_REQUEST_KINDS = 4       # captured kinds of request (cameras present, candidate counts) kept at a time
+
     def _graphed_request(self, batch, idx, sampler_idx, action_prefix, delay, noise, n: int) -> Tensor:
         """One request as ONE graph launch: input copies, replay, output copies."""
+        from .. import normalize
         from ...runtime.graphs import CudaGraphRunner
         cfg = self.config
         B, device = batch["state"].shape[0], batch["state"].device
@@ -1042,7 +1046,7 @@ class PI05Policy(PreTrainedPolicy):
 
         def fn(values, idx, sampler_idx, lang_tokens, lang_masks, noise, action_prefix, frozen):
             b = dict(zip(keys, values))
-            nb = self.normalize_inputs(b, idx)
+            nb = self.normalize_inputs(b, idx, check=False)
             images, img_masks = self.prepare_images(nb)
             state = nb["state"]
             state = state[:, -1] if state.dim() == 3 else state
@@ -1050,18 +1054,26 @@ class PI05Policy(PreTrainedPolicy):
                                                 noise=noise, frozen=frozen, n_candidates=n,
                                                 state=state if cfg.state_type == "continuous" else None)
             real = feat.shape[0] if feat is not None else actions.shape[-1]
-            actions = self.unnormalize_outputs({"actions": actions[:, :, :real]}, sampler_idx)["actions"]
+            actions = self.unnormalize_outputs({"actions": actions[:, :, :real]}, sampler_idx, check=False)["actions"]
             if cfg.predict_response:
                 return actions, self.model.last_response_tokens, self.model.last_response_masks
             return (actions,)
 
         # the captured kernels read the statistics by address: replaced buffers (an injection) mean a new capture
         stats = tuple(p.data_ptr() for m in (self.normalize_inputs, self.unnormalize_outputs) for p in m.parameters())
-        signature = (tuple(keys), n, stats)
-        if getattr(self, "_graph_runner", None) is None or self._request_signature != signature:
-            self._request_signature, self._graph_runner = signature, CudaGraphRunner(fn)
-        out = self._graph_runner(tuple(batch[k] for k in keys), idx, sampler_idx, batch["lang_tokens"].to(device),
-                                 batch["lang_masks"].to(device).bool(), noise.float(), action_prefix.float(), frozen)
+        if self._request_stats != stats:
+            self._request_runners, self._request_stats = {}, stats
+        signature = (tuple(keys), n, cfg.predict_response, cfg.response_max_length, cfg.num_steps)
+        runner = self._request_runners.pop(signature, None) or CudaGraphRunner(fn)
+        while len(self._request_runners) >= self.MAX_REQUEST_KINDS:        # the one that was used longest ago goes
+            self._request_runners.pop(next(iter(self._request_runners)))
+        self._request_runners[signature] = self._graph_runner = runner
+        infinite = normalize.infinite_verdict(self.normalize_inputs, self.unnormalize_outputs)
+        out = runner(tuple(batch[k] for k in keys), idx, sampler_idx, batch["lang_tokens"].to(device),
+                     batch["lang_masks"].to(device).bool(), noise.float(), action_prefix.float(), frozen)
+        if infinite():
+            self.normalize_inputs.refuse_infinite(keys, idx)
+            self.unnormalize_outputs.refuse_infinite(["actions"], sampler_idx)
         self.model.last_response_tokens = self.model.last_response_masks = None
         if cfg.predict_response:
             self.model.last_response_tokens, self.model.last_response_masks = out[1].clone(), out[2].clone()

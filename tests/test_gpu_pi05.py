@@ -4,7 +4,8 @@ replayed from a CUDA graph."""
 import pytest
 import torch
 
-from helpers import tiny_batch, tiny_pi05
+from helpers import tiny_batch, tiny_pi05, tiny_pi05_config
+from opentau_b200.datasets.synthetic import identity_stats
 
 pytestmark = pytest.mark.gpu
 
@@ -80,3 +81,42 @@ def test_cuda_graph_sampler_matches_eager():
     assert torch.equal(g1, g2)
     assert not torch.allclose(other, g1)
     assert pol._graph_runner.num_graphs == 1
+
+
+def test_replayed_requests_refuse_infinite_statistics_of_their_own_rows():
+    """Two datasets, the second without usable statistics: requests of the first are served, requests of the second are
+    refused, also when the graph is already captured and the buffer was written through ``.data``."""
+    from opentau_b200.policies.pi05.modeling_pi05 import PI05Policy
+    torch.manual_seed(2)
+    pol = PI05Policy(tiny_pi05_config("cuda"), per_dataset_stats=[identity_stats(), identity_stats()],
+                     dataset_names=["a", "b"]).to("cuda").to(torch.bfloat16).eval()
+    for stat in (*pol.normalize_inputs.parameters(), *pol.unnormalize_outputs.parameters()):
+        stat.data[1] = float("inf")
+    b = tiny_batch(device="cuda")
+    B = b["state"].shape[0]
+    noise = torch.randn(B, 10, 32, device="cuda")
+    first = dict(b, dataset_index=torch.zeros(B, dtype=torch.long, device="cuda"))
+    second = dict(b, dataset_index=torch.ones(B, dtype=torch.long, device="cuda"))
+    eager = pol.sample_actions(first, noise=noise)
+    pol.enable_cuda_graphs(True)
+    torch.testing.assert_close(pol.sample_actions(first, noise=noise), eager, rtol=1e-3, atol=1e-3)
+    with pytest.raises(AssertionError, match="infinity"):
+        pol.sample_actions(second, noise=noise)
+    pol.normalize_inputs.buffer_state["max"].data[0] = float("inf")
+    with pytest.raises(AssertionError, match="infinity"):
+        pol.sample_actions(first, noise=noise)
+
+
+def test_replayed_requests_of_several_kinds_keep_their_captures():
+    """Serving one and several candidates in turn captures each kind once."""
+    from opentau_b200.policies.candidates import MEDOID, configure_candidates
+    pol = tiny_pi05(seed=2).to("cuda").to(torch.bfloat16).eval()
+    b = tiny_batch(device="cuda")
+    B = b["state"].shape[0]
+    configure_candidates(pol, 3, MEDOID, device=torch.device("cuda"))
+    pol.enable_cuda_graphs(True)
+    runners = {}
+    for n in (1, 3, 1, 3):
+        pol.sample_actions(b, noise=torch.randn(B * n, 10, 32, device="cuda"), n_candidates=n)
+        assert runners.setdefault(n, pol._graph_runner) is pol._graph_runner and pol._graph_runner.num_graphs == 1
+    assert runners[1] is not runners[3]

@@ -401,3 +401,22 @@ def test_zero_variance_guard_reports_real_deviations_once(caplog):
         healthy({"other": torch.zeros(1)})
         healthy({"other": torch.zeros(1)})
     assert caplog.text.count("'state' was missing from the batch during normalization") == 1
+
+
+@pytest.mark.parametrize("name", ["min", "max"])
+def test_infinite_statistics_are_refused_however_they_were_written(name):
+    """A write through ``.data`` leaves neither address nor version of the parameter changed: the check reads values."""
+    from opentau_b200.policies.normalize import infinite_verdict
+    pol = tiny_pi05()
+    stat = pol.normalize_inputs.buffer_state[name]
+    idx = torch.zeros(2, dtype=torch.long)
+    batch = {"state": torch.randn(2, 32)}
+    pol.normalize_inputs(batch, idx)
+    assert not infinite_verdict(pol.normalize_inputs, pol.unnormalize_outputs)()
+    stat.data[0, 3] = float("inf")
+    assert infinite_verdict(pol.normalize_inputs, pol.unnormalize_outputs)()
+    with pytest.raises(AssertionError, match="infinity"):
+        pol.normalize_inputs(batch, idx)
+    with pytest.raises(AssertionError, match="infinity"):
+        pol.normalize_inputs.refuse_infinite(["state"], idx)
+    pol.normalize_inputs.refuse_infinite(["camera0"], idx)                 # not a feature of this call
