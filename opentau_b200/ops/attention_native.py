@@ -3,7 +3,7 @@
 from __future__ import annotations
 
 import os
-from ctypes import c_float, c_int, c_longlong, c_void_p
+from ctypes import byref, c_float, c_int, c_longlong, c_void_p
 
 import torch
 from torch import Tensor
@@ -95,8 +95,9 @@ def attn_fwd(q: Tensor, k: Tensor, v: Tensor, q_blk: Tensor, k_blk: Tensor, q_va
 
 
 def attn_bwd(do: Tensor, q: Tensor, k: Tensor, v: Tensor, o: Tensor, lse: Tensor, q_blk: Tensor, k_blk: Tensor,
-             q_valid: Tensor, k_valid: Tensor, scale: float):
-    """Returns ``(dq, dk, dv)``; ``delta`` scratch and outputs are allocated here."""
+             q_valid: Tensor, k_valid: Tensor, scale: float, splits: tuple[int, int, int] | None = None):
+    """Returns ``(dq, dk, dv)``; scratch and outputs are allocated here.  ``splits`` forces the parts that the streamed
+    blocks of dQ, dK and dV are dealt to."""
     from . import cuda_ops
     B, Sq, H, D = q.shape
     Sk, Hkv = k.shape[1], k.shape[2]
@@ -112,10 +113,18 @@ def attn_bwd(do: Tensor, q: Tensor, k: Tensor, v: Tensor, o: Tensor, lse: Tensor
     kb = k_blk.to(torch.int32).contiguous()
     qv = _u8(q_valid)
     kv = _u8(k_valid)
-    rc = _lib.load("attention_bwd_tcgen05").otb_attn_bwd(
+    lib = _lib.load("attention_bwd_tcgen05")
+    if splits is None:
+        n = (c_int(), c_int(), c_int())
+        lib.otb_attn_bwd_splits(c_int(B), c_int(Sq), c_int(Sk), c_int(H), c_int(Hkv), c_int(D), *(byref(x) for x in n))
+        splits = tuple(x.value for x in n)
+    parts = [torch.empty(m, *t.shape, dtype=torch.float32, device=q.device) if m > 1 else None
+             for m, t in zip(splits, (dq, dk, dv))]
+    rc = lib.otb_attn_bwd(
         c_void_p(q.data_ptr()), c_void_p(k.data_ptr()), c_void_p(v.data_ptr()), c_void_p(o.data_ptr()),
         c_void_p(do.data_ptr()), c_void_p(lse.data_ptr()), c_void_p(delta.data_ptr()), c_void_p(dq.data_ptr()),
-        c_void_p(dk.data_ptr()), c_void_p(dv.data_ptr()), c_void_p(qb.data_ptr()), c_void_p(kb.data_ptr()),
+        c_void_p(dk.data_ptr()), c_void_p(dv.data_ptr()), *(c_void_p(t.data_ptr() if t is not None else 0) for t in parts),
+        *(c_int(m) for m in splits), c_void_p(qb.data_ptr()), c_void_p(kb.data_ptr()),
         c_void_p(qv.data_ptr()), c_void_p(kv.data_ptr()), c_int(B), c_int(Sq), c_int(Sk), c_int(H), c_int(Hkv),
         c_int(D), c_longlong(q.stride(0)), c_longlong(q.stride(1)), c_longlong(q.stride(2)),
         c_longlong(k.stride(0)), c_longlong(k.stride(1)), c_longlong(k.stride(2)),
@@ -123,7 +132,7 @@ def attn_bwd(do: Tensor, q: Tensor, k: Tensor, v: Tensor, o: Tensor, lse: Tensor
         c_float(scale), c_void_p(cuda_ops.status_pointer()), cuda_ops._stream())
     if rc != 0:
         raise RuntimeError(f"native attn_bwd failed with code {rc} (B={B} Sq={Sq} Sk={Sk} H={H} Hkv={Hkv} D={D})")
-    cuda_ops.launch_count += 4
+    cuda_ops.launch_count += 4 + sum(m > 1 for m in splits)
     return dq, dk, dv
 
 

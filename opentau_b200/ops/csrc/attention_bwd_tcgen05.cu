@@ -36,6 +36,8 @@ struct BwdParams {
   const float* lse;     // (B, H, Sq), natural log
   const float* delta;   // (B, H, Sq)
   __nv_bfloat16* out;   // dq (B,Sq,H,D) | dk, dv (B,Sk,Hkv,D), contiguous
+  float* parts;         // splits > 1: fp32 sums of each part instead, (splits, ...) of the same layout
+  int splits;           // blocks that share a tile's streamed blocks
   KernelStatus* status;
 };
 
@@ -91,7 +93,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant
   int* range_smem = reinterpret_cast<int*>(tmem_slot + 2);   // [0] = first block, [1] = end (exclusive, in elements)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  const int tile = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z % p.B, split = blockIdx.z / p.B;
   const int g = p.g;
   const int pos_per_tile = BW_M / g;   // MODE_DQ: positions per row tile
   const int pos_per_blk = BN / g;      // MODE_DK/DV: positions per streamed query block
@@ -205,6 +207,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant
     blk0 = first / pos_per_blk;
     const int endb = (range_smem[1] + pos_per_blk - 1) / pos_per_blk;
     nblk = max(1, endb - blk0);
+  }
+  bool none = false;                     // my part has no block: its sum is zero (one block is run all the same)
+  if (p.splits > 1) {
+    const int lo = (int)((long long)nblk * split / p.splits), hi = (int)((long long)nblk * (split + 1) / p.splits);
+    none = lo == hi;
+    blk0 += lo;
+    nblk = max(1, hi - lo);
   }
 
   if (warp == 0) {
@@ -449,6 +458,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant
     mbar_wait(acc_full, 0, abort_flag, p.status, KID_ATTN_BWD, 9, 0);
     tc_fence_after();
     __nv_bfloat16* orow = p.out + out_off;
+    float* prow = nullptr;
+    if (p.splits > 1)
+      prow = p.parts + (long long)split * p.B * (MODE == MODE_DQ ? (long long)p.Sq * p.H : (long long)p.Sk * p.Hkv) * p.D +
+             out_off;
     const int n16 = p.Dmma / 16;
     const int a_lo = half ? (n16 + 1) / 2 : 0, a_hi = half ? n16 : (n16 + 1) / 2;
 #pragma unroll 1
@@ -461,7 +474,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant
 #pragma unroll
         for (int h8 = 0; h8 < 2; ++h8) {
           const int col = c * 16 + h8 * 8;
-          if (col < p.D) {
+          if (col < p.D && prow != nullptr) {
+#pragma unroll
+            for (int e = 0; e < 8; e += 4)
+              *reinterpret_cast<float4*>(prow + col + e) =
+                  none ? make_float4(0.f, 0.f, 0.f, 0.f)
+                       : make_float4(__uint_as_float(r[h8 * 8 + e]), __uint_as_float(r[h8 * 8 + e + 1]),
+                                     __uint_as_float(r[h8 * 8 + e + 2]), __uint_as_float(r[h8 * 8 + e + 3]));
+          } else if (col < p.D) {
             uint4 o;
             o.x = pack_bf16(__uint_as_float(r[h8 * 8 + 0]), __uint_as_float(r[h8 * 8 + 1]));
             o.y = pack_bf16(__uint_as_float(r[h8 * 8 + 2]), __uint_as_float(r[h8 * 8 + 3]));
@@ -528,6 +548,29 @@ struct Strides {
   long long sb, ss, sh;
 };
 
+// out[i] = bf16(sum over `splits` parts of 8 n8 floats each, in order)
+__global__ void attn_bwd_sum_kernel(const float* __restrict__ parts, __nv_bfloat16* __restrict__ out, long long n8,
+                                    int splits) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= n8) return;
+  float a[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) a[e] = 0.f;
+  for (int s = 0; s < splits; ++s) {
+    const float4* src = reinterpret_cast<const float4*>(parts + (s * n8 + i) * 8);
+    const float4 u = src[0], w = src[1];
+    a[0] += u.x; a[1] += u.y; a[2] += u.z; a[3] += u.w;
+    a[4] += w.x; a[5] += w.y; a[6] += w.z; a[7] += w.w;
+  }
+  *reinterpret_cast<uint4*>(out + i * 8) =
+      make_uint4(pack_bf16(a[0], a[1]), pack_bf16(a[2], a[3]), pack_bf16(a[4], a[5]), pack_bf16(a[6], a[7]));
+}
+
+template <int MODE>
+static long long bwd_tiles(int Sq, int Sk, int g) {
+  return MODE == MODE_DQ ? (Sq + BW_M / g - 1) / (BW_M / g) : (Sk + BW_M - 1) / BW_M;
+}
+
 template <int MODE, int DPAD, int BN>
 static int launch_bwd(const void* q, Strides qs, const void* k, Strides ks, const void* v, Strides vs, const void* d_o,
                       const BwdParams& p, cudaStream_t stream) {
@@ -563,22 +606,73 @@ static int launch_bwd(const void* q, Strides qs, const void* k, Strides ks, cons
     r = make_map4b(&y2, d_o, p.D, p.H, p.Sq, p.B, dos.sh, dos.ss, dos.sb, g, BN / g);
     if (r) return 4000 + r;
   }
-  dim3 grid;
-  if (MODE == MODE_DQ) grid = dim3((p.Sq + BW_M / g - 1) / (BW_M / g), p.Hkv, p.B);
-  else grid = dim3((p.Sk + BW_M - 1) / BW_M, p.Hkv, p.B);
+  const dim3 grid((unsigned)bwd_tiles<MODE>(p.Sq, p.Sk, g), p.Hkv, p.B * p.splits);
   kern<<<grid, 320, L::TOTAL, stream>>>(f1, f2, y1, y2, p);
+  if (p.splits > 1) {
+    const long long n8 = (long long)p.B * (MODE == MODE_DQ ? (long long)p.Sq * p.H : (long long)p.Sk * p.Hkv) * p.D / 8;
+    attn_bwd_sum_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(p.parts, p.out, n8, p.splits);
+  }
   return (int)cudaGetLastError();
+}
+
+constexpr int BWD_MAX_SPLITS = 16;
+
+// Into how many parts a tile's streamed blocks are dealt.  One block fills an SM, so the time is rounds x the blocks a part
+// streams, plus what every part does once (fixed tiles, first scores, epilogue: about PER_PART blocks' worth) and the
+// sums that are written and read in fp32 (charged to the parts of the whole launch).  One sample of 4096 keys under one kv
+// head is 32 dK and 32 dV tiles, which left 116 of 148 SMs idle: forward + backward 2.85 ms without parts, 1.27 ms with
+// (8 heads on 1, width 256, 1024 causal positions); a pi0.5 training step at batch 8 (80 tiles) 172.5 -> 167.6 ms.
+static int pick_bwd_splits(long long tiles, int blocks, int B, double sum_cost) {
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (sms <= 0) return 1;
+  }
+  constexpr double PER_PART = 4.0;
+  int best = 1;
+  double best_cost = 0;
+  for (int s = 1; s <= BWD_MAX_SPLITS && s * 4 <= (blocks > 4 ? blocks : 4) && (long long)B * s <= 65535; ++s) {
+    const double cost = (double)((tiles * s + sms - 1) / sms) * ((double)((blocks + s - 1) / s) + PER_PART) +
+                        (s > 1 ? sum_cost * (s + 1) : 0.0);
+    if (s == 1 || cost < best_cost) {
+      best = s;
+      best_cost = cost;
+    }
+  }
+  return best;
 }
 
 }  // namespace otb
 
 using namespace otb;
 
+// columns of a streamed block by padded head width, for dQ and dK / for dV
+static constexpr int bwd_bn(int dpad) { return dpad == 256 ? 32 : 64; }
+static constexpr int bwd_bn_v(int dpad) { return dpad == 64 ? 128 : 64; }
+
+// Parts of the three products; `dq`, `dk`, `dv` above 1 want fp32 scratch of that many outputs each.  Sk must be the
+// streamed length of dQ.
+extern "C" void otb_attn_bwd_splits(int B, int Sq, int Sk, int H, int Hkv, int D, int* dq, int* dk, int* dv) {
+  const int g = H / Hkv, dpad = D <= 64 ? 64 : (D <= 128 ? 128 : 256);
+  const int bn = bwd_bn(dpad), bnv = bwd_bn_v(dpad);
+  const long long kv = (long long)Hkv * B;
+  // a block of 32 x 256 takes about 1 us, a dV block of 64 x 256 0.8, others in proportion; fp32 sums move at about 4 TB/s
+  const double us = 1.0 * bn * dpad / (32 * 256), us_v = 0.8 * bnv * dpad / (64 * 256);
+  const double q_sum = 4.0 * B * Sq * H * D / 4e6, k_sum = 4.0 * B * Sk * Hkv * D / 4e6;
+  *dq = pick_bwd_splits(bwd_tiles<MODE_DQ>(Sq, Sk, g) * kv, (Sk + bn - 1) / bn, B, q_sum / us);
+  *dk = pick_bwd_splits(bwd_tiles<MODE_DK>(Sq, Sk, g) * kv, (int)(((long long)Sq * g + bn - 1) / bn), B, k_sum / us);
+  *dv = pick_bwd_splits(bwd_tiles<MODE_DV>(Sq, Sk, g) * kv, (int)(((long long)Sq * g + bnv - 1) / bnv), B, k_sum / us_v);
+}
+
 // q (B,Sq,H,D), k/v (B,Sk,Hkv,D) with element strides; o, do: (B,Sq,H,D) contiguous; lse (B,H,Sq);
-// delta: scratch (B,H,Sq) fp32; dq (B,Sq,H,D), dk/dv (B,Sk,Hkv,D) contiguous outputs.
+// delta: scratch (B,H,Sq) fp32; dq (B,Sq,H,D), dk/dv (B,Sk,Hkv,D) contiguous outputs; *_parts: the scratch that
+// otb_attn_bwd_splits asks for (null where the parts are 1).
 extern "C" int otb_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
-                            const float* lse, float* delta, void* dq, void* dk, void* dv, const int* q_blk,
-                            const int* k_blk, const unsigned char* q_valid, const unsigned char* k_valid, int B,
+                            const float* lse, float* delta, void* dq, void* dk, void* dv, float* dq_parts,
+                            float* dk_parts, float* dv_parts, int dq_splits, int dk_splits, int dv_splits,
+                            const int* q_blk, const int* k_blk, const unsigned char* q_valid, const unsigned char* k_valid, int B,
                             int Sq, int Sk, int H, int Hkv, int D, long long q_sb, long long q_ss, long long q_sh,
                             long long k_sb, long long k_ss, long long k_sh, long long v_sb, long long v_ss,
                             long long v_sh, float scale, void* status, cudaStream_t stream) {
@@ -589,6 +683,12 @@ extern "C" int otb_attn_bwd(const void* q, const void* k, const void* v, const v
   const long long strides[9] = {q_sb, q_ss, q_sh, k_sb, k_ss, k_sh, v_sb, v_ss, v_sh};
   for (int i = 0; i < 9; ++i)
     if (strides[i] % 8) return -5;
+  const int splits[3] = {dq_splits, dk_splits, dv_splits};
+  float* const parts[3] = {dq_parts, dk_parts, dv_parts};
+  for (int i = 0; i < 3; ++i)
+    if (splits[i] < 1 || splits[i] > BWD_MAX_SPLITS || (splits[i] > 1 && parts[i] == nullptr) ||
+        (reinterpret_cast<uintptr_t>(parts[i]) & 15))
+      return -7;
   {
     const long long rows = (long long)B * Sq * H;
     const int threads = 256;
@@ -608,19 +708,25 @@ extern "C" int otb_attn_bwd(const void* q, const void* k, const void* v, const v
   const Strides qs = {q_sb, q_ss, q_sh}, ks = {k_sb, k_ss, k_sh}, vs = {v_sb, v_ss, v_sh};
   const int dpad = D <= 64 ? 64 : (D <= 128 ? 128 : 256);
   int r = 0;
-#define RUN3(DP, BN_QK, BN_V)                                                          \
+#define RUN3(DP)                                                                       \
   p.out = static_cast<__nv_bfloat16*>(dq);                                             \
-  r = launch_bwd<MODE_DQ, DP, BN_QK>(q, qs, k, ks, v, vs, d_o, p, stream);              \
+  p.parts = dq_parts;                                                                  \
+  p.splits = dq_splits;                                                                \
+  r = launch_bwd<MODE_DQ, DP, bwd_bn(DP)>(q, qs, k, ks, v, vs, d_o, p, stream);         \
   if (r) return r;                                                                     \
   p.out = static_cast<__nv_bfloat16*>(dk);                                             \
-  r = launch_bwd<MODE_DK, DP, BN_QK>(q, qs, k, ks, v, vs, d_o, p, stream);              \
+  p.parts = dk_parts;                                                                  \
+  p.splits = dk_splits;                                                                \
+  r = launch_bwd<MODE_DK, DP, bwd_bn(DP)>(q, qs, k, ks, v, vs, d_o, p, stream);         \
   if (r) return 100000 + r;                                                            \
   p.out = static_cast<__nv_bfloat16*>(dv);                                             \
-  r = launch_bwd<MODE_DV, DP, BN_V>(q, qs, k, ks, v, vs, d_o, p, stream);               \
+  p.parts = dv_parts;                                                                  \
+  p.splits = dv_splits;                                                                \
+  r = launch_bwd<MODE_DV, DP, bwd_bn_v(DP)>(q, qs, k, ks, v, vs, d_o, p, stream);       \
   if (r) return 200000 + r;
-  if (dpad == 64) { RUN3(64, 64, 128) }
-  else if (dpad == 128) { RUN3(128, 64, 64) }
-  else { RUN3(256, 32, 64) }
+  if (dpad == 64) { RUN3(64) }
+  else if (dpad == 128) { RUN3(128) }
+  else { RUN3(256) }
 #undef RUN3
   return 0;
 }

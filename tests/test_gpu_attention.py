@@ -235,3 +235,33 @@ def test_fp32_attention_through_autograd_on_gpu(monkeypatch):
     torch.testing.assert_close(dq_g[vq], dq_c[vq], rtol=5e-4, atol=1e-4)
     torch.testing.assert_close(dk_g[vq], dk_c[vq], rtol=5e-4, atol=1e-4)
     torch.testing.assert_close(dv_g[vq], dv_c[vq], rtol=5e-4, atol=1e-4)
+
+
+def _rel(got, want):
+    return ((got.double() - want).norm() / want.norm().clamp_min(1e-30)).item()
+
+
+@pytest.mark.parametrize("D,H,Hkv", [(256, 8, 1), (128, 8, 2), (64, 4, 4), (72, 16, 16)])
+@pytest.mark.parametrize("splits", [(2, 3, 2), (4, 16, 7)])
+def test_split_backward_matches_the_unsplit_one(D, H, Hkv, splits):
+    """Parts of every size, empty ones among them (a causal tail leaves late key tiles with few query blocks).  Split sums
+    differ from the running one by rounding in fp32 and agree after the one rounding to bf16 but for ties (2^-8)."""
+    from opentau_b200.ops import attention_native, cuda_ops
+    B, S = 2, 333
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q, k, v, do = (torch.randn(*shape, device="cuda", generator=g).to(torch.bfloat16)
+                   for shape in ((B, S, H, D), (B, S, Hkv, D), (B, S, Hkv, D), (B, S, H * D)))
+    blk = (torch.arange(S, device="cuda") - 40).clamp_min(0).expand(B, -1).int().contiguous()
+    valid = torch.ones(B, S, dtype=torch.bool, device="cuda")
+    valid[1, 300:] = False
+    args = (q, k, v, blk, blk, valid, valid, D ** -0.5)
+    o, lse = attention_native.attn_fwd(*args)
+    args = (do, q, k, v, o, lse, blk, blk, valid, valid, D ** -0.5)
+    one = attention_native.attn_bwd(*args, splits=(1, 1, 1))
+    got = attention_native.attn_bwd(*args, splits=splits)
+    cuda_ops.check_status()
+    for name, x, w in zip(("dq", "dk", "dv"), got, one):
+        x, w = x[valid], w[valid]
+        assert _rel(x, w.double()) < 2 ** -8, name
+    for x in got[1:]:
+        assert float(x[1, 300:].abs().max()) == 0.0
