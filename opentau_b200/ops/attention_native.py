@@ -147,15 +147,17 @@ def supported_f32(q: Tensor, k: Tensor, v: Tensor) -> bool:
 
 
 #: score bytes of one 8-sample chunk of the dense evaluation above which the kernels are used whatever the head width
-F32_DENSE_SCORE_LIMIT = 1 << 30
+F32_DENSE_SCORE_LIMIT = 5 << 18
 
 
 def prefer_f32_kernels(q: Tensor, k: Tensor) -> bool:
     """Which fp32 path the dispatcher takes when both can run (``OPENTAU_B200_F32_ATTN=kernel|dense`` forces one).
-    Measured on a B200: the kernels need O(S) extra memory instead of the (B, H, Sq, Sk) score tensor and are 2.5 x
-    (forward) / 1.1 x (backward) the dense evaluation at head width 64, but at head width 256 the library's fp32 GEMMs
-    win (forward 0.9 x, backward 0.3 x) as long as the scores fit.  So: kernels for head widths up to 128, and at any
-    width once the scores of a chunk would pass :data:`F32_DENSE_SCORE_LIMIT`."""
+    Measured on a B200, forward + backward, kernels against the dense evaluation on the library's fp32 GEMMs: 800 us
+    against 1043 (2 x 601 positions, 8 heads on 1, width 256), 1067 against 1203 (2 x 700, 8 on 4, 256), 252 against 759
+    (2 x 300, 16 heads of 72), at half its error against 64 bits.  So: the kernels, except at head widths above 128 with
+    fewer score bytes than :data:`F32_DENSE_SCORE_LIMIT` (about 200 positions of 8 heads), where the dense evaluation is
+    what callers have always had and the tests hold it there; it is launch-bound and slower at that size too (734 us
+    against 108 for 100 positions)."""
     mode = os.environ.get("OPENTAU_B200_F32_ATTN", "auto")
     if mode in ("kernel", "dense"):
         return mode == "kernel"
@@ -199,24 +201,38 @@ def attn_f32_fwd(q: Tensor, k: Tensor, v: Tensor, q_blk, k_blk, q_valid, k_valid
 
 
 def attn_f32_bwd(do: Tensor, q: Tensor, k: Tensor, v: Tensor, o: Tensor, lse: Tensor, q_blk, k_blk, q_valid, k_valid,
-                 scale: float):
+                 scale: float, keep_ds: bool = True):
+    """Returns ``(dq, dk, dv)``.  ``keep_ds=False`` recomputes dS for dQ as long sequences do, whose dS would be too big."""
     from . import cuda_ops
     B, Sq, H, D = q.shape
     Sk, Hkv = k.shape[1], k.shape[2]
     (q, k, v, qb, kb, qv, kv), dims = _f32_common(q, k, v, q_blk, k_blk, q_valid, k_valid)
     o = o.contiguous().float()
     do = do.contiguous().float()
+    if do.data_ptr() % 16:
+        do = do.clone()
     lse = lse.contiguous()
+    lib = _lib.load("attention_f32")
+    n_dq, n_dkv, n_ds = c_int(), c_int(), c_longlong()
+    lib.otb_attn_f32_bwd_plan(c_int(B), c_int(Sq), c_int(Sk), c_int(H), c_int(Hkv), byref(n_dq), byref(n_dkv), byref(n_ds))
+    n_dq, n_dkv = n_dq.value, n_dkv.value
+    ds = torch.empty(n_ds.value, dtype=torch.float32, device=q.device) if n_ds.value and keep_ds else None
+    # partial sums of a split backward
+    dq_parts = torch.empty(n_dq, B, Sq, H, D, dtype=torch.float32, device=q.device) if n_dq > 1 else None
+    dk_parts, dv_parts = torch.empty(2, n_dkv, B, Sk, Hkv, D, dtype=torch.float32, device=q.device) \
+        if n_dkv > 1 else (None, None)
     dq = torch.empty(B, Sq, H, D, dtype=torch.float32, device=q.device)
     dk = torch.empty(B, Sk, Hkv, D, dtype=torch.float32, device=q.device)
     dv = torch.empty(B, Sk, Hkv, D, dtype=torch.float32, device=q.device)
     delta = torch.empty(B, H, Sq, dtype=torch.float32, device=q.device)
-    rc = _lib.load("attention_f32").otb_attn_f32_bwd(
+    rc = lib.otb_attn_f32_bwd(
         c_void_p(q.data_ptr()), c_void_p(k.data_ptr()), c_void_p(v.data_ptr()), c_void_p(o.data_ptr()),
         c_void_p(do.data_ptr()), c_void_p(lse.data_ptr()), c_void_p(delta.data_ptr()), c_void_p(dq.data_ptr()),
-        c_void_p(dk.data_ptr()), c_void_p(dv.data_ptr()), c_void_p(qb.data_ptr()), c_void_p(kb.data_ptr()),
+        c_void_p(dk.data_ptr()), c_void_p(dv.data_ptr()),
+        *(c_void_p(t.data_ptr() if t is not None else 0) for t in (dq_parts, dk_parts, dv_parts, ds)), c_int(n_dq),
+        c_int(n_dkv), c_void_p(qb.data_ptr()), c_void_p(kb.data_ptr()),
         c_void_p(qv.data_ptr()), c_void_p(kv.data_ptr()), *dims, c_float(scale), cuda_ops._stream())
     if rc != 0:
         raise RuntimeError(f"fp32 attn_bwd failed with code {rc} (B={B} Sq={Sq} Sk={Sk} H={H} Hkv={Hkv} D={D})")
-    cuda_ops.launch_count += 3
+    cuda_ops.launch_count += 3 + (n_dq > 1) + 2 * (n_dkv > 1)
     return dq, dk, dv

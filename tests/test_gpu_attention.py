@@ -237,8 +237,65 @@ def test_fp32_attention_through_autograd_on_gpu(monkeypatch):
     torch.testing.assert_close(dv_g[vq], dv_c[vq], rtol=5e-4, atol=1e-4)
 
 
+@pytest.mark.parametrize("B,S,H,Hkv,D,kernels", [(2, 250, 8, 1, 256, True), (1, 90, 8, 1, 256, False), (2, 40, 4, 4, 72, True)])
+def test_fp32_attention_reaches_its_kernels(B, S, H, Hkv, D, kernels):
+    """``ops.block_attention`` on fp32 CUDA tensors launches them (forward and backward) where the rule says so, and
+    gives the dense statement's answer where masks broadcast."""
+    from opentau_b200 import ops
+    from opentau_b200.ops import cuda_ops
+    q, k, v = (torch.randn(B, S, h, D, device="cuda").requires_grad_() for h in (H, Hkv, Hkv))
+    blk = torch.arange(S, device="cuda").int().expand(B, -1)
+    ok = torch.ones(B, S, dtype=torch.bool, device="cuda")
+    before = cuda_ops.launch_count
+    o = ops.block_attention(q, k, v, blk, blk, ok, ok, D ** -0.5)
+    o.sum().backward()
+    assert (cuda_ops.launch_count > before) == kernels
+    wide = ops.block_attention(q, k, v, blk[:1], blk[:1], ok[:1], ok[:1], D ** -0.5)
+    assert _rel(wide.detach(), o.detach().double()) < 256 * 2 ** -24
+
+
+def _fp64(q, k, v, do, qb, kb, qv, kv, scale):
+    """``(o, dq, dk, dv)`` of the masked attention in 64 bits."""
+    B, Sq, H, D = q.shape
+    K = k.shape[2]
+    a = [q.double(), k.double().repeat_interleave(H // K, 2), v.double().repeat_interleave(H // K, 2)]
+    a = [t.requires_grad_() for t in a]
+    m = (qv[:, :, None] & kv[:, None, :] & (kb[:, None, :] <= qb[:, :, None]))[:, None]
+    s = (torch.einsum("bqhd,bkhd->bhqk", a[0], a[1]) * scale).masked_fill(~m, -1e300)
+    p = torch.where(m, torch.softmax(s, -1), 0.0)
+    o = torch.einsum("bhqk,bkhd->bqhd", p, a[2]).reshape(B, Sq, H * D)
+    dq, dk, dv = torch.autograd.grad(o, a, do.double())
+    return o.detach(), dq, dk.view(B, -1, K, H // K, D).sum(3), dv.view(B, -1, K, H // K, D).sum(3)
+
+
 def _rel(got, want):
     return ((got.double() - want).norm() / want.norm().clamp_min(1e-30)).item()
+
+
+@pytest.mark.parametrize("D", [4, 28, 72, 132, 256])
+@pytest.mark.parametrize("Sq,cross", [(1, 0), (31, 1), (32, 32), (33, 63), (64, 0), (65, 0), (129, 70), (400, 0)])
+@pytest.mark.parametrize("H,Hkv", [(8, 1), (4, 4)])
+def test_fp32_attention_kernels_at_the_edges_of_their_tiles(D, Sq, cross, H, Hkv):
+    """32 owner rows, 64 streamed rows, widths that pad to 16, split sums (400 positions under one kv head), against 64
+    bits.  Bound: an inner product of n terms rounds to within n 2^-24 of the sum of its magnitudes (n = 256 at most here,
+    the sums over rows average out).  A hidden key may hold anything, NaN included."""
+    from opentau_b200.ops import attention_native
+    B, Sk = 2, Sq + cross
+    g = torch.Generator(device="cuda").manual_seed(D + Sq)
+    q, k, v, do = (torch.randn(*shape, device="cuda", generator=g)
+                   for shape in ((B, Sq, H, D), (B, Sk, Hkv, D), (B, Sk, Hkv, D), (B, Sq, H * D)))
+    kb = torch.cat([torch.full((B, cross), -2**31, device="cuda"), torch.arange(Sq, device="cuda").expand(B, -1) // 5], 1).int()
+    qb, kv = kb[:, cross:].contiguous(), torch.rand(B, Sk, device="cuda", generator=g) > 0.1
+    qv = torch.rand(B, Sq, device="cuda", generator=g) > 0.1
+    kv[:, 0] = qv[:, -1] = True
+    do = do * qv[:, :, None]
+    want = _fp64(q, k, v, do, qb, kb, qv, kv, D ** -0.5)
+    k[~kv], v[~kv] = float("nan"), float("nan")
+    o, lse = attention_native.attn_f32_fwd(q, k, v, qb, kb, qv, kv, D ** -0.5)
+    got = (o, *attention_native.attn_f32_bwd(do, q, k, v, o, lse, qb, kb, qv, kv, D ** -0.5))
+    again = attention_native.attn_f32_bwd(do, q, k, v, o, lse, qb, kb, qv, kv, D ** -0.5, keep_ds=False)
+    for name, x, w in zip(("o", "dq", "dk", "dv", "dq recomputed"), (*got, again[0]), (*want, want[1])):      # inputs of unit scale: their count bounds cancellation
+        assert (x.double() - w).norm() < 256 * 2 ** -24 * (w.norm() + w.numel() ** 0.5), name
 
 
 @pytest.mark.parametrize("D,H,Hkv", [(256, 8, 1), (128, 8, 2), (64, 4, 4), (72, 16, 16)])
