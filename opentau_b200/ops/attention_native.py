@@ -59,8 +59,17 @@ def split_kv(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int) -> int:
     return max(1, min(8, NUM_SMS // ctas, nblk // 2))
 
 
+def split_cluster(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int) -> int:
+    """CTAs of the cluster that shares the keys of a 64-row query tile and merges on chip (1: not this path)."""
+    g = H // Hkv
+    if g > 64 or 64 % g or -(-Sk // (64 if D > 128 else 128)) < 3:
+        return 1
+    return _lib.load("attention_tcgen05").otb_attn_cluster_fit(c_int(D), c_longlong(-(-Sq // (64 // g)) * Hkv * B))
+
+
 def attn_fwd(q: Tensor, k: Tensor, v: Tensor, q_blk: Tensor, k_blk: Tensor, q_valid: Tensor, k_valid: Tensor,
-             scale: float, nsplit: int | None = None):
+             scale: float, nsplit: int | None = None, cluster: bool = False):
+    """Returns ``(o, lse)``.  ``nsplit`` forces the CTAs that share a tile's keys, ``cluster`` that they merge on chip."""
     from . import cuda_ops
     B, Sq, H, D = q.shape
     Sk, Hkv = k.shape[1], k.shape[2]
@@ -78,8 +87,15 @@ def attn_fwd(q: Tensor, k: Tensor, v: Tensor, q_blk: Tensor, k_blk: Tensor, q_va
             c_longlong(q.stride(0)), c_longlong(q.stride(1)), c_longlong(q.stride(2)),
             c_longlong(k.stride(0)), c_longlong(k.stride(1)), c_longlong(k.stride(2)),
             c_longlong(v.stride(0)), c_longlong(v.stride(1)), c_longlong(v.stride(2)), c_float(scale)]
-    nsplit = split_kv(B, Sq, Sk, H, Hkv, D) if nsplit is None else nsplit
-    if nsplit > 1:
+    if nsplit is None:
+        nsplit = split_cluster(B, Sq, Sk, H, Hkv, D)
+        cluster = nsplit > 1
+        if not cluster:
+            nsplit = split_kv(B, Sq, Sk, H, Hkv, D)
+    if nsplit > 1 and cluster:
+        rc = lib.otb_attn_fwd_splitkv(*args, c_int(nsplit), c_void_p(0), c_void_p(0),
+                                      c_void_p(cuda_ops.status_pointer()), cuda_ops._stream())
+    elif nsplit > 1:
         part_o = torch.empty(nsplit, B, Sq, H, D, dtype=torch.float32, device=q.device)
         part_ml = torch.empty(nsplit, B, H, Sq, 2, dtype=torch.float32, device=q.device)
         rc = lib.otb_attn_fwd_splitkv(*args, c_int(nsplit), c_void_p(part_o.data_ptr()),

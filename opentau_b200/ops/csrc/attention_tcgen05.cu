@@ -13,6 +13,12 @@
 // Per KV block j:  MMA issues S[j+1] = Q K_{j+1}^T early, softmax turns S[j] into bf16 P in shared
 // memory (128B-swizzled, K-major), MMA issues O += P V_j.  O is rescaled lazily: only when the running
 // row maximum grew by more than 2^8 since the maximum in use, so the common case touches O never.
+//
+// Few query tiles against many keys (a denoising step or a decoded token against a cached prefix) share the key blocks of
+// a tile among `nsplit` CTAs.  Where the tiles are few enough (SPLIT_CLUSTER) those CTAs are one cluster and the partials
+// never leave the chip's shared memory: a tile holds 64 rows, every CTA leaves its fp32 partial (with the row's maximum
+// and sum behind it) in its own shared memory, sends each peer the rows that peer owns with one bulk copy, and merges its
+// own rows.  Otherwise (SPLIT_GLOBAL) the partials go to global memory and attn_combine_kernel merges them.
 #include "common.cuh"
 #include <limits.h>
 
@@ -20,6 +26,8 @@ namespace otb {
 
 constexpr unsigned KID_ATTN = 2;
 constexpr int ATT_M = 128;
+constexpr int CL_ROWS = 64;        // rows of a tile whose key blocks a cluster shares
+enum { SPLIT_GLOBAL = 0, SPLIT_CLUSTER = 1 };
 
 struct AttnParams {
   int B, Sq, Sk, H, Hkv, D, Dmma, g;
@@ -54,6 +62,11 @@ struct AttnSmem {
   static constexpr int OFF_KMM = OFF_RED + 2 * ATT_M * 4;  // int kmm[2][BN/32][2]: min / max block id per 32 keys
   static constexpr int OFF_BAR = OFF_KMM + 2 * (BN / 32) * 2 * 4;
   static constexpr int NBAR = 16;
+  // a cluster's partials lie over the operand tiles: [row][DPAD + 4] floats (the pad spreads the banks and carries the
+  // row's maximum and sum), mine of all rows, then the peers' of the rows I own
+  static constexpr int PART_LD = DPAD + 4;
+  static constexpr int OFF_PEER = CL_ROWS * PART_LD * 4;
+  static_assert(OFF_PEER + (CL_ROWS + 8) * PART_LD * 4 <= OFF_META, "the partials must fit over the operand tiles");
   static constexpr int USED = OFF_BAR + NBAR * 8 + 32;
   // room for rounding the base up to 1024 bytes (the kernel has no static shared memory, so the base normally is
   // aligned already); capped at the 227 KB a CTA may own, and checked at run time
@@ -67,7 +80,7 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-template <int DPAD, int BN>
+template <int DPAD, int BN, int SPLIT>
 __global__ void __launch_bounds__(320, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
                 const __grid_constant__ CUtensorMap tma_v, AttnParams p) {
@@ -89,6 +102,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   uint64_t* p_full = bars + 9;     // [2]
   uint64_t* p_free = bars + 11;    // [2]
   uint64_t* o_full = bars + 13;
+  uint64_t* recv_bar = bars + 14;  // the peers' partials of my rows have landed (SPLIT_CLUSTER)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NBAR);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* kv_end_smem = reinterpret_cast<int*>(tmem_slot + 2);
@@ -100,10 +114,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   }
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile = blockIdx.x / p.nsplit, split = blockIdx.x % p.nsplit, kvh = blockIdx.y, b = blockIdx.z;
+  constexpr bool CL = SPLIT == SPLIT_CLUSTER;        // the cluster lies along y
+  const int tile = CL ? blockIdx.x : blockIdx.x / p.nsplit, split = CL ? (int)cluster_ctarank() : blockIdx.x % p.nsplit;
+  const int kvh = CL ? blockIdx.y / p.nsplit : blockIdx.y, b = blockIdx.z;
   const int g = p.g;
-  const int pos_per_tile = ATT_M / g;
+  constexpr int ROWS = CL ? CL_ROWS : ATT_M;
+  const int pos_per_tile = ROWS / g;
   const int p0 = tile * pos_per_tile;
+  // SPLIT_CLUSTER: the tile's valid rows, dealt to the CTAs in order; mine are [t0, t0 + own)
+  const int rows_valid = min(pos_per_tile, p.Sq - p0) * g;
+  const int rpr = (rows_valid + p.nsplit - 1) / p.nsplit;
+  const int t0 = split * rpr, own = max(0, min(rpr, rows_valid - t0));
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -116,9 +137,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       mbar_init(&p_free[i], 1);
     }
     mbar_init(o_full, 1);
+    if (CL) mbar_init(recv_bar, 1);
     *abort_flag = 0;
     *kv_end_smem = 0;
     mbar_fence_init();
+    if (CL) mbar_expect_tx(recv_bar, (uint32_t)((p.nsplit - 1) * own * L::PART_LD * 4));
     tma_prefetch_desc(&tma_q);
     tma_prefetch_desc(&tma_k);
     tma_prefetch_desc(&tma_v);
@@ -190,7 +213,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one()) {
-      mbar_expect_tx(q_full, L::Q_BYTES);
+      mbar_expect_tx(q_full, L::Q_BYTES * ROWS / ATT_M);        // the rows past a 64-row tile are never looked at
 #pragma unroll
       for (int c = 0; c < L::NCHUNK; ++c)
         tma_load_4d(sQ + c * (ATT_M * 128), &tma_q, q_full, c * 64, kvh * g, p0, b);
@@ -261,7 +284,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     const int st = threadIdx.x - 64;             // 0..255 index among softmax threads
     const int pos = p0 + row / g;
     const int head = kvh * g + row % g;
-    const bool row_in = pos < p.Sq;
+    const bool row_in = pos < p.Sq && row < ROWS;
     const bool q_ok = row_in && p.q_valid[(long long)b * p.Sq + pos] != 0;
     const int qb = q_ok ? p.q_blk[(long long)b * p.Sq + pos] : INT_MIN;
     const uint32_t lane_off = uint32_t(quad * 32) << 16;
@@ -412,8 +435,100 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     l += red[(half ^ 1) * ATT_M + row];
     mbar_wait(o_full, 0, abort_flag, p.status, KID_ATTN, 9, 0);
     tc_fence_after();
-    const float inv_l = l > 0.f ? 1.f / l : 0.f;
     const uint32_t o_addr = tmem_O + lane_off;
+    if constexpr (CL) {
+      float* part = reinterpret_cast<float*>(smem);
+      if (quad * 32 < rows_valid) {                  // warp-uniform; every MMA of mine has retired: the tiles are free
+        float* dst = part + row * L::PART_LD;
+#pragma unroll 1
+        for (int c = o_lo; c < o_hi; c += 2) {
+          uint32_t ro[32];
+          __syncwarp();
+          tmem_ld_x16(o_addr + c * 16, ro);
+          if (c + 1 < o_hi) tmem_ld_x16(o_addr + c * 16 + 16, ro + 16);
+          tmem_wait_ld();
+          const int n = c + 1 < o_hi ? 8 : 4;
+#pragma unroll
+          for (int q4 = 0; q4 < 8; ++q4)
+            if (q4 < n)
+              *reinterpret_cast<uint4*>(dst + c * 16 + q4 * 4) =
+                  make_uint4(ro[q4 * 4 + 0], ro[q4 * 4 + 1], ro[q4 * 4 + 2], ro[q4 * 4 + 3]);
+        }
+        if (half == 0) *reinterpret_cast<float2*>(dst + DPAD) = make_float2(m_used, l);
+      }
+      fence_async_smem();                            // the bulk copies read what was just written
+      cluster_arrive();                              // after my last MMA: peers may write over my tiles
+      cluster_wait();
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (st < p.nsplit && st != split) {
+        const int cnt = min(rpr, rows_valid - st * rpr);
+        if (cnt > 0)
+          bulk_to_peer(map_rank(smem_u32(smem + L::OFF_PEER) + (uint32_t)((split < st ? split : split - 1) * rpr) * (L::PART_LD * 4u),
+                                (uint32_t)st),
+                       smem_u32(part + st * rpr * L::PART_LD), (uint32_t)cnt * (L::PART_LD * 4u),
+                       map_rank(smem_u32(recv_bar), (uint32_t)st));
+      }
+      if (own > 0) mbar_wait(recv_bar, 0, abort_flag, p.status, KID_ATTN, 10, 0);
+      __syncwarp();
+      cluster_arrive();                              // my rows have all arrived; waited for before leaving
+      const float* peers = reinterpret_cast<const float*>(smem + L::OFF_PEER);
+#pragma unroll 1
+      for (int t = warp - 2; t < own && !*abort_flag; t += 8) {
+        const auto slot_row = [&](int sp) {
+          return sp == split ? part + (t0 + t) * L::PART_LD : peers + ((sp < split ? sp : sp - 1) * rpr + t) * L::PART_LD;
+        };
+        // lane s < nsplit holds split s: (maximum, row sum); M = max m_s, O = sum O_s 2^(m_s - M) / sum l_s 2^(m_s - M)
+        float m_s = -INFINITY, l_s = 0.f;
+        if (lane < p.nsplit) {
+          const float2 ml = *reinterpret_cast<const float2*>(slot_row(lane) + DPAD);
+          l_s = ml.y;
+          m_s = ml.y > 0.f ? ml.x : -INFINITY;
+        }
+        float M = m_s;
+#pragma unroll
+        for (int off = 4; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));   // nsplit <= 8
+        const float w_s = (m_s == -INFINITY) ? 0.f : fast_exp2(m_s - M);
+        float sum = l_s * w_s;
+#pragma unroll
+        for (int off = 4; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+        M = __shfl_sync(0xffffffffu, M, 0);
+        sum = __shfl_sync(0xffffffffu, sum, 0);
+        const float inv = sum > 0.f ? 1.f / sum : 0.f;
+        float acc[DPAD / 32];
+#pragma unroll
+        for (int e = 0; e < DPAD / 32; ++e) acc[e] = 0.f;
+        constexpr int V = DPAD >= 128 ? 4 : 2;       // floats per lane and piece
+        for (int sp = 0; sp < p.nsplit; ++sp) {
+          const float w = __shfl_sync(0xffffffffu, w_s, sp) * inv;
+          if (w == 0.f) continue;                    // nothing visible there
+          const float* src = slot_row(sp) + lane * V;
+#pragma unroll
+          for (int c = 0; c < DPAD / (32 * V); ++c) {
+            float v[V];
+            if (V == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(src + c * 32 * V);
+            else *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(src + c * 32 * V);
+#pragma unroll
+            for (int e = 0; e < V; ++e) acc[c * V + e] += v[e] * w;
+          }
+        }
+        const int r = t0 + t, rpos = p0 + r / g, rhead = kvh * g + r % g;
+        __nv_bfloat16* orow = p.o + (((long long)b * p.Sq + rpos) * p.H + rhead) * p.D;
+#pragma unroll
+        for (int c = 0; c < DPAD / (32 * V); ++c) {
+          const int colo = c * 32 * V + lane * V;
+          if (colo < p.D) {
+            if (V == 4)
+              *reinterpret_cast<uint2*>(orow + colo) =
+                  make_uint2(pack_bf16(acc[c * V], acc[c * V + 1]), pack_bf16(acc[c * V + V - 2], acc[c * V + V - 1]));
+            else
+              *reinterpret_cast<uint32_t*>(orow + colo) = pack_bf16(acc[c * V], acc[c * V + 1]);
+          }
+        }
+        if (lane == 0)
+          p.lse[((long long)b * p.H + rhead) * p.Sq + rpos] = sum > 0.f ? (M + log2f(sum)) * 0.6931471805599453f : 0.f;
+      }
+    } else {
+    const float inv_l = l > 0.f ? 1.f / l : 0.f;
     __nv_bfloat16* orow = p.o + (((long long)b * p.Sq + pos) * p.H + head) * p.D;
     float* prow_o = p.nsplit > 1
                         ? p.part_o + ((((long long)split * p.B + b) * p.Sq + pos) * p.H + head) * (long long)p.D
@@ -456,12 +571,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         p.lse[((long long)b * p.H + head) * p.Sq + pos] = lse;
       }
     }
+    }
     tc_fence_before();
+  }
+
+  if (CL && warp < 2) {
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    cluster_arrive();
   }
 
   // ---------------------------------------------------------------------- teardown
   tc_fence_before();
   __syncthreads();
+  if (CL) cluster_wait();                            // every copy out of my shared memory has arrived at its owner
   if (warp == 1) {
     if (*abort_flag) {
       for (int i = 0; i < 2000; ++i) __nanosleep(1000);
@@ -533,21 +657,23 @@ static int make_map4(CUtensorMap* m, const void* base, int D, int Hx, int S, int
   return make_tmap_bf16(m, base, 4, dims, strides, box);
 }
 
-template <int DPAD, int BN>
+template <int DPAD, int BN, int SPLIT>
 static int launch_attn(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p,
                        cudaStream_t stream) {
   using L = AttnSmem<DPAD, BN>;
   static bool configured = false;
-  auto kern = attn_fwd_kernel<DPAD, BN>;
+  auto kern = attn_fwd_kernel<DPAD, BN, SPLIT>;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  const int pos_per_tile = ATT_M / p.g;
-  dim3 grid(((p.Sq + pos_per_tile - 1) / pos_per_tile) * p.nsplit, p.Hkv, p.B);
-  cudaError_t e = launch_pdl(kern, grid, dim3(320), (size_t)L::TOTAL, stream, 0u, tq, tk, tv, p);
-  if (e != cudaSuccess || p.nsplit == 1) return (int)e;
+  const int pos_per_tile = (SPLIT == SPLIT_CLUSTER ? CL_ROWS : ATT_M) / p.g;
+  dim3 grid((p.Sq + pos_per_tile - 1) / pos_per_tile, p.Hkv, p.B);
+  (SPLIT == SPLIT_CLUSTER ? grid.y : grid.x) *= p.nsplit;
+  cudaError_t e = launch_pdl(kern, grid, dim3(320), (size_t)L::TOTAL, stream,
+                             SPLIT == SPLIT_CLUSTER ? (unsigned)p.nsplit : 0u, tq, tk, tv, p);
+  if (e != cudaSuccess || p.nsplit == 1 || SPLIT == SPLIT_CLUSTER) return (int)e;
   const long long rows = (long long)p.B * p.Sq * p.H;
   e = launch_pdl(attn_combine_kernel, dim3((unsigned)((rows * 32 + 255) / 256)), dim3(256), 0, stream, 0u,
                  (const float*)p.part_o, (const float2*)p.part_ml, p.o, p.lse, p.nsplit, p.B, p.Sq, p.H, p.D);
@@ -564,10 +690,13 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
                          int Sk, int H, int Hkv, int D, long long q_sb, long long q_ss, long long q_sh, long long k_sb,
                          long long k_ss, long long k_sh, long long v_sb, long long v_ss, long long v_sh, float scale,
                          int nsplit, float* part_o, float* part_ml, void* status, cudaStream_t stream) {
-  if (nsplit < 1 || nsplit > 8 || (nsplit > 1 && (part_o == nullptr || part_ml == nullptr || D % 4))) return -7;
+  if (nsplit < 1 || nsplit > 8) return -7;
+  // split without scratch: one cluster per tile of 64 rows merges on chip
+  const bool cluster = nsplit > 1 && part_o == nullptr;
+  if (nsplit > 1 && !cluster && (part_ml == nullptr || D % 4)) return -7;
   if (B <= 0 || Sq <= 0 || Sk <= 0 || H <= 0 || Hkv <= 0 || H % Hkv) return -2;
   const int g = H / Hkv;
-  if (g > 128 || (128 % g)) return -3;
+  if (g > 128 || (128 % g) || (cluster && g > CL_ROWS)) return -3;
   if (D % 8 || D > 256 || D < 16) return -4;
   const long long strides[9] = {q_sb, q_ss, q_sh, k_sb, k_ss, k_sh, v_sb, v_ss, v_sh};
   for (int i = 0; i < 9; ++i)
@@ -590,17 +719,20 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
   const int dpad = D <= 64 ? 64 : (D <= 128 ? 128 : 256);
   const int bn = dpad == 256 ? 64 : 128;
   CUtensorMap tq, tk, tv;
-  int r = make_map4(&tq, q, D, H, Sq, B, q_sh, q_ss, q_sb, g, ATT_M / g);
+  int r = make_map4(&tq, q, D, H, Sq, B, q_sh, q_ss, q_sb, g, (cluster ? CL_ROWS : ATT_M) / g);
   if (r) return 1000 + r;
   r = make_map4(&tk, k, D, Hkv, Sk, B, k_sh, k_ss, k_sb, 1, bn);
   if (r) return 2000 + r;
   r = make_map4(&tv, v, D, Hkv, Sk, B, v_sh, v_ss, v_sb, 1, bn);
   if (r) return 3000 + r;
+#define RUN(DP, BLK) (cluster ? launch_attn<DP, BLK, SPLIT_CLUSTER>(tq, tk, tv, p, stream) \
+                              : launch_attn<DP, BLK, SPLIT_GLOBAL>(tq, tk, tv, p, stream))
   switch (dpad) {
-    case 64: return launch_attn<64, 128>(tq, tk, tv, p, stream);
-    case 128: return launch_attn<128, 128>(tq, tk, tv, p, stream);
-    default: return launch_attn<256, 64>(tq, tk, tv, p, stream);
+    case 64: return RUN(64, 128);
+    case 128: return RUN(128, 128);
+    default: return RUN(256, 64);
   }
+#undef RUN
 }
 
 extern "C" int otb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const int* q_blk,
@@ -613,7 +745,7 @@ extern "C" int otb_attn_fwd(const void* q, const void* k, const void* v, void* o
 }
 
 // Split-KV form: `nsplit` (2..8) CTAs per query tile share the key blocks; part_o holds nsplit*B*Sq*H*D floats and
-// part_ml 2*nsplit*B*H*Sq floats of scratch.  Same result as otb_attn_fwd up to fp32 rounding of the merge.
+// part_ml 2*nsplit*B*H*Sq floats of scratch, or both are null and a cluster merges on chip.  Same result as otb_attn_fwd up to fp32 rounding of the merge.
 extern "C" int otb_attn_fwd_splitkv(const void* q, const void* k, const void* v, void* o, float* lse, const int* q_blk,
                                     const int* k_blk, const unsigned char* q_valid, const unsigned char* k_valid,
                                     int B, int Sq, int Sk, int H, int Hkv, int D, long long q_sb, long long q_ss,
@@ -622,6 +754,46 @@ extern "C" int otb_attn_fwd_splitkv(const void* q, const void* k, const void* v,
                                     float* part_ml, void* status, cudaStream_t stream) {
   return attn_fwd_impl(q, k, v, o, lse, q_blk, k_blk, q_valid, k_valid, B, Sq, Sk, H, Hkv, D, q_sb, q_ss, q_sh, k_sb,
                        k_ss, k_sh, v_sb, v_ss, v_sh, scale, nsplit, part_o, part_ml, status, stream);
+}
+
+template <int DPAD, int BN>
+static int max_clusters(int n) {
+  using L = AttnSmem<DPAD, BN>;
+  auto kern = attn_fwd_kernel<DPAD, BN, SPLIT_CLUSTER>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL) != cudaSuccess) return 0;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(1, (unsigned)n, 1);
+  cfg.blockDim = dim3(320);
+  cfg.dynamicSmemBytes = L::TOTAL;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 1;
+  attr.val.clusterDim.y = (unsigned)n;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  return cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess ? clusters : 0;
+}
+
+// CTAs per cluster for `tiles` tiles of 64 rows: the most (up to 8) whose clusters are all resident at once, since a second
+// round costs more than anything a larger cluster saves; 1 if that leaves fewer than 3.  Measured at 50 queries of 8 heads
+// on 1, width 256, against the merge through global memory: 10.5 us against 17.2 (7 tiles, 1018 keys, 8 CTAs), 12.5 against
+// 17.0 (28 tiles, 639 keys, 4), 16.9 against 19.7 (42 tiles, 900 keys, 3); pairs gain nothing (56 tiles: 20.4 against 20.2)
+// and clusters that do not fit lose (28 tiles with 8: 20.5).  One query: 7.6 against 11.4 us.
+extern "C" int otb_attn_cluster_fit(int D, long long tiles) {
+  static int cap[3][9] = {};                         // -1: none
+  const int which = D <= 64 ? 0 : (D <= 128 ? 1 : 2);
+  for (int n = 8; n >= 3; --n) {
+    int c = cap[which][n];
+    if (c == 0) {
+      c = which == 0 ? max_clusters<64, 128>(n) : which == 1 ? max_clusters<128, 128>(n) : max_clusters<256, 64>(n);
+      cap[which][n] = c = c > 0 ? c : -1;
+    }
+    if (tiles <= c) return n;
+  }
+  return 1;
 }
 
 // key-block width the forward kernel uses for this head dimension (callers size split-KV from it)

@@ -167,6 +167,31 @@ def test_split_kv_matches_single_pass(B, Sq, Sk, H, Hkv, D, nsplit):
     torch.testing.assert_close(got_lse, want_lse, atol=1e-3, rtol=1e-3)
 
 
+@pytest.mark.parametrize("nsplit", [2, 3, 7, 8])
+@pytest.mark.parametrize("H,Hkv,D", [(8, 1, 256), (8, 4, 256), (4, 1, 64), (16, 16, 72), (32, 8, 128), (64, 1, 40)])
+@pytest.mark.parametrize("Sq,Sk", [(1, 77), (1, 1019), (50, 322), (51, 1018), (9, 130)])
+def test_cluster_merge_matches_single_pass(H, Hkv, D, Sq, Sk, nsplit):
+    """Keys of a 64-row tile shared by a cluster: tiles with one row and partly filled ones, ranks that own no row, splits
+    without a key, rows that see nothing.  Differs from one pass by fp32 rounding of the merge before bf16 (2^-8)."""
+    from opentau_b200.ops import attention_native, cuda_ops
+    B = 2
+    g = torch.Generator(device="cuda").manual_seed(Sk)
+    q, k, v = (torch.randn(B, S, h, D, device="cuda", generator=g).to(torch.bfloat16)
+               for S, h in ((Sq, H), (Sk, Hkv), (Sk, Hkv)))
+    kb = torch.cat([torch.full((B, Sk - Sq), -2**31, device="cuda"), torch.arange(Sq, device="cuda").expand(B, -1) // 7], 1).int()
+    qb, kv = kb[:, Sk - Sq:].contiguous(), torch.rand(B, Sk, device="cuda", generator=g) > 0.2
+    kv[1, :] = False                                       # nothing to see for this sample
+    qv = torch.ones(B, Sq, dtype=torch.bool, device="cuda")
+    qv[:, Sq // 2 + 1:Sq // 2 + 3] = False
+    args = (q, k, v, qb, kb, qv, kv, D ** -0.5)
+    want_o, want_lse = attention_native.attn_fwd(*args, nsplit=1)
+    o, lse = attention_native.attn_fwd(*args, nsplit=nsplit, cluster=True)
+    cuda_ops.check_status()
+    assert _rel(o, want_o.double()) < 2 ** -8
+    torch.testing.assert_close(lse, want_lse, atol=1e-4, rtol=1e-5)
+    assert float(o[1].abs().max()) == 0.0
+
+
 @pytest.mark.parametrize("D", [32, 72, 128, 160, 256])
 @pytest.mark.parametrize("H,Hkv", [(8, 1), (6, 3), (4, 4)])
 @pytest.mark.parametrize("Sq,cross", [(50, 0), (131, 0), (50, 203), (33, 64)])
