@@ -547,69 +547,132 @@ __global__ void qkv_post_kernel(const __nv_bfloat16* __restrict__ qkv, long long
 // SigLIP patch embedding in ONE kernel and in fp32 (the model keeps this island in fp32 under every bf16 cast):
 //   out[b, gy*gw + gx, n] = bias[n] + pos[gy*gw + gx, n] + sum_{c,py,px} W[n, (c,py,px)] * pix[b, c, gy*p+py, gx*p+px]
 // The non-overlapping patches are gathered straight from the image (no unfolded copy), the product runs on the fp32
-// pipes as a 64 x 64 x 16 shared-memory tiled GEMM with 4 x 4 outputs per thread, and bias, position table and the
-// cast to the encoder dtype are the epilogue.  PixT = float or bf16, OutT = float or bf16.
+// pipes, and bias, position table and the cast to the encoder dtype are the epilogue.  PixT = float or bf16, OutT = float
+// or bf16.
+//
+// A block computes 64 patches x 64 features.  Its four groups of 64 threads take a quarter of the taps each, 8 x 8 outputs
+// per thread (a 128-bit shared load takes four cycles, so 4 x 4 outputs per thread would stop at half the arithmetic
+// peak), and their sums are added at the end.  The next 32 taps are on their way from global memory while a tile is
+// multiplied; where a tap lies in the image comes from a table in shared memory instead of divisions.
+constexpr int PE_M = 64, PE_N = 64, PE_K = 32, PE_LD = 68, PE_TAPS = 2048;
 template <typename PixT, typename OutT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 patch_embed_kernel(const PixT* __restrict__ pix, const float* __restrict__ w, const float* __restrict__ bias,
                    const float* __restrict__ pos, OutT* __restrict__ out, int B, int C, int H, int W, int p, int N) {
-  constexpr int BM = 64, BN = 64, BK = 16;
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Bs[BK][BN + 4];
-  const int gh = H / p, gw = W / p, P = gh * gw, K = C * p * p;
+  __shared__ __align__(16) float tiles[4][PE_K * PE_LD];        // patches 0 / 1, features 0 / 1, tap-major
+  __shared__ int tap_off[PE_TAPS];                              // offset of taps [chunk, chunk + PE_TAPS) inside an image
+  const int gw = W / p, P = (H / p) * gw, K = C * p * p;
   const long long M = (long long)B * P;
-  const long long m0 = (long long)blockIdx.x * BM;
-  const int n0 = blockIdx.y * BN;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;       // 16 x 16 threads, 4 x 4 outputs each
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    // A tile: 64 patches x 16 taps, gathered from the image
-    for (int e = threadIdx.x; e < BM * BK; e += 256) {
-      const int mm = e / BK, kk = e % BK;
-      const long long m = m0 + mm;
-      const int k = k0 + kk;
-      float v = 0.f;
-      if (m < M && k < K) {
-        const int b = int(m / P), pi = int(m % P), gy = pi / gw, gx = pi % gw;
-        const int c = k / (p * p), r = k % (p * p), py = r / p, px = r % p;
-        const PixT x = pix[(((long long)b * C + c) * H + gy * p + py) * W + gx * p + px];
-        if constexpr (sizeof(PixT) == 4) v = x; else v = __bfloat162float(x);
-      }
-      As[kk][mm] = v;
-    }
-    // B tile: 64 output features x 16 taps of the flattened convolution weight
-    for (int e = threadIdx.x; e < BN * BK; e += 256) {
-      const int nn = e / BK, kk = e % BK;
-      const int n = n0 + nn, k = k0 + kk;
-      Bs[kk][nn] = (n < N && k < K) ? w[(long long)n * K + k] : 0.f;
-    }
-    __syncthreads();
+  const long long m0 = (long long)blockIdx.x * PE_M;
+  const int n0 = blockIdx.y * PE_N;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // loads: this thread's rows are lr and lr + 4 of both tiles, its taps lk + 8 j (stores of a warp: 32 different banks)
+  const int lk = lane & 7, lr = warp * 8 + (lane >> 3);
+  const PixT* arow[2];
+  const float* brow[2];
 #pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      float a[4], bb[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bb[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], bb[j], acc[i][j]);
-    }
-    __syncthreads();
+  for (int i = 0; i < 2; ++i) {
+    const long long m = m0 + lr + 4 * i;
+    const int pi = int(m % P), gy = pi / gw, gx = pi % gw;
+    arow[i] = m < M ? pix + ((m / P) * C * H + gy * p) * (long long)W + gx * p : nullptr;
+    brow[i] = n0 + lr + 4 * i < N ? w + (long long)(n0 + lr + 4 * i) * K : nullptr;
   }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const long long m = m0 + ty * 4 + i;
-    if (m >= M) continue;
-    const int pi = int(m % P);
+  float av[8], bv[8];
+  const auto fetch = [&](int k0) {
+    if (k0 % PE_TAPS == 0) {
+      __syncthreads();                                          // the previous chunk is no longer read
+      for (int i = threadIdx.x; i < PE_TAPS && k0 + i < K; i += 256) {
+        const int k = k0 + i, c = k / (p * p), r = k % (p * p);
+        tap_off[i] = (c * H + r / p) * W + r % p;
+      }
+      __syncthreads();
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n >= N) continue;
-      const float v = acc[i][j] + bias[n] + pos[(long long)pi * N + n];
-      if constexpr (sizeof(OutT) == 4) out[m * N + n] = v; else out[m * N + n] = __float2bfloat16(v);
+      const int k = k0 + lk + 8 * j;
+      const int off = k < K ? tap_off[k % PE_TAPS] : 0;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        av[2 * j + i] = 0.f;
+        if (k < K && arow[i] != nullptr) {
+          if constexpr (sizeof(PixT) == 4) av[2 * j + i] = arow[i][off];
+          else av[2 * j + i] = __bfloat162float(arow[i][off]);
+        }
+        bv[2 * j + i] = k < K && brow[i] != nullptr ? brow[i][k] : 0.f;
+      }
     }
+  };
+  const int grp = threadIdx.x >> 6, ty = (threadIdx.x >> 3) & 7, tx = threadIdx.x & 7;   // 8 x 8 threads per group
+  float acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  fetch(0);
+  int buf = 0;
+  for (int k0 = 0; k0 < K; k0 += PE_K, buf ^= 1) {
+    float* as = tiles[buf];
+    float* bs = tiles[2 + buf];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        as[(lk + 8 * j) * PE_LD + lr + 4 * i] = av[2 * j + i];
+        bs[(lk + 8 * j) * PE_LD + lr + 4 * i] = bv[2 * j + i];
+      }
+    __syncthreads();                                            // the other buffer was last read before this barrier
+    if (k0 + PE_K < K) fetch(k0 + PE_K);
+#pragma unroll
+    for (int kk = 0; kk < PE_K / 4; ++kk) {
+      const float* ar = as + (grp * (PE_K / 4) + kk) * PE_LD + ty * 4;
+      const float* br = bs + (grp * (PE_K / 4) + kk) * PE_LD + tx * 4;
+      float a[8], b[8];
+      *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(ar);
+      *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(ar + 32);
+      *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(br);
+      *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(br + 32);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+    }
+  }
+  // the groups' sums: 2, 3 onto 0, 1, then 1 onto 0, whose sums all threads store
+  float* sum = &tiles[0][0];                                    // [2][64][PE_LD]
+  const auto put = [&](float* dst) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float* r = dst + (ty * 4 + (i & 3) + 32 * (i >> 2)) * PE_LD + tx * 4;
+      *reinterpret_cast<float4*>(r) = *reinterpret_cast<const float4*>(&acc[i][0]);
+      *reinterpret_cast<float4*>(r + 32) = *reinterpret_cast<const float4*>(&acc[i][4]);
+    }
+  };
+  const auto add = [&](const float* src) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float* r = src + (ty * 4 + (i & 3) + 32 * (i >> 2)) * PE_LD + tx * 4;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[i][j] += r[(j & 3) + 32 * (j >> 2)];
+    }
+  };
+  __syncthreads();
+  if (grp >= 2) put(sum + (grp - 2) * PE_M * PE_LD);
+  __syncthreads();
+  if (grp < 2) add(sum + grp * PE_M * PE_LD);
+  __syncthreads();
+  if (grp == 1) put(sum);
+  __syncthreads();
+  if (grp == 0) {
+    add(sum);
+    put(sum);
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < PE_M * PE_N; e += 256) {
+    const long long m = m0 + (e >> 6);
+    const int n = n0 + (e & 63);
+    if (m >= M || n >= N) continue;
+    const float v = sum[(e >> 6) * PE_LD + (e & 63)] + bias[n] + pos[(m % P) * N + n];
+    if constexpr (sizeof(OutT) == 4) out[m * N + n] = v; else out[m * N + n] = __float2bfloat16(v);
   }
 }
 

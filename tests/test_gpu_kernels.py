@@ -510,3 +510,17 @@ def test_norm_backward_adds_the_residual_gradient_in_the_kernel(H):
     a1 = cuda_ops.ada_rms_bwd(dy, x, mod, rstd_a, dres)
     torch.testing.assert_close(a1[0].float(), a0[0].float() + dres.float(), rtol=1e-2, atol=2e-2)
     assert torch.equal(a0[1], a1[1]) and torch.equal(a0[2], a1[2])
+
+
+@pytest.mark.parametrize("B,C,H,W,p,N", [(1, 1, 4, 4, 2, 8), (2, 3, 28, 56, 14, 72), (5, 3, 70, 70, 14, 65), (1, 3, 64, 64, 32, 130)])
+def test_patch_embed_at_the_edges_of_its_tiles(B, C, H, W, p, N, dev):
+    """Fewer taps than a tile (4), ragged patches and features, more taps than the offset table holds (3072).  Bound: n
+    products and additions round to within n 2^-24 of the sum of magnitudes, of which the 2-norm sees the square root."""
+    from opentau_b200 import ops
+    g = torch.Generator(device=dev).manual_seed(N)
+    pix, w = torch.rand(B, C, H, W, device=dev, generator=g) * 2 - 1, torch.randn(N, C, p, p, device=dev, generator=g)
+    b, pos = torch.randn(N, device=dev, generator=g), torch.randn((H // p) * (W // p), N, device=dev, generator=g)
+    got = ops.patch_embed(pix, w, b, pos, p, torch.float32)
+    x = pix.double().view(B, C, H // p, p, W // p, p).permute(0, 2, 4, 1, 3, 5).reshape(B, -1, C * p * p)
+    want = x @ w.double().view(N, -1).t() + b.double() + pos.double()
+    assert (got.double() - want).norm() < max(8, (C * p * p) ** 0.5) * 2 ** -24 * want.norm()
