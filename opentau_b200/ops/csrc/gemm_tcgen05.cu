@@ -225,6 +225,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();                             // after the TMEM allocation (see common.cuh)
+  pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -446,6 +448,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   cluster_sync_all();                                  // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();                             // after the TMEM allocation (see common.cuh)
+  pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
@@ -568,8 +572,7 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
   }
   int num_tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
   int grid = num_tiles < g_num_sms ? num_tiles : g_num_sms;
-  kern<<<grid, 192, L::TOTAL, stream>>>(ta, tb, p);
-  return (int)cudaGetLastError();
+  return (int)launch_pdl(kern, dim3((unsigned)grid), dim3(192), (size_t)L::TOTAL, stream, 0u, ta, tb, p);
 }
 
 template <int STAGES>
@@ -585,8 +588,8 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const 
   const int num_tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + 255) / 256);
   int pairs = g_num_sms / 2;
   if (num_tiles < pairs) pairs = num_tiles;
-  kern<<<2 * pairs, 192, L::TOTAL, stream>>>(ta, tb, p);     // cluster size 2 comes from __cluster_dims__
-  return (int)cudaGetLastError();
+  // cluster size 2 comes from __cluster_dims__
+  return (int)launch_pdl(kern, dim3((unsigned)(2 * pairs)), dim3(192), (size_t)L::TOTAL, stream, 0u, ta, tb, p);
 }
 
 }  // namespace otb
