@@ -201,7 +201,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int num_n = (p.N + BN - 1) / BN;
   const int num_tiles = num_m * num_n;
   const int num_kb = (p.K + BK - 1) / BK;
-  constexpr uint32_t TMEM_COLS = 2 * BN;  // 128 / 256 / 512: powers of two >= 32
+  constexpr uint32_t TMEM_COLS = BN <= 64 ? 128 : (BN <= 128 ? 256 : 512);   // two accumulators, a power of two
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -601,7 +601,7 @@ extern "C" int otb_gemm_bf16(const void* A, const void* B, void* out, int M, int
                              long long ldb, long long ldo, int a_mn_major, int b_mn_major, const void* bias,
                              const void* residual, long long ldr, void* out2, long long ldo2, int flags,
                              int bn_override, void* status, cudaStream_t stream) {
-  // bn_override: 0 = choose; 64 / 128 / 256 = that column tile on one CTA; 512 = the CTA-pair kernel (256 x 256 tiles)
+  // bn_override: 0 = choose; 64 / 128 / 160 / 192 / 256 = that column tile on one CTA; 512 = the CTA-pair kernel (256 x 256 tiles)
   if (M <= 0 || N <= 0 || K <= 0) return -2;
   if ((lda % 8) || (ldb % 8) || (ldo % 8) || (N % 8)) return -3;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(out)) & 15) return -4;
@@ -614,26 +614,33 @@ extern "C" int otb_gemm_bf16(const void* A, const void* B, void* out, int M, int
     if (g_num_sms <= 0) return -7;
   }
   int bn = bn_override;
+  // 160 columns are no multiple of the 64-column slabs of an MN-major B, nor of the gated MLP's gate / up pairs of 32
+  const bool no160 = b_mn_major || (flags & (EPI_GLU_GELU | EPI_GLU_SILU));
   // Big products: two SMs per 256 x 256 tile (measured 1.10 - 1.26x the single-CTA kernel on the training shapes).
   // The exception is a weight gradient with a narrow output (both operands MN-major, N <= 2048), where it measured
   // 0.97x.
-  if (bn == 0 && g_pair_default && M >= 1024 && N >= 1024 && (long long)((M + 255) / 256) * ((N + 255) / 256) >= 74 &&
-      !(a_mn_major && b_mn_major && N <= 2048))
-    bn = 512;
+  const bool pair_ok = g_pair_default && !(a_mn_major && b_mn_major && N <= 2048);
+  const long long pair_tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
+  const int pairs = g_num_sms / 2;
+  if (bn == 0 && pair_ok && M >= 1024 && N >= 1024 && pair_tiles >= 4 * pairs) bn = 512;
   if (bn == 0) {
-    // Column tile of the one-CTA kernel: the cheapest of waves x k-blocks x (time per k-block) + drain, with the times
-    // measured on 200 - 968 rows (us per 64-deep k-block 0.20 / 0.21 / 0.35 and drain 1.3 / 2.3 / 4.0 for 64 / 128 / 256
-    // columns: the narrow tiles are bound by the load latency, so their k-blocks cost the same).  200 x 2560 x 1024 runs
-    // 7.6 us on 64 columns against 8.8 / 12.3, 968 x 2048 x 2048 13.6 us on 128 against 18.3 / 20.5.
-    const int cand[3] = {64, 128, 256};
-    const double per_kb[3] = {0.20, 0.21, 0.35}, drain[3] = {1.3, 2.3, 4.0};
+    // Otherwise a launch is a few rounds of tiles, and what the last round leaves empty decides: the cheapest of
+    // rounds x k-blocks x (time per k-block) + (launch, first load, drain), in us, as measured inside a replayed graph on
+    // 200 - 3072 rows.  Up to 128 columns a k-block is bound by the load latency and costs the same.  Of 64 / 128 / 256 columns
+    // or pairs alone, 1024 x 2560 x 10240 took 57.8 us (160 columns: 44.9), 968 x 2560 x 2048 18.8 (160: 13.5),
+    // 2356 x 2048 x 16384 159 (160: 137), 3072 x 1152 x 1152 13.7 (192: 11.0).
+    const int cand[6] = {64, 128, 160, 192, 256, 512};
+    const double per_kb[6] = {0.21, 0.223, 0.245, 0.27, 0.346, 0.305}, once[6] = {3.5, 5.0, 5.6, 6.6, 8.5, 9.0};
     const long long m_tiles = (M + BM - 1) / BM;
     const double kbs = (K + BK - 1) / BK;
     double best = 0;
-    for (int i = 0; i < 3; ++i) {
-      if (i > 0 && cand[i] >= 2 * N) break;                       // a tile at least half empty
-      const long long tiles = m_tiles * ((N + cand[i] - 1) / cand[i]);
-      const double t = (double)((tiles + g_num_sms - 1) / g_num_sms) * kbs * per_kb[i] + drain[i];
+    for (int i = 0; i < 6; ++i) {
+      const bool pair = cand[i] == 512;
+      if (i > 0 && (pair ? 256 : cand[i]) >= 2 * N) break;        // a tile at least half empty
+      if ((cand[i] == 160 && no160) || (pair && (!pair_ok || M <= 256))) continue;
+      const long long rounds = pair ? (pair_tiles + pairs - 1) / pairs
+                                    : (m_tiles * ((N + cand[i] - 1) / cand[i]) + g_num_sms - 1) / g_num_sms;
+      const double t = (double)rounds * kbs * per_kb[i] + once[i];
       if (bn == 0 || t < best) {
         best = t;
         bn = cand[i];
@@ -666,6 +673,8 @@ extern "C" int otb_gemm_bf16(const void* A, const void* B, void* out, int M, int
   p.status = static_cast<KernelStatus*>(status);
   switch (bn) {
     case 256: return launch_gemm<256, 4>(ta, tb, p, stream);
+    case 192: return launch_gemm<192, 5>(ta, tb, p, stream);
+    case 160: return no160 ? -8 : launch_gemm<160, 6>(ta, tb, p, stream);
     case 128: return launch_gemm<128, 6>(ta, tb, p, stream);
     case 64: return launch_gemm<64, 8>(ta, tb, p, stream);
     case 512: return launch_gemm_pair<6>(ta, tb, p, stream);

@@ -512,6 +512,26 @@ def test_norm_backward_adds_the_residual_gradient_in_the_kernel(H):
     assert torch.equal(a0[1], a1[1]) and torch.equal(a0[2], a1[2])
 
 
+@pytest.mark.parametrize("bn", [160, 192])
+@pytest.mark.parametrize("M,N,K", [(1, 160, 64), (129, 328, 72), (300, 1152, 200), (968, 2560, 136)])
+def test_wide_column_tiles_give_the_bits_of_the_others(bn, M, N, K, dev):
+    """A column tile only decides which CTA sums an output: 160 and 192 columns give the 256-column tile's bits, with
+    every epilogue and layout they take."""
+    from opentau_b200.ops import cuda_ops
+    g = torch.Generator(device=dev).manual_seed(M)
+    x, w, res = (torch.randn(*s, device=dev, generator=g).to(torch.bfloat16) for s in ((M, K), (N, K), (M, N)))
+    bias = torch.randn(N, device=dev, generator=g)
+    for kw in (dict(), dict(bias=bias, residual=res), dict(bias=bias, act="gelu_tanh"), dict(out_dtype=torch.float32)):
+        assert torch.equal(cuda_ops.gemm(x, w, "nt", bn=bn, **kw), cuda_ops.gemm(x, w, "nt", bn=256, **kw))
+    if bn == 192:
+        wt = w.t().contiguous()
+        assert torch.equal(cuda_ops.gemm(x, wt, "nn", bn=bn), cuda_ops.gemm(x, wt, "nn", bn=256))
+        if N % 64 == 0:
+            for a, b in zip(cuda_ops.gemm(x, w, "nt", glu="silu", bn=bn), cuda_ops.gemm(x, w, "nt", glu="silu", bn=256)):
+                assert torch.equal(a, b)
+    cuda_ops.check_status()
+
+
 @pytest.mark.parametrize("B,C,H,W,p,N", [(1, 1, 4, 4, 2, 8), (2, 3, 28, 56, 14, 72), (5, 3, 70, 70, 14, 65), (1, 3, 64, 64, 32, 130)])
 def test_patch_embed_at_the_edges_of_its_tiles(B, C, H, W, p, N, dev):
     """Fewer taps than a tile (4), ragged patches and features, more taps than the offset table holds (3072).  Bound: n
