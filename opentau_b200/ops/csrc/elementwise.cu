@@ -577,7 +577,8 @@ patch_embed_kernel(const PixT* __restrict__ pix, const float* __restrict__ w, co
     arow[i] = m < M ? pix + ((m / P) * C * H + gy * p) * (long long)W + gx * p : nullptr;
     brow[i] = n0 + lr + 4 * i < N ? w + (long long)(n0 + lr + 4 * i) * K : nullptr;
   }
-  float av[8], bv[8];
+  PixT av[8];                                                   // as loaded: converting here would wait for the load
+  float bv[8];
   const auto fetch = [&](int k0) {
     if (k0 % PE_TAPS == 0) {
       __syncthreads();                                          // the previous chunk is no longer read
@@ -593,11 +594,7 @@ patch_embed_kernel(const PixT* __restrict__ pix, const float* __restrict__ w, co
       const int off = k < K ? tap_off[k % PE_TAPS] : 0;
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        av[2 * j + i] = 0.f;
-        if (k < K && arow[i] != nullptr) {
-          if constexpr (sizeof(PixT) == 4) av[2 * j + i] = arow[i][off];
-          else av[2 * j + i] = __bfloat162float(arow[i][off]);
-        }
+        av[2 * j + i] = k < K && arow[i] != nullptr ? arow[i][off] : PixT(0.f);
         bv[2 * j + i] = k < K && brow[i] != nullptr ? brow[i][k] : 0.f;
       }
     }
@@ -617,7 +614,7 @@ patch_embed_kernel(const PixT* __restrict__ pix, const float* __restrict__ w, co
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        as[(lk + 8 * j) * PE_LD + lr + 4 * i] = av[2 * j + i];
+        as[(lk + 8 * j) * PE_LD + lr + 4 * i] = (float)av[2 * j + i];
         bs[(lk + 8 * j) * PE_LD + lr + 4 * i] = bv[2 * j + i];
       }
     __syncthreads();                                            // the other buffer was last read before this barrier
