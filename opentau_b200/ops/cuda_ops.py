@@ -64,14 +64,16 @@ def check_status(reset: bool = True) -> None:
 SKINNY = os.environ.get("OPENTAU_B200_SKINNY_GEMM", "1") != "0"
 
 
-def use_skinny(layout: str, M: int, N: int, accumulate: bool, bn: int) -> bool:
-    """``x @ W^T`` with few rows goes to the weight-streaming split-K kernel."""
+def use_skinny(layout: str, M: int, N: int, accumulate: bool, bn: int, K: int = 0, gated: bool = True) -> bool:
+    """``x @ W^T`` with few rows goes to the weight-streaming split-K kernel.  ``K`` and ``gated`` (the product ends in a
+    gated residual, which only that kernel fuses) narrow the rule at 65 to 256 rows."""
     if not SKINNY or layout != "nt" or accumulate or bn:
         return False
-    # measured inside a replayed graph: up to 64 rows the split-K kernel always wins (50 x 8192 x 1024 7.8 us against
-    # 10.2); at 65..256 rows only where the persistent kernel has too few tiles for the chip (200 x 1024 x 4096 14.5 us
-    # against 17.2, but 200 x 2560 x 1024 11.8 against 7.6)
-    return M <= 64 or (M <= 256 and N <= 2048)
+    # measured inside a replayed graph: up to 64 rows the split-K kernel always wins (50 x 8192 x 1024 6.4 us against
+    # 9.1, 50 x 1024 x 4096 6.0 against 16.2); at 65..256 rows only where the persistent kernel has too few tiles for the
+    # chip and a long sum (200 x 1024 x 4096 12.8 us against 16.3, but 200 x 1024 x 2048 11.5 against 9.8 and 256 x 768 x 768
+    # 11.1 against 6.0, where it needs the 2.3 us it saves on the gated residual's launch)
+    return M <= 64 or (M <= 256 and N <= 2048 and (gated or K >= 3072))
 
 
 class _SkinnyArgs(ctypes.Structure):
@@ -170,7 +172,7 @@ def gemm(a: Tensor, b: Tensor, layout: str, bias: Tensor | None = None, residual
         ldo2 = glu_out.stride(0)
     if splits and (layout != "nt" or accumulate):
         raise ValueError("the split-K kernel computes a @ b^T without accumulation")
-    skinny = bool(splits) or use_skinny(layout, M, N, accumulate, bn)
+    skinny = bool(splits) or use_skinny(layout, M, N, accumulate, bn, K, gate is not None)
     g_stride, g_rows = 0, 1
     if gate is not None:
         # out = residual + gate * (a @ b^T): rows of N gates, one per `M / gate rows` consecutive output rows
@@ -247,7 +249,7 @@ def rows_linear(x: Tensor, w: Tensor, bias: Tensor | None = None, *, norm: RowNo
     if norm is not None:
         x = norm.apply(x)
     gate = gated_by.gate if gated_by is not None else None
-    if not use_skinny("nt", R, N, False, 0):
+    if not use_skinny("nt", R, N, False, 0, K, gate is not None):
         if gate is not None:
             y = gemm(x, w, "nt", bias=bias)
             out = torch.empty_like(y)
