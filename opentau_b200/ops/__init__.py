@@ -249,9 +249,9 @@ def mha(q: Tensor, k: Tensor, v: Tensor, scale: float, add_mask: Tensor | None =
     B, S, _, _ = q.shape
     Sk = k.shape[1]
     zq = torch.zeros(B, S, dtype=torch.int32, device=q.device)
-    zk = torch.zeros(B, Sk, dtype=torch.int32, device=q.device)
     oq = torch.ones(B, S, dtype=torch.bool, device=q.device)
-    ok = torch.ones(B, Sk, dtype=torch.bool, device=q.device)
+    zk, ok = (zq, oq) if Sk == S else (torch.zeros(B, Sk, dtype=torch.int32, device=q.device),
+                                       torch.ones(B, Sk, dtype=torch.bool, device=q.device))
     return fused.block_attention(q, k, v, zq, zk, oq, ok, scale)
 
 

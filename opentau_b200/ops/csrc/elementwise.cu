@@ -311,6 +311,8 @@ __global__ void ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bf
                               const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
                               float* __restrict__ mean_out, float* __restrict__ rstd_out, int H, float eps) {
   __shared__ float red[32];
+  pdl_launch_dependents();
+  pdl_wait();
   const long long row = blockIdx.x;
   const __nv_bfloat16* xr = x + row * (long long)H;
   float v[MAXV][8];
@@ -478,6 +480,8 @@ __global__ void rope_kernel(const __nv_bfloat16* __restrict__ x, long long sb, l
 // After the fused q/k/v projection of ONE tower (no autograd): per (token, head) split the row, RMS-normalise q and
 // k heads (Qwen3 / Gemma-3 qk-norm; optional), rotate q and k, and write q densely and k / v through strides, so
 // that new keys and values can land directly behind the cached prefix.  One warp per (token, head slot).
+// A lane holds four pairs (i, i + D / 2): consecutive ones where every row allows 64-bit accesses (VEC), else 32 apart.
+template <bool VEC>
 __global__ void qkv_post_kernel(const __nv_bfloat16* __restrict__ qkv, long long ld, const __nv_bfloat16* __restrict__ qw,
                                 const __nv_bfloat16* __restrict__ kw, float eps, int unit_offset,
                                 const float* __restrict__ cosb, const float* __restrict__ sinb,
@@ -501,26 +505,56 @@ __global__ void qkv_post_kernel(const __nv_bfloat16* __restrict__ qkv, long long
   else if (kind == 1) dst = k_out + b * k_sb + t * k_ss + (long long)(slot - H) * D;
   else dst = v_out + b * v_sb + t * v_ss + (long long)(slot - H - Hkv) * D;
   if (kind == 2) {
-    for (int i = lane; i < D; i += 32) dst[i] = src[i];
+    if (VEC) {
+      for (int i = lane * 4; i < D; i += 128) *reinterpret_cast<uint2*>(dst + i) = *reinterpret_cast<const uint2*>(src + i);
+    } else {
+      for (int i = lane; i < D; i += 32) dst[i] = src[i];
+    }
     return;
   }
-  float x1[4], x2[4];                                          // D <= 256: at most 4 pairs per lane
-  float ss = 0.f;
+  const auto at = [&](int j) { return VEC ? lane * 4 + j : lane + 32 * j; };      // D <= 256: at most 4 pairs per lane
+  const auto load4 = [&](const __nv_bfloat16* p, float* v) {
+    if (VEC) {
+      if (at(0) >= half) {
+        v[0] = v[1] = v[2] = v[3] = 0.f;
+        return;
+      }
+      const uint2 u = *reinterpret_cast<const uint2*>(p + at(0));
+      const float2 a = unpack_bf16(u.x), b2 = unpack_bf16(u.y);
+      v[0] = a.x; v[1] = a.y; v[2] = b2.x; v[3] = b2.y;
+    } else {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int i = lane + 32 * j;
-    x1[j] = i < half ? __bfloat162float(src[i]) : 0.f;
-    x2[j] = i < half ? __bfloat162float(src[i + half]) : 0.f;
-    ss += x1[j] * x1[j] + x2[j] * x2[j];
+      for (int j = 0; j < 4; ++j) v[j] = at(j) < half ? __bfloat162float(p[at(j)]) : 0.f;
+    }
+  };
+  float x1[4], x2[4], c[4], sn[4];
+  load4(src, x1);
+  load4(src + half, x2);
+  const float* cp = cosb + tok * half;
+  const float* sp = sinb + tok * half;
+  if (VEC) {
+    if (at(0) < half) {
+      *reinterpret_cast<float4*>(c) = *reinterpret_cast<const float4*>(cp + at(0));
+      *reinterpret_cast<float4*>(sn) = *reinterpret_cast<const float4*>(sp + at(0));
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      c[j] = at(j) < half ? cp[at(j)] : 0.f;
+      sn[j] = at(j) < half ? sp[at(j)] : 0.f;
+    }
   }
   const __nv_bfloat16* w = kind == 0 ? qw : kw;
   if (w != nullptr) {
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) ss += x1[j] * x1[j] + x2[j] * x2[j];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     const float rstd = rsqrtf(ss / D + eps);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int i = lane + 32 * j;
+      const int i = at(j);
       if (i < half) {
         const float w1 = __bfloat162float(w[i]) + (unit_offset ? 1.f : 0.f);
         const float w2 = __bfloat162float(w[i + half]) + (unit_offset ? 1.f : 0.f);
@@ -530,15 +564,25 @@ __global__ void qkv_post_kernel(const __nv_bfloat16* __restrict__ qkv, long long
       }
     }
   }
-  const float* cp = cosb + tok * half;
-  const float* sp = sinb + tok * half;
+  if (VEC) {
+    if (at(0) < half) {
+      float a[4], b2[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int i = lane + 32 * j;
-    if (i < half) {
-      const float c = cp[i], sn = sp[i];
-      dst[i] = __float2bfloat16(x1[j] * c - x2[j] * sn);
-      dst[i + half] = __float2bfloat16(x2[j] * c + x1[j] * sn);
+      for (int j = 0; j < 4; ++j) {
+        a[j] = x1[j] * c[j] - x2[j] * sn[j];
+        b2[j] = x2[j] * c[j] + x1[j] * sn[j];
+      }
+      *reinterpret_cast<uint2*>(dst + at(0)) = make_uint2(pack_bf16(a[0], a[1]), pack_bf16(a[2], a[3]));
+      *reinterpret_cast<uint2*>(dst + half + at(0)) = make_uint2(pack_bf16(b2[0], b2[1]), pack_bf16(b2[2], b2[3]));
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int i = at(j);
+      if (i < half) {
+        dst[i] = __float2bfloat16(x1[j] * c[j] - x2[j] * sn[j]);
+        dst[i + half] = __float2bfloat16(x2[j] * c[j] + x1[j] * sn[j]);
+      }
     }
   }
 }
@@ -1026,7 +1070,7 @@ extern "C" int otb_ln_fwd(const void* x, const void* w, const void* b, void* y, 
                           long long rows, int H, float eps, cudaStream_t stream) {
   if (H % 8 || rows <= 0) return -1;
   dim3 grid((unsigned)rows);
-  LAUNCH_BY_H(ln_fwd_kernel, H, (const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, mean, rstd, H, eps);
+  LAUNCH_BY_H_PDL(ln_fwd_kernel, H, (const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, mean, rstd, H, eps);
   return (int)cudaGetLastError();
 }
 
@@ -1066,9 +1110,14 @@ extern "C" int otb_qkv_post(const void* qkv, long long ld, const void* qw, const
   if (D % 2 || D > 256 || B <= 0 || T <= 0) return -1;
   const long long warps = (long long)B * T * (H + 2 * Hkv);
   const unsigned blocks = (unsigned)((warps * 32 + 255) / 256);
-  cudaError_t e = launch_pdl(qkv_post_kernel, dim3(blocks), dim3(256), 0, stream, 0u, (const bf16*)qkv, ld,
-                             (const bf16*)qw, (const bf16*)kw, eps, unit_offset, cosb, sinb, (bf16*)q_out, (bf16*)k_out,
-                             k_sb, k_ss, (bf16*)v_out, v_sb, v_ss, B, T, H, Hkv, D);
+  // 64-bit accesses: four values of a half head at a time, every row of every tensor on an 8-byte boundary (tables: 16)
+  const bool vec = D % 8 == 0 && ld % 4 == 0 && k_sb % 4 == 0 && k_ss % 4 == 0 && v_sb % 4 == 0 && v_ss % 4 == 0 &&
+                   ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) |
+                     reinterpret_cast<uintptr_t>(k_out) | reinterpret_cast<uintptr_t>(v_out)) & 7) == 0 &&
+                   ((reinterpret_cast<uintptr_t>(cosb) | reinterpret_cast<uintptr_t>(sinb)) & 15) == 0;
+  cudaError_t e = launch_pdl(vec ? qkv_post_kernel<true> : qkv_post_kernel<false>, dim3(blocks), dim3(256), 0, stream, 0u,
+                             (const bf16*)qkv, ld, (const bf16*)qw, (const bf16*)kw, eps, unit_offset, cosb, sinb,
+                             (bf16*)q_out, (bf16*)k_out, k_sb, k_ss, (bf16*)v_out, v_sb, v_ss, B, T, H, Hkv, D);
   return (int)e;
 }
 

@@ -544,3 +544,19 @@ def test_patch_embed_at_the_edges_of_its_tiles(B, C, H, W, p, N, dev):
     x = pix.double().view(B, C, H // p, p, W // p, p).permute(0, 2, 4, 1, 3, 5).reshape(B, -1, C * p * p)
     want = x @ w.double().view(N, -1).t() + b.double() + pos.double()
     assert (got.double() - want).norm() < max(8, (C * p * p) ** 0.5) * 2 ** -24 * want.norm()
+
+
+@pytest.mark.parametrize("D", [8, 64, 72, 256])
+def test_qkv_post_off_its_alignment_gives_the_same_values(D, dev):
+    """Rows that start on a 2-byte boundary take 16-bit accesses; the arithmetic is the same but for the compiler's choice
+    of fused multiply-adds (one rounding to bf16, 2^-8)."""
+    from opentau_b200 import ops
+    B, T, H, Hkv = 2, 5, 4, 2
+    W = (H + 2 * Hkv) * D
+    wide = torch.randn(B, T, W + 1, device=dev).to(torch.bfloat16)
+    cos, sin = (torch.randn(B, T, D // 2, device=dev) for _ in range(2))
+    with torch.no_grad():
+        want = ops.qkv_post(wide[..., 1:].contiguous(), H, Hkv, D, None, None, cos, sin)
+        got = ops.qkv_post(wide[..., 1:], H, Hkv, D, None, None, cos, sin)
+    for a, b in zip(got, want):
+        torch.testing.assert_close(a, b, rtol=2 ** -7, atol=0)
