@@ -3,6 +3,7 @@
 from __future__ import annotations
 
 import os
+from functools import lru_cache
 from ctypes import byref, c_float, c_int, c_longlong, c_void_p
 
 import torch
@@ -61,6 +62,7 @@ def split_kv(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int) -> int:
     return max(1, min(8, NUM_SMS // ctas, nblk // 2))
 
 
+@lru_cache(maxsize=1024)
 def split_cluster(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int) -> int:
     """CTAs of the cluster that shares the keys of a 64-row query tile and merges on chip (1: not this path)."""
     g = H // Hkv
@@ -112,6 +114,15 @@ def attn_fwd(q: Tensor, k: Tensor, v: Tensor, q_blk: Tensor, k_blk: Tensor, q_va
     return o, lse
 
 
+@lru_cache(maxsize=1024)
+def bwd_splits(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int) -> tuple[int, int, int]:
+    """Parts that the streamed blocks of dQ, dK and dV are dealt to (a function of the sizes alone)."""
+    n = (c_int(), c_int(), c_int())
+    _lib.load("attention_bwd_tcgen05").otb_attn_bwd_splits(c_int(B), c_int(Sq), c_int(Sk), c_int(H), c_int(Hkv), c_int(D),
+                                                           *(byref(x) for x in n))
+    return tuple(x.value for x in n)
+
+
 def attn_bwd(do: Tensor, q: Tensor, k: Tensor, v: Tensor, o: Tensor, lse: Tensor, q_blk: Tensor, k_blk: Tensor,
              q_valid: Tensor, k_valid: Tensor, scale: float, splits: tuple[int, int, int] | None = None):
     """Returns ``(dq, dk, dv)``; scratch and outputs are allocated here.  ``splits`` forces the parts that the streamed
@@ -133,9 +144,7 @@ def attn_bwd(do: Tensor, q: Tensor, k: Tensor, v: Tensor, o: Tensor, lse: Tensor
     kv = _u8(k_valid)
     lib = _lib.load("attention_bwd_tcgen05")
     if splits is None:
-        n = (c_int(), c_int(), c_int())
-        lib.otb_attn_bwd_splits(c_int(B), c_int(Sq), c_int(Sk), c_int(H), c_int(Hkv), c_int(D), *(byref(x) for x in n))
-        splits = tuple(x.value for x in n)
+        splits = bwd_splits(B, Sq, Sk, H, Hkv, D)
     parts = [torch.empty(m, *t.shape, dtype=torch.float32, device=q.device) if m > 1 else None
              for m, t in zip(splits, (dq, dk, dv))]
     rc = lib.otb_attn_bwd(
