@@ -166,8 +166,7 @@ def gated_mlp_gated_residual(x: Tensor, w_gate_up: Tensor, w_down: Tensor, act: 
     if gate is not None and x.dim() == 3 and _native_nograd(x, w_gate_up, residual, gate):
         from . import cuda_ops
         rows, g2 = x.shape[0] * x.shape[1], _gate_rows(gate, x)
-        if g2 is not None and cuda_ops.use_skinny("nt", rows, w_down.shape[0], False, 0) \
-                and cuda_ops.use_skinny("nt", rows, w_gate_up.shape[0], False, 0):
+        if g2 is not None and cuda_ops.use_skinny("nt", rows, w_down.shape[0], False, 0):
             h = cuda_ops.gemm(x.reshape(rows, -1), w_gate_up, "nt", glu=act, store_out=False)
             out = cuda_ops.gemm(h, w_down, "nt", residual=residual.reshape(rows, -1).contiguous(), gate=g2)
             return out.view(*x.shape[:-1], w_down.shape[0])

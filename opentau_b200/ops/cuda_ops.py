@@ -65,15 +65,19 @@ SKINNY = os.environ.get("OPENTAU_B200_SKINNY_GEMM", "1") != "0"
 
 
 def use_skinny(layout: str, M: int, N: int, accumulate: bool, bn: int, K: int = 0, gated: bool = True) -> bool:
-    """``x @ W^T`` with few rows goes to the weight-streaming split-K kernel.  ``K`` and ``gated`` (the product ends in a
-    gated residual, which only that kernel fuses) narrow the rule at 65 to 256 rows."""
+    """``x @ W^T`` with few rows goes to the weight-streaming split-K kernel.  ``gated``: the product ends in a gated
+    residual, which only that kernel fuses (the gate then multiplies the fp32 sum)."""
     if not SKINNY or layout != "nt" or accumulate or bn:
         return False
+    if gated:
+        # the alternative rounds the sum to bf16 in front of the gate: every few-row product keeps the fusion, but for
+        # more columns than the 128 x 256 tiles of the persistent kernel need to fill the chip
+        return M <= 128 or (M <= 256 and N <= 8192)
     # measured inside a replayed graph: up to 64 rows the split-K kernel always wins (50 x 8192 x 1024 6.4 us against
     # 9.1, 50 x 1024 x 4096 6.0 against 16.2); at 65..256 rows only where the persistent kernel has too few tiles for the
     # chip and a long sum (200 x 1024 x 4096 12.8 us against 16.3, but 200 x 1024 x 2048 11.5 against 9.8 and 256 x 768 x 768
-    # 11.1 against 6.0, where it needs the 2.3 us it saves on the gated residual's launch)
-    return M <= 64 or (M <= 256 and N <= 2048 and (gated or K >= 3072))
+    # 11.1 against 6.0)
+    return M <= 64 or (M <= 256 and N <= 2048 and K >= 3072)
 
 
 class _SkinnyArgs(ctypes.Structure):

@@ -560,3 +560,25 @@ def test_qkv_post_off_its_alignment_gives_the_same_values(D, dev):
         got = ops.qkv_post(wide[..., 1:], H, Hkv, D, None, None, cos, sin)
     for a, b in zip(got, want):
         torch.testing.assert_close(a, b, rtol=2 ** -7, atol=0)
+
+
+@pytest.mark.parametrize("rows,cols,mlp", [(65, 1024, 4096), (130, 2048, 4096), (250, 4096, 512), (128, 2056, 96)])
+def test_gated_mlp_at_65_to_256_rows_gates_the_fp32_sum(rows, cols, mlp, dev):
+    """Two launches (gate / up, down with its gate and residual) whatever the widths, and one rounding behind the down
+    product's sum.  One rounding to bf16 moves values spread over their binades by 0.42 x 2^-8 in the 2-norm, a second one in
+    front of the gate by sqrt(2) of that: the bound lies between."""
+    from opentau_b200 import ops
+    from opentau_b200.ops import cuda_ops
+    g = torch.Generator(device=dev).manual_seed(rows)
+    x, wgu, wd, res, gate = (torch.randn(*s, device=dev, generator=g).mul_(k).to(torch.bfloat16) for s, k in (
+        ((1, rows, 64), 1.0), ((2 * mlp, 64), 0.1), ((cols, mlp), 0.05), ((1, rows, cols), 1e-3), ((1, 1, cols), 1.0)))
+    with torch.no_grad():
+        before = cuda_ops.launch_count
+        got = ops.gated_mlp_gated_residual(x, wgu, wd, "silu", res, gate)
+        assert cuda_ops.launch_count - before == 2
+        h = cuda_ops.gemm(x[0], wgu, "nt", glu="silu", store_out=False)
+        one = ops.linear_gated_residual(h[None], wd, None, res, gate)
+    want = res.double() + gate.double() * (h.double() @ wd.double().t())
+    for y in (got, one):
+        assert (y.double() - want).norm() < 0.5 * 2 ** -8 * want.norm()
+    cuda_ops.check_status()

@@ -249,3 +249,12 @@ def test_forked_norms_give_the_gradients_of_norm_plus_residual():
     with torch.no_grad():
         h, xr = ops.rms_norm_fork(x, w)
         assert xr is x                                                                       # nothing to fork
+
+
+@pytest.mark.parametrize("rows", [1, 65, 128, 129, 256])
+@pytest.mark.parametrize("cols", [1024, 2056, 4096, 8192])
+def test_gated_few_row_products_keep_the_gate_in_their_epilogue(rows, cols):
+    """The few-row kernel alone multiplies the gate into the fp32 sum: every width that ever took it does."""
+    from opentau_b200.ops import cuda_ops
+    assert cuda_ops.use_skinny("nt", rows, cols, False, 0, 2048, True)
+    assert cuda_ops.use_skinny("nt", rows, cols, False, 0)               # what ``gemm(gate=...)`` accepts
