@@ -27,7 +27,7 @@
 // kernel adds in a fixed order: with one kv head, 38 key blocks would leave three quarters of the chip idle.
 //
 //   forward : online softmax; writes O (B,Sq,H*D) and the natural-log LSE (B,H,Sq); a row that sees no key gets
-//             O = 0 and LSE = 0
+//             O = 0 and LSE = 0, one with a NaN among its visible scores NaN in both, as the dense evaluation does
 //   dQ      : P is recomputed from LSE; dS = P * (dP - delta) * scale; dQ += dS K
 //   dK / dV : the heads of the GQA group are one stream, so the sum over the group happens in registers (no atomics)
 //   delta   : rowsum(O * dO), one warp per row
@@ -64,6 +64,13 @@ __device__ __forceinline__ float warp_sum(float x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
   return x;
+}
+
+// The larger of two numbers, NaN if either is (fmaxf would drop it).
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
 }
 
 __device__ __forceinline__ void cp_async16(float* dst, const float* src, bool read) {
@@ -287,6 +294,7 @@ __global__ void __launch_bounds__(F32_THREADS, G == 1 ? 2 : 1) attn_f32_fwd_kern
   const bool row_ok = (own.ok >> row) & 1;
   const int row_blk = row_ok ? p.q_blk[(long long)b * p.Sq + q0 + row] : INT_MIN;
   float m = -INFINITY, l = 0.f;
+  unsigned seen = 0;                                 // visible keys met so far by this thread
   const int grp = warp >> 2, r0 = 8 * (warp & 3), col = lane * 4 < Dp ? lane * 4 : 0;
   float acc[8][4 * G];
 #pragma unroll
@@ -319,12 +327,13 @@ __global__ void __launch_bounds__(F32_THREADS, G == 1 ? 2 : 1) attn_f32_fwd_kern
         if (row_ok && ((cur >> j) & 1ull) && kblk[cur0 + j] <= row_blk) {
           vis |= 1u << e;
           s[e] *= p.scale;
-          mt = fmaxf(mt, s[e]);
+          mt = max_nan(mt, s[e]);
         }
       }
+      seen |= vis;
 #pragma unroll
-      for (int x = 4; x > 0; x >>= 1) mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, x));
-      const float mn = fmaxf(m, mt);
+      for (int x = 4; x > 0; x >>= 1) mt = max_nan(mt, __shfl_xor_sync(0xffffffffu, mt, x));
+      const float mn = max_nan(m, mt);
       float corr = 1.f, sum = 0.f;
       if (mn != -INFINITY) corr = m == -INFINITY ? 0.f : expf(m - mn);
 #pragma unroll
@@ -354,10 +363,13 @@ __global__ void __launch_bounds__(F32_THREADS, G == 1 ? 2 : 1) attn_f32_fwd_kern
   cp_async_wait<0>();
   __syncthreads();
   // the second group's sums go through shared memory (over K); 1 / l through the factors
-  const bool any = l > 0.f;
+#pragma unroll
+  for (int x = 4; x > 0; x >>= 1) seen |= __shfl_xor_sync(0xffffffffu, seen, x);
   if (part == 0) {
-    sC[row] = any ? 1.f / l : 0.f;
-    if (q0 + row < p.Sq) lse[((long long)b * p.H + h) * p.Sq + q0 + row] = any ? m + logf(l) : 0.f;
+    // a maximum that is no finite number is the LSE, and no probability is one: 1 / l is NaN (of l = 0: all scores -inf)
+    const bool finite = fabsf(m) < INFINITY;
+    sC[row] = !seen ? 0.f : finite ? 1.f / l : NAN;
+    if (q0 + row < p.Sq) lse[((long long)b * p.H + h) * p.Sq + q0 + row] = !seen ? 0.f : finite ? m + logf(l) : m;
   }
   if (grp == 1 && lane * 4 < Dp) {
 #pragma unroll

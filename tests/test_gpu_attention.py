@@ -347,3 +347,40 @@ def test_split_backward_matches_the_unsplit_one(D, H, Hkv, splits):
         assert _rel(x, w.double()) < 2 ** -8, name
     for x in got[1:]:
         assert float(x[1, 300:].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("bad_keys", [False, True])
+@pytest.mark.parametrize("H,Hkv,D", [(4, 1, 64), (8, 1, 256)])
+def test_fp32_attention_keeps_nan_and_infinite_scores(H, Hkv, D, bad_keys):
+    """A NaN or infinite row or key of the inputs shows in ``block_attention``'s output where the dense evaluation shows
+    it: a row of nothing but NaN or -inf scores is not one that sees no key."""
+    from opentau_b200 import ops
+    from opentau_b200.ops import prims
+    B, S = 1, 260
+    g = torch.Generator().manual_seed(D)
+    q, k, v, do = (torch.randn(B, S, h, D, generator=g) for h in (H, Hkv, Hkv, H))
+    k[..., 0] = 2.0
+    q[0, 5, 0], q[0, 70, H - 1, 3] = float("nan"), float("nan")      # all scores of a row NaN
+    q[0, 33, 1, 0], q[0, 200, 0, 0] = 3e38, -3e38                    # all +inf, all -inf
+    if bad_keys:
+        k[0, 250] = float("nan")                                     # for the rows that see it
+    blk = (torch.arange(S) // 20).int()[None]
+    ok = torch.ones(B, S, dtype=torch.bool)
+    ok[0, 100:110] = False                                           # rows that see nothing stay zero
+    args = (blk, blk, ok, ok, D ** -0.5)
+    dev_args = (*(t.cuda() for t in args[:4]), args[4])
+    o_w, lse_w = prims.attn_fwd(q, k, v, *args)
+    a = [t.cuda().requires_grad_() for t in (q, k, v)]
+    lse = prims.attn_fwd(*(t.detach() for t in a), *dev_args)[1]
+    o = ops.block_attention(*a, *dev_args)
+    pairs = [("o", o.detach(), o_w), ("lse", lse, lse_w)]
+    if not bad_keys:                # (the dense backward also spreads NaN between rows and keys that do not meet)
+        dq_w, _, dv_w = prims.attn_bwd(do.reshape(B, S, -1), q, k, v, o_w, lse_w, *args)
+        dq, _, dv = torch.autograd.grad(o, a, do.reshape(B, S, -1).cuda())
+        pairs += [("dq", dq, dq_w), ("dv", dv, dv_w)]
+    for name, x, w in pairs:
+        x = x.cpu()
+        assert torch.equal(x.isnan(), w.isnan()) and torch.equal(x.isposinf(), w.isposinf()), name
+        assert torch.equal(x.isneginf(), w.isneginf()), name
+        torch.testing.assert_close(x[w.isfinite()], w[w.isfinite()], rtol=1e-4, atol=1e-4)
+    assert not o_w[0, 105].any() and not lse_w[0, :, 105].any()
