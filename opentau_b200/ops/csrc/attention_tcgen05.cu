@@ -499,8 +499,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         for (int e = 0; e < DPAD / 32; ++e) acc[e] = 0.f;
         constexpr int V = DPAD >= 128 ? 4 : 2;       // floats per lane and piece
         for (int sp = 0; sp < p.nsplit; ++sp) {
-          const float w = __shfl_sync(0xffffffffu, w_s, sp) * inv;
-          if (w == 0.f) continue;                    // nothing visible there
+          const float w = __shfl_sync(0xffffffffu, w_s, sp) * inv;   // 0 where nothing is visible; a NaN there stays one
           const float* src = slot_row(sp) + lane * V;
 #pragma unroll
           for (int c = 0; c < DPAD / (32 * V); ++c) {

@@ -192,6 +192,28 @@ def test_cluster_merge_matches_single_pass(H, Hkv, D, Sq, Sk, nsplit):
     assert float(o[1].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("nsplit", [3, 8])
+@pytest.mark.parametrize("H,Hkv,D", [(8, 1, 256), (4, 1, 64), (16, 16, 72)])
+def test_cluster_merge_keeps_nan(H, Hkv, D, nsplit):
+    """A NaN in a query row or in a key's value reaches the same outputs as in one pass: a partial whose weight is zero
+    because its row sum is NaN is not one that saw nothing."""
+    from opentau_b200.ops import attention_native, cuda_ops
+    B, Sq, Sk = 2, 50, 700
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q, k, v = (torch.randn(B, S, h, D, device="cuda", generator=g).to(torch.bfloat16)
+               for S, h in ((Sq, H), (Sk, Hkv), (Sk, Hkv)))
+    q[0, 7, H // 2, 1] = q[1, 20] = v[1, 500, 0, 3] = float("nan")
+    zero, ok = (lambda S: torch.zeros(B, S, dtype=torch.int32, device="cuda"),
+                lambda S: torch.ones(B, S, dtype=torch.bool, device="cuda"))
+    args = (q, k, v, zero(Sq), zero(Sk), ok(Sq), ok(Sk), D ** -0.5)
+    want = attention_native.attn_fwd(*args, nsplit=1)[0]
+    got = attention_native.attn_fwd(*args, nsplit=nsplit, cluster=True)[0]
+    cuda_ops.check_status()
+    assert torch.equal(got.isnan(), want.isnan())
+    assert want.view(B, Sq, H, D)[0, 7, H // 2].isnan().all() and want.view(B, Sq, H, D)[1, 20].isnan().all()
+    assert want.view(B, Sq, H, D)[1, 30, 0, 3].isnan() and not want[0, 8].isnan().any()
+
+
 @pytest.mark.parametrize("D", [32, 72, 128, 160, 256])
 @pytest.mark.parametrize("H,Hkv", [(8, 1), (6, 3), (4, 4)])
 @pytest.mark.parametrize("Sq,cross", [(50, 0), (131, 0), (50, 203), (33, 64)])
