@@ -19,7 +19,7 @@ import torch
 from torch import Tensor, nn
 
 from .. import ops
-from .layers import AdaRMSNorm, DecoderLayer, Tower, TowerConfig
+from .layers import AdaRMSNorm, DecoderLayer, GatedMLP, Linear, RMSNorm, Tower, TowerConfig, is_plain
 
 
 @dataclass
@@ -237,13 +237,28 @@ class DualStreamDecoder(nn.Module):
 
     # -- few-row inference: one tower behind a cached prefix ----------------------------------------
     def can_run_rows(self, ti: int, x: Tensor) -> bool:
-        """Whether :meth:`rows_pass` covers tower ``ti`` (pre-norm layers whose widths the vector loads take, weights
-        resident and dense); other towers take :meth:`forward`."""
-        cfg = self.towers[ti].cfg
-        w = self.towers[ti].layers[0].self_attn.qkv_proj.weight
-        return (ops.can_fuse_qkv_post(x, cfg.head_dim) and not cfg.sandwich_norms and self.param_gate is None
-                and not self.training and w.dtype == torch.bfloat16 and cfg.hidden_size % 8 == 0
-                and cfg.intermediate_size % 32 == 0 and (cfg.num_attention_heads * cfg.head_dim) % 8 == 0)
+        """Whether :meth:`rows_pass` covers tower ``ti`` for embeddings like ``x`` (pre-norm layers whose widths the vector
+        loads take, bf16 weights resident, nothing but the layers' own arithmetic in their modules); other towers take
+        :meth:`forward`."""
+        tower, cfg = self.towers[ti], self.towers[ti].cfg
+        if not (ops.can_fuse_qkv_post(x, cfg.head_dim) and not cfg.sandwich_norms and self.param_gate is None
+                and not self.training and cfg.hidden_size % 8 == 0 and cfg.intermediate_size % 32 == 0
+                and (cfg.num_attention_heads * cfg.head_dim) % 8 == 0):
+            return False
+        # the pass reads parameters where the layers would call modules
+        kind = AdaRMSNorm if cfg.use_adarms else RMSNorm
+        norms, weights = [tower.norm], []
+        for layer in tower.layers:
+            attn, mlp = layer.self_attn, layer.mlp
+            norms += [layer.input_layernorm, layer.post_attention_layernorm]
+            if not (is_plain(attn.qkv_proj, Linear) and is_plain(attn.o_proj, Linear) and is_plain(mlp, GatedMLP)):
+                return False
+            weights += [attn.qkv_proj.weight, attn.o_proj.weight, mlp.gate_up_proj.weight, mlp.down_proj.weight]
+        if not all(is_plain(n, kind) for n in norms):
+            return False
+        if cfg.use_adarms:
+            weights += [n.dense.weight for n in norms]
+        return all(w.dtype == torch.bfloat16 for w in weights)
 
     def rows_pass(self, ti: int, x: Tensor, cache: KVCache, q_blk: Tensor, q_valid: Tensor, k_blk: Tensor,
                   k_valid: Tensor, tables, mods: list[Tensor] | None = None,

@@ -18,6 +18,12 @@ from torch import Tensor, nn
 from .. import ops
 
 
+def is_plain(m: nn.Module, kind: type) -> bool:
+    """Whether calling ``m`` runs ``kind``'s forward pass and nothing else (no wrapper in its place, no hook, no patched
+    method), so that a caller may read its parameters instead."""
+    return type(m) is kind and not (m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__)
+
+
 class Linear(nn.Module):
     """``nn.Linear``-compatible parameters; forward goes through ``ops.linear`` (tcgen05 GEMM)."""
 

@@ -104,6 +104,12 @@ def _skinny_launch(x: Tensor, w: Tensor, out: Tensor | None, M: int, N: int, K: 
     launch_count += 1
 
 
+def _operand(t: Tensor) -> Tensor:
+    """A bf16 operand whose rows the TMA can load (16-byte aligned starts)."""
+    assert t.dtype == torch.bfloat16, "gemm expects bf16 operands"
+    return t.contiguous() if t.stride(-1) != 1 or (t.stride(0) % 8) or (t.data_ptr() % 16) else t
+
+
 def gemm(a: Tensor, b: Tensor, layout: str, bias: Tensor | None = None, residual: Tensor | None = None,
          out: Tensor | None = None, accumulate: bool = False, out_dtype: torch.dtype | None = None,
          glu: str | None = None, glu_out: Tensor | None = None, store_out: bool = True, act: str | None = None,
@@ -111,11 +117,7 @@ def gemm(a: Tensor, b: Tensor, layout: str, bias: Tensor | None = None, residual
     """tcgen05 GEMM.  layout 'nt': a(M,K) b(N,K); 'nn': a(M,K) b(K,N); 'tn': a(K,M) b(K,N).  ``bn`` forces the column
     tile of the persistent kernel, ``splits`` (1, 2, 4, 8) forces the weight-streaming split-K kernel."""
     global launch_count
-    assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16, "gemm expects bf16 operands"
-    if a.stride(-1) != 1 or (a.stride(0) % 8) or (a.data_ptr() % 16):
-        a = a.contiguous()
-    if b.stride(-1) != 1 or (b.stride(0) % 8) or (b.data_ptr() % 16):
-        b = b.contiguous()
+    a, b = _operand(a), _operand(b)
     if layout == "nt":
         M, K = a.shape
         N, Kb = b.shape
@@ -224,7 +226,10 @@ class RowNorm:
         """The norm as its own launch."""
         global launch_count
         R, H = x2.shape
-        y = torch.empty_like(x2)
+        if x2.dtype != torch.bfloat16 or x2.stride(1) != 1 or (self.mod is not None and (
+                self.mod.dtype != torch.bfloat16 or self.mod.stride(1) != 1 or self.mod.shape[1] != 3 * H)):
+            raise ValueError("RowNorm takes bf16 rows and bf16 modulation rows")
+        y = torch.empty(R, H, dtype=x2.dtype, device=x2.device)
         wt = self.weight.to(torch.bfloat16).contiguous() if self.weight is not None else None
         mode = 0 if wt is None else (1 if self.unit_offset else 2)
         _check(_lib.load("elementwise").otb_rms_fwd(
@@ -248,11 +253,22 @@ def rows_linear(x: Tensor, w: Tensor, bias: Tensor | None = None, *, norm: RowNo
     against 2.3 + 6.6 for 50 rows: the code that runs once per launch from a cold instruction cache outweighs the
     launch)."""
     global launch_count
-    R, K = x.shape
-    N = w.shape[0]
     if norm is not None:
         x = norm.apply(x)
+    x, w = _operand(x), _operand(w)
+    R, K = x.shape
+    N = w.shape[0]
     gate = gated_by.gate if gated_by is not None else None
+    if w.shape[1] != K:
+        raise ValueError(f"inner dimensions differ: {tuple(x.shape)} x {tuple(w.shape)}")
+    if residual is not None and (residual.shape != (R, N) or residual.dtype != torch.bfloat16 or not residual.is_contiguous()):
+        raise ValueError("bad residual for rows_linear")
+    if gate is not None and (gate.shape[1] != N or gate.dtype != torch.bfloat16 or gate.stride(1) != 1 or residual is None):
+        raise ValueError("bad gate for rows_linear")
+    if bias is not None:
+        if bias.numel() != N or bias.dtype not in (torch.bfloat16, torch.float32):
+            raise ValueError("bad bias for rows_linear")
+        bias = bias.contiguous()
     if not use_skinny("nt", R, N, False, 0, K, gate is not None):
         if gate is not None:
             y = gemm(x, w, "nt", bias=bias)

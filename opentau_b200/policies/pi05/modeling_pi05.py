@@ -25,7 +25,7 @@ from torch import Tensor, nn
 
 from ... import ops
 from ...models.dual_stream import DualStreamDecoder, KVCache
-from ...models.layers import Linear, Tower, TowerConfig
+from ...models.layers import Linear, Tower, TowerConfig, is_plain
 from ...datasets.action_indexing import add_chunk_start_state, subtract_chunk_start_state
 from ...models.siglip import MultiModalProjector, SiglipConfig, SiglipVisionModel
 from ...utils.tokenizer import load_action_tokenizer, load_text_tokenizer, pad_tokens
@@ -499,10 +499,11 @@ class PI05FlowMatching(nn.Module):
             raise ValueError("response generation needs a tokenizer with bos, eos and pad ids")
         mrope = getattr(self, "_mrope", False)
         L, base, dec = cfg.response_max_length, cache.length, pwe.decoder
-        d = pwe.vlm_cfg.hidden_size
-        probe = cache.k.new_empty(0, 1, d)
-        in_place = (cache.writable_room() >= L and dec.can_run_rows(0, probe)
-                    and pwe.lm_head_weight().shape[0] % 8 == 0)       # the few-row product stores eight logits at a time
+        first = torch.full((B, 1), bos, dtype=torch.long, device=device)
+        emb, head = pwe.embed_language_tokens(first), pwe.lm_head_weight()
+        in_place = (cache.writable_room() >= L and cache.k.dtype == head.dtype == torch.bfloat16
+                    and self._passes_straight_to_decoder() and dec.can_run_rows(0, emb)
+                    and head.shape[0] % 8 == 0)                       # the few-row product stores eight logits at a time
         blk_all = self._const(("resp_blk", B, base, L, str(device)),
                               lambda: torch.zeros(B, base + L, dtype=torch.int32, device=device))
         valid_all = torch.cat([cache.valid[:, :base], torch.zeros(B, L, dtype=torch.bool, device=device)], dim=1)
@@ -512,7 +513,7 @@ class PI05FlowMatching(nn.Module):
         ended = None
         logits = None
         for step in range(L):
-            nxt = torch.full((B, 1), bos, dtype=torch.long, device=device) if step == 0 else logits.argmax(dim=-1)
+            nxt = first if step == 0 else logits.argmax(dim=-1)
             live = one
             if step > 1:
                 live = ~ended
@@ -520,7 +521,8 @@ class PI05FlowMatching(nn.Module):
             tokens.append(nxt), lives.append(live)
             stop = (nxt == eos) | (nxt == pad)
             ended = stop if ended is None else ended | stop
-            emb = pwe.embed_language_tokens(nxt)
+            if step > 0:
+                emb = pwe.embed_language_tokens(nxt)
             pos = offset                                            # a finished sample's pad takes no new position
             offset = offset + live.long()
             if in_place:
@@ -633,11 +635,20 @@ class PI05FlowMatching(nn.Module):
             x_t = ops.euler_step(x_t, v_t, dt, frozen if has_prefix else None, action_prefix)
         return x_t
 
+    def _passes_straight_to_decoder(self) -> bool:
+        """Whether the wrapper's forward pass is the decoder's and nothing hangs on either."""
+        return not any(m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__
+                       for m in (self.wrapper, self.wrapper.decoder))
+
     def _can_plan_loop(self, cache: KVCache, x_t: Tensor) -> bool:
         """Whether :meth:`_planned_loop` covers this policy: the suffix is the action chunk alone, conditioned on time
-        through adaptive norms (a subclass that changes either keeps the step-by-step loop)."""
+        through adaptive norms (a subclass that changes either keeps the step-by-step loop), in bf16 from the action
+        projection to the velocity head."""
         cls, dec = type(self), self.wrapper.decoder
         if cls.denoise_step is not PI05FlowMatching.denoise_step or cls.embed_suffix is not PI05FlowMatching.embed_suffix:
+            return False
+        if not all(is_plain(m, Linear) and m.weight.dtype == torch.bfloat16
+                   for m in (self.action_in_proj, self.action_out_proj)) or not self._passes_straight_to_decoder():
             return False
         ti, T = len(dec.towers) - 1, x_t.shape[1]
         w_in = self.action_in_proj.weight

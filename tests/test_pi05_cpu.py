@@ -211,3 +211,72 @@ def test_stacked_adaptive_norm_weights_follow_in_place_updates():
     out = pol.train()(b)                                                # training still reaches the individual parameters
     (out["MSE"] + out["CE"]).backward()
     assert first.grad is not None and first.grad.abs().sum() > 0
+
+
+def test_row_pass_is_refused_where_modules_do_more_than_their_parameters(monkeypatch):
+    """The few-row pass reads weights where the layers call modules: it steps aside for weights of another type, hooks,
+    wrappers and patched methods anywhere on its way, from the action projection to the velocity head."""
+    from types import SimpleNamespace
+
+    from torch import nn
+
+    from opentau_b200 import ops
+    pol = tiny_pi05().to(torch.bfloat16).eval()
+    m, dec = pol.model, pol.model.wrapper.decoder
+    monkeypatch.setattr(ops, "can_fuse_qkv_post", lambda x, d: True)          # what a CUDA device answers
+    k = SimpleNamespace(is_cuda=True, shape=(2, 1, 64, 1, 64), new_empty=lambda *s: torch.empty(*s, dtype=torch.bfloat16))
+    cache, x_t = SimpleNamespace(k=k, length=20), torch.empty(1, 10, 32)
+
+    def plans() -> bool:
+        return m._can_plan_loop(cache, x_t)
+
+    assert plans() and dec.can_run_rows(0, torch.empty(0)) and m._passes_straight_to_decoder()
+    layer = dec.towers[1].layers[-1]
+    for mod in (m.action_in_proj, m.action_out_proj, layer.self_attn.qkv_proj, layer.self_attn.o_proj,
+                layer.mlp.gate_up_proj, layer.mlp.down_proj, layer.input_layernorm.dense, dec.towers[1].norm.dense):
+        mod.float()
+        assert not plans(), mod
+        mod.to(torch.bfloat16)
+        assert plans()
+    for mod in (m.action_in_proj, m.action_out_proj, layer.self_attn.qkv_proj, layer.self_attn.o_proj, layer.mlp,
+                layer.input_layernorm, layer.post_attention_layernorm, dec.towers[1].norm, m.wrapper, dec):
+        for add in (mod.register_forward_hook, mod.register_forward_pre_hook):
+            handle = add(lambda *a: None)
+            assert not plans(), mod
+            handle.remove()
+        mod.forward = mod.forward
+        assert not plans(), mod
+        del mod.forward
+        assert plans()
+
+    class Wrapped(nn.Module):
+        def __init__(self, inner):
+            super().__init__()
+            self.inner = inner
+
+    for name in ("qkv_proj", "o_proj"):
+        inner = getattr(layer.self_attn, name)
+        setattr(layer.self_attn, name, Wrapped(inner))
+        assert not plans()
+        setattr(layer.self_attn, name, inner)
+    layer.mlp, mlp = Wrapped(layer.mlp), layer.mlp
+    assert not plans()
+    layer.mlp = mlp
+    assert plans()
+    dec.towers[0].layers[0].mlp.down_proj.float()
+    assert plans() and not dec.can_run_rows(0, torch.empty(0))
+
+
+def test_row_products_refuse_operands_they_would_misread():
+    import pytest
+
+    from opentau_b200.ops import cuda_ops
+    x, w, f = torch.zeros(4, 16, dtype=torch.bfloat16), torch.zeros(24, 16, dtype=torch.bfloat16), torch.float32
+    norm = cuda_ops.RowNorm(1e-6, mod=torch.zeros(3, 72))
+    for args, kw in (((x.float(), w), {}), ((x, w.float()), {}), ((x[:, :8], w), {}),
+                     ((x, w), dict(residual=torch.zeros(4, 24, dtype=f))), ((x, w), dict(residual=x)),
+                     ((x, w), dict(bias=torch.zeros(16))), ((x, w), dict(bias=torch.zeros(24, dtype=torch.float64))),
+                     ((x, w), dict(residual=torch.zeros(4, 24, dtype=torch.bfloat16), gated_by=norm)),
+                     ((x, w), dict(norm=cuda_ops.RowNorm(1e-6, mod=torch.zeros(3, 48))))):
+        with pytest.raises((ValueError, AssertionError)):
+            cuda_ops.rows_linear(*args, **kw)
