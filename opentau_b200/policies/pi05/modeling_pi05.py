@@ -1016,7 +1016,7 @@ class PI05Policy(PreTrainedPolicy):
     def enable_cuda_graphs(self, flag: bool = True) -> None:
         """Replay the sampler (prefix pass + Euler loop) from a CUDA graph: one launch per action chunk."""
         self._use_graphs = bool(flag)
-        self._graph_runner = self._sampler_runner = None
+        self._graph_runner = None
         self._request_runners, self._request_stats = {}, None
 
     def _ensure_eval(self) -> None:
@@ -1035,20 +1035,33 @@ class PI05Policy(PreTrainedPolicy):
                 and cls._prefix_kwargs is PI05Policy._prefix_kwargs
                 and not (normalize.SNAP_WARN_TOL > 0 and self.normalize_inputs._snapping_possible()))
 
-    MAX_REQUEST_KINDS = 4       # captured kinds of request (cameras present, candidate counts) kept at a time
+    MAX_REQUEST_KINDS = 8       # captured kinds of request (cameras present, candidate counts, ...) kept at a time
 
-    def _graphed_request(self, batch, idx, sampler_idx, action_prefix, delay, noise, n: int) -> Tensor:
-        """One request as ONE graph launch: input copies, replay, output copies."""
-        from .. import normalize
+    def _runner(self, signature: tuple, fn):
+        """The captures of one kind of request: all that ``fn`` takes from the call it was made in is in ``signature``."""
         from ...runtime.graphs import CudaGraphRunner
+        runner = self._request_runners.pop(signature, None) or CudaGraphRunner(fn)
+        while len(self._request_runners) >= self.MAX_REQUEST_KINDS:        # the one that was used longest ago goes
+            self._request_runners.pop(next(iter(self._request_runners)))
+        self._request_runners[signature] = self._graph_runner = runner
+        return runner
+
+    def _graph_inputs(self, noise, action_prefix, delay, B: int, n: int, device):
+        """``(noise, action_prefix, frozen)`` as tensors of fixed shape."""
         cfg = self.config
-        B, device = batch["state"].shape[0], batch["state"].device
         if noise is None:
             noise = self.model.sample_noise((B * n, cfg.chunk_size, cfg.max_action_dim), device)
         if action_prefix is None:
             action_prefix = self.model._const(("no_prefix", B, str(device)), lambda: torch.zeros(
                 B, cfg.chunk_size, cfg.max_action_dim, device=device))
-        frozen = self.model.frozen_mask(delay, B, device)
+        return noise.float(), action_prefix.float(), self.model.frozen_mask(delay, B, device)
+
+    def _graphed_request(self, batch, idx, sampler_idx, action_prefix, delay, noise, n: int) -> Tensor:
+        """One request as ONE graph launch: input copies, replay, output copies."""
+        from .. import normalize
+        cfg = self.config
+        B, device = batch["state"].shape[0], batch["state"].device
+        noise, action_prefix, frozen = self._graph_inputs(noise, action_prefix, delay, B, n, device)
         keys = ["state", *sorted(k for k in batch if (k in cfg.image_features or k.startswith("camera"))
                                  and isinstance(batch[k], Tensor))]
         if batch.get("img_is_pad") is not None:
@@ -1061,7 +1074,8 @@ class PI05Policy(PreTrainedPolicy):
             images, img_masks = self.prepare_images(nb)
             state = nb["state"]
             state = state[:, -1] if state.dim() == 3 else state
-            actions = self.model.sample_actions(images, img_masks, lang_tokens, lang_masks, action_prefix=action_prefix,
+            actions = self.model.sample_actions(images, img_masks, lang_tokens, lang_masks,
+                                                action_prefix=action_prefix,
                                                 noise=noise, frozen=frozen, n_candidates=n,
                                                 state=state if cfg.state_type == "continuous" else None)
             real = feat.shape[0] if feat is not None else actions.shape[-1]
@@ -1074,14 +1088,10 @@ class PI05Policy(PreTrainedPolicy):
         stats = tuple(p.data_ptr() for m in (self.normalize_inputs, self.unnormalize_outputs) for p in m.parameters())
         if self._request_stats != stats:
             self._request_runners, self._request_stats = {}, stats
-        signature = (tuple(keys), n, cfg.predict_response, cfg.response_max_length, cfg.num_steps)
-        runner = self._request_runners.pop(signature, None) or CudaGraphRunner(fn)
-        while len(self._request_runners) >= self.MAX_REQUEST_KINDS:        # the one that was used longest ago goes
-            self._request_runners.pop(next(iter(self._request_runners)))
-        self._request_runners[signature] = self._graph_runner = runner
+        runner = self._runner((tuple(keys), n, cfg.predict_response, cfg.response_max_length, cfg.num_steps), fn)
         infinite = normalize.infinite_verdict(self.normalize_inputs, self.unnormalize_outputs)
         out = runner(tuple(batch[k] for k in keys), idx, sampler_idx, batch["lang_tokens"].to(device),
-                     batch["lang_masks"].to(device).bool(), noise.float(), action_prefix.float(), frozen)
+                     batch["lang_masks"].to(device).bool(), noise, action_prefix, frozen)
         if infinite():
             self.normalize_inputs.refuse_infinite(keys, idx)
             self.unnormalize_outputs.refuse_infinite(["actions"], sampler_idx)
@@ -1091,26 +1101,21 @@ class PI05Policy(PreTrainedPolicy):
         return out[0].clone()
 
     def _graphed_sample(self, images, img_masks, lang_tokens, lang_masks, action_prefix, delay, noise, state, n):
-        from ...runtime.graphs import CudaGraphRunner
         cfg = self.config
         B = lang_tokens.shape[0]
         device = lang_tokens.device
-        if noise is None:
-            noise = self.model.sample_noise((B * n, cfg.chunk_size, cfg.max_action_dim), device)
-        if action_prefix is None:
-            action_prefix = torch.zeros(B, cfg.chunk_size, cfg.max_action_dim, device=device)
-        frozen = self.model.frozen_mask(delay, B, device).contiguous()
+        noise, action_prefix, frozen = self._graph_inputs(noise, action_prefix, delay, B, n, device)
         has_state = state is not None
-        if getattr(self, "_sampler_runner", None) is None:
-            def fn(images, img_masks, lang_tokens, lang_masks, noise, action_prefix, frozen, state):
-                return self.model.sample_actions(list(images), list(img_masks), lang_tokens, lang_masks,
-                                                 action_prefix=action_prefix, noise=noise, frozen=frozen,
-                                                 state=state if has_state else None, n_candidates=n)
-            self._sampler_runner = CudaGraphRunner(fn)
+
+        def fn(images, img_masks, lang_tokens, lang_masks, noise, action_prefix, frozen, state):
+            return self.model.sample_actions(list(images), list(img_masks), lang_tokens, lang_masks,
+                                             action_prefix=action_prefix, noise=noise, frozen=frozen,
+                                             state=state if has_state else None, n_candidates=n)
+
         st = state if has_state else torch.zeros(1, device=device)
-        out = self._sampler_runner(tuple(images), tuple(img_masks), lang_tokens, lang_masks.bool(), noise.float(),
-                                 action_prefix.float(), frozen, st)
-        return out.clone()
+        runner = self._runner(("sampler", len(images), n, has_state, cfg.num_steps), fn)
+        return runner(tuple(images), tuple(img_masks), lang_tokens, lang_masks.bool(), noise, action_prefix, frozen,
+                      st).clone()
 
     @torch.no_grad()
     def select_action(self, batch: dict[str, Any], noise: Tensor | None = None) -> Tensor:

@@ -120,3 +120,36 @@ def test_replayed_requests_of_several_kinds_keep_their_captures():
         pol.sample_actions(b, noise=torch.randn(B * n, 10, 32, device="cuda"), n_candidates=n)
         assert runners.setdefault(n, pol._graph_runner) is pol._graph_runner and pol._graph_runner.num_graphs == 1
     assert runners[1] is not runners[3]
+
+
+def _open_policy(**over):
+    """A tiny policy whose adaptive norms are open, as a trained checkpoint's are (zero at the start of training)."""
+    from opentau_b200.models.layers import AdaRMSNorm
+    pol = tiny_pi05(seed=2, **over).to("cuda").to(torch.bfloat16).eval()
+    with torch.no_grad():
+        for m in pol.modules():
+            if isinstance(m, AdaRMSNorm):
+                m.dense.weight.normal_(std=0.1)
+                m.dense.bias.normal_(std=0.3)
+    return pol
+
+
+def test_replayed_samplers_follow_candidates_and_steps():
+    """Text prompts replay the sampler alone: other candidate counts and step counts are other captures, each with the
+    eager call's actions."""
+    from opentau_b200.policies.candidates import MEDOID, configure_candidates
+    pol = _open_policy()
+    b = {k: v for k, v in tiny_batch(device="cuda").items() if not k.startswith("lang_")}
+    B = b["state"].shape[0]
+    b["prompt"] = ["pick up the cup"] * B
+    configure_candidates(pol, 3, MEDOID, device=torch.device("cuda"))
+    for n, steps in ((1, 10), (3, 10), (1, 5), (1, 10)):
+        pol.config.num_steps = steps
+        noise = torch.randn(B * n, 10, 32, device="cuda")
+        pol._use_graphs = False
+        eager = pol.sample_actions(b, noise=noise, n_candidates=n)
+        if not hasattr(pol, "_request_runners"):
+            pol.enable_cuda_graphs(True)
+        pol._use_graphs = True
+        torch.testing.assert_close(pol.sample_actions(b, noise=noise, n_candidates=n), eager, rtol=1e-3, atol=1e-3)
+    assert len(pol._request_runners) == 3
