@@ -1047,21 +1047,23 @@ class PI05Policy(PreTrainedPolicy):
         return runner
 
     def _graph_inputs(self, noise, action_prefix, delay, B: int, n: int, device):
-        """``(noise, action_prefix, frozen)`` as tensors of fixed shape."""
+        """``(noise, action_prefix, frozen, held)`` as tensors of fixed shape.  ``held``: frozen rows are held at the prefix;
+        without one they run at time 0 and stay free, unless nothing is frozen, when any prefix does."""
         cfg = self.config
         if noise is None:
             noise = self.model.sample_noise((B * n, cfg.chunk_size, cfg.max_action_dim), device)
+        held = action_prefix is not None or (isinstance(delay, int) and delay <= 0)
         if action_prefix is None:
             action_prefix = self.model._const(("no_prefix", B, str(device)), lambda: torch.zeros(
                 B, cfg.chunk_size, cfg.max_action_dim, device=device))
-        return noise.float(), action_prefix.float(), self.model.frozen_mask(delay, B, device)
+        return noise.float(), action_prefix.float(), self.model.frozen_mask(delay, B, device), held
 
     def _graphed_request(self, batch, idx, sampler_idx, action_prefix, delay, noise, n: int) -> Tensor:
         """One request as ONE graph launch: input copies, replay, output copies."""
         from .. import normalize
         cfg = self.config
         B, device = batch["state"].shape[0], batch["state"].device
-        noise, action_prefix, frozen = self._graph_inputs(noise, action_prefix, delay, B, n, device)
+        noise, action_prefix, frozen, held = self._graph_inputs(noise, action_prefix, delay, B, n, device)
         keys = ["state", *sorted(k for k in batch if (k in cfg.image_features or k.startswith("camera"))
                                  and isinstance(batch[k], Tensor))]
         if batch.get("img_is_pad") is not None:
@@ -1075,7 +1077,7 @@ class PI05Policy(PreTrainedPolicy):
             state = nb["state"]
             state = state[:, -1] if state.dim() == 3 else state
             actions = self.model.sample_actions(images, img_masks, lang_tokens, lang_masks,
-                                                action_prefix=action_prefix,
+                                                action_prefix=action_prefix if held else None,
                                                 noise=noise, frozen=frozen, n_candidates=n,
                                                 state=state if cfg.state_type == "continuous" else None)
             real = feat.shape[0] if feat is not None else actions.shape[-1]
@@ -1088,7 +1090,7 @@ class PI05Policy(PreTrainedPolicy):
         stats = tuple(p.data_ptr() for m in (self.normalize_inputs, self.unnormalize_outputs) for p in m.parameters())
         if self._request_stats != stats:
             self._request_runners, self._request_stats = {}, stats
-        runner = self._runner((tuple(keys), n, cfg.predict_response, cfg.response_max_length, cfg.num_steps), fn)
+        runner = self._runner((tuple(keys), n, held, cfg.predict_response, cfg.response_max_length, cfg.num_steps), fn)
         infinite = normalize.infinite_verdict(self.normalize_inputs, self.unnormalize_outputs)
         out = runner(tuple(batch[k] for k in keys), idx, sampler_idx, batch["lang_tokens"].to(device),
                      batch["lang_masks"].to(device).bool(), noise, action_prefix, frozen)
@@ -1104,16 +1106,16 @@ class PI05Policy(PreTrainedPolicy):
         cfg = self.config
         B = lang_tokens.shape[0]
         device = lang_tokens.device
-        noise, action_prefix, frozen = self._graph_inputs(noise, action_prefix, delay, B, n, device)
+        noise, action_prefix, frozen, held = self._graph_inputs(noise, action_prefix, delay, B, n, device)
         has_state = state is not None
 
         def fn(images, img_masks, lang_tokens, lang_masks, noise, action_prefix, frozen, state):
             return self.model.sample_actions(list(images), list(img_masks), lang_tokens, lang_masks,
-                                             action_prefix=action_prefix, noise=noise, frozen=frozen,
+                                             action_prefix=action_prefix if held else None, noise=noise, frozen=frozen,
                                              state=state if has_state else None, n_candidates=n)
 
         st = state if has_state else torch.zeros(1, device=device)
-        runner = self._runner(("sampler", len(images), n, has_state, cfg.num_steps), fn)
+        runner = self._runner(("sampler", len(images), n, held, has_state, cfg.num_steps), fn)
         return runner(tuple(images), tuple(img_masks), lang_tokens, lang_masks.bool(), noise, action_prefix, frozen,
                       st).clone()
 

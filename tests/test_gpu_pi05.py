@@ -153,3 +153,22 @@ def test_replayed_samplers_follow_candidates_and_steps():
         pol._use_graphs = True
         torch.testing.assert_close(pol.sample_actions(b, noise=noise, n_candidates=n), eager, rtol=1e-3, atol=1e-3)
     assert len(pol._request_runners) == 3
+
+
+@pytest.mark.parametrize("text", [False, True])
+@pytest.mark.parametrize("delay", [3, "per sample"])
+def test_frozen_rows_without_a_prefix_stay_free_when_replayed(text, delay):
+    """A delay without committed actions only sets the frozen rows' diffusion time; with a prefix they are held at it."""
+    pol = _open_policy()
+    b = tiny_batch(device="cuda")
+    B = b["state"].shape[0]
+    if text:
+        b = {k: v for k, v in b.items() if not k.startswith("lang_")} | {"prompt": ["pick up the cup"] * B}
+    if delay != 3:
+        delay = torch.arange(B, device="cuda") % 4
+    noise, prefix = torch.randn(B, 10, 32, device="cuda"), torch.randn(B, 10, 32, device="cuda")
+    calls = (dict(delay=delay), dict(delay=delay, action_prefix=prefix), dict())
+    eager = [pol.sample_actions(b, noise=noise, **kw) for kw in calls]
+    pol.enable_cuda_graphs(True)
+    for kw, want in zip(calls, eager):
+        torch.testing.assert_close(pol.sample_actions(b, noise=noise, **kw), want, rtol=1e-3, atol=1e-3)
