@@ -1020,10 +1020,17 @@ class PI05Policy(PreTrainedPolicy):
         self._request_runners, self._request_stats = {}, None
 
     def _ensure_eval(self) -> None:
-        """``self.eval()`` when anything the forward pass reads is in training mode (the recursion over every module
-        costs more than the host side of a replayed chunk)."""
-        if self.training or self.model.training or self.model.wrapper.training or self.model.wrapper.decoder.training:
-            self.eval()
+        """``self.eval()`` when any module is in training mode: reading the flags of 634 modules takes 0.08 ms, setting them
+        2.3 ms."""
+        todo: list = [self]
+        for m in todo:
+            if m is None:
+                continue
+            if m.training:
+                self.eval()
+                return
+            if m._modules:
+                todo.extend(m._modules.values())
 
     def _request_fits_graph(self, batch) -> bool:
         """Whether a whole request (normalisation, image preparation, sampler, un-normalisation) can be captured: the

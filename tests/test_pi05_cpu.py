@@ -280,3 +280,12 @@ def test_row_products_refuse_operands_they_would_misread():
                      ((x, w), dict(norm=cuda_ops.RowNorm(1e-6, mod=torch.zeros(3, 48))))):
         with pytest.raises((ValueError, AssertionError)):
             cuda_ops.rows_linear(*args, **kw)
+
+
+def test_sampling_puts_every_module_in_eval_mode():
+    pol = tiny_pi05(dropout=0.1).eval()
+    for part in (pol, pol.model.wrapper.paligemma.vision_tower, pol.model.wrapper.gemma_expert.model.layers[1].mlp,
+                 pol.normalize_inputs):
+        part.train()
+        pol.sample_actions(tiny_batch())
+        assert not any(m.training for m in pol.modules())
