@@ -1102,7 +1102,7 @@ class PI05Policy(PreTrainedPolicy):
         out = runner(tuple(batch[k] for k in keys), idx, sampler_idx, batch["lang_tokens"].to(device),
                      batch["lang_masks"].to(device).bool(), noise, action_prefix, frozen)
         if infinite():
-            self.normalize_inputs.refuse_infinite(keys, idx)
+            self.normalize_inputs.refuse_infinite(batch, idx)            # of every feature that came, captured or not
             self.unnormalize_outputs.refuse_infinite(["actions"], sampler_idx)
         self.model.last_response_tokens = self.model.last_response_masks = None
         if cfg.predict_response:

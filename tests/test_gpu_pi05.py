@@ -172,3 +172,20 @@ def test_frozen_rows_without_a_prefix_stay_free_when_replayed(text, delay):
     pol.enable_cuda_graphs(True)
     for kw, want in zip(calls, eager):
         torch.testing.assert_close(pol.sample_actions(b, noise=noise, **kw), want, rtol=1e-3, atol=1e-3)
+
+
+def test_replayed_requests_refuse_infinite_statistics_of_every_feature_that_comes():
+    """An input that the sampler does not read is normalised, and refused, all the same."""
+    from opentau_b200.configs.types import FeatureType, NormalizationMode, PolicyFeature
+    from opentau_b200.policies.pi05.modeling_pi05 import PI05Policy
+    cfg = tiny_pi05_config("cuda")
+    cfg.input_features["environment"] = PolicyFeature(FeatureType.ENV, (4,))
+    cfg.normalization_mapping = dict(cfg.normalization_mapping, ENV=NormalizationMode.MIN_MAX)
+    stats = dict(identity_stats(), environment={"min": torch.zeros(4), "max": torch.full((4,), float("inf"))})
+    pol = PI05Policy(cfg, per_dataset_stats=[stats]).to("cuda").to(torch.bfloat16).eval()
+    b = tiny_batch(device="cuda")
+    for graphs in (False, True):
+        pol.enable_cuda_graphs(graphs)
+        pol.sample_actions(b)
+        with pytest.raises(AssertionError, match="infinity"):
+            pol.sample_actions(dict(b, environment=torch.zeros(b["state"].shape[0], 4, device="cuda")))
