@@ -508,7 +508,7 @@ class PI05FlowMatching(nn.Module):
                               lambda: torch.zeros(B, base + L, dtype=torch.int32, device=device))
         valid_all = torch.cat([cache.valid[:, :base], torch.zeros(B, L, dtype=torch.bool, device=device)], dim=1)
         one = torch.ones(B, 1, dtype=torch.bool, device=device)
-        tokens, lives = [], []
+        tokens, lives = [first[:, :0]], [one[:, :0]]
         offset = prefix_len.clone()
         ended = None
         logits = None

@@ -73,3 +73,11 @@ def test_an_early_eos_pads_the_rest():
     # an all-zero head gives equal logits: arg-max is id 0 = pad, which ends the sample just like <eos>
     assert bool((toks[:, 0] == tok.bos_token_id).all())
     assert bool((toks[:, 2:] == tok.pad_token_id).all()) and not bool(masks[:, 2:].any())
+
+
+def test_a_response_of_no_tokens_is_an_empty_one():
+    pol = tiny_pi05(predict_response=True, response_max_length=0).eval()
+    b = tiny_batch()
+    pol.sample_actions(b)
+    assert pol.model.last_response_tokens.shape == pol.model.last_response_masks.shape == (b["state"].shape[0], 0)
+    assert pol.last_response == [""] * b["state"].shape[0]
