@@ -45,15 +45,22 @@ def _copy_into(dst: Any, src: Any) -> None:
 class CudaGraphRunner:
     """Wraps ``fn(*tensors) -> Tensor | tuple``; each new input signature is warmed up eagerly, captured,
     then replayed.  Outputs are returned as views of the graph's static output buffers: copy them if they
-    must survive the next call."""
+    must survive the next call.
 
-    def __init__(self, fn: Callable, warmup: int = 1):
-        self.fn, self.warmup = fn, warmup
+    ``defer``: the first call of a signature runs eagerly and is the warm-up; the second one captures.  For functions of
+    thousands of launches, whose capture costs as much as the call itself."""
+
+    def __init__(self, fn: Callable, warmup: int = 1, defer: bool = False):
+        self.fn, self.warmup = fn, 0 if defer else warmup
         self._graphs: dict[tuple, tuple] = {}
+        self._met = set() if defer else None         # signatures that have run eagerly
 
     def __call__(self, *args):
         key = _signature(args)
         entry = self._graphs.get(key)
+        if entry is None and self._met is not None and key not in self._met:
+            self._met.add(key)
+            return self.fn(*args)
         if entry is None:
             entry = self._capture(args)
             self._graphs[key] = entry

@@ -189,3 +189,19 @@ def test_replayed_requests_refuse_infinite_statistics_of_every_feature_that_come
         pol.sample_actions(b)
         with pytest.raises(AssertionError, match="infinity"):
             pol.sample_actions(dict(b, environment=torch.zeros(b["state"].shape[0], 4, device="cuda")))
+
+
+def test_replayed_responses_match_the_eager_ones():
+    """The first request of a kind with a response runs eagerly, the second captures, later ones replay: the same tokens and
+    actions each time, and those of a policy without graphs."""
+    pol = _open_policy(predict_response=True, response_max_length=6)
+    b = tiny_batch(device="cuda")
+    noise = torch.randn(b["state"].shape[0], 10, 32, device="cuda")
+    want = pol.sample_actions(b, noise=noise)
+    tokens, masks = pol.model.last_response_tokens, pol.model.last_response_masks
+    pol.enable_cuda_graphs(True)
+    for graphs in (0, 1, 1):
+        got = pol.sample_actions(b, noise=noise)
+        assert pol._graph_runner.num_graphs == graphs
+        assert torch.equal(pol.model.last_response_tokens, tokens) and torch.equal(pol.model.last_response_masks, masks)
+        torch.testing.assert_close(got, want, rtol=1e-3, atol=1e-3)
