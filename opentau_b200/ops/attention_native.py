@@ -170,7 +170,8 @@ def supported_f32(q: Tensor, k: Tensor, v: Tensor) -> bool:
     if not _enabled() or q.dtype != torch.float32 or not q.is_cuda:
         return False
     D, H, Hkv = q.shape[3], q.shape[2], k.shape[2]
-    return k.dtype == v.dtype == torch.float32 and D % 4 == 0 and 4 <= D <= 256 and H % Hkv == 0
+    return (k.dtype == v.dtype == torch.float32 and D % 4 == 0 and 4 <= D <= 256 and H % Hkv == 0
+            and q.shape[0] <= 65535 and H <= 65535)                    # samples and heads are grid dimensions
 
 
 #: score bytes of one 8-sample chunk of the dense evaluation above which the kernels are used whatever the head width

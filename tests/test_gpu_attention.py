@@ -406,3 +406,18 @@ def test_fp32_attention_keeps_nan_and_infinite_scores(H, Hkv, D, bad_keys):
         assert torch.equal(x.isneginf(), w.isneginf()), name
         torch.testing.assert_close(x[w.isfinite()], w[w.isfinite()], rtol=1e-4, atol=1e-4)
     assert not o_w[0, 105].any() and not lse_w[0, :, 105].any()
+
+
+def test_fp32_attention_takes_more_sequences_than_a_grid_has_rows():
+    """65 536 sequences of a few positions (temporal attention of a batch of clips) take the dense evaluation."""
+    from opentau_b200 import ops
+    B, S, H, D = 65536, 3, 1, 8
+    q, k, v = (torch.randn(B, S, H, D, device="cuda").requires_grad_() for _ in range(3))
+    blk = torch.arange(S, device="cuda").int().expand(B, -1)
+    ok = torch.ones(B, S, dtype=torch.bool, device="cuda")
+    o = ops.block_attention(q, k, v, blk, blk, ok, ok, D ** -0.5)
+    grads = torch.autograd.grad(o.square().sum(), (q, k, v))
+    a = [t.detach()[-40:].requires_grad_() for t in (q, k, v)]
+    w = ops.block_attention(*a, blk[:40], blk[:40], ok[:40], ok[:40], D ** -0.5)
+    for x, y in zip((o, *grads), (w, *torch.autograd.grad(w.square().sum(), a))):
+        torch.testing.assert_close(x[-40:], y, rtol=1e-5, atol=1e-5)
