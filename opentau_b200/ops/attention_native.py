@@ -242,7 +242,8 @@ def attn_f32_bwd(do: Tensor, q: Tensor, k: Tensor, v: Tensor, o: Tensor, lse: Te
     lse = lse.contiguous()
     lib = _lib.load("attention_f32")
     n_dq, n_dkv, n_ds = c_int(), c_int(), c_longlong()
-    lib.otb_attn_f32_bwd_plan(c_int(B), c_int(Sq), c_int(Sk), c_int(H), c_int(Hkv), byref(n_dq), byref(n_dkv), byref(n_ds))
+    lib.otb_attn_f32_bwd_plan(c_int(B), c_int(Sq), c_int(Sk), c_int(H), c_int(Hkv), c_int(D), byref(n_dq), byref(n_dkv),
+                              byref(n_ds))
     n_dq, n_dkv = n_dq.value, n_dkv.value
     ds = torch.empty(n_ds.value, dtype=torch.float32, device=q.device) if n_ds.value and keep_ds else None
     # partial sums of a split backward

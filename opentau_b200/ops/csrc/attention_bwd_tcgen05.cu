@@ -616,6 +616,7 @@ static int launch_bwd(const void* q, Strides qs, const void* k, Strides ks, cons
 }
 
 constexpr int BWD_MAX_SPLITS = 16;
+constexpr double BWD_MAX_SCRATCH = 256.0 * (1 << 20);   // bytes of one output's parts; past it a tile's share is small anyway
 
 // Into how many parts a tile's streamed blocks are dealt.  One block fills an SM, so the time is rounds x the blocks a part
 // streams, plus what every part does once (fixed tiles, first scores, epilogue: about PER_PART blocks' worth) and the
@@ -623,7 +624,7 @@ constexpr int BWD_MAX_SPLITS = 16;
 // short sequences are bound by what the host issues.  One sample of 4096 keys under one kv
 // head is 32 dK and 32 dV tiles, which left 116 of 148 SMs idle: forward + backward 2.85 ms without parts, 1.27 ms with
 // (8 heads on 1, width 256, 1024 causal positions); a pi0.5 training step at batch 8 (80 tiles) 172.5 -> 167.6 ms.
-static int pick_bwd_splits(long long tiles, int blocks, int B, double sum_cost, double extra) {
+static int pick_bwd_splits(long long tiles, int blocks, int B, double out_bytes, double sum_cost, double extra) {
   static int sms = 0;
   if (sms == 0) {
     int dev = 0;
@@ -634,7 +635,8 @@ static int pick_bwd_splits(long long tiles, int blocks, int B, double sum_cost, 
   constexpr double PER_PART = 4.0;
   int best = 1;
   double best_cost = 0;
-  for (int s = 1; s <= BWD_MAX_SPLITS && s * 4 <= (blocks > 4 ? blocks : 4) && (long long)B * s <= 65535; ++s) {
+  for (int s = 1; s <= BWD_MAX_SPLITS && s * 4 <= (blocks > 4 ? blocks : 4) && (long long)B * s <= 65535 &&
+                  (s == 1 || s * out_bytes <= BWD_MAX_SCRATCH); ++s) {
     const double cost = (double)((tiles * s + sms - 1) / sms) * ((double)((blocks + s - 1) / s) + PER_PART) +
                         (s > 1 ? sum_cost * (s + 1) + extra : 0.0);
     if (s == 1 || cost < best_cost) {
@@ -661,10 +663,12 @@ extern "C" void otb_attn_bwd_splits(int B, int Sq, int Sk, int H, int Hkv, int D
   const long long kv = (long long)Hkv * B;
   // a block of 32 x 256 takes about 1 us, a dV block of 64 x 256 0.8, others in proportion; fp32 sums move at about 4 TB/s
   const double us = 1.0 * bn * dpad / (32 * 256), us_v = 0.8 * bnv * dpad / (64 * 256);
-  const double q_sum = 4.0 * B * Sq * H * D / 4e6, k_sum = 4.0 * B * Sk * Hkv * D / 4e6;
-  *dq = pick_bwd_splits(bwd_tiles<MODE_DQ>(Sq, Sk, g) * kv, (Sk + bn - 1) / bn, B, q_sum / us, 15.0 / us);
-  *dk = pick_bwd_splits(bwd_tiles<MODE_DK>(Sq, Sk, g) * kv, (int)(((long long)Sq * g + bn - 1) / bn), B, k_sum / us, 15.0 / us);
-  *dv = pick_bwd_splits(bwd_tiles<MODE_DV>(Sq, Sk, g) * kv, (int)(((long long)Sq * g + bnv - 1) / bnv), B, k_sum / us_v, 15.0 / us_v);
+  const double q_out = 4.0 * B * Sq * H * D, k_out = 4.0 * B * Sk * Hkv * D, q_sum = q_out / 4e6, k_sum = k_out / 4e6;
+  *dq = pick_bwd_splits(bwd_tiles<MODE_DQ>(Sq, Sk, g) * kv, (Sk + bn - 1) / bn, B, q_out, q_sum / us, 15.0 / us);
+  *dk = pick_bwd_splits(bwd_tiles<MODE_DK>(Sq, Sk, g) * kv, (int)(((long long)Sq * g + bn - 1) / bn), B, k_out, k_sum / us,
+                        15.0 / us);
+  *dv = pick_bwd_splits(bwd_tiles<MODE_DV>(Sq, Sk, g) * kv, (int)(((long long)Sq * g + bnv - 1) / bnv), B, k_out, k_sum / us_v,
+                        15.0 / us_v);
 }
 
 // q (B,Sq,H,D), k/v (B,Sk,Hkv,D) with element strides; o, do: (B,Sq,H,D) contiguous; lse (B,H,Sq);

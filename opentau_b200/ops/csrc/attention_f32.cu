@@ -46,6 +46,7 @@ constexpr int F32_STR = 64;       // streamed rows per tile
 constexpr int F32_THREADS = 256;
 constexpr int F32_PLD = F32_STR + 4;
 constexpr int F32_MAX_SPLITS = 8;
+constexpr long long F32_MAX_SCRATCH = 256ll << 20;      // bytes of dS, and of one output's parts
 
 struct F32Params {
   const float* q;
@@ -715,7 +716,7 @@ static int set_smem(K kern, size_t bytes) {
 
 // Into how many parts the streamed tiles are dealt: the fewest rounds of one block per SM for the work there is, and a
 // hundredth of it charged per part (its partial sums are written and read once more).
-static int pick_splits(long long blocks, long long steps, int B) {
+static int pick_splits(long long blocks, long long steps, int B, long long out_bytes) {
   static int sms = 0;
   if (sms == 0) {
     int dev = 0;
@@ -725,7 +726,8 @@ static int pick_splits(long long blocks, long long steps, int B) {
   }
   int best = 1;
   double best_cost = 0;
-  for (int s = 1; s <= F32_MAX_SPLITS && s <= steps && (long long)B * s <= 65535; ++s) {
+  for (int s = 1; s <= F32_MAX_SPLITS && s <= steps && (long long)B * s <= 65535 && (s == 1 || s * out_bytes <= F32_MAX_SCRATCH);
+       ++s) {
     const long long per = (steps + s - 1) / s;
     const double cost = (double)((blocks * s + sms - 1) / sms) * per * (1.0 + 0.01 * (s - 1));
     if (s == 1 || cost < best_cost) {
@@ -776,12 +778,13 @@ extern "C" int otb_attn_f32_fwd(const float* q, const float* k, const float* v, 
 
 // Scratch of the backward: `dq` and `dkv` above 1 want that many outputs each (the parts that the streamed tiles are dealt
 // to); `ds` floats for dS, 0 where it would pass 256 MB and is recomputed instead.
-extern "C" void otb_attn_f32_bwd_plan(int B, int Sq, int Sk, int H, int Hkv, int* dq, int* dkv, long long* ds) {
+extern "C" void otb_attn_f32_bwd_plan(int B, int Sq, int Sk, int H, int Hkv, int D, int* dq, int* dkv, long long* ds) {
   const long long qt = (Sq + F32_STR - 1) / F32_STR, kt = (Sk + F32_STR - 1) / F32_STR;
-  *dq = pick_splits((long long)((Sq + F32_OWN - 1) / F32_OWN) * H * B, kt, B);
-  *dkv = pick_splits((long long)((Sk + F32_OWN - 1) / F32_OWN) * Hkv * B, qt * (H / Hkv), B);
+  *dq = pick_splits((long long)((Sq + F32_OWN - 1) / F32_OWN) * H * B, kt, B, 4ll * B * Sq * H * D);
+  *dkv = pick_splits((long long)((Sk + F32_OWN - 1) / F32_OWN) * Hkv * B, qt * (H / Hkv), B,
+                     4ll * B * Sk * Hkv * D);
   const long long n = (long long)B * H * Sk * qt * F32_STR;
-  *ds = n <= (64ll << 20) ? n : 0;
+  *ds = n * 4 <= F32_MAX_SCRATCH ? n : 0;
 }
 
 // o, d_o (B,Sq,H,D) contiguous; delta: scratch (B,H,Sq); dq (B,Sq,H,D), dk / dv (B,Sk,Hkv,D) contiguous outputs; dq_parts:

@@ -421,3 +421,21 @@ def test_fp32_attention_takes_more_sequences_than_a_grid_has_rows():
     w = ops.block_attention(*a, blk[:40], blk[:40], ok[:40], ok[:40], D ** -0.5)
     for x, y in zip((o, *grads), (w, *torch.autograd.grad(w.square().sum(), a))):
         torch.testing.assert_close(x[-40:], y, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("H,Hkv,D", [(8, 1, 256), (8, 4, 256), (16, 16, 72), (32, 1, 128)])
+@pytest.mark.parametrize("B,S", [(1, 400), (1, 4096), (8, 1300), (1, 131072), (8, 65536)])
+def test_split_backward_scratch_is_bounded(H, Hkv, D, B, S):
+    """The parts of one output never pass 256 MB, in bf16's backward as in fp32's (sizes only: nothing is allocated)."""
+    from ctypes import byref, c_int, c_longlong
+    from opentau_b200.ops import _lib, attention_native
+    outs = [4 * B * S * H * D] + [4 * B * S * Hkv * D] * 2
+    parts = [attention_native.bwd_splits(B, S, S, H, Hkv, D)]
+    dq, dkv, ds = c_int(), c_int(), c_longlong()
+    _lib.load("attention_f32").otb_attn_f32_bwd_plan(B, S, S, H, Hkv, D, byref(dq), byref(dkv), byref(ds))
+    parts.append((dq.value, dkv.value, dkv.value))
+    for m in parts:
+        assert all(n >= 1 and (n == 1 or n * out <= 1 << 28) for n, out in zip(m, outs)), m
+    assert 4 * ds.value <= 1 << 28
+    if (B, S, H, Hkv) == (1, 4096, 8, 1):
+        assert min(parts[0][1:]) > 4                        # where they pay they are kept
