@@ -632,7 +632,7 @@ static int pick_bwd_splits(long long tiles, int blocks, int B, double out_bytes,
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (sms <= 0) return 1;
   }
-  constexpr double PER_PART = 4.0;
+  constexpr double PER_PART = 4.0, MUST_WIN = 0.95;
   int best = 1;
   double best_cost = 0;
   for (int s = 1; s <= BWD_MAX_SPLITS && s * 4 <= (blocks > 4 ? blocks : 4) && (long long)B * s <= 65535 &&
@@ -641,7 +641,7 @@ static int pick_bwd_splits(long long tiles, int blocks, int B, double out_bytes,
                         (s > 1 ? sum_cost * (s + 1) + extra : 0.0);
     if (s == 1 || cost < best_cost) {
       best = s;
-      best_cost = cost;
+      best_cost = s == 1 ? MUST_WIN * cost : cost;
     }
   }
   return best;
