@@ -59,8 +59,9 @@ class CudaGraphRunner:
         key = _signature(args)
         entry = self._graphs.get(key)
         if entry is None and self._met is not None and key not in self._met:
+            out = self.fn(*args)
             self._met.add(key)
-            return self.fn(*args)
+            return out
         if entry is None:
             entry = self._capture(args)
             self._graphs[key] = entry

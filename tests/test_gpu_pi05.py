@@ -129,8 +129,10 @@ def _open_policy(**over):
     with torch.no_grad():
         for m in pol.modules():
             if isinstance(m, AdaRMSNorm):
-                m.dense.weight.normal_(std=0.1)
+                m.dense.weight.normal_(std=0.05)
                 m.dense.bias.normal_(std=0.3)
+        pol.model.time_mlp_in.weight.normal_(std=0.15)
+        pol.model.time_mlp_out.weight.normal_(std=0.15)
     return pol
 
 
@@ -205,3 +207,42 @@ def test_replayed_responses_match_the_eager_ones():
         assert pol._graph_runner.num_graphs == graphs
         assert torch.equal(pol.model.last_response_tokens, tokens) and torch.equal(pol.model.last_response_masks, masks)
         torch.testing.assert_close(got, want, rtol=1e-3, atol=1e-3)
+
+
+@pytest.mark.parametrize("B", [4, 12, 30])                 # 40, 120 and 300 rows: each way the row products take
+@pytest.mark.parametrize("delay", [0, 3, "per sample"])
+@pytest.mark.parametrize("prefix", [False, True])
+def test_planned_loop_matches_the_step_by_step_one(B, delay, prefix, monkeypatch):
+    """Conditions of all steps computed at once and picked per token (frozen ones at time 0) give the velocities of the
+    loop that computes them step by step.  Both round to bf16 (2^-8 at most, in their own order) what a step adds to the sample;
+    other frozen rows move the result by a third."""
+    pol = _open_policy()
+    b = tiny_batch(device="cuda", batch_size=B)
+    if delay == "per sample":
+        delay = torch.arange(B, device="cuda") % 6
+    kw = dict(noise=torch.randn(B, 10, 32, device="cuda"), delay=delay)
+    if prefix:
+        kw["action_prefix"] = torch.randn(B, 10, 32, device="cuda")
+    got = pol.sample_actions(b, **kw)
+    calls = []
+    monkeypatch.setattr(pol.model, "_can_plan_loop", lambda *a: calls.append(a))
+    want = pol.sample_actions(b, **kw)
+    assert calls
+    move = want - kw["noise"]
+    assert (got - want).norm() < 2 ** -8 * move.norm()
+    if not (prefix and delay == 0):
+        other = pol.sample_actions(b, **dict(kw, delay=6))
+        assert (other - want).norm() > 2 ** -3 * move.norm()    # frozen rows are seen by the others
+
+def test_replayed_candidates_are_the_eager_ones():
+    from opentau_b200.policies.candidates import MEDOID, configure_candidates
+    pol = _open_policy()
+    b = tiny_batch(device="cuda")
+    B = b["state"].shape[0]
+    configure_candidates(pol, 3, MEDOID, device=torch.device("cuda"))
+    for n in (3, 7):
+        noise = torch.randn(B * n, 10, 32, device="cuda")
+        pol.enable_cuda_graphs(False)
+        want = pol.sample_actions(b, noise=noise, n_candidates=n)
+        pol.enable_cuda_graphs(True)
+        torch.testing.assert_close(pol.sample_actions(b, noise=noise, n_candidates=n), want, rtol=1e-3, atol=1e-3)
