@@ -180,6 +180,8 @@ def supported_f32(q: Tensor, k: Tensor, v: Tensor) -> bool:
             and q.shape[0] <= 65535 and H <= 65535)                    # samples and heads are grid dimensions
 
 
+#: bytes of dS that the backward keeps (``F32_MAX_DS`` of ``csrc/attention_f32.cu``)
+F32_DS_LIMIT = 2 << 30
 #: score bytes of one 8-sample chunk of the dense evaluation above which the kernels are used whatever the head width
 F32_DENSE_SCORE_LIMIT = 5 << 18
 

@@ -46,7 +46,10 @@ constexpr int F32_STR = 64;       // streamed rows per tile
 constexpr int F32_THREADS = 256;
 constexpr int F32_PLD = F32_STR + 4;
 constexpr int F32_MAX_SPLITS = 8;
-constexpr long long F32_MAX_SCRATCH = 256ll << 20;      // bytes of dS, and of one output's parts
+constexpr long long F32_MAX_SCRATCH = 256ll << 20;      // bytes of one output's parts
+// Bytes of dS.  The dense evaluation holds five tensors of that size; without it the backward computes seven products
+// instead of five (8 x 1227 positions, 8 heads on 1 of 256, nothing hidden: 11.9 ms; 16 x 601, 16 heads of 72: 6.1).
+constexpr long long F32_MAX_DS = 2ll << 30;
 
 struct F32Params {
   const float* q;
@@ -777,14 +780,14 @@ extern "C" int otb_attn_f32_fwd(const float* q, const float* k, const float* v, 
 }
 
 // Scratch of the backward: `dq` and `dkv` above 1 want that many outputs each (the parts that the streamed tiles are dealt
-// to); `ds` floats for dS, 0 where it would pass 256 MB and is recomputed instead.
+// to); `ds` floats for dS, 0 where it would pass F32_MAX_DS and is recomputed instead.
 extern "C" void otb_attn_f32_bwd_plan(int B, int Sq, int Sk, int H, int Hkv, int D, int* dq, int* dkv, long long* ds) {
   const long long qt = (Sq + F32_STR - 1) / F32_STR, kt = (Sk + F32_STR - 1) / F32_STR;
   *dq = pick_splits((long long)((Sq + F32_OWN - 1) / F32_OWN) * H * B, kt, B, 4ll * B * Sq * H * D);
   *dkv = pick_splits((long long)((Sk + F32_OWN - 1) / F32_OWN) * Hkv * B, qt * (H / Hkv), B,
                      4ll * B * Sk * Hkv * D);
   const long long n = (long long)B * H * Sk * qt * F32_STR;
-  *ds = n * 4 <= F32_MAX_SCRATCH ? n : 0;
+  *ds = n * 4 <= F32_MAX_DS ? n : 0;
 }
 
 // o, d_o (B,Sq,H,D) contiguous; delta: scratch (B,H,Sq); dq (B,Sq,H,D), dk / dv (B,Sk,Hkv,D) contiguous outputs; dq_parts:

@@ -436,6 +436,6 @@ def test_split_backward_scratch_is_bounded(H, Hkv, D, B, S):
     parts.append((dq.value, dkv.value, dkv.value))
     for m in parts:
         assert all(n >= 1 and (n == 1 or n * out <= 1 << 28) for n, out in zip(m, outs)), m
-    assert 4 * ds.value <= 1 << 28
+    assert 4 * ds.value <= attention_native.F32_DS_LIMIT
     if (B, S, H, Hkv) == (1, 4096, 8, 1):
         assert min(parts[0][1:]) > 4                        # where they pay they are kept
