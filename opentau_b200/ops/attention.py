@@ -78,6 +78,6 @@ def attn_bwd(do, q, k, v, o, lse, q_blk, k_blk, q_valid, k_valid, scale):
     from . import attention_native
     if attention_native.supported_bwd(q, k, v):
         return attention_native.attn_bwd(do, q, k, v, o, lse, q_blk, k_blk, q_valid, k_valid, scale)
-    if attention_native.supported_f32(q, k, v) and attention_native.prefer_f32_kernels(q, k):
+    if attention_native.supported_f32(q, k, v) and attention_native.prefer_f32_kernels(q, k, True):
         return attention_native.attn_f32_bwd(do, q, k, v, o, lse, q_blk, k_blk, q_valid, k_valid, scale)
     return dense_attn_bwd(do, q, k, v, o, lse, q_blk, k_blk, q_valid, k_valid, scale)

@@ -180,26 +180,48 @@ def supported_f32(q: Tensor, k: Tensor, v: Tensor) -> bool:
             and q.shape[0] <= 65535 and H <= 65535)                    # samples and heads are grid dimensions
 
 
+#: score bytes of one 8-sample chunk up to which head widths above 128 stay on the dense evaluation
+F32_DENSE_SCORE_LIMIT = 5 << 18
+#: score bytes of a call above which the dense evaluation, which holds several such tensors, is not considered
+F32_DENSE_MEMORY_LIMIT = 8 << 30
 #: bytes of dS that the backward keeps (``F32_MAX_DS`` of ``csrc/attention_f32.cu``)
 F32_DS_LIMIT = 2 << 30
-#: score bytes of one 8-sample chunk of the dense evaluation above which the kernels are used whatever the head width
-F32_DENSE_SCORE_LIMIT = 5 << 18
 
 
-def prefer_f32_kernels(q: Tensor, k: Tensor) -> bool:
-    """Which fp32 path the dispatcher takes when both can run (``OPENTAU_B200_F32_ATTN=kernel|dense`` forces one).
-    Measured on a B200, forward + backward, kernels against the dense evaluation on the library's fp32 GEMMs: 800 us
-    against 1043 (2 x 601 positions, 8 heads on 1, width 256), 1067 against 1203 (2 x 700, 8 on 4, 256), 252 against 759
-    (2 x 300, 16 heads of 72), at half its error against 64 bits.  So: the kernels, except at head widths above 128 with
-    fewer score bytes than :data:`F32_DENSE_SCORE_LIMIT` (about 200 positions of 8 heads), where the dense evaluation is
-    what callers have always had and the tests hold it there; it is launch-bound and slower at that size too (734 us
-    against 108 for 100 positions)."""
+@lru_cache(maxsize=1024)
+def _f32_kernels_pay(B: int, Sq: int, Sk: int, H: int, D: int, backward: bool) -> bool:
+    """Whether the fp32 kernels are about as fast as the dense evaluation (or faster), from sizes alone and for masks that
+    hide nothing (the kernels skip hidden tiles).  Microseconds, fitted to a B200 at head widths 64 - 256, 1 - 4096 samples
+    and 1 - 1227 positions: a forward block takes ``5 + D / 34`` for 32 queries x 64 keys; the backward a constant per
+    million of the pairs it computes, 32 keys x 64 queries at a time; the dense evaluation its launches, then a constant per
+    million pairs.  Padding decides: with 4 queries of 4096 samples against themselves (16 heads of 72) the kernels take
+    2779 forward and 6484 backward, dense 974 and 2531; with 64 queries of 64 samples 111 and 280 against 317 and 643."""
+    tiles = lambda n, of: -(-n // of)  # noqa: E731
+    pairs = B * H * Sq * Sk / 1e6
+    if not backward:
+        kernels = tiles(B * H * tiles(Sq, 32), NUM_SMS) * tiles(Sk, 64) * (5 + D / 34)
+        return kernels <= 1.15 * max(265, 100 + (28 + 0.06 * D) * pairs)
+    padded = B * H * tiles(Sk, 32) * 32 * tiles(Sq, 64) * 64 / 1e6
+    kernels = padded * (42 + 0.06 * D if D <= 128 else 56 + 0.133 * D)
+    if B * H * Sk * tiles(Sq, 64) * 64 * 4 > F32_DS_LIMIT:
+        kernels *= 1.4                                          # dS is recomputed for dQ
+    return kernels <= max(600, 1.2 * (130 + (35 + 0.17 * D) * pairs))
+
+
+def prefer_f32_kernels(q: Tensor, k: Tensor, backward: bool = False) -> bool:
+    """Which fp32 path the dispatcher takes when both can run (``OPENTAU_B200_F32_ATTN=kernel|dense`` forces one): the
+    kernels, at half the dense evaluation's error against 64 bits and without its score tensors, unless they would be
+    clearly slower (:func:`_f32_kernels_pay`).  Head widths above 128 with fewer score bytes than
+    :data:`F32_DENSE_SCORE_LIMIT` (about 200 positions of 8 heads) stay dense, as tests hold it; that is launch-bound and
+    slower (734 us against 108, forward + backward, for 100 positions of 8 heads on 1 of 256)."""
     mode = os.environ.get("OPENTAU_B200_F32_ATTN", "auto")
     if mode in ("kernel", "dense"):
         return mode == "kernel"
     B, Sq, H, D = q.shape
-    scores = min(B, 8) * H * Sq * k.shape[1] * 4
-    return D <= 128 or scores > F32_DENSE_SCORE_LIMIT
+    Sk = k.shape[1]
+    if D > 128 and min(B, 8) * H * Sq * Sk * 4 <= F32_DENSE_SCORE_LIMIT:
+        return False
+    return B * H * Sq * Sk * 4 > F32_DENSE_MEMORY_LIMIT or _f32_kernels_pay(B, Sq, Sk, H, D, backward)
 
 
 def _prep_f32(t: Tensor) -> Tensor:

@@ -262,7 +262,7 @@ def rope_fwd(x: Tensor, cos: Tensor, sin: Tensor, inverse: bool = False) -> Tens
 
 
 # ----------------------------------------------------------------------------- attention
-def _f32_kernels(q, k, v, q_blk, k_blk, q_valid, k_valid) -> bool:
+def _f32_kernels(q, k, v, q_blk, k_blk, q_valid, k_valid, backward=False) -> bool:
     """Whether fp32 attention runs on its own kernels: what they cover, with masks of exactly the sequences' shapes (the
     dense statement below also broadcasts and takes empty ones)."""
     if not q.is_cuda or q.dtype != torch.float32 or oracle_mode() or not (q.numel() and k.numel()):
@@ -271,7 +271,7 @@ def _f32_kernels(q, k, v, q_blk, k_blk, q_valid, k_valid) -> bool:
     sq, sk = tuple(q.shape[:2]), tuple(k.shape[:2])
     return (tuple(q_blk.shape) == tuple(q_valid.shape) == sq and tuple(k_blk.shape) == tuple(k_valid.shape) == sk
             and sq[0] == sk[0] and v.shape == k.shape and q.shape[3] == k.shape[3]
-            and attention_native.supported_f32(q, k, v) and attention_native.prefer_f32_kernels(q, k))
+            and attention_native.supported_f32(q, k, v) and attention_native.prefer_f32_kernels(q, k, backward))
 
 
 def attn_fwd(q, k, v, q_blk, k_blk, q_valid, k_valid, scale) -> tuple[Tensor, Tensor]:
@@ -296,7 +296,7 @@ def attn_fwd(q, k, v, q_blk, k_blk, q_valid, k_valid, scale) -> tuple[Tensor, Te
 
 def attn_bwd(do, q, k, v, o, lse, q_blk, k_blk, q_valid, k_valid, scale):
     """Returns ``(dq, dk, dv)`` shaped like q, k, v (dk/dv summed over the GQA group)."""
-    if _cuda(q) or _f32_kernels(q, k, v, q_blk, k_blk, q_valid, k_valid):
+    if _cuda(q) or _f32_kernels(q, k, v, q_blk, k_blk, q_valid, k_valid, True):
         from . import cuda_ops
         return cuda_ops.attn_bwd(do, q, k, v, o, lse, q_blk, k_blk, q_valid, k_valid, scale)
     B, Sq, H, D = q.shape

@@ -439,3 +439,30 @@ def test_split_backward_scratch_is_bounded(H, Hkv, D, B, S):
     assert 4 * ds.value <= attention_native.F32_DS_LIMIT
     if (B, S, H, Hkv) == (1, 4096, 8, 1):
         assert min(parts[0][1:]) > 4                        # where they pay they are kept
+
+
+@pytest.mark.parametrize("forward", [True, False])
+@pytest.mark.parametrize("backward", [True, False])
+def test_fp32_attention_may_take_either_path_in_each_direction(forward, backward, monkeypatch):
+    """Kernels and dense evaluation hand each other O and LSE: every combination gives the 64-bit gradients to fp32
+    rounding (256 * 2^-24 of the norm: inner products of at most 256 terms)."""
+    from opentau_b200 import ops
+    from opentau_b200.ops import attention_native, cuda_ops
+    monkeypatch.setattr(attention_native, "_f32_kernels_pay", lambda *a: backward if a[-1] else forward)
+    B, S, H, Hkv, D = 2, 75, 6, 2, 72
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v, do = (torch.randn(B, S, h, D, device="cuda", generator=g) for h in (H, Hkv, Hkv, H))
+    blk = (torch.arange(S, device="cuda") // 9).int().expand(B, -1).contiguous()
+    ok = torch.rand(B, S, device="cuda", generator=g) > 0.15
+    ok[:, 0] = True
+    do = (do * ok[:, :, None, None]).reshape(B, S, -1)
+    want = _fp64(q, k, v, do, blk, blk, ok, ok, D ** -0.5)
+    a = [t.requires_grad_() for t in (q, k, v)]
+    before = cuda_ops.launch_count
+    o = ops.block_attention(*a, blk, blk, ok, ok, D ** -0.5)
+    assert (cuda_ops.launch_count > before) == forward
+    before = cuda_ops.launch_count
+    grads = torch.autograd.grad(o, a, do)
+    assert (cuda_ops.launch_count > before) == backward
+    for x, w in zip((o.detach(), *grads), want):
+        assert _rel(x, w) < 256 * 2 ** -24

@@ -258,3 +258,16 @@ def test_gated_few_row_products_keep_the_gate_in_their_epilogue(rows, cols):
     from opentau_b200.ops import cuda_ops
     assert cuda_ops.use_skinny("nt", rows, cols, False, 0, 2048, True)
     assert cuda_ops.use_skinny("nt", rows, cols, False, 0)               # what ``gemm(gate=...)`` accepts
+
+
+def test_fp32_attention_rule_follows_the_padding():
+    """Sizes measured on both sides: few positions of many sequences leave the kernels' tiles empty and are clearly faster
+    dense; full tiles, and calls that the dense evaluation cannot even launch in the time, are the kernels'."""
+    from opentau_b200.ops.attention_native import _f32_kernels_pay as pay
+    for size in ((4096, 4, 4, 16, 72), (16384, 16, 16, 8, 64), (64, 1, 1000, 32, 128), (512, 8, 1000, 8, 256), (1, 1, 4000, 32, 128)):
+        assert not pay(*size, False), size
+    for size in ((4096, 4, 4, 16, 72), (64, 1, 300, 16, 72), (512, 1, 300, 8, 64), (512, 8, 1000, 8, 256)):
+        assert not pay(*size, True), size
+    for size in ((2, 601, 601, 8, 256), (2, 700, 700, 8, 256), (1, 100, 100, 16, 72), (64, 64, 64, 16, 72), (256, 300, 300, 8, 64),
+                 (1, 50, 1000, 8, 256), (8, 1, 1000, 16, 72), (16, 601, 601, 16, 72), (4, 1227, 1227, 32, 128)):
+        assert pay(*size, False) and pay(*size, True), size
