@@ -621,8 +621,8 @@ constexpr double BWD_MAX_SCRATCH = 256.0 * (1 << 20);   // bytes of one output's
 // Into how many parts a tile's streamed blocks are dealt.  One block fills an SM, so the time is rounds x the blocks a part
 // streams, plus what every part does once (fixed tiles, first scores, epilogue: about PER_PART blocks' worth) and the
 // sums that are written and read in fp32 (charged to the parts of the whole launch) by one more launch, `extra` blocks' worth:
-// short sequences are bound by what the host issues.  One sample of 4096 keys under one kv
-// head is 32 dK and 32 dV tiles, which left 116 of 148 SMs idle: forward + backward 2.85 ms without parts, 1.27 ms with
+// short sequences are bound by what the host issues, so parts must win a twentieth as well.  One sample of 4096 keys under one
+// kv head is 32 dK and 32 dV tiles, which left 116 of 148 SMs idle: forward + backward 2.85 ms without parts, 1.15 ms with
 // (8 heads on 1, width 256, 1024 causal positions); a pi0.5 training step at batch 8 (80 tiles) 172.5 -> 167.6 ms.
 static int pick_bwd_splits(long long tiles, int blocks, int B, double out_bytes, double sum_cost, double extra) {
   static int sms = 0;

@@ -48,7 +48,8 @@ constexpr int F32_PLD = F32_STR + 4;
 constexpr int F32_MAX_SPLITS = 8;
 constexpr long long F32_MAX_SCRATCH = 256ll << 20;      // bytes of one output's parts
 // Bytes of dS.  The dense evaluation holds five tensors of that size; without it the backward computes seven products
-// instead of five (8 x 1227 positions, 8 heads on 1 of 256, nothing hidden: 11.9 ms; 16 x 601, 16 heads of 72: 6.1).
+// instead of five (forward + backward with nothing hidden: 8 x 1227 positions, 8 heads on 1 of 256, 15.9 ms against 12.5;
+// 16 x 601, 16 heads of 72, 8.1 against 6.2).
 constexpr long long F32_MAX_DS = 2ll << 30;
 
 struct F32Params {

@@ -527,49 +527,49 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
           p.lse[((long long)b * p.H + rhead) * p.Sq + rpos] = sum > 0.f ? (M + log2f(sum)) * 0.6931471805599453f : 0.f;
       }
     } else {
-    const float inv_l = l > 0.f ? 1.f / l : 0.f;
-    __nv_bfloat16* orow = p.o + (((long long)b * p.Sq + pos) * p.H + head) * p.D;
-    float* prow_o = p.nsplit > 1
-                        ? p.part_o + ((((long long)split * p.B + b) * p.Sq + pos) * p.H + head) * (long long)p.D
-                        : nullptr;
+      const float inv_l = l > 0.f ? 1.f / l : 0.f;
+      __nv_bfloat16* orow = p.o + (((long long)b * p.Sq + pos) * p.H + head) * p.D;
+      float* prow_o = p.nsplit > 1
+                          ? p.part_o + ((((long long)split * p.B + b) * p.Sq + pos) * p.H + head) * (long long)p.D
+                          : nullptr;
 #pragma unroll 1
-    for (int c = o_lo; c < o_hi; ++c) {
-      uint32_t ro[16];
-      __syncwarp();
-      tmem_ld_x16(o_addr + c * 16, ro);
-      tmem_wait_ld();
-      if (row_in && prow_o != nullptr) {
+      for (int c = o_lo; c < o_hi; ++c) {
+        uint32_t ro[16];
+        __syncwarp();
+        tmem_ld_x16(o_addr + c * 16, ro);
+        tmem_wait_ld();
+        if (row_in && prow_o != nullptr) {
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          const int col = c * 16 + q4 * 4;
-          if (col < p.D)
-            *reinterpret_cast<float4*>(prow_o + col) =
-                make_float4(__uint_as_float(ro[q4 * 4 + 0]), __uint_as_float(ro[q4 * 4 + 1]),
-                            __uint_as_float(ro[q4 * 4 + 2]), __uint_as_float(ro[q4 * 4 + 3]));
-        }
-      } else if (row_in) {
+          for (int q4 = 0; q4 < 4; ++q4) {
+            const int col = c * 16 + q4 * 4;
+            if (col < p.D)
+              *reinterpret_cast<float4*>(prow_o + col) =
+                  make_float4(__uint_as_float(ro[q4 * 4 + 0]), __uint_as_float(ro[q4 * 4 + 1]),
+                              __uint_as_float(ro[q4 * 4 + 2]), __uint_as_float(ro[q4 * 4 + 3]));
+          }
+        } else if (row_in) {
 #pragma unroll
-        for (int h8 = 0; h8 < 2; ++h8) {
-          const int col = c * 16 + h8 * 8;
-          if (col < p.D) {
-            uint4 o;
-            o.x = pack_bf16(__uint_as_float(ro[h8 * 8 + 0]) * inv_l, __uint_as_float(ro[h8 * 8 + 1]) * inv_l);
-            o.y = pack_bf16(__uint_as_float(ro[h8 * 8 + 2]) * inv_l, __uint_as_float(ro[h8 * 8 + 3]) * inv_l);
-            o.z = pack_bf16(__uint_as_float(ro[h8 * 8 + 4]) * inv_l, __uint_as_float(ro[h8 * 8 + 5]) * inv_l);
-            o.w = pack_bf16(__uint_as_float(ro[h8 * 8 + 6]) * inv_l, __uint_as_float(ro[h8 * 8 + 7]) * inv_l);
-            *reinterpret_cast<uint4*>(orow + col) = o;
+          for (int h8 = 0; h8 < 2; ++h8) {
+            const int col = c * 16 + h8 * 8;
+            if (col < p.D) {
+              uint4 o;
+              o.x = pack_bf16(__uint_as_float(ro[h8 * 8 + 0]) * inv_l, __uint_as_float(ro[h8 * 8 + 1]) * inv_l);
+              o.y = pack_bf16(__uint_as_float(ro[h8 * 8 + 2]) * inv_l, __uint_as_float(ro[h8 * 8 + 3]) * inv_l);
+              o.z = pack_bf16(__uint_as_float(ro[h8 * 8 + 4]) * inv_l, __uint_as_float(ro[h8 * 8 + 5]) * inv_l);
+              o.w = pack_bf16(__uint_as_float(ro[h8 * 8 + 6]) * inv_l, __uint_as_float(ro[h8 * 8 + 7]) * inv_l);
+              *reinterpret_cast<uint4*>(orow + col) = o;
+            }
           }
         }
       }
-    }
-    if (row_in && half == 0) {
-      if (p.nsplit > 1) {
-        p.part_ml[(((long long)split * p.B + b) * p.H + head) * p.Sq + pos] = make_float2(m_used, l);
-      } else {
-        const float lse = l > 0.f ? (m_used + log2f(l)) * 0.6931471805599453f : 0.f;
-        p.lse[((long long)b * p.H + head) * p.Sq + pos] = lse;
+      if (row_in && half == 0) {
+        if (p.nsplit > 1) {
+          p.part_ml[(((long long)split * p.B + b) * p.H + head) * p.Sq + pos] = make_float2(m_used, l);
+        } else {
+          const float lse = l > 0.f ? (m_used + log2f(l)) * 0.6931471805599453f : 0.f;
+          p.lse[((long long)b * p.H + head) * p.Sq + pos] = lse;
+        }
       }
-    }
     }
     tc_fence_before();
   }
