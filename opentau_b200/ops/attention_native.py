@@ -191,23 +191,27 @@ F32_DS_LIMIT = 2 << 30
 
 
 @lru_cache(maxsize=1024)
-def _f32_kernels_pay(B: int, Sq: int, Sk: int, H: int, D: int, backward: bool) -> bool:
+def _f32_kernels_pay(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int, backward: bool) -> bool:
     """Whether the fp32 kernels are about as fast as the dense evaluation (or faster), from sizes alone and for masks that
-    hide nothing (the kernels skip hidden tiles).  Microseconds, fitted to a B200 at head widths 64 - 256, 1 - 4096 samples
-    and 1 - 1227 positions: a forward block takes ``5 + D / 34`` for 32 queries x 64 keys; the backward a constant per
-    million of the pairs it computes, 32 keys x 64 queries at a time; the dense evaluation its launches, then a constant per
-    million pairs.  Padding decides: with 4 queries of 4096 samples against themselves (16 heads of 72) the kernels take
-    2779 forward and 6484 backward, dense 974 and 2531; with 64 queries of 64 samples 111 and 280 against 317 and 643."""
+    hide nothing (the kernels skip hidden tiles).  Microseconds, fitted to 460 sizes on a B200 (head widths 64 - 256, 1 -
+    16384 samples, 1 - 4000 positions): rounds of blocks of 32 queries x 64 keys, in the backward the pairs of 32 keys x 64
+    queries that are computed; for the dense evaluation its launches, its passes over pairs and operands and its batched
+    products.  Padding decides: 4 queries of 4096 samples against themselves (16 heads of 72) take the kernels 2779
+    forward and 6484 backward, dense 974 and 2531; 64 of 64 samples 111 and 280 against 317 and 643.  The backward
+    is charged a quarter less than it takes on such masks (the kernels' forward wins that back, and what a mask hides they
+    skip): by this rule no measured size takes more than 1.2 times the faster path forward, 1.25 forward and
+    backward (1.35 at head width 160)."""
     tiles = lambda n, of: -(-n // of)  # noqa: E731
-    pairs = B * H * Sq * Sk / 1e6
+    pairs, elements = B * H * Sq * Sk / 1e6, B * D * (Sq * H + Sk * Hkv) / 1e6
     if not backward:
-        kernels = tiles(B * H * tiles(Sq, 32), NUM_SMS) * tiles(Sk, 64) * (5 + D / 34)
-        return kernels <= 1.15 * max(265, 100 + (28 + 0.06 * D) * pairs)
-    padded = B * H * tiles(Sk, 32) * 32 * tiles(Sq, 64) * 64 / 1e6
-    kernels = padded * (42 + 0.06 * D if D <= 128 else 56 + 0.133 * D)
+        kernels = tiles(B * H * tiles(Sq, 32), NUM_SMS) * tiles(Sk, 64) * (5 + D / 48 if D <= 128 else 7 + D / 45)
+        dense = 170 + pairs * (24 + 0.06 * D) + 5 * elements + 0.01 * B * Hkv
+        return kernels <= 1.15 * max(265, dense)
+    kernels = B * H * tiles(Sk, 32) * 32 * tiles(Sq, 64) * 64 / 1e6 * (40 + 0.06 * D if D <= 128 else 56 + 0.133 * D)
     if B * H * Sk * tiles(Sq, 64) * 64 * 4 > F32_DS_LIMIT:
         kernels *= 1.4                                          # dS is recomputed for dQ
-    return kernels <= max(600, 1.2 * (130 + (35 + 0.17 * D) * pairs))
+    dense = 290 + pairs * (20 + 0.18 * D) + 10 * elements + 0.02 * B * Hkv
+    return kernels <= 1.35 * max(600, dense)
 
 
 def prefer_f32_kernels(q: Tensor, k: Tensor, backward: bool = False) -> bool:
@@ -223,7 +227,8 @@ def prefer_f32_kernels(q: Tensor, k: Tensor, backward: bool = False) -> bool:
     Sk = k.shape[1]
     if D > 128 and min(B, 8) * H * Sq * Sk * 4 <= F32_DENSE_SCORE_LIMIT:
         return False
-    return B * H * Sq * Sk * 4 > F32_DENSE_MEMORY_LIMIT or _f32_kernels_pay(B, Sq, Sk, H, D, backward)
+    return B * H * Sq * Sk * 4 > F32_DENSE_MEMORY_LIMIT or _f32_kernels_pay(B, Sq, Sk, H, k.shape[2], D,
+                                                                                  backward)
 
 
 def _prep_f32(t: Tensor) -> Tensor:

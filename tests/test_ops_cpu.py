@@ -264,10 +264,12 @@ def test_fp32_attention_rule_follows_the_padding():
     """Sizes measured on both sides: few positions of many sequences leave the kernels' tiles empty and are clearly faster
     dense; full tiles, and calls that the dense evaluation cannot even launch in the time, are the kernels'."""
     from opentau_b200.ops.attention_native import _f32_kernels_pay as pay
-    for size in ((4096, 4, 4, 16, 72), (16384, 16, 16, 8, 64), (64, 1, 1000, 32, 128), (512, 8, 1000, 8, 256), (1, 1, 4000, 32, 128)):
+    for size in ((4096, 4, 4, 16, 16, 72), (16384, 16, 16, 8, 8, 64), (64, 1, 1000, 32, 8, 128), (512, 8, 1000, 8, 1, 256),
+                 (1, 1, 4000, 32, 8, 128)):
         assert not pay(*size, False), size
-    for size in ((4096, 4, 4, 16, 72), (64, 1, 300, 16, 72), (512, 1, 300, 8, 64), (512, 8, 1000, 8, 256)):
+    for size in ((4096, 4, 4, 16, 16, 72), (64, 1, 300, 16, 16, 72), (512, 1, 300, 8, 8, 64), (512, 8, 1000, 8, 1, 256)):
         assert not pay(*size, True), size
-    for size in ((2, 601, 601, 8, 256), (2, 700, 700, 8, 256), (1, 100, 100, 16, 72), (64, 64, 64, 16, 72), (256, 300, 300, 8, 64),
-                 (1, 50, 1000, 8, 256), (8, 1, 1000, 16, 72), (16, 601, 601, 16, 72), (4, 1227, 1227, 32, 128)):
+    for size in ((2, 601, 601, 8, 1, 256), (2, 700, 700, 8, 4, 256), (1, 100, 100, 16, 16, 72), (64, 64, 64, 16, 16, 72),
+                 (64, 300, 300, 8, 8, 64), (1, 50, 1000, 8, 1, 256), (8, 1, 1000, 16, 16, 72), (16, 601, 601, 16, 16, 72),
+                 (4, 1227, 1227, 32, 8, 128)):
         assert pay(*size, False) and pay(*size, True), size
