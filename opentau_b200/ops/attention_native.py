@@ -282,7 +282,12 @@ def attn_f32_bwd(do: Tensor, q: Tensor, k: Tensor, v: Tensor, o: Tensor, lse: Te
     lib.otb_attn_f32_bwd_plan(c_int(B), c_int(Sq), c_int(Sk), c_int(H), c_int(Hkv), c_int(D), byref(n_dq), byref(n_dkv),
                               byref(n_ds))
     n_dq, n_dkv = n_dq.value, n_dkv.value
-    ds = torch.empty(n_ds.value, dtype=torch.float32, device=q.device) if n_ds.value and keep_ds else None
+    ds = None
+    if n_ds.value and keep_ds:
+        try:
+            ds = torch.empty(n_ds.value, dtype=torch.float32, device=q.device)
+        except torch.cuda.OutOfMemoryError:                     # no room to keep it: recomputed
+            pass
     # partial sums of a split backward
     dq_parts = torch.empty(n_dq, B, Sq, H, D, dtype=torch.float32, device=q.device) if n_dq > 1 else None
     dk_parts, dv_parts = torch.empty(2, n_dkv, B, Sk, Hkv, D, dtype=torch.float32, device=q.device) \

@@ -466,3 +466,25 @@ def test_fp32_attention_may_take_either_path_in_each_direction(forward, backward
     assert (cuda_ops.launch_count > before) == backward
     for x, w in zip((o.detach(), *grads), want):
         assert _rel(x, w) < 256 * 2 ** -24
+
+
+def test_fp32_backward_recomputes_ds_where_there_is_no_room_for_it(monkeypatch):
+    from opentau_b200.ops import attention_native
+    B, S, H, D = 1, 70, 2, 64
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v, do = (torch.randn(B, S, H, D, device="cuda", generator=g) for _ in range(4))
+    blk = torch.arange(S, device="cuda").int()[None]
+    args = (blk, blk, torch.ones(B, S, dtype=torch.bool, device="cuda"), torch.ones(B, S, dtype=torch.bool, device="cuda"), D ** -0.5)
+    o, lse = attention_native.attn_f32_fwd(q, k, v, *args)
+    want = attention_native.attn_f32_bwd(do.reshape(B, S, -1), q, k, v, o, lse, *args, keep_ds=False)
+    empty = torch.empty
+
+    def full(*size, **kw):
+        if len(size) == 1:                                  # the scratch of dS alone has one dimension
+            raise torch.cuda.OutOfMemoryError("no room")
+        return empty(*size, **kw)
+
+    monkeypatch.setattr(torch, "empty", full)
+    got = attention_native.attn_f32_bwd(do.reshape(B, S, -1), q, k, v, o, lse, *args)
+    for x, y in zip(got, want):
+        assert torch.equal(x, y)
