@@ -246,3 +246,17 @@ def test_replayed_candidates_are_the_eager_ones():
         want = pol.sample_actions(b, noise=noise, n_candidates=n)
         pol.enable_cuda_graphs(True)
         torch.testing.assert_close(pol.sample_actions(b, noise=noise, n_candidates=n), want, rtol=1e-3, atol=1e-3)
+
+
+def test_replayed_requests_leave_every_module_in_eval_mode():
+    """A vision tower left in training mode is out of it after the call, also when the request is replayed, and a capture is
+    made in eval mode."""
+    pol = _open_policy(dropout=0.1)
+    b = tiny_batch(device="cuda")
+    noise = torch.randn(b["state"].shape[0], 10, 32, device="cuda")
+    want = pol.sample_actions(b, noise=noise)
+    pol.enable_cuda_graphs(True)
+    for part in (pol, pol.model.wrapper.paligemma.vision_tower, pol.model.wrapper.decoder):
+        part.train()
+        torch.testing.assert_close(pol.sample_actions(b, noise=noise), want, rtol=1e-3, atol=1e-3)
+        assert not any(m.training for m in pol.modules())
