@@ -15,8 +15,13 @@
 //
 // P is recomputed from the saved log-sum-exp (no running maximum needed); delta = rowsum(O o dO) comes
 // from a small pre-kernel.  Splitting dK and dV keeps each accumulator (128 x D fp32 = up to 256 TMEM
-// columns) next to double-buffered score tiles inside the 512-column tensor memory at D = 256.
+// columns) beside the first fixed tile and the scores inside the 512-column tensor memory at D = 256.
 // Results are deterministic: no atomics, fixed accumulation order.
+//
+// Order of a block j in the MMA warp: S of block j + 1 (its columns are free once S of j has been read, so it runs under the
+// elementwise work), the accumulation of j, dP of j + 1 (over the columns that held dS of j).  Measured against 32-wide blocks
+// with all operands in shared memory: 4096 positions, 8 heads on 1, width 256, 1024 of them causal: forward + backward 1145 ->
+// 718 us; a pi0.5 training step 164.4 -> 158.0 ms (all weights, batch 8), 214.7 -> 203.7 ms (expert only, batch 16).
 #include "common.cuh"
 #include <limits.h>
 
@@ -35,31 +40,51 @@ struct BwdParams {
   const unsigned char* k_valid;
   const float* lse;     // (B, H, Sq), natural log
   const float* delta;   // (B, H, Sq)
+  const __nv_bfloat16 *f1, *f2;   // tensors of the fixed tiles that go to tensor memory, and their strides in elements
+  long long f1_sb, f1_ss, f1_sh, f2_sb, f2_ss, f2_sh;
   __nv_bfloat16* out;   // dq (B,Sq,H,D) | dk, dv (B,Sk,Hkv,D), contiguous
   float* parts;         // splits > 1: fp32 sums of each part instead, (splits, ...) of the same layout
   int splits;           // blocks that share a tile's streamed blocks
   KernelStatus* status;
 };
 
+// Tensor memory (512 columns of 32 bits) and shared memory of one CTA.
+//
+// The product that every block pays twice is the score product, and its A operand, the fixed tile, is what it used to
+// spend its time on: with both operands in shared memory an M = 128 instruction of width N reads 4096 + 32 N bytes for N / 2
+// clocks of arithmetic (shared memory: 128 bytes a clock), so 32-wide blocks kept the pipe at most 40 % busy.  A fixed tile is
+// therefore moved into tensor memory once (two bf16 to a column), where an instruction reads only its 32 N bytes of B from
+// shared memory; P and dS take the place of the scores they were made from and are the A operand of the accumulation from
+// there.  At width 256 that is columns 128 (first fixed tile) + 64 + 64 (S, dP) + 256 (accumulator); the second fixed tile
+// stays in shared memory.  Without the first tile and the dS tiles there, blocks are 64 wide in five 32 KB slots.
+// Clocks of tensor pipe a 64-wide block at width 256: S 512, dP 768 (bound by operand reads), accumulation 512.
 template <int MODE, int DPAD, int BN>
 struct BwdSmem {
-  static constexpr int NF = MODE == MODE_DV ? 1 : 2;          // fixed tiles
+  static constexpr bool TWO = MODE != MODE_DV;                // second score product (dP)
+  static constexpr bool F2_TMEM = TWO && DPAD <= 128;         // second fixed tile in tensor memory too
+  static constexpr bool F2_SMEM = TWO && !F2_TMEM;
   static constexpr int NCHUNK = DPAD / 64;
   static constexpr int F_BYTES = BW_M * DPAD * 2;
   static constexpr int Y_BYTES = BN * DPAD * 2;
-  static constexpr int STAGE_BYTES = 2 * Y_BYTES;
-  static constexpr int T_CHUNKS = (BN + 63) / 64;
-  static constexpr int T_BYTES = T_CHUNKS * BW_M * 128;
+  static constexpr int NY1 = 3;                               // ring of the operand that S and (not in DV) the accumulation read
+  static constexpr int NY2 = F2_SMEM ? 2 : 3;                 // ring of the other one
   static constexpr int OFF_F = 0;
-  static constexpr int OFF_Y = NF * F_BYTES;
-  static constexpr int OFF_T = OFF_Y + 2 * STAGE_BYTES;
-  static constexpr int OFF_META = OFF_T + 2 * T_BYTES;        // per slot: int blk[BN], float lse2[BN], float delta[BN]
-  static constexpr int OFF_KMM = OFF_META + 2 * BN * 12;       // int kmm[2][BN/32][2]: min / max block id per 32 columns
+  static constexpr int OFF_Y1 = F2_SMEM ? F_BYTES : 0;
+  static constexpr int OFF_Y2 = OFF_Y1 + NY1 * Y_BYTES;
+  static constexpr int OFF_META = OFF_Y2 + NY2 * Y_BYTES;     // per slot: int blk[BN], float lse2[BN], float delta[BN]
+  static constexpr int OFF_KMM = OFF_META + 2 * BN * 12;      // int kmm[2][BN/32][2]: min / max block id per 32 columns
   static constexpr int OFF_BAR = OFF_KMM + 2 * (BN / 32) * 2 * 4;
-  static constexpr int NBAR = 16;
-  static constexpr int TOTAL = OFF_BAR + NBAR * 8 + 32 + 1024;
-  static constexpr int NS = MODE == MODE_DV ? 1 : 2;          // score tiles per block
-  static constexpr int TMEM_ACC = 2 * NS * BN;                // accumulator column offset
+  static constexpr int NBAR = 22;
+  static constexpr int USED = OFF_BAR + NBAR * 8 + 32;
+  static constexpr int TOTAL = USED + 1024;
+  static_assert(TOTAL <= 232448, "shared memory budget");
+  static constexpr int NS = TWO ? 1 : 2;                      // S tiles in flight
+  static constexpr int TM_F1 = 0;
+  static constexpr int TM_F2 = DPAD / 2;
+  static constexpr int TM_S = TM_F2 + (F2_TMEM ? DPAD / 2 : 0);
+  static constexpr int TM_DP = TM_S + NS * BN;
+  static constexpr int TM_ACC = TM_DP + (TWO ? BN : 0);
+  static_assert(TM_ACC + DPAD <= 512, "tensor memory budget");
 };
 
 __device__ __forceinline__ float bw_exp2(float x) {
@@ -70,24 +95,27 @@ __device__ __forceinline__ float bw_exp2(float x) {
 
 template <int MODE, int DPAD, int BN>
 __global__ void __launch_bounds__(320, 1)
-attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant__ CUtensorMap tm_f2,
-                const __grid_constant__ CUtensorMap tm_y1, const __grid_constant__ CUtensorMap tm_y2, BwdParams p) {
+attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_f2, const __grid_constant__ CUtensorMap tm_y1,
+                const __grid_constant__ CUtensorMap tm_y2, BwdParams p) {
   using L = BwdSmem<MODE, DPAD, BN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sF = smem + L::OFF_F;
-  uint8_t* sY = smem + L::OFF_Y;
-  uint8_t* sT = smem + L::OFF_T;
+  uint8_t* sY1 = smem + L::OFF_Y1;
+  uint8_t* sY2 = smem + L::OFF_Y2;
   int* meta_blk = reinterpret_cast<int*>(smem + L::OFF_META);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
-  uint64_t* f_full = bars + 0;
-  uint64_t* y_full = bars + 1;    // [2]
-  uint64_t* y_empty = bars + 3;   // [2]
-  uint64_t* s_full = bars + 5;    // [2]
-  uint64_t* s_free = bars + 7;    // [2]
-  uint64_t* t_full = bars + 9;    // [2]
-  uint64_t* t_free = bars + 11;   // [2]
-  uint64_t* acc_full = bars + 13;
+  uint64_t* f_full = bars + 0;     // the fixed tile in shared memory has landed
+  uint64_t* a_full = bars + 1;     // the fixed tiles are in tensor memory
+  uint64_t* y1_full = bars + 2;    // [3]
+  uint64_t* y1_empty = bars + 5;   // [3]
+  uint64_t* y2_full = bars + 8;    // [3]
+  uint64_t* y2_empty = bars + 11;  // [3]
+  uint64_t* s_full = bars + 14;    // [2]
+  uint64_t* s_free = bars + 16;    // S has been read (TWO)
+  uint64_t* dp_full = bars + 17;
+  uint64_t* t_full = bars + 18;    // [2] P or dS is in tensor memory
+  uint64_t* acc_full = bars + 20;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NBAR);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* range_smem = reinterpret_cast<int*>(tmem_slot + 2);   // [0] = first block, [1] = end (exclusive, in elements)
@@ -100,23 +128,27 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant
 
   if (threadIdx.x == 0) {
     mbar_init(f_full, 1);
+    mbar_init(a_full, 256);
+    for (int i = 0; i < 3; ++i) {
+      mbar_init(&y1_full[i], 1);
+      mbar_init(&y1_empty[i], 1);
+      mbar_init(&y2_full[i], 1);
+      mbar_init(&y2_empty[i], 1);
+    }
+    mbar_init(s_free, 256);
+    mbar_init(dp_full, 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&y_full[i], 1);
-      mbar_init(&y_empty[i], 1);
       mbar_init(&s_full[i], 1);
-      mbar_init(&s_free[i], 256);
       mbar_init(&t_full[i], 256);
-      mbar_init(&t_free[i], 1);
     }
     mbar_init(acc_full, 1);
     *abort_flag = 0;
     range_smem[0] = INT_MAX;
     range_smem[1] = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&tm_f1);
     tma_prefetch_desc(&tm_y1);
     tma_prefetch_desc(&tm_y2);
-    if (MODE != MODE_DV) tma_prefetch_desc(&tm_f2);
+    if (L::F2_SMEM) tma_prefetch_desc(&tm_f2);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
@@ -126,7 +158,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_acc = tmem_base + L::TMEM_ACC;
+  const uint32_t tmem_acc = tmem_base + L::TM_ACC;
 
   // ---- range of streamed blocks that can contain a visible (query, key) pair
   __shared__ int s_ext, s_any;
@@ -219,81 +251,113 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one()) {
-      mbar_expect_tx(f_full, L::NF * L::F_BYTES);
-#pragma unroll
-      for (int c = 0; c < L::NCHUNK; ++c) {
-        if (MODE == MODE_DQ) {
-          tma_load_4d(sF + c * (BW_M * 128), &tm_f1, f_full, c * 64, kvh * g, tile * pos_per_tile, b);
-          tma_load_4d(sF + L::F_BYTES + c * (BW_M * 128), &tm_f2, f_full, c * 64, kvh * g, tile * pos_per_tile, b);
-        } else {
-          tma_load_4d(sF + c * (BW_M * 128), &tm_f1, f_full, c * 64, kvh, tile * BW_M, b);
-          if (MODE == MODE_DK)
-            tma_load_4d(sF + L::F_BYTES + c * (BW_M * 128), &tm_f2, f_full, c * 64, kvh, tile * BW_M, b);
-        }
-      }
-      for (int j = 0; j < nblk; ++j) {
-        const int slot = j & 1, u = j >> 1;
-        mbar_wait(&y_empty[slot], (u & 1) ^ 1, abort_flag, p.status, KID_ATTN_BWD, 1, j);
-        uint8_t* y1 = sY + slot * L::STAGE_BYTES;
-        uint8_t* y2 = y1 + L::Y_BYTES;
-        mbar_expect_tx(&y_full[slot], L::STAGE_BYTES);
-        const int blk = blk0 + j;
+      if (L::F2_SMEM) {
+        mbar_expect_tx(f_full, L::F_BYTES);
 #pragma unroll
         for (int c = 0; c < L::NCHUNK; ++c) {
-          if (MODE == MODE_DQ) {
-            tma_load_4d(y1 + c * (BN * 128), &tm_y1, &y_full[slot], c * 64, kvh, blk * BN, b);
-            tma_load_4d(y2 + c * (BN * 128), &tm_y2, &y_full[slot], c * 64, kvh, blk * BN, b);
-          } else {
-            tma_load_4d(y1 + c * (BN * 128), &tm_y1, &y_full[slot], c * 64, kvh * g, blk * pos_per_blk, b);
-            tma_load_4d(y2 + c * (BN * 128), &tm_y2, &y_full[slot], c * 64, kvh * g, blk * pos_per_blk, b);
-          }
+          if (MODE == MODE_DQ) tma_load_4d(sF + c * (BW_M * 128), &tm_f2, f_full, c * 64, kvh * g, tile * pos_per_tile, b);
+          else tma_load_4d(sF + c * (BW_M * 128), &tm_f2, f_full, c * 64, kvh, tile * BW_M, b);
         }
+      }
+      int s1 = 0, s2 = 0;
+      uint32_t ph1 = 1, ph2 = 1;                     // a ring's first round does not wait
+      for (int j = 0; j < nblk; ++j) {
+        const int blk = blk0 + j;
+        mbar_wait(&y1_empty[s1], ph1, abort_flag, p.status, KID_ATTN_BWD, 1, j);
+        mbar_expect_tx(&y1_full[s1], L::Y_BYTES);
+#pragma unroll
+        for (int c = 0; c < L::NCHUNK; ++c) {
+          uint8_t* y = sY1 + s1 * L::Y_BYTES + c * (BN * 128);
+          if (MODE == MODE_DQ) tma_load_4d(y, &tm_y1, &y1_full[s1], c * 64, kvh, blk * BN, b);
+          else tma_load_4d(y, &tm_y1, &y1_full[s1], c * 64, kvh * g, blk * pos_per_blk, b);
+        }
+        if (++s1 == L::NY1) { s1 = 0; ph1 ^= 1; }
+        mbar_wait(&y2_empty[s2], ph2, abort_flag, p.status, KID_ATTN_BWD, 8, j);
+        mbar_expect_tx(&y2_full[s2], L::Y_BYTES);
+#pragma unroll
+        for (int c = 0; c < L::NCHUNK; ++c) {
+          uint8_t* y = sY2 + s2 * L::Y_BYTES + c * (BN * 128);
+          if (MODE == MODE_DQ) tma_load_4d(y, &tm_y2, &y2_full[s2], c * 64, kvh, blk * BN, b);
+          else tma_load_4d(y, &tm_y2, &y2_full[s2], c * 64, kvh * g, blk * pos_per_blk, b);
+        }
+        if (++s2 == L::NY2) { s2 = 0; ph2 ^= 1; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
+    // Instructions of one CTA run in the order they are issued, so dP of block j + 1 (and, with two S tiles, S of block
+    // j + 2) may be issued straight behind the accumulation that reads dS (P) of block j from the same columns.
     if (elect_one()) {
       const uint32_t idesc_s = make_idesc_bf16(BW_M, BN, 0, 0);
       const uint32_t idesc_acc = make_idesc_bf16(BW_M, p.Dmma, 0, 1);
       const int ksteps = p.Dmma / 16;
-      const uint32_t f_addr = smem_u32(sF);
-      auto issue_scores = [&](int j) {
-        const int slot = j & 1, u = j >> 1;
-        mbar_wait(&y_full[slot], u & 1, abort_flag, p.status, KID_ATTN_BWD, 2, j);
-        mbar_wait(&s_free[slot], (u & 1) ^ 1, abort_flag, p.status, KID_ATTN_BWD, 3, j);
+      // scores of block j against a fixed tile in tensor memory
+      auto scores_tmem = [&](uint32_t d, uint32_t f, uint32_t y) {
+        for (int kk = 0; kk < ksteps; ++kk) {
+          uint64_t bd = make_smem_desc(y + (kk >> 2) * (BN * 128) + (kk & 3) * 32, 16, 1024);
+          umma_ts(d, f + kk * 8, bd, idesc_s, kk != 0 ? 1u : 0u);
+        }
+      };
+      int s1 = 0, s2 = 0;                            // ring slots of the next S and of the next dP (DV: accumulation)
+      uint32_t ph1 = 0, ph2 = 0;
+      auto issue_s = [&](int j) {
+        mbar_wait(&y1_full[s1], ph1, abort_flag, p.status, KID_ATTN_BWD, 2, j);
+        if (L::TWO && j > 0) mbar_wait(s_free, (j - 1) & 1, abort_flag, p.status, KID_ATTN_BWD, 3, j);
         tc_fence_after();
-        const uint32_t y_addr = smem_u32(sY + slot * L::STAGE_BYTES);
-#pragma unroll
-        for (int s = 0; s < L::NS; ++s) {
-          const uint32_t fa = f_addr + s * L::F_BYTES;
-          const uint32_t ya = y_addr + s * L::Y_BYTES;
-          const uint32_t d = tmem_base + slot * (L::NS * BN) + s * BN;
+        const int buf = L::TWO ? 0 : (j & 1);
+        scores_tmem(tmem_base + L::TM_S + buf * BN, tmem_base + L::TM_F1, smem_u32(sY1 + s1 * L::Y_BYTES));
+        umma_commit(&s_full[buf]);
+        if (!L::TWO) umma_commit(&y1_empty[s1]);     // DV reads this operand nowhere else
+        if (++s1 == L::NY1) { s1 = 0; ph1 ^= 1; }
+      };
+      auto issue_dp = [&](int j) {
+        mbar_wait(&y2_full[s2], ph2, abort_flag, p.status, KID_ATTN_BWD, 10, j);
+        tc_fence_after();
+        const uint32_t y = smem_u32(sY2 + s2 * L::Y_BYTES), d = tmem_base + L::TM_DP;
+        if (L::F2_TMEM) {
+          scores_tmem(d, tmem_base + L::TM_F2, y);
+        } else {
+          const uint32_t fa = smem_u32(sF);
           for (int kk = 0; kk < ksteps; ++kk) {
             const int c = kk >> 2, w = kk & 3;
             uint64_t ad = make_smem_desc(fa + c * (BW_M * 128) + w * 32, 16, 1024);
-            uint64_t bd = make_smem_desc(ya + c * (BN * 128) + w * 32, 16, 1024);
+            uint64_t bd = make_smem_desc(y + c * (BN * 128) + w * 32, 16, 1024);
             umma_ss(d, ad, bd, idesc_s, kk != 0 ? 1u : 0u);
           }
         }
-        umma_commit(&s_full[slot]);
+        umma_commit(dp_full);
+        umma_commit(&y2_empty[s2]);
+        if (++s2 == L::NY2) { s2 = 0; ph2 ^= 1; }
       };
-      mbar_wait(f_full, 0, abort_flag, p.status, KID_ATTN_BWD, 4, 0);
-      issue_scores(0);
+      mbar_wait(a_full, 0, abort_flag, p.status, KID_ATTN_BWD, 4, 0);
+      if (L::F2_SMEM) mbar_wait(f_full, 0, abort_flag, p.status, KID_ATTN_BWD, 11, 0);
+      tc_fence_after();
+      issue_s(0);
+      if (L::TWO) issue_dp(0);
+      int sa = 0;                                    // ring slot of the accumulation's operand
       for (int j = 0; j < nblk; ++j) {
-        const int slot = j & 1, u = j >> 1;
-        if (j + 1 < nblk) issue_scores(j + 1);
-        mbar_wait(&t_full[slot], u & 1, abort_flag, p.status, KID_ATTN_BWD, 5, j);
+        if (j + 1 < nblk) issue_s(j + 1);
+        const int buf = L::TWO ? 0 : (j & 1);
+        if (!L::TWO) mbar_wait(&y2_full[s2], ph2, abort_flag, p.status, KID_ATTN_BWD, 10, j);
+        mbar_wait(&t_full[buf], (L::TWO ? j : (j >> 1)) & 1, abort_flag, p.status, KID_ATTN_BWD, 5, j);
         tc_fence_after();
-        const uint32_t t_addr = smem_u32(sT + slot * L::T_BYTES);
-        const uint32_t yb = smem_u32(sY + slot * L::STAGE_BYTES + (MODE == MODE_DV ? L::Y_BYTES : 0));
+        const uint32_t t = tmem_base + (L::TWO ? L::TM_DP : L::TM_S + buf * BN);
+        const uint32_t yb = smem_u32(L::TWO ? sY1 + sa * L::Y_BYTES : sY2 + s2 * L::Y_BYTES);
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk) {
-          uint64_t ad = make_smem_desc(t_addr + (kk >> 2) * (BW_M * 128) + (kk & 3) * 32, 16, 1024);
+          // each half of a block's columns was written over the first columns of its own scores
+          const uint32_t at = t + (kk / (BN / 32)) * (BN / 2) + (kk % (BN / 32)) * 8;
           uint64_t bd = make_smem_desc(yb + kk * 2048, BN * 128, 1024);
-          umma_ss(tmem_acc, ad, bd, idesc_acc, (j | kk) != 0 ? 1u : 0u);
+          umma_ts(tmem_acc, at, bd, idesc_acc, (j | kk) != 0 ? 1u : 0u);
         }
-        umma_commit(&y_empty[slot]);
-        umma_commit(&t_free[slot]);
+        if (L::TWO) {
+          umma_commit(&y1_empty[sa]);
+          if (++sa == L::NY1) sa = 0;
+          if (j + 1 < nblk) issue_dp(j + 1);
+        } else {
+          umma_commit(&y2_empty[s2]);
+          if (++s2 == L::NY2) { s2 = 0; ph2 ^= 1; }
+        }
       }
       umma_commit(acc_full);
     }
@@ -305,8 +369,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant
     const int st = threadIdx.x - 64;             // 0..255
     int* kmm = reinterpret_cast<int*>(smem + L::OFF_KMM);
     constexpr int HB = BN / 2;                   // columns per thread per block
-    constexpr int PIECE = HB >= 32 ? 32 : 16;    // columns per TMEM read
-    constexpr int NP = HB / PIECE;
+    static_assert(HB % 32 == 0, "TMEM reads are 32 columns wide");
     const uint32_t lane_off = uint32_t(quad * 32) << 16;
     float* meta_lse = reinterpret_cast<float*>(meta_blk + 2 * BN);
     float* meta_delta = meta_lse + 2 * BN;
@@ -318,6 +381,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant
     float row_lse2 = 0.f, row_delta = 0.f;
     long long out_off;
     bool row_in;
+    const __nv_bfloat16 *f1_row, *f2_row;
     if (MODE == MODE_DQ) {
       const int pos = tile * pos_per_tile + row / g;
       const int head = kvh * g + row % g;
@@ -329,130 +393,170 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_f1, const __grid_constant
         row_delta = p.delta[((long long)b * p.H + head) * p.Sq + pos];
       }
       out_off = (((long long)b * p.Sq + pos) * p.H + head) * p.D;
+      f1_row = p.f1 + b * p.f1_sb + pos * p.f1_ss + head * p.f1_sh;
+      f2_row = p.f2 + out_off;                   // dO is laid out like dQ
     } else {
       const int key = tile * BW_M + row;
       row_in = key < p.Sk;
       row_ok = row_in && p.k_valid[(long long)b * p.Sk + key] != 0;
       if (row_ok) row_blk = p.k_blk[(long long)b * p.Sk + key];
       out_off = (((long long)b * p.Sk + key) * p.Hkv + kvh) * p.D;
+      f1_row = p.f1 + b * p.f1_sb + key * p.f1_ss + kvh * p.f1_sh;
+      f2_row = p.f2 + b * p.f2_sb + key * p.f2_ss + kvh * p.f2_sh;
     }
 
-    for (int j = 0; j < nblk; ++j) {
-      const int slot = j & 1, u = j >> 1;
-      const int blk = blk0 + j;
-      if (st < BN) {
-        if (MODE == MODE_DQ) {
-          const int key = blk * BN + st;
-          int kb = INT_MAX;
-          if (key < p.Sk) {
-            const int kbv = p.k_blk[(long long)b * p.Sk + key];
-            const int kvv = p.k_valid[(long long)b * p.Sk + key];
-            kb = kvv ? kbv : INT_MAX;
-          }
-          meta_blk[slot * BN + st] = kb;
-          const int mn = __reduce_min_sync(0xffffffffu, kb), mxk = __reduce_max_sync(0xffffffffu, kb);
-          if (lane == 0) {
-            kmm[(slot * (BN / 32) + st / 32) * 2 + 0] = mn;
-            kmm[(slot * (BN / 32) + st / 32) * 2 + 1] = mxk;
-          }
-        } else {
-          const int pos = blk * pos_per_blk + st / g;
-          const int head = kvh * g + st % g;
-          int qb = INT_MIN;
-          float l2 = INFINITY, dl = 0.f;
-          if (pos < p.Sq) {
-            // four independent loads; the validity only selects afterwards
-            const int qvv = p.q_valid[(long long)b * p.Sq + pos];
-            const int qbv = p.q_blk[(long long)b * p.Sq + pos];
-            const float lv = p.lse[((long long)b * p.H + head) * p.Sq + pos];
-            const float dv2 = p.delta[((long long)b * p.H + head) * p.Sq + pos];
-            if (qvv) {
-              qb = qbv;
-              l2 = lv * LOG2E;
-              dl = dv2;
-            }
-          }
-          meta_blk[slot * BN + st] = qb;
-          meta_lse[slot * BN + st] = l2;
-          meta_delta[slot * BN + st] = dl;
-          const int mn = __reduce_min_sync(0xffffffffu, qb), mxk = __reduce_max_sync(0xffffffffu, qb);
-          if (lane == 0) {
-            kmm[(slot * (BN / 32) + st / 32) * 2 + 0] = mn;
-            kmm[(slot * (BN / 32) + st / 32) * 2 + 1] = mxk;
-          }
-        }
-      }
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      const int* mb = meta_blk + slot * BN;
-      const float* ml = meta_lse + slot * BN;
-      const float* md = meta_delta + slot * BN;
-      mbar_wait(&s_full[slot], u & 1, abort_flag, p.status, KID_ATTN_BWD, 6, j);
-      tc_fence_after();
-      if (j >= 2) mbar_wait(&t_free[slot], (u - 1) & 1, abort_flag, p.status, KID_ATTN_BWD, 7, j);
-      const uint32_t s_addr = tmem_base + slot * (L::NS * BN) + lane_off;
-      uint8_t* trow = sT + slot * L::T_BYTES + row * 128;
+    // ---- fixed tiles -> tensor memory: this thread's row, its half of the head width
+    auto fixed_tile = [&](const __nv_bfloat16* src, int col) {
+      constexpr int CW = DPAD / 4 < 32 ? DPAD / 4 : 32;      // 32-bit columns a piece: the half row is one or two pieces
 #pragma unroll
-      for (int c = 0; c < NP; ++c) {
-        const int col0 = half * HB + c * PIECE;
-        uint32_t rs[PIECE];
-        uint32_t rd[PIECE];
+      for (int c = 0; c < DPAD / 4; c += CW) {
+        uint32_t r[CW];
+#pragma unroll
+        for (int e = 0; e < CW; e += 4) {
+          const int d = 2 * (half * (DPAD / 4) + c + e);
+          uint4 v = make_uint4(0u, 0u, 0u, 0u);
+          if (row_in && d < p.D) v = *reinterpret_cast<const uint4*>(src + d);
+          r[e] = v.x; r[e + 1] = v.y; r[e + 2] = v.z; r[e + 3] = v.w;
+        }
         __syncwarp();
-        if (PIECE == 32) {
-          tmem_ld_x32(s_addr + col0, rs);
-          if (MODE != MODE_DV) tmem_ld_x32(s_addr + BN + col0, rd);
-        } else {
-          tmem_ld_x16(s_addr + col0, rs);
-          if (MODE != MODE_DV) tmem_ld_x16(s_addr + BN + col0, rd);
+        const uint32_t dst = tmem_base + col + lane_off + half * (DPAD / 4) + c;
+        if (CW == 32) tmem_st_x32(dst, r);
+        else tmem_st_x16(dst, r);
+      }
+    };
+    fixed_tile(f1_row, L::TM_F1);
+    if (L::F2_TMEM) fixed_tile(f2_row, L::TM_F2);
+    tmem_wait_st();
+    tc_fence_before();
+    mbar_arrive(a_full);
+
+    // ---- what a block's columns carry (thread st < BN: one column), fetched one block ahead
+    int nx_blk = 0;
+    float nx_lse = 0.f, nx_delta = 0.f;
+    auto fetch_meta = [&](int j) {
+      if (st >= BN) return;
+      if (MODE == MODE_DQ) {
+        const int key = (blk0 + j) * BN + st;
+        nx_blk = INT_MAX;
+        if (key < p.Sk) {
+          const int kbv = p.k_blk[(long long)b * p.Sk + key];
+          const int kvv = p.k_valid[(long long)b * p.Sk + key];
+          nx_blk = kvv ? kbv : INT_MAX;
         }
-        // visibility of this group of columns for this row: 2 = all, 0 = none, 1 = test each
-        const int gi = (slot * (BN / 32) + col0 / 32) * 2;
-        const int gmin = kmm[gi], gmax = kmm[gi + 1];
-        int cls;
-        if (MODE == MODE_DQ) cls = (!row_ok || gmin > row_blk) ? 0 : (gmax <= row_blk ? 2 : 1);
-        else cls = (!row_ok || gmax < row_blk) ? 0 : (gmin >= row_blk ? 2 : 1);
-        tmem_wait_ld();
-        uint32_t packed[PIECE / 2];
-        if (cls == 0) {
-#pragma unroll
-          for (int e = 0; e < PIECE / 2; ++e) packed[e] = 0u;
-        } else {
-#pragma unroll
-          for (int e = 0; e < PIECE; e += 2) {
-            float v[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int col = col0 + e + h;
-              bool vis = true;
-              float l2, dl;
-              if (MODE == MODE_DQ) {
-                if (cls == 1) vis = mb[col] <= row_blk;
-                l2 = row_lse2;
-                dl = row_delta;
-              } else {
-                if (cls == 1) vis = row_blk <= mb[col];
-                l2 = ml[col];
-                dl = md[col];
-              }
-              float pr = vis ? bw_exp2(fmaf(__uint_as_float(rs[e + h]), p.scale_log2, -l2)) : 0.f;
-              if (MODE == MODE_DV) v[h] = pr;
-              else v[h] = pr * (__uint_as_float(rd[e + h]) - dl) * p.scale;
-            }
-            packed[e >> 1] = pack_bf16(v[0], v[1]);
+      } else {
+        const int pos = (blk0 + j) * pos_per_blk + st / g;
+        const int head = kvh * g + st % g;
+        nx_blk = INT_MIN;
+        nx_lse = INFINITY;
+        nx_delta = 0.f;
+        if (pos < p.Sq) {
+          // four independent loads; the validity only selects afterwards
+          const int qvv = p.q_valid[(long long)b * p.Sq + pos];
+          const int qbv = p.q_blk[(long long)b * p.Sq + pos];
+          const float lv = p.lse[((long long)b * p.H + head) * p.Sq + pos];
+          const float dv2 = p.delta[((long long)b * p.H + head) * p.Sq + pos];
+          if (qvv) {
+            nx_blk = qbv;
+            nx_lse = lv * LOG2E;
+            nx_delta = dv2;
           }
         }
-        const int chunk = col0 / 64;
-        const int unit0 = (col0 % 64) / 8;
-#pragma unroll
-        for (int q4 = 0; q4 < PIECE / 8; ++q4) {
-          const int unit = (unit0 + q4) ^ (row & 7);
-          uint4 val = make_uint4(packed[q4 * 4 + 0], packed[q4 * 4 + 1], packed[q4 * 4 + 2], packed[q4 * 4 + 3]);
-          *reinterpret_cast<uint4*>(trow + chunk * (BW_M * 128) + unit * 16) = val;
+      }
+    };
+    fetch_meta(0);
+    for (int j = 0; j < nblk; ++j) {
+      const int slot = j & 1;
+      if (st < BN) {                             // whole warps
+        meta_blk[slot * BN + st] = nx_blk;
+        if (MODE != MODE_DQ) {
+          meta_lse[slot * BN + st] = nx_lse;
+          meta_delta[slot * BN + st] = nx_delta;
+        }
+        const int mn = __reduce_min_sync(0xffffffffu, nx_blk), mxk = __reduce_max_sync(0xffffffffu, nx_blk);
+        if (lane == 0) {
+          kmm[(slot * (BN / 32) + st / 32) * 2 + 0] = mn;
+          kmm[(slot * (BN / 32) + st / 32) * 2 + 1] = mxk;
         }
       }
+      if (j + 1 < nblk) fetch_meta(j + 1);
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      const int* mb = meta_blk + slot * BN + half * HB;
+      const float* ml = meta_lse + slot * BN + half * HB;
+      const float* md = meta_delta + slot * BN + half * HB;
+      const int buf = L::TWO ? 0 : slot;
+      const uint32_t s_addr = tmem_base + L::TM_S + buf * BN + half * HB + lane_off;
+      const uint32_t d_addr = tmem_base + L::TM_DP + half * HB + lane_off;
+      const uint32_t t_addr = L::TWO ? d_addr : s_addr;
+      mbar_wait(&s_full[buf], (L::TWO ? j : (j >> 1)) & 1, abort_flag, p.status, KID_ATTN_BWD, 6, j);
+      tc_fence_after();
+      uint32_t rs[HB];
+#pragma unroll
+      for (int c = 0; c < HB; c += 32) {
+        __syncwarp();
+        tmem_ld_x32(s_addr + c, rs + c);
+      }
+      tmem_wait_ld();
+      if (L::TWO) {
+        tc_fence_before();
+        mbar_arrive(s_free);
+      }
+      // ---- P, over the scores; visibility per group of 32 columns for this row: 2 = all, 0 = none, 1 = test each
+      int cls[HB / 32];
+#pragma unroll
+      for (int c = 0; c < HB / 32; ++c) {
+        const int gi = (slot * (BN / 32) + half * (HB / 32) + c) * 2;
+        const int gmin = kmm[gi], gmax = kmm[gi + 1];
+        if (MODE == MODE_DQ) cls[c] = (!row_ok || gmin > row_blk) ? 0 : (gmax <= row_blk ? 2 : 1);
+        else cls[c] = (!row_ok || gmax < row_blk) ? 0 : (gmin >= row_blk ? 2 : 1);
+        if (cls[c] != 0) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            const int col = c * 32 + e;
+            const float l2 = MODE == MODE_DQ ? row_lse2 : ml[col];
+            rs[col] = __float_as_uint(bw_exp2(fmaf(__uint_as_float(rs[col]), p.scale_log2, -l2)));
+          }
+          if (cls[c] == 1) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) {
+              const int col = c * 32 + e;
+              if (!(MODE == MODE_DQ ? mb[col] <= row_blk : row_blk <= mb[col])) rs[col] = 0u;
+            }
+          }
+        }
+      }
+      if (L::TWO) {
+        mbar_wait(dp_full, j & 1, abort_flag, p.status, KID_ATTN_BWD, 7, j);
+        tc_fence_after();
+      }
+      // every score of mine has to be read before its columns are written
+      uint32_t packed[HB / 2];
+#pragma unroll
+      for (int c = 0; c < HB / 32; ++c) {
+        uint32_t rd[32];
+        if (L::TWO) {
+          __syncwarp();
+          tmem_ld_x32(d_addr + c * 32, rd);
+          tmem_wait_ld();
+        }
+#pragma unroll
+        for (int e = 0; e < 32; e += 2) {
+          const int col = c * 32 + e;
+          float v[2];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const float pr = __uint_as_float(rs[col + h]);
+            if (!L::TWO) v[h] = pr;
+            else v[h] = pr * (__uint_as_float(rd[e + h]) - (MODE == MODE_DQ ? row_delta : md[col + h])) * p.scale;
+          }
+          packed[col >> 1] = cls[c] == 0 ? 0u : pack_bf16(v[0], v[1]);
+        }
+      }
+      __syncwarp();
+      if (HB == 64) tmem_st_x32(t_addr, packed);
+      else tmem_st_x16(t_addr, packed);
+      tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(&s_free[slot]);
-      fence_async_smem();
-      mbar_arrive(&t_full[slot]);
+      mbar_arrive(&t_full[buf]);
     }
 
     mbar_wait(acc_full, 0, abort_flag, p.status, KID_ATTN_BWD, 9, 0);
@@ -573,7 +677,7 @@ static long long bwd_tiles(int Sq, int Sk, int g) {
 
 template <int MODE, int DPAD, int BN>
 static int launch_bwd(const void* q, Strides qs, const void* k, Strides ks, const void* v, Strides vs, const void* d_o,
-                      const BwdParams& p, cudaStream_t stream) {
+                      BwdParams p, cudaStream_t stream) {
   using L = BwdSmem<MODE, DPAD, BN>;
   static bool configured = false;
   auto kern = attn_bwd_kernel<MODE, DPAD, BN>;
@@ -584,12 +688,15 @@ static int launch_bwd(const void* q, Strides qs, const void* k, Strides ks, cons
   }
   const int g = p.g;
   if (MODE != MODE_DQ && (BN % g)) return -20;
-  CUtensorMap f1, f2, y1, y2;
+  CUtensorMap f2, y1, y2;
   const Strides dos = {(long long)p.Sq * p.H * p.D, (long long)p.H * p.D, (long long)p.D};
+  const Strides f1s = MODE == MODE_DQ ? qs : ks, f2s = MODE == MODE_DQ ? dos : vs;
+  p.f1 = static_cast<const __nv_bfloat16*>(MODE == MODE_DQ ? q : k);
+  p.f2 = static_cast<const __nv_bfloat16*>(MODE == MODE_DQ ? d_o : v);
+  p.f1_sb = f1s.sb; p.f1_ss = f1s.ss; p.f1_sh = f1s.sh;
+  p.f2_sb = f2s.sb; p.f2_ss = f2s.ss; p.f2_sh = f2s.sh;
   int r;
   if (MODE == MODE_DQ) {
-    r = make_map4b(&f1, q, p.D, p.H, p.Sq, p.B, qs.sh, qs.ss, qs.sb, g, BW_M / g);
-    if (r) return 1000 + r;
     r = make_map4b(&f2, d_o, p.D, p.H, p.Sq, p.B, dos.sh, dos.ss, dos.sb, g, BW_M / g);
     if (r) return 2000 + r;
     r = make_map4b(&y1, k, p.D, p.Hkv, p.Sk, p.B, ks.sh, ks.ss, ks.sb, 1, BN);
@@ -597,8 +704,6 @@ static int launch_bwd(const void* q, Strides qs, const void* k, Strides ks, cons
     r = make_map4b(&y2, v, p.D, p.Hkv, p.Sk, p.B, vs.sh, vs.ss, vs.sb, 1, BN);
     if (r) return 4000 + r;
   } else {
-    r = make_map4b(&f1, k, p.D, p.Hkv, p.Sk, p.B, ks.sh, ks.ss, ks.sb, 1, BW_M);
-    if (r) return 1000 + r;
     r = make_map4b(&f2, v, p.D, p.Hkv, p.Sk, p.B, vs.sh, vs.ss, vs.sb, 1, BW_M);
     if (r) return 2000 + r;
     r = make_map4b(&y1, q, p.D, p.H, p.Sq, p.B, qs.sh, qs.ss, qs.sb, g, BN / g);
@@ -607,7 +712,7 @@ static int launch_bwd(const void* q, Strides qs, const void* k, Strides ks, cons
     if (r) return 4000 + r;
   }
   const dim3 grid((unsigned)bwd_tiles<MODE>(p.Sq, p.Sk, g), p.Hkv, p.B * p.splits);
-  kern<<<grid, 320, L::TOTAL, stream>>>(f1, f2, y1, y2, p);
+  kern<<<grid, 320, L::TOTAL, stream>>>(f2, y1, y2, p);
   if (p.splits > 1) {
     const long long n8 = (long long)p.B * (MODE == MODE_DQ ? (long long)p.Sq * p.H : (long long)p.Sk * p.Hkv) * p.D / 8;
     attn_bwd_sum_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(p.parts, p.out, n8, p.splits);
@@ -651,23 +756,22 @@ static int pick_bwd_splits(long long tiles, int blocks, int B, double out_bytes,
 
 using namespace otb;
 
-// columns of a streamed block by padded head width, for dQ and dK / for dV
-static constexpr int bwd_bn(int dpad) { return dpad == 256 ? 32 : 64; }
-static constexpr int bwd_bn_v(int dpad) { return dpad == 64 ? 128 : 64; }
+// columns of a streamed block by padded head width
+static constexpr int bwd_bn(int dpad) { return dpad == 256 ? 64 : 128; }
 
 // Parts of the three products; `dq`, `dk`, `dv` above 1 want fp32 scratch of that many outputs each.  Sk must be the
 // streamed length of dQ.
 extern "C" void otb_attn_bwd_splits(int B, int Sq, int Sk, int H, int Hkv, int D, int* dq, int* dk, int* dv) {
   const int g = H / Hkv, dpad = D <= 64 ? 64 : (D <= 128 ? 128 : 256);
-  const int bn = bwd_bn(dpad), bnv = bwd_bn_v(dpad);
+  const int bn = bwd_bn(dpad);
   const long long kv = (long long)Hkv * B;
-  // a block of 32 x 256 takes about 1 us, a dV block of 64 x 256 0.8, others in proportion; fp32 sums move at about 4 TB/s
-  const double us = 1.0 * bn * dpad / (32 * 256), us_v = 0.8 * bnv * dpad / (64 * 256);
+  // a block of 64 x 256 takes about 1.1 us (dV: 0.65), others in proportion; fp32 sums move at about 4 TB/s
+  const double us = 1.1 * bn * dpad / (64 * 256), us_v = 0.65 * bn * dpad / (64 * 256);
   const double q_out = 4.0 * B * Sq * H * D, k_out = 4.0 * B * Sk * Hkv * D, q_sum = q_out / 4e6, k_sum = k_out / 4e6;
   *dq = pick_bwd_splits(bwd_tiles<MODE_DQ>(Sq, Sk, g) * kv, (Sk + bn - 1) / bn, B, q_out, q_sum / us, 15.0 / us);
   *dk = pick_bwd_splits(bwd_tiles<MODE_DK>(Sq, Sk, g) * kv, (int)(((long long)Sq * g + bn - 1) / bn), B, k_out, k_sum / us,
                         15.0 / us);
-  *dv = pick_bwd_splits(bwd_tiles<MODE_DV>(Sq, Sk, g) * kv, (int)(((long long)Sq * g + bnv - 1) / bnv), B, k_out, k_sum / us_v,
+  *dv = pick_bwd_splits(bwd_tiles<MODE_DV>(Sq, Sk, g) * kv, (int)(((long long)Sq * g + bn - 1) / bn), B, k_out, k_sum / us_v,
                         15.0 / us_v);
 }
 
@@ -727,7 +831,7 @@ extern "C" int otb_attn_bwd(const void* q, const void* k, const void* v, const v
   p.out = static_cast<__nv_bfloat16*>(dv);                                             \
   p.parts = dv_parts;                                                                  \
   p.splits = dv_splits;                                                                \
-  r = launch_bwd<MODE_DV, DP, bwd_bn_v(DP)>(q, qs, k, ks, v, vs, d_o, p, stream);       \
+  r = launch_bwd<MODE_DV, DP, bwd_bn(DP)>(q, qs, k, ks, v, vs, d_o, p, stream);       \
   if (r) return 200000 + r;
   if (dpad == 64) { RUN3(64) }
   else if (dpad == 128) { RUN3(128) }

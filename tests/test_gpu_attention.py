@@ -345,6 +345,33 @@ def test_fp32_attention_kernels_at_the_edges_of_their_tiles(D, Sq, cross, H, Hkv
         assert (x.double() - w).norm() < 256 * 2 ** -24 * (w.norm() + w.numel() ** 0.5), name
 
 
+@pytest.mark.parametrize("D,H,Hkv,S", [(256, 8, 1, 513), (256, 2, 2, 1000), (200, 4, 4, 449), (136, 8, 4, 65), (128, 4, 2, 1025),
+                                       (96, 2, 2, 129), (64, 8, 1, 900), (24, 4, 4, 1000), (16, 32, 1, 130)])
+def test_backward_with_fixed_tiles_in_tensor_memory(D, H, Hkv, S):
+    """Rings that wrap twice, last blocks and tiles of one column or row, head widths off the 64-column pieces, against 64 bits.
+    P, dS and the results are rounded to bf16 (2^-9 each): the sums' relative error stays below two of them."""
+    from opentau_b200.ops import attention_native, cuda_ops
+    B = 2
+    g = torch.Generator(device="cuda").manual_seed(D + S)
+    q, k, v, do = (torch.randn(*shape, device="cuda", generator=g).to(torch.bfloat16)
+                   for shape in ((B, S, H, D), (B, S, Hkv, D), (B, S, Hkv, D), (B, S, H, D)))
+    blk = (torch.arange(S, device="cuda") - S // 2).clamp_min(0).expand(B, -1).int().contiguous()
+    valid = torch.ones(B, S, dtype=torch.bool, device="cuda")
+    valid[1, S - 7:] = False
+    o, lse = attention_native.attn_fwd(q, k, v, blk, blk, valid, valid, D ** -0.5)
+    do[~valid] = 0
+    got = attention_native.attn_bwd(do.view(B, S, -1), q, k, v, o, lse, blk, blk, valid, valid, D ** -0.5)
+    cuda_ops.check_status()
+    qd, kd, vd = (t.double().requires_grad_() for t in (q, k, v))
+    see = valid[:, None, :, None] & valid[:, None, None, :] & (blk[:, None, None, :] <= blk[:, None, :, None])
+    s = torch.einsum("bqhd,bkhd->bhqk", qd, kd.repeat_interleave(H // Hkv, 2)) * D ** -0.5
+    p = s.masked_fill(~see, -1e30).softmax(-1).masked_fill(~see, 0.0)
+    out = torch.einsum("bhqk,bkhd->bqhd", p, vd.repeat_interleave(H // Hkv, 2))
+    want = torch.autograd.grad(out, (qd, kd, vd), do.double())
+    for name, x, w in zip(("dq", "dk", "dv"), got, want):
+        assert _rel(x, w) < 2 ** -8, (name, _rel(x, w))
+
+
 @pytest.mark.parametrize("D,H,Hkv", [(256, 8, 1), (128, 8, 2), (64, 4, 4), (72, 16, 16)])
 @pytest.mark.parametrize("splits", [(2, 3, 2), (4, 16, 7)])
 def test_split_backward_matches_the_unsplit_one(D, H, Hkv, splits):
