@@ -883,52 +883,51 @@ __global__ void adamw_kernel(float* __restrict__ p32, const G* __restrict__ g, f
   }
 }
 
-// Same update, 8 elements per thread: 128-bit accesses on every stream (two per fp32 array, one per bf16 array)
-// and 8 independent loads in flight before the first use.  The launcher picks it when every pointer is 16-byte
-// aligned; the last n % 8 elements go through the scalar kernel.
-__device__ __forceinline__ void load8f(const float* p, float* v) {
-  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+// Same update, 4 elements per thread in 128-bit accesses.  The launcher picks it when every pointer is 16-byte aligned; the
+// last n % 4 elements go through the scalar kernel.
+__device__ __forceinline__ void load4g(const __nv_bfloat16* p, float* v) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
-__device__ __forceinline__ void store8f(float* p, const float* v) {
-  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-  *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+__device__ __forceinline__ void load4g(const float* p, float* v) {
+  *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
 }
-__device__ __forceinline__ void load8g(const __nv_bfloat16* p, float* v) { load8(p, v); }
-__device__ __forceinline__ void load8g(const float* p, float* v) { load8f(p, v); }
 
+// One block per 1024 elements: 28 bytes an element through HBM, 4.55 ms for 2^30 elements (6.6 TB/s, the copy's rate).  Eight
+// elements per thread of blocks that stride over the whole range keep more pages open: 5.58 ms; eight without the stride 5.47,
+// four with it 5.15.
 template <typename G>
-__global__ void __launch_bounds__(256) adamw_vec8_kernel(float* __restrict__ p32, const G* __restrict__ g,
+__global__ void __launch_bounds__(256) adamw_vec4_kernel(float* __restrict__ p32, const G* __restrict__ g,
                                                          float* __restrict__ m, float* __restrict__ v,
                                                          __nv_bfloat16* __restrict__ p16, long long nvec, float lr,
                                                          float beta1, float beta2, float eps, float wd, float bc1,
                                                          float bc2, const float* __restrict__ scale_ptr) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= nvec) return;
+  const long long i = t * 4;
+  float gr[4], pp[4], mm[4], vv[4];
+  load4g(g + i, gr);
+  *reinterpret_cast<float4*>(pp) = *reinterpret_cast<const float4*>(p32 + i);
+  *reinterpret_cast<float4*>(mm) = *reinterpret_cast<const float4*>(m + i);
+  *reinterpret_cast<float4*>(vv) = *reinterpret_cast<const float4*>(v + i);
   const float gs = scale_ptr ? scale_ptr[0] : 1.f;
   const float inv_bc1 = 1.f / bc1, inv_sqrt_bc2 = rsqrtf(bc2);
   const float decay = 1.f - lr * wd, step = lr * inv_bc1;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nvec;
-       t += (long long)gridDim.x * blockDim.x) {
-    const long long i = t * 8;
-    float gr[8], pp[8], mm[8], vv[8];
-    load8g(g + i, gr);
-    load8f(p32 + i, pp);
-    load8f(m + i, mm);
-    load8f(v + i, vv);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const float gk = gr[k] * gs;
-      float pk = pp[k] * decay;
-      mm[k] = beta1 * mm[k] + (1.f - beta1) * gk;
-      vv[k] = beta2 * vv[k] + (1.f - beta2) * gk * gk;
-      const float denom = sqrtf(vv[k]) * inv_sqrt_bc2 + eps;
-      pk -= step * mm[k] / denom;
-      pp[k] = pk;
-    }
-    store8f(p32 + i, pp);
-    store8f(m + i, mm);
-    store8f(v + i, vv);
-    if (p16) store8(p16 + i, pp);
+  for (int k = 0; k < 4; ++k) {
+    const float gk = gr[k] * gs;
+    float pk = pp[k] * decay;
+    mm[k] = beta1 * mm[k] + (1.f - beta1) * gk;
+    vv[k] = beta2 * vv[k] + (1.f - beta2) * gk * gk;
+    const float denom = sqrtf(vv[k]) * inv_sqrt_bc2 + eps;
+    pk -= step * mm[k] / denom;
+    pp[k] = pk;
   }
+  *reinterpret_cast<float4*>(p32 + i) = *reinterpret_cast<const float4*>(pp);
+  *reinterpret_cast<float4*>(m + i) = *reinterpret_cast<const float4*>(mm);
+  *reinterpret_cast<float4*>(v + i) = *reinterpret_cast<const float4*>(vv);
+  if (p16) *reinterpret_cast<uint2*>(p16 + i) = make_uint2(pack_bf16(pp[0], pp[1]), pack_bf16(pp[2], pp[3]));
 }
 
 // ------------------------------------------------------------------------------------------ images
@@ -1196,18 +1195,19 @@ extern "C" int otb_adamw(float* p32, const void* g, int g_is_bf16, float* m, flo
                          const float* scale_ptr, cudaStream_t stream) {
   auto aligned16 = [](const void* q) { return q == nullptr || (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   long long done = 0;
-  if (n >= 8 && aligned16(p32) && aligned16(g) && aligned16(m) && aligned16(v) && aligned16(p16)) {
-    const long long nvec = n / 8;
-    const int grid = grid_for(nvec, 256, 148 * 8);
-    if (g_is_bf16)
-      adamw_vec8_kernel<bf16><<<grid, 256, 0, stream>>>(p32, (const bf16*)g, m, v, (bf16*)p16, nvec, lr, beta1, beta2,
+  const long long most = 0x7fffffffll * 1024;            // blocks of a launch
+  if (aligned16(p32) && aligned16(g) && aligned16(m) && aligned16(v) && aligned16(p16)) {
+    const long long nvec = (n < most ? n : most) / 4;
+    const unsigned grid = (unsigned)((nvec + 255) / 256);
+    if (grid > 0 && g_is_bf16)
+      adamw_vec4_kernel<bf16><<<grid, 256, 0, stream>>>(p32, (const bf16*)g, m, v, (bf16*)p16, nvec, lr, beta1, beta2,
                                                         eps, wd, bc1, bc2, scale_ptr);
-    else
-      adamw_vec8_kernel<float><<<grid, 256, 0, stream>>>(p32, (const float*)g, m, v, (bf16*)p16, nvec, lr, beta1,
+    else if (grid > 0)
+      adamw_vec4_kernel<float><<<grid, 256, 0, stream>>>(p32, (const float*)g, m, v, (bf16*)p16, nvec, lr, beta1,
                                                          beta2, eps, wd, bc1, bc2, scale_ptr);
-    done = nvec * 8;
+    done = nvec * 4;
   }
-  const long long rest = n - done;       // everything when unaligned, else the last n % 8 elements
+  const long long rest = n - done;       // everything when unaligned, else the last n % 4 elements
   if (rest > 0) {
     const int grid = grid_for(rest, 512, 148 * 8);
     bf16* p16r = p16 ? (bf16*)p16 + done : nullptr;
