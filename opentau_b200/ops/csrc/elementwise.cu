@@ -379,12 +379,15 @@ __global__ void glu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat
   }
 }
 
+// One piece per thread without a stride over the rows: 9816 x 16384 takes 243 us (6.6 TB/s) against 256 with 2368 blocks that
+// stride.
 __global__ void glu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dh,
                                __nv_bfloat16* __restrict__ dgu, long long M, int I, int act) {
   const long long nvec = M * (long long)(I >> 3);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nvec;
        t += (long long)gridDim.x * blockDim.x) {
-    const long long row = t / (I >> 3);
+    // 32-bit division where it is enough: the 64-bit one is a hundred instructions
+    const long long row = nvec <= 0xffffffffLL ? (long long)((unsigned)t / (unsigned)(I >> 3)) : t / (I >> 3);
     const int c = int(t - row * (I >> 3)) * 8;
     const int blk = c >> 5, off = c & 31;
     const long long base = row * (2LL * I) + blk * 64 + off;
@@ -1082,7 +1085,7 @@ extern "C" int otb_glu_fwd(const void* gu, void* h, long long M, int I, int act,
 extern "C" int otb_glu_bwd(const void* gu, const void* dh, void* dgu, long long M, int I, int act,
                            cudaStream_t stream) {
   if (I % 32) return -1;
-  glu_bwd_kernel<<<grid_for(M * (I / 8), 256), 256, 0, stream>>>((const bf16*)gu, (const bf16*)dh, (bf16*)dgu, M, I,
+  glu_bwd_kernel<<<grid_for(M * (I / 8), 256, 1 << 30), 256, 0, stream>>>((const bf16*)gu, (const bf16*)dh, (bf16*)dgu, M, I,
                                                                  act);
   return (int)cudaGetLastError();
 }
