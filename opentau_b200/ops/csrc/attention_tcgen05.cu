@@ -27,7 +27,7 @@ namespace otb {
 constexpr unsigned KID_ATTN = 2;
 constexpr int ATT_M = 128;
 constexpr int CL_ROWS = 64;        // rows of a tile whose key blocks a cluster shares
-enum { SPLIT_GLOBAL = 0, SPLIT_CLUSTER = 1 };
+enum { SPLIT_GLOBAL = 0, SPLIT_CLUSTER = 1, SPLIT_TWO = 2 };     // SPLIT_TWO: no split, two CTAs per SM
 
 struct AttnParams {
   int B, Sq, Sk, H, Hkv, D, Dmma, g;
@@ -47,13 +47,20 @@ struct AttnParams {
   KernelStatus* status;
 };
 
-template <int DPAD, int BN>
+// TSP: P is written over the scores in tensor memory and is the A operand of the PV product from there.  Without P in shared
+// memory and with 64-wide blocks a CTA is 99 KB and 256 columns, so two share an SM: the softmax of one block is a chain of
+// tensor-memory reads, an exchange and exponentials that one CTA's eight warps leave three quarters open (ncu: issue slots 25 %
+// busy, tensor pipe 14 %, at 16 heads of 72).
+constexpr bool attn_tsp(int split) { return split == SPLIT_TWO; }
+
+template <int DPAD, int BN, int SPLIT>
 struct AttnSmem {
+  static constexpr bool TSP = attn_tsp(SPLIT);
   static constexpr int NCHUNK = DPAD / 64;
   static constexpr int Q_BYTES = ATT_M * DPAD * 2;
   static constexpr int KV_TILE = BN * DPAD * 2;        // one K or V tile
   static constexpr int STAGE_BYTES = 2 * KV_TILE;      // K and V of one block
-  static constexpr int P_BYTES = ATT_M * BN * 2;
+  static constexpr int P_BYTES = TSP ? 0 : ATT_M * BN * 2;
   static constexpr int OFF_Q = 0;
   static constexpr int OFF_KV = Q_BYTES;
   static constexpr int OFF_P = OFF_KV + 2 * STAGE_BYTES;
@@ -66,12 +73,14 @@ struct AttnSmem {
   // row's maximum and sum), mine of all rows, then the peers' of the rows I own
   static constexpr int PART_LD = DPAD + 4;
   static constexpr int OFF_PEER = CL_ROWS * PART_LD * 4;
-  static_assert(OFF_PEER + (CL_ROWS + 8) * PART_LD * 4 <= OFF_META, "the partials must fit over the operand tiles");
+  static_assert(SPLIT != SPLIT_CLUSTER || OFF_PEER + (CL_ROWS + 8) * PART_LD * 4 <= OFF_META, "the partials must fit over the operand tiles");
   static constexpr int USED = OFF_BAR + NBAR * 8 + 32;
   // room for rounding the base up to 1024 bytes (the kernel has no static shared memory, so the base normally is
   // aligned already); capped at the 227 KB a CTA may own, and checked at run time
   static constexpr int TOTAL = USED + 1024 <= 232448 ? USED + 1024 : 232448;
   static_assert(USED <= 232448, "shared memory budget");
+  static constexpr int TMEM_COLS = TSP ? 256 : 512;    // two S tiles, O
+  static_assert(2 * BN + DPAD <= TMEM_COLS, "tensor memory budget");
 };
 
 __device__ __forceinline__ float fast_exp2(float x) {
@@ -81,10 +90,11 @@ __device__ __forceinline__ float fast_exp2(float x) {
 }
 
 template <int DPAD, int BN, int SPLIT>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(320, attn_tsp(SPLIT) ? 2 : 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
                 const __grid_constant__ CUtensorMap tma_v, AttnParams p) {
-  using L = AttnSmem<DPAD, BN>;
+  using L = AttnSmem<DPAD, BN, SPLIT>;
+  constexpr bool TSP = L::TSP;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem + L::OFF_Q;
@@ -147,7 +157,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     tma_prefetch_desc(&tma_v);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 512);
+    tmem_alloc(tmem_slot, L::TMEM_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -240,7 +250,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       auto issue_qk = [&](int j) {
         const int slot = j & 1, u = j >> 1;
         mbar_wait(&kv_full[slot], u & 1, abort_flag, p.status, KID_ATTN, 2, j);
-        mbar_wait(&s_free[slot], (u & 1) ^ 1, abort_flag, p.status, KID_ATTN, 3, j);
+        // TSP: the scores of block j - 2 gave way to their P, and instructions run in the order they are issued
+        if (!TSP) mbar_wait(&s_free[slot], (u & 1) ^ 1, abort_flag, p.status, KID_ATTN, 3, j);
         tc_fence_after();
         const uint32_t k_addr = smem_u32(sKV + slot * L::STAGE_BYTES);
         for (int kk = 0; kk < ksteps_qk; ++kk) {
@@ -262,9 +273,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         const uint32_t v_addr = smem_u32(sKV + slot * L::STAGE_BYTES + L::KV_TILE);
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk) {
-          uint64_t ad = make_smem_desc(p_addr + (kk >> 2) * (ATT_M * 128) + (kk & 3) * 32, 16, 1024);
           uint64_t bd = make_smem_desc(v_addr + kk * 2048, BN * 128, 1024);
-          umma_ss(tmem_O, ad, bd, idesc_pv, (j | kk) != 0 ? 1u : 0u);
+          if (TSP) {
+            // each half of the columns was written over the first columns of its own scores
+            umma_ts(tmem_O, tmem_S + slot * BN + (kk / (BN / 32)) * (BN / 2) + (kk % (BN / 32)) * 8, bd, idesc_pv,
+                    (j | kk) != 0 ? 1u : 0u);
+          } else {
+            uint64_t ad = make_smem_desc(p_addr + (kk >> 2) * (ATT_M * 128) + (kk & 3) * 32, 16, 1024);
+            umma_ss(tmem_O, ad, bd, idesc_pv, (j | kk) != 0 ? 1u : 0u);
+          }
         }
         umma_commit(&kv_empty[slot]);
         umma_commit(&p_free[slot]);
@@ -337,14 +354,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       tmem_wait_ld();
 #pragma unroll
       for (int c = 0; c < NCH; ++c) {
+        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // four chains instead of one
         if (cls[c] == 2) {
 #pragma unroll
-          for (int e = 0; e < 32; ++e) mx = fmaxf(mx, __uint_as_float(r[c][e]));
+          for (int e = 0; e < 32; ++e) m4[e & 3] = fmaxf(m4[e & 3], __uint_as_float(r[c][e]));
         } else if (cls[c] == 1) {
 #pragma unroll
           for (int e = 0; e < 32; ++e)
-            if (km[c * 32 + e] <= qb) mx = fmaxf(mx, __uint_as_float(r[c][e]));
+            if (km[c * 32 + e] <= qb) m4[e & 3] = fmaxf(m4[e & 3], __uint_as_float(r[c][e]));
         }
+        mx = fmaxf(mx, fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));
       }
       mx *= scale;                                // scale > 0: max commutes with it
       red[half * ATT_M + row] = mx;
@@ -361,7 +380,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         m_used = m_new;
       }
       // P buffer `slot` was last read by PV(j-2)
-      if (j >= 2) mbar_wait(&p_free[slot], ((u - 1) & 1), abort_flag, p.status, KID_ATTN, 7, j);
+      if (!TSP && j >= 2) mbar_wait(&p_free[slot], ((u - 1) & 1), abort_flag, p.status, KID_ATTN, 7, j);
       if (any_want && j > 0) {
         // O may only be touched once PV(j-1) has retired
         const int ps = (j - 1) & 1, pu = (j - 1) >> 1;
@@ -409,6 +428,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
 #pragma unroll
           for (int e = 0; e < 16; ++e) packed[e] = 0u;
         }
+        if constexpr (TSP) {
+          static_assert(NCH == 1, "a thread's scores are one piece");
+          __syncwarp();
+          tmem_st_x16(s_addr, packed);
+          continue;
+        }
         // 32 keys = 64 bytes = four 16-byte units; unit index within the 128-byte row is XOR-swizzled
         const int col = c0 + c * 32;
         const int chunk = col / 64;                // 64-key chunk (16 KB apart)
@@ -422,9 +447,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       }
       l += lsum;
       // S buffer is free for QK(j+2); P is visible to the tensor core (async proxy)
-      tc_fence_before();
-      mbar_arrive(&s_free[slot]);
-      fence_async_smem();
+      if constexpr (TSP) {
+        tmem_wait_st();
+        tc_fence_before();
+      } else {
+        tc_fence_before();
+        mbar_arrive(&s_free[slot]);
+        fence_async_smem();
+      }
       mbar_arrive(&p_full[slot]);
     }
 
@@ -591,7 +621,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     }
     __syncwarp();
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, L::TMEM_COLS);
   }
 }
 
@@ -659,7 +689,7 @@ static int make_map4(CUtensorMap* m, const void* base, int D, int Hx, int S, int
 template <int DPAD, int BN, int SPLIT>
 static int launch_attn(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p,
                        cudaStream_t stream) {
-  using L = AttnSmem<DPAD, BN>;
+  using L = AttnSmem<DPAD, BN, SPLIT>;
   static bool configured = false;
   auto kern = attn_fwd_kernel<DPAD, BN, SPLIT>;
   if (!configured) {
@@ -682,6 +712,16 @@ static int launch_attn(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
 }  // namespace otb
 
 using namespace otb;
+
+static int sm_count() {
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  return sms;
+}
 
 // q: (B,Sq,H,D) strides (q_sb,q_ss,q_sh,1); k,v: (B,Sk,Hkv,D); o: (B,Sq,H,D) contiguous; lse: (B,H,Sq).
 static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, float* lse, const int* q_blk,
@@ -716,7 +756,12 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
   p.part_ml = reinterpret_cast<float2*>(part_ml);
   p.status = static_cast<KernelStatus*>(status);
   const int dpad = D <= 64 ? 64 : (D <= 128 ? 128 : 256);
-  const int bn = dpad == 256 ? 64 : 128;
+  // Head widths up to 128, more tiles than SMs: two CTAs per SM.  us inside a replayed graph, one CTA per SM against two: 16 heads
+  // of 72, 24 x 256 positions 52.3 / 34.4 (768 tiles), 3 x 1024 61.6 / 53.1, 8 x 256 18.6 / 13.2; 32 heads of 128 on 8, 2 x 2048
+  // 228.6 / 178.7, 700 31.2 / 23.1 (176 tiles); with a tile per SM there is nothing to share it with: 3 x 256 of 72 9.7 / 11.1 (96
+  // tiles), 300 of 128 11.0 / 13.3 (80)
+  const bool two = dpad <= 128 && nsplit == 1 && (long long)((Sq + ATT_M / g - 1) / (ATT_M / g)) * Hkv * B > sm_count();
+  const int bn = dpad == 256 || two ? 64 : 128;
   CUtensorMap tq, tk, tv;
   int r = make_map4(&tq, q, D, H, Sq, B, q_sh, q_ss, q_sb, g, (cluster ? CL_ROWS : ATT_M) / g);
   if (r) return 1000 + r;
@@ -727,8 +772,8 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
 #define RUN(DP, BLK) (cluster ? launch_attn<DP, BLK, SPLIT_CLUSTER>(tq, tk, tv, p, stream) \
                               : launch_attn<DP, BLK, SPLIT_GLOBAL>(tq, tk, tv, p, stream))
   switch (dpad) {
-    case 64: return RUN(64, 128);
-    case 128: return RUN(128, 128);
+    case 64: return two ? launch_attn<64, 64, SPLIT_TWO>(tq, tk, tv, p, stream) : RUN(64, 128);
+    case 128: return two ? launch_attn<128, 64, SPLIT_TWO>(tq, tk, tv, p, stream) : RUN(128, 128);
     default: return RUN(256, 64);
   }
 #undef RUN
@@ -757,7 +802,7 @@ extern "C" int otb_attn_fwd_splitkv(const void* q, const void* k, const void* v,
 
 template <int DPAD, int BN>
 static int max_clusters(int n) {
-  using L = AttnSmem<DPAD, BN>;
+  using L = AttnSmem<DPAD, BN, SPLIT_CLUSTER>;
   auto kern = attn_fwd_kernel<DPAD, BN, SPLIT_CLUSTER>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL) != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg;

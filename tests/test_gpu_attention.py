@@ -345,6 +345,29 @@ def test_fp32_attention_kernels_at_the_edges_of_their_tiles(D, Sq, cross, H, Hkv
         assert (x.double() - w).norm() < 256 * 2 ** -24 * (w.norm() + w.numel() ** 0.5), name
 
 
+@pytest.mark.parametrize("B,S,H,Hkv,D", [(4, 333, 16, 16, 72), (2, 1300, 8, 1, 128), (3, 200, 32, 32, 64), (5, 129, 16, 16, 24),
+                                         (2, 641, 16, 16, 96), (160, 65, 1, 1, 128)])
+def test_forward_with_two_tiles_per_sm(B, S, H, Hkv, D):
+    """More tiles than SMs up to width 128: probabilities in tensor memory, last blocks and tiles of one row, rows that see
+    nothing, against 64 bits.  Probabilities and results are rounded to bf16, 2^-9 each."""
+    from opentau_b200.ops import attention_native, cuda_ops
+    g = torch.Generator(device="cuda").manual_seed(D + S)
+    q, k, v = (torch.randn(B, S, h, D, device="cuda", generator=g).to(torch.bfloat16) for h in (H, Hkv, Hkv))
+    blk = (torch.arange(S, device="cuda") - S // 2).clamp_min(0).expand(B, -1).int().contiguous()
+    valid = torch.ones(B, S, dtype=torch.bool, device="cuda")
+    valid[1, S - 7:] = False
+    o, lse = attention_native.attn_fwd(q, k, v, blk, blk, valid, valid, D ** -0.5)
+    cuda_ops.check_status()
+    see = valid[:, None, :, None] & valid[:, None, None, :] & (blk[:, None, None, :] <= blk[:, None, :, None])
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double().repeat_interleave(H // Hkv, 2)) * D ** -0.5
+    s = s.masked_fill(~see, float("-inf"))
+    want = torch.einsum("bhqk,bkhd->bqhd", s.softmax(-1).nan_to_num(0.0), v.double().repeat_interleave(H // Hkv, 2))
+    assert _rel(o.view_as(q), want) < 2 ** -8
+    ref = torch.logsumexp(s, -1)
+    ref = torch.where(ref.isinf(), torch.zeros_like(ref), ref)
+    assert (lse.double() - ref).abs().max() < 1e-3
+
+
 @pytest.mark.parametrize("D,H,Hkv,S", [(256, 8, 1, 513), (256, 2, 2, 1000), (200, 4, 4, 449), (136, 8, 4, 65), (128, 4, 2, 1025),
                                        (96, 2, 2, 129), (64, 8, 1, 900), (24, 4, 4, 1000), (16, 32, 1, 130)])
 def test_backward_with_fixed_tiles_in_tensor_memory(D, H, Hkv, S):
