@@ -16,7 +16,7 @@
 //
 // Few query tiles against many keys (a denoising step or a decoded token against a cached prefix) share the key blocks of
 // a tile among `nsplit` CTAs.  Where the tiles are few enough (SPLIT_CLUSTER) those CTAs are one cluster and the partials
-// never leave the chip's shared memory: a tile holds 64 rows, every CTA leaves its fp32 partial (with the row's maximum
+// never leave the chip's shared memory: a tile holds 64 or 32 rows, every CTA leaves its fp32 partial (with the row's maximum
 // and sum behind it) in its own shared memory, sends each peer the rows that peer owns with one bulk copy, and merges its
 // own rows.  Otherwise (SPLIT_GLOBAL) the partials go to global memory and attn_combine_kernel merges them.
 #include "common.cuh"
@@ -26,7 +26,7 @@ namespace otb {
 
 constexpr unsigned KID_ATTN = 2;
 constexpr int ATT_M = 128;
-constexpr int CL_ROWS = 64;        // rows of a tile whose key blocks a cluster shares
+constexpr int CL_ROWS = 64;        // rows, at most, of a tile whose key blocks a cluster shares
 enum { SPLIT_GLOBAL = 0, SPLIT_CLUSTER = 1, SPLIT_TWO = 2 };     // SPLIT_TWO: no split, two CTAs per SM
 
 struct AttnParams {
@@ -42,6 +42,7 @@ struct AttnParams {
   // share of the key blocks and leaves an unnormalised partial; attn_combine_kernel merges the partials
   int skip_reach;                   // visit every key block: skip the prologue scan for the last reachable key
   int nsplit;                       // 1: write o / lse directly
+  int cl_rows;                      // SPLIT_CLUSTER: rows of a tile (32 or 64)
   float* part_o;                    // (nsplit, B, Sq, H, D) fp32, accumulators expressed against part m
   float2* part_ml;                  // (nsplit, B, H, Sq): (running maximum in log2 units, row sum)
   KernelStatus* status;
@@ -83,6 +84,10 @@ struct AttnSmem {
   static_assert(2 * BN + DPAD <= TMEM_COLS, "tensor memory budget");
 };
 
+__device__ __forceinline__ void l2_prefetch_4d(const CUtensorMap* m, int x, int y, int z, int w) {
+  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];"
+               ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -128,7 +133,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   const int tile = CL ? blockIdx.x : blockIdx.x / p.nsplit, split = CL ? (int)cluster_ctarank() : blockIdx.x % p.nsplit;
   const int kvh = CL ? blockIdx.y / p.nsplit : blockIdx.y, b = blockIdx.z;
   const int g = p.g;
-  constexpr int ROWS = CL ? CL_ROWS : ATT_M;
+  const int ROWS = CL ? p.cl_rows : ATT_M;
   const int pos_per_tile = ROWS / g;
   const int p0 = tile * pos_per_tile;
   // SPLIT_CLUSTER: the tile's valid rows, dealt to the CTAs in order; mine are [t0, t0 + own)
@@ -167,6 +172,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   const uint32_t tmem_S = tmem_base;            // two buffers of BN columns
   const uint32_t tmem_O = tmem_base + 2 * BN;   // Dmma columns
   pdl_launch_dependents();                      // after the TMEM allocation (see common.cuh)
+  if (CL && threadIdx.x == 0) {
+    // the cached keys and values have left L2 since the last pass: on their way while the preceding kernel finishes
+    const int all = (p.Sk + BN - 1) / BN, per = (all + p.nsplit - 1) / p.nsplit;
+    for (int j = split * per; j < min(all, (split + 1) * per); ++j)
+      for (int c = 0; c < L::NCHUNK; ++c) {
+        l2_prefetch_4d(&tma_k, c * 64, kvh, j * BN, b);
+        l2_prefetch_4d(&tma_v, c * 64, kvh, j * BN, b);
+      }
+  }
   pdl_wait();                                   // q / k / v and the masks come from the preceding kernels
 
   // ---- how many keys can this tile reach?  1 + the last key index j that is valid and has
@@ -697,7 +711,7 @@ static int launch_attn(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  const int pos_per_tile = (SPLIT == SPLIT_CLUSTER ? CL_ROWS : ATT_M) / p.g;
+  const int pos_per_tile = (SPLIT == SPLIT_CLUSTER ? p.cl_rows : ATT_M) / p.g;
   dim3 grid((p.Sq + pos_per_tile - 1) / pos_per_tile, p.Hkv, p.B);
   (SPLIT == SPLIT_CLUSTER ? grid.y : grid.x) *= p.nsplit;
   cudaError_t e = launch_pdl(kern, grid, dim3(320), (size_t)L::TOTAL, stream,
@@ -721,6 +735,40 @@ static int sm_count() {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   }
   return sms;
+}
+
+template <int DPAD, int BN>
+static int max_clusters(int n) {
+  using L = AttnSmem<DPAD, BN, SPLIT_CLUSTER>;
+  auto kern = attn_fwd_kernel<DPAD, BN, SPLIT_CLUSTER>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL) != cudaSuccess) return 0;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(1, (unsigned)n, 1);
+  cfg.blockDim = dim3(320);
+  cfg.dynamicSmemBytes = L::TOTAL;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 1;
+  attr.val.clusterDim.y = (unsigned)n;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  return cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess ? clusters : 0;
+}
+
+// whether `tiles` clusters of `n` CTAs are resident at once
+static bool cluster_fits(int D, int n, long long tiles) {
+  static int cap[3][9] = {};                         // -1: none
+  if (n < 1 || n > 8) return false;
+  const int which = D <= 64 ? 0 : (D <= 128 ? 1 : 2);
+  int c = cap[which][n];
+  if (c == 0) {
+    c = which == 0 ? max_clusters<64, 128>(n) : which == 1 ? max_clusters<128, 128>(n) : max_clusters<256, 64>(n);
+    cap[which][n] = c = c > 0 ? c : -1;
+  }
+  return tiles <= c;
 }
 
 // q: (B,Sq,H,D) strides (q_sb,q_ss,q_sh,1); k,v: (B,Sk,Hkv,D); o: (B,Sq,H,D) contiguous; lse: (B,H,Sq).
@@ -763,7 +811,11 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
   const bool two = dpad <= 128 && nsplit == 1 && (long long)((Sq + ATT_M / g - 1) / (ATT_M / g)) * Hkv * B > sm_count();
   const int bn = dpad == 256 || two ? 64 : 128;
   CUtensorMap tq, tk, tv;
-  int r = make_map4(&tq, q, D, H, Sq, B, q_sh, q_ss, q_sb, g, (cluster ? CL_ROWS : ATT_M) / g);
+  // 32-row tiles halve what a cluster's CTAs send one another, where twice the clusters are still resident at once (50 queries of
+  // 8 heads on 1, 1018 keys: 13 clusters, 10.2 -> 9.2 us; 16 queries, 400 keys: 8.9 -> 7.3)
+  p.cl_rows = CL_ROWS;
+  if (cluster && g <= 32 && cluster_fits(D, nsplit, ((long long)Sq * g + 31) / 32 * Hkv * B)) p.cl_rows = 32;
+  int r = make_map4(&tq, q, D, H, Sq, B, q_sh, q_ss, q_sb, g, (cluster ? p.cl_rows : ATT_M) / g);
   if (r) return 1000 + r;
   r = make_map4(&tk, k, D, Hkv, Sk, B, k_sh, k_ss, k_sb, 1, bn);
   if (r) return 2000 + r;
@@ -800,43 +852,14 @@ extern "C" int otb_attn_fwd_splitkv(const void* q, const void* k, const void* v,
                        k_ss, k_sh, v_sb, v_ss, v_sh, scale, nsplit, part_o, part_ml, status, stream);
 }
 
-template <int DPAD, int BN>
-static int max_clusters(int n) {
-  using L = AttnSmem<DPAD, BN, SPLIT_CLUSTER>;
-  auto kern = attn_fwd_kernel<DPAD, BN, SPLIT_CLUSTER>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL) != cudaSuccess) return 0;
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(1, (unsigned)n, 1);
-  cfg.blockDim = dim3(320);
-  cfg.dynamicSmemBytes = L::TOTAL;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = 1;
-  attr.val.clusterDim.y = (unsigned)n;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  int clusters = 0;
-  return cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess ? clusters : 0;
-}
-
 // CTAs per cluster for `tiles` tiles of 64 rows: the most (up to 8) whose clusters are all resident at once, since a second
 // round costs more than anything a larger cluster saves; 1 if that leaves fewer than 3.  Measured at 50 queries of 8 heads
 // on 1, width 256, against the merge through global memory: 10.5 us against 17.2 (7 tiles, 1018 keys, 8 CTAs), 12.5 against
 // 17.0 (28 tiles, 639 keys, 4), 16.9 against 19.7 (42 tiles, 900 keys, 3); pairs gain nothing (56 tiles: 20.4 against 20.2)
 // and clusters that do not fit lose (28 tiles with 8: 20.5).  One query: 7.6 against 11.4 us.
 extern "C" int otb_attn_cluster_fit(int D, long long tiles) {
-  static int cap[3][9] = {};                         // -1: none
-  const int which = D <= 64 ? 0 : (D <= 128 ? 1 : 2);
-  for (int n = 8; n >= 3; --n) {
-    int c = cap[which][n];
-    if (c == 0) {
-      c = which == 0 ? max_clusters<64, 128>(n) : which == 1 ? max_clusters<128, 128>(n) : max_clusters<256, 64>(n);
-      cap[which][n] = c = c > 0 ? c : -1;
-    }
-    if (tiles <= c) return n;
-  }
+  for (int n = 8; n >= 3; --n)
+    if (cluster_fits(D, n, tiles)) return n;
   return 1;
 }
 

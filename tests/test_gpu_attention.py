@@ -368,6 +368,29 @@ def test_forward_with_two_tiles_per_sm(B, S, H, Hkv, D):
     assert (lse.double() - ref).abs().max() < 1e-3
 
 
+@pytest.mark.parametrize("B,Sq,Sk,H,Hkv,D", [(1, 50, 1018, 8, 1, 256), (1, 60, 1018, 8, 1, 256), (1, 1, 700, 8, 1, 256),
+                                             (1, 50, 1074, 8, 4, 256), (2, 17, 400, 4, 2, 128), (1, 33, 322, 32, 1, 64),
+                                             (1, 3, 515, 64, 1, 64)])
+def test_cluster_tiles_of_32_and_64_rows(B, Sq, Sk, H, Hkv, D):
+    """Tiles whose keys a cluster shares, on both sides of the line between 32 and 64 rows, against 64 bits."""
+    from opentau_b200.ops import attention_native, cuda_ops
+    g = torch.Generator(device="cuda").manual_seed(Sq + Sk)
+    q, k, v = (torch.randn(B, n, h, D, device="cuda", generator=g).to(torch.bfloat16) for n, h in ((Sq, H), (Sk, Hkv), (Sk, Hkv)))
+    k_ok = torch.rand(B, Sk, device="cuda", generator=g) > 0.2
+    q_ok = torch.ones(B, Sq, dtype=torch.bool, device="cuda")
+    q_ok[-1, -1] = Sq == 1
+    zq, zk = (torch.zeros(B, n, dtype=torch.int32, device="cuda") for n in (Sq, Sk))
+    assert attention_native.split_cluster(B, Sq, Sk, H, Hkv, D) > 1
+    o, lse = attention_native.attn_fwd(q, k, v, zq, zk, q_ok, k_ok, D ** -0.5)
+    cuda_ops.check_status()
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double().repeat_interleave(H // Hkv, 2)) * D ** -0.5
+    s = s.masked_fill(~(q_ok[:, None, :, None] & k_ok[:, None, None]), float("-inf"))
+    want = torch.einsum("bhqk,bkhd->bqhd", s.softmax(-1).nan_to_num(0.0), v.double().repeat_interleave(H // Hkv, 2))
+    assert _rel(o.view_as(q), want) < 2 ** -8
+    ref = torch.logsumexp(s, -1)
+    assert (lse.double() - torch.where(ref.isinf(), torch.zeros_like(ref), ref)).abs().max() < 1e-3
+
+
 @pytest.mark.parametrize("D,H,Hkv,S", [(256, 8, 1, 513), (256, 2, 2, 1000), (200, 4, 4, 449), (136, 8, 4, 65), (128, 4, 2, 1025),
                                        (96, 2, 2, 129), (64, 8, 1, 900), (24, 4, 4, 1000), (16, 32, 1, 130)])
 def test_backward_with_fixed_tiles_in_tensor_memory(D, H, Hkv, S):
