@@ -333,6 +333,34 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
 
 static int g_sk_sms = 0;
 
+// Clusters of `n` CTAs that are resident at once, two CTAs to an SM (tokens tiles of at most 64).  A GPC's SMs do not divide
+// by every size: 30 clusters of eight, not 37.
+static int resident_clusters(int n) {
+  static int cap[9] = {};                            // -1: none
+  int& c = cap[n];
+  if (c == 0) {
+    auto kern = gemm_skinny_kernel<64, -1>;
+    int got = 0;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(1, (unsigned)n, 1);
+    cfg.blockDim = dim3(SK_THREADS);
+    cfg.dynamicSmemBytes = 111 * 1024;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 1;
+    attr.val.clusterDim.y = (unsigned)n;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&got, kern, &cfg) != cudaSuccess)
+      got = 0;
+    c = got > 0 ? got : -1;
+  }
+  return c > 0 ? c : 0;
+}
+
 template <int MAXT, int EPI>
 static int launch_skinny_epi(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyParams& p, int n_tiles, int chunks,
                          int smem_bytes, cudaStream_t stream) {
@@ -428,6 +456,21 @@ extern "C" int otb_gemm_skinny_bf16(const OtbSkinnyArgs* a, cudaStream_t stream)
     for (int s = 2; s <= 8; ++s) {
       const long long ctas = (long long)n_tiles * chunks * s;
       if (ctas <= slots && num_kb / s >= 2 && (ctas <= g_sk_sms || num_kb / s >= 4) && reduction_fits(nt, s)) splits = s;
+    }
+    // More than 64 rows: chunks of 64 instead, where that leaves two to four CTAs to a sum.  A CTA then sends a quarter of the
+    // partials (they set the pace at 200 tokens) and two share an SM; the weights are read once per chunk, from L2.  A pi0.5
+    // request with 200 rows (two such products a layer) 24.52 -> 23.16 ms, with 400 rows, where the persistent kernel and a
+    // gated residual of its own were the alternative, 22.4 -> 21.5; up to eight CTAs to a sum: 23.38 and 21.54, two: 24.65, 21.45.
+    if (M > 64) {
+      const int c64 = (M + 63) / 64;
+      const long long units = (long long)n_tiles * c64;
+      for (int s = 4; s >= 2; --s)
+        if (num_kb / s >= 4 && units * s <= 2LL * g_sk_sms && units <= resident_clusters(s)) {
+          splits = s;
+          chunks = c64;
+          nt = ((M + chunks - 1) / chunks + 15) / 16 * 16;
+          break;
+        }
     }
   }
   if (splits < 1 || splits > 8) return -8;

@@ -270,7 +270,9 @@ def rows_linear(x: Tensor, w: Tensor, bias: Tensor | None = None, *, norm: RowNo
         if bias.numel() != N or bias.dtype not in (torch.bfloat16, torch.float32):
             raise ValueError("bad bias for rows_linear")
         bias = bias.contiguous()
-    if not use_skinny("nt", R, N, False, 0, K, gate is not None):
+    # gated products of a few hundred rows keep the gate in the epilogue as well (chunks of 64 rows: 400 rows 22.4 -> 21.5 ms a request)
+    wide = SKINNY and gate is not None and R <= 640 and N <= 2048
+    if not wide and not use_skinny("nt", R, N, False, 0, K, gate is not None):
         if gate is not None:
             y = gemm(x, w, "nt", bias=bias)
             out = torch.empty_like(y)

@@ -582,3 +582,23 @@ def test_gated_mlp_at_65_to_256_rows_gates_the_fp32_sum(rows, cols, mlp, dev):
     for y in (got, one):
         assert (y.double() - want).norm() < 0.5 * 2 ** -8 * want.norm()
     cuda_ops.check_status()
+
+
+@pytest.mark.parametrize("R,N,K", [(65, 1024, 2048), (129, 1280, 1088), (200, 1024, 4096), (256, 1032, 2048), (257, 1024, 2048),
+                                   (400, 1024, 4096), (600, 1280, 5120), (640, 2048, 512), (641, 1024, 2048)])
+def test_gated_rows_in_chunks(R, N, K, dev):
+    """More than 64 rows run as chunks of at most 64: ragged last chunks, odd column tiles, sums that several CTAs share.  The
+    gate multiplies the fp32 sum, so only the one rounding to bf16 (2^-9) is left."""
+    from opentau_b200.ops import cuda_ops
+    g = torch.Generator(device="cuda").manual_seed(R + N)
+    x, w, res = (torch.randn(*s, device=dev, generator=g).to(torch.bfloat16) for s in ((R, K), (N, K), (R, N)))
+    mod = torch.randn(3, 3 * N, device=dev, generator=g).to(torch.bfloat16)
+    idx = torch.randint(0, 3, (R,), device=dev, generator=g).to(torch.int32)
+    norm = cuda_ops.RowNorm(1e-6, mod=mod, idx=idx)
+    before = cuda_ops.launch_count
+    got = cuda_ops.rows_linear(x, w, residual=res, gated_by=norm)
+    assert (cuda_ops.launch_count - before == 1) == (R <= 640)
+    cuda_ops.check_status()
+    want = res.double() + mod.double()[idx.long(), 2 * N:] * (x.double() @ w.double().T)
+    assert (got.double() - want).norm() < (2 ** -8 if R <= 640 else 2 ** -7) * want.norm()
+    assert torch.equal(got, cuda_ops.rows_linear(x, w, residual=res, gated_by=norm))
