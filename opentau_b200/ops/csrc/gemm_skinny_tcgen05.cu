@@ -436,8 +436,8 @@ extern "C" int otb_gemm_skinny_bf16(const OtbSkinnyArgs* a, cudaStream_t stream)
     cudaDeviceGetAttribute(&g_sk_sms, cudaDevAttrMultiProcessorCount, dev);
     if (g_sk_sms <= 0) return -7;
   }
-  // Tokens per CTA: as few chunks of at most 256 as cover M, all of one size (a multiple of the MMA's 16): 200 rows run
-  // as one 208-token tile, 400 as two, instead of padding to powers of two.
+  // Tokens per CTA: as few chunks of at most 256 as cover M, all of one size (a multiple of the MMA's 16) instead of padding
+  // to powers of two; where a sum is shared, chunks of 64 may take their place (below).
   int chunks = (M + 255) / 256;
   int nt = ((M + chunks - 1) / chunks + 15) / 16 * 16;
   // my partial tile (over the ring) and the peers' partials of my tokens must fit side by side
