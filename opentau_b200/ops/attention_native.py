@@ -147,6 +147,8 @@ def attn_bwd(do: Tensor, q: Tensor, k: Tensor, v: Tensor, o: Tensor, lse: Tensor
     q, k, v = _prep(q), _prep(k), _prep(v)
     o = o.contiguous()
     do = do.contiguous()
+    if do.data_ptr() % 16:                                      # a gradient may be any view; the kernels read 16 bytes at a time
+        do = do.clone()
     lse = lse.contiguous()
     dq = torch.empty(B, Sq, H, D, dtype=q.dtype, device=q.device)
     dk = torch.empty(B, Sk, Hkv, D, dtype=q.dtype, device=q.device)

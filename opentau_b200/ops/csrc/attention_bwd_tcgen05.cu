@@ -792,6 +792,10 @@ extern "C" int otb_attn_bwd(const void* q, const void* k, const void* v, const v
   const long long strides[9] = {q_sb, q_ss, q_sh, k_sb, k_ss, k_sh, v_sb, v_ss, v_sh};
   for (int i = 0; i < 9; ++i)
     if (strides[i] % 8) return -5;
+  // rows are read and written in 128-bit pieces by the kernels themselves, not only through tensor maps
+  const void* const bases[8] = {q, k, v, o, d_o, dq, dk, dv};
+  for (int i = 0; i < 8; ++i)
+    if (reinterpret_cast<uintptr_t>(bases[i]) & 15) return -6;
   const int splits[3] = {dq_splits, dk_splits, dv_splits};
   float* const parts[3] = {dq_parts, dk_parts, dv_parts};
   for (int i = 0; i < 3; ++i)

@@ -273,3 +273,18 @@ def test_fp32_attention_rule_follows_the_padding():
                  (64, 300, 300, 8, 8, 64), (1, 50, 1000, 8, 1, 256), (8, 1, 1000, 16, 16, 72), (16, 601, 601, 16, 16, 72),
                  (4, 1227, 1227, 32, 8, 128)):
         assert pay(*size, False) and pay(*size, True), size
+
+
+@pytest.mark.parametrize("which", range(8))
+def test_attention_backward_refuses_misaligned_tensors_before_any_launch(which):
+    """The bf16 backward reads and writes 16 bytes at a time: q, k, v, o, dO, dQ, dK and dV that start elsewhere are refused on the
+    host (the addresses here are numbers that nothing may look at)."""
+    from opentau_b200.ops import attention_native, build
+    if not build.lib_path("attention_bwd_tcgen05").exists():
+        pytest.skip("native libraries are not built")
+    fn = attention_native._entry("attention_bwd_tcgen05", "otb_attn_bwd", 13 * "p" + 3 * "i" + 4 * "p" + 6 * "i" + 9 * "l" + "fpp")
+    base = [1 << 20] * 10                                   # q k v o dO lse delta dQ dK dV
+    base[(0, 1, 2, 3, 4, 7, 8, 9)[which]] += 8
+    B, S, H, D = 1, 64, 4, 64
+    strides = (S * H * D, H * D, D) * 3
+    assert fn(*base, 0, 0, 0, 1, 1, 1, *[1 << 20] * 4, B, S, S, H, H, D, *strides, 0.125, 0, 0) == -6
