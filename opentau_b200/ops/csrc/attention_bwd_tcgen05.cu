@@ -285,8 +285,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_f2, const __grid_constant
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    // Instructions of one CTA run in the order they are issued, so dP of block j + 1 (and, with two S tiles, S of block
-    // j + 2) may be issued straight behind the accumulation that reads dS (P) of block j from the same columns.
+    // dP of block j + 1 (with two S tiles: S of block j + 1) goes over the columns that held dS of block j (P of j - 1).
+    // Only instructions with one accumulator and shape are promised to run in the order they are issued, so it waits for
+    // the commit of the accumulation that reads them.
     if (elect_one()) {
       const uint32_t idesc_s = make_idesc_bf16(BW_M, BN, 0, 0);
       const uint32_t idesc_acc = make_idesc_bf16(BW_M, p.Dmma, 0, 1);
@@ -302,7 +303,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_f2, const __grid_constant
       uint32_t ph1 = 0, ph2 = 0;
       auto issue_s = [&](int j) {
         mbar_wait(&y1_full[s1], ph1, abort_flag, p.status, KID_ATTN_BWD, 2, j);
-        if (L::TWO && j > 0) mbar_wait(s_free, (j - 1) & 1, abort_flag, p.status, KID_ATTN_BWD, 3, j);
+        if (L::TWO) {
+          if (j > 0) mbar_wait(s_free, (j - 1) & 1, abort_flag, p.status, KID_ATTN_BWD, 3, j);
+        } else if (j > 1) {
+          mbar_wait(&y2_empty[(j - 2) % L::NY2], ((j - 2) / L::NY2) & 1, abort_flag, p.status, KID_ATTN_BWD, 12, j);
+        }
         tc_fence_after();
         const int buf = L::TWO ? 0 : (j & 1);
         scores_tmem(tmem_base + L::TM_S + buf * BN, tmem_base + L::TM_F1, smem_u32(sY1 + s1 * L::Y_BYTES));
@@ -312,6 +317,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_f2, const __grid_constant
       };
       auto issue_dp = [&](int j) {
         mbar_wait(&y2_full[s2], ph2, abort_flag, p.status, KID_ATTN_BWD, 10, j);
+        if (j > 0) mbar_wait(&y1_empty[(j - 1) % L::NY1], ((j - 1) / L::NY1) & 1, abort_flag, p.status, KID_ATTN_BWD, 13, j);
         tc_fence_after();
         const uint32_t y = smem_u32(sY2 + s2 * L::Y_BYTES), d = tmem_base + L::TM_DP;
         if (L::F2_TMEM) {

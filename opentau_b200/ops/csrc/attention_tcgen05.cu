@@ -264,7 +264,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       auto issue_qk = [&](int j) {
         const int slot = j & 1, u = j >> 1;
         mbar_wait(&kv_full[slot], u & 1, abort_flag, p.status, KID_ATTN, 2, j);
-        // TSP: the scores of block j - 2 gave way to their P, and instructions run in the order they are issued
+        // TSP: the scores of block j - 2 gave way to their P.  Block j's keys are in the slot of block j - 2, which the
+        // producer filled behind the commit of the PV product that read that P: kv_full stands for both
         if (!TSP) mbar_wait(&s_free[slot], (u & 1) ^ 1, abort_flag, p.status, KID_ATTN, 3, j);
         tc_fence_after();
         const uint32_t k_addr = smem_u32(sKV + slot * L::STAGE_BYTES);
