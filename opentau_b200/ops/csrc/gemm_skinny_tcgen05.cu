@@ -31,6 +31,7 @@ constexpr int SK_UMMA_K = 16;
 constexpr int SK_THREADS = 320;
 constexpr int SK_WORKERS = 256;
 constexpr int SK_MAX_STAGES = 12;
+constexpr int SK_TAIL = 1024 /* barriers */ + 1024 /* alignment */;
 
 enum SkinnyFlags {  // same values as the big GEMM's epilogue flags
   SK_BIAS = 1,
@@ -333,19 +334,19 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
 
 static int g_sk_sms = 0;
 
-// Clusters of `n` CTAs that are resident at once, two CTAs to an SM (tokens tiles of at most 64).  A GPC's SMs do not divide
-// by every size: 30 clusters of eight, not 37.
+// Clusters of `n` CTAs that are resident at once with one CTA to an SM (a GPC's SMs do not divide by every size: 15 of eight
+// on a B200, not 18).  Token tiles of at most 64 put two to an SM, which the query does not count.
 static int resident_clusters(int n) {
   static int cap[9] = {};                            // -1: none
   int& c = cap[n];
   if (c == 0) {
-    auto kern = gemm_skinny_kernel<64, -1>;
+    auto kern = gemm_skinny_kernel<256, -1>;
     int got = 0;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(1, (unsigned)n, 1);
     cfg.blockDim = dim3(SK_THREADS);
-    cfg.dynamicSmemBytes = 111 * 1024;
+    cfg.dynamicSmemBytes = 224 * 1024;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = 1;
@@ -359,6 +360,84 @@ static int resident_clusters(int n) {
     c = got > 0 ? got : -1;
   }
   return c > 0 ? c : 0;
+}
+
+// How a product is dealt out: token chunks of `nt` (a multiple of the MMA's 16) and the CTAs that share a sum over K.
+struct SkinnyPlan {
+  int chunks, nt, splits, stages;
+  int stage_bytes, ring, buf_bytes;    // shared memory: a stage; ring or my partial tile, whichever is larger; the peers' partials
+};
+
+// Fills in chunks, token tile and shared memory for `chunks` and `splits`; false where they do not fit.  The ring is as deep as
+// the CTA's k-blocks need or the budget gives (my own partial overlays it), the peers' partials lie behind it, then barriers.
+// 111 KB keeps two CTAs on an SM while there are at most 64 tokens; wider tiles take the SM alone.
+static bool layout_plan(int M, int K, int chunks, int splits, SkinnyPlan* p) {
+  const int nt = ((M + chunks - 1) / chunks + 15) / 16 * 16;
+  const int num_kb = (K + SK_BK - 1) / SK_BK, per = (num_kb + splits - 1) / splits;
+  p->chunks = (M + nt - 1) / nt;
+  p->nt = nt;
+  p->splits = splits;
+  p->stage_bytes = (SK_BW * SK_BK * 2 + nt * SK_BK * 2 + 1023) / 1024 * 1024;
+  const int tile_bytes = (nt <= 64 ? nt : (nt + 31) / 32 * 32) * SK_BW * 4;
+  p->buf_bytes = (nt + splits - 1) / splits * SK_BW * 4 * (splits - 1);
+  const int room = (nt > 64 ? 224 : 111) * 1024 - SK_TAIL - p->buf_bytes;
+  int stages = room / p->stage_bytes;
+  if (stages > per) stages = per;
+  if (stages > SK_MAX_STAGES) stages = SK_MAX_STAGES;
+  p->stages = stages;
+  p->ring = stages * p->stage_bytes > tile_bytes ? stages * p->stage_bytes : tile_bytes;
+  return nt <= 256 && stages >= 1 && tile_bytes <= room;
+}
+
+// The plan of an M x N x K product on `sms` SMs; clusters(n): clusters of n CTAs resident at once, one CTA to an SM.
+//
+// Up to 64 rows: one token tile, and the largest cluster size whose grid is resident at once and leaves every CTA two k-blocks;
+// going beyond ONE CTA per SM only pays while each CTA still streams four k-blocks (a launch of two-k-block CTAs that fills every
+// SM twice keeps the next kernel of the chain from becoming resident early).
+//
+// More rows: of the token tiles from 32 to 256 and 1 to 8 CTAs to a sum, the cheapest that is resident at once.  A CTA
+// pays for its k-blocks, for every round of the ring behind the first, for the partials it sends, for its own tokens' epilogue,
+// and the launch for its CTAs: microseconds fitted to 3400 resident plans at 65 - 640 rows, 128 - 2048 columns, K 256 - 8192 inside a
+// replayed graph with cold weights (rms error 6 %; the plan taken costs 1.5 % more than the best one in the mean, 13 % at most).
+// The weights are read once per chunk, from L2.  With the norm behind them, us, against one tile of up to 256 rows and
+// against chunks of 64 that two to four CTAs share (what ran before): 100 x 1024 x 4096 9.3 / 11.2 -> 8.0, 200 x 1024 x 4096 15.1 /
+// 12.2 -> 9.7, 256 x 1280 x 5120 31.8 / 16.4 -> 12.5, 200 x 128 x 256 13.8 / 13.8 -> 4.7.
+template <typename F>
+static bool choose_plan(int M, int N, int K, int sms, F clusters, SkinnyPlan* best) {
+  const int n_tiles = (N + SK_BW - 1) / SK_BW, num_kb = (K + SK_BK - 1) / SK_BK;
+  const int one = (M + 255) / 256;
+  if (M <= 64) {
+    int splits = 1;
+    for (int s = 2; s <= 8; ++s) {
+      const long long ctas = (long long)n_tiles * s;
+      if (ctas <= 2LL * sms && num_kb / s >= 2 && (ctas <= sms || num_kb / s >= 4)) splits = s;
+    }
+    return layout_plan(M, K, one, splits, best);
+  }
+  bool found = false;
+  double best_cost = 0.0;
+  for (int nt = 256, last = 0; nt >= 32; nt -= 16) {
+    const int chunks = (M + nt - 1) / nt;
+    if (chunks == last) continue;
+    last = chunks;
+    for (int s = 1; s <= 8; ++s) {
+      SkinnyPlan c;
+      const int per = (num_kb + s - 1) / s;
+      if ((s - 1) * per >= num_kb || !layout_plan(M, K, chunks, s, &c)) continue;
+      const long long units = (long long)n_tiles * c.chunks;
+      // the last places do not fill: 26 clusters of five of 80 tokens, or 90 of three of 48, took a second round
+      if (units > (c.nt <= 64 ? 2LL * clusters(s) - 2 : clusters(s) - (s > 2 ? 1LL : 0LL))) continue;
+      const double cost = per * (0.05 + 0.0004 * c.nt) + 0.8 * (per > c.stages ? (double)(per - c.stages) / c.stages : 0.0) +
+                          0.03 * c.nt * (s - 1) / s + 0.075 * ((c.nt + s - 1) / s) + 1.25 * (double)(units * s) / sms;
+      if (!found || cost < best_cost) {
+        found = true;
+        best_cost = cost;
+        *best = c;
+      }
+    }
+  }
+  // more CTAs than the chip holds whatever the tile: the widest tiles
+  return found || layout_plan(M, K, one, 1, best);
 }
 
 template <int MAXT, int EPI>
@@ -412,8 +491,22 @@ struct OtbSkinnyArgs {
   int rows_per_gate, flags, splits;
 };
 
+// The plan that a launch with `splits` 0 takes, for `sms` SMs that hold clusters[n] clusters of n CTAs (null: of this device).
+// plan: token chunks, tokens per CTA, CTAs to a sum, stages of the ring, bytes of shared memory.
+extern "C" int otb_gemm_skinny_plan(int M, int N, int K, int sms, const int* clusters, int* plan) {
+  if (M <= 0 || N <= 0 || K <= 0 || sms <= 0) return -2;
+  SkinnyPlan p;
+  if (!choose_plan(M, N, K, sms, [&](int n) { return clusters != nullptr ? clusters[n] : resident_clusters(n); }, &p)) return -13;
+  plan[0] = p.chunks;
+  plan[1] = p.nt;
+  plan[2] = p.splits;
+  plan[3] = p.stages;
+  plan[4] = p.ring + p.buf_bytes + SK_TAIL;
+  return 0;
+}
+
 // out[M,N] = X[M,K] W[N,K]^T (+ epilogue).  Returns 0, a CUDA / driver error code, or a negative argument-check
-// code.  `splits`: 0 = choose (see the rule at the selection below).
+// code.  `splits`: 0 = choose (choose_plan).
 extern "C" int otb_gemm_skinny_bf16(const OtbSkinnyArgs* a, cudaStream_t stream) {
   const int M = a->M, N = a->N, K = a->K, flags = a->flags;
   if (M <= 0 || N <= 0 || K <= 0 || (N % 8)) return -2;
@@ -436,67 +529,22 @@ extern "C" int otb_gemm_skinny_bf16(const OtbSkinnyArgs* a, cudaStream_t stream)
     cudaDeviceGetAttribute(&g_sk_sms, cudaDevAttrMultiProcessorCount, dev);
     if (g_sk_sms <= 0) return -7;
   }
-  // Tokens per CTA: as few chunks of at most 256 as cover M, all of one size (a multiple of the MMA's 16) instead of padding
-  // to powers of two; where a sum is shared, chunks of 64 may take their place (below).
-  int chunks = (M + 255) / 256;
-  int nt = ((M + chunks - 1) / chunks + 15) / 16 * 16;
-  // my partial tile (over the ring) and the peers' partials of my tokens must fit side by side
-  const auto reduction_fits = [](int tokens, int s) {
-    return (((tokens + 31) / 32 * 32) + (tokens + s - 1) / s * (s - 1)) * SK_BW * 4 <= 222 * 1024;
-  };
+  SkinnyPlan plan;
+  if (a->splits < 0 || a->splits > 8) return -8;
+  bool ok;
+  if (a->splits == 0) {
+    ok = choose_plan(M, N, K, g_sk_sms, resident_clusters, &plan);
+  } else {
+    // a forced split: as few chunks of at most 256 as cover M, narrower where the partials do not fit side by side
+    ok = layout_plan(M, K, (M + 255) / 256, a->splits, &plan) || layout_plan(M, K, (M + 127) / 128, a->splits, &plan);
+  }
+  if (!ok) return -13;
   const int n_tiles = (N + SK_BW - 1) / SK_BW;
-  const int num_kb = (K + SK_BK - 1) / SK_BK;
-  int splits = a->splits;
-  if (splits == 0) {
-    // Largest cluster size whose grid is resident at once and leaves every CTA two k-blocks; going beyond ONE CTA per
-    // SM only pays while each CTA still streams four k-blocks (a launch of two-k-block CTAs that fills every SM twice
-    // keeps the next kernel of the chain from becoming resident early).
-    const long long slots = (long long)g_sk_sms * (nt <= 64 ? 2 : 1);
-    splits = 1;
-    for (int s = 2; s <= 8; ++s) {
-      const long long ctas = (long long)n_tiles * chunks * s;
-      if (ctas <= slots && num_kb / s >= 2 && (ctas <= g_sk_sms || num_kb / s >= 4) && reduction_fits(nt, s)) splits = s;
-    }
-    // More than 64 rows: chunks of 64 instead, where that leaves two to four CTAs to a sum.  A CTA then sends a quarter of the
-    // partials (they set the pace at 200 tokens) and two share an SM; the weights are read once per chunk, from L2.  A pi0.5
-    // request with 200 rows (two such products a layer) 24.52 -> 23.16 ms, with 400 rows, where the persistent kernel and a
-    // gated residual of its own were the alternative, 22.4 -> 21.5; up to eight CTAs to a sum: 23.38 and 21.54, two: 24.65, 21.45.
-    if (M > 64) {
-      const int c64 = (M + 63) / 64;
-      const long long units = (long long)n_tiles * c64;
-      for (int s = 4; s >= 2; --s)
-        if (num_kb / s >= 4 && units * s <= 2LL * g_sk_sms && units <= resident_clusters(s)) {
-          splits = s;
-          chunks = c64;
-          nt = ((M + chunks - 1) / chunks + 15) / 16 * 16;
-          break;
-        }
-    }
-  }
-  if (splits < 1 || splits > 8) return -8;
-  if (!reduction_fits(nt, splits)) {                          // a forced split: narrower token tiles
-    chunks = (M + 127) / 128;
-    nt = ((M + chunks - 1) / chunks + 15) / 16 * 16;
-  }
-  // Shared memory: the ring (as deep as the CTA's k-blocks need or the budget gives; my own partial overlays it), the
-  // peers' partials behind it, barriers.  111 KB keeps two CTAs on an SM while there are at most 64 tokens;
-  // wider tiles take the SM alone.
-  const int stage_bytes = (SK_BW * SK_BK * 2 + nt * SK_BK * 2 + 1023) / 1024 * 1024;
-  const int tile_bytes = (nt <= 64 ? nt : (nt + 31) / 32 * 32) * SK_BW * 4;   // my partial tile, over the ring
-  const int buf_bytes = (nt + splits - 1) / splits * SK_BW * 4 * (splits - 1);
-  const int budget = nt > 64 ? 224 * 1024 : 111 * 1024;
-  const int tail = 1024 /* barriers */ + 1024 /* alignment */;
-  const int tile_over = tile_bytes > budget - tail - buf_bytes;
-  const int per = (num_kb + splits - 1) / splits;
-  int stages = (budget - tail - buf_bytes) / stage_bytes;
-  if (stages > per) stages = per;
-  if (stages > SK_MAX_STAGES) stages = SK_MAX_STAGES;
-  if (stages < 1 || tile_over) return -13;
-  const int ring = stages * stage_bytes > tile_bytes ? stages * stage_bytes : tile_bytes;
+  const int chunks = plan.chunks, nt = plan.nt, splits = plan.splits;
   SkinnyParams p;
-  p.buf_offset = ring;
-  p.bar_offset = ring + buf_bytes;
-  const int smem_bytes = p.bar_offset + tail;
+  p.buf_offset = plan.ring;
+  p.bar_offset = plan.ring + plan.buf_bytes;
+  const int smem_bytes = p.bar_offset + SK_TAIL;
   CUtensorMap tw, tx;
   {
     uint64_t dims[2], strides[1];
@@ -520,9 +568,9 @@ extern "C" int otb_gemm_skinny_bf16(const OtbSkinnyArgs* a, cudaStream_t stream)
   p.mod_idx = a->mod_idx;
   p.flags = flags;
   p.splits = splits;
-  p.stages = stages;
+  p.stages = plan.stages;
   p.nt = nt;
-  p.stage_bytes = stage_bytes;
+  p.stage_bytes = plan.stage_bytes;
   p.tmem_cols = nt <= 32 ? 32 : (nt <= 64 ? 64 : (nt <= 128 ? 128 : 256));
   p.status = static_cast<KernelStatus*>(a->status);
   if (nt <= 64) return launch_skinny<64>(tw, tx, p, n_tiles, chunks, smem_bytes, stream);

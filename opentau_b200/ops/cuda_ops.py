@@ -72,8 +72,10 @@ def use_skinny(layout: str, M: int, N: int, accumulate: bool, bn: int, K: int = 
         return False
     if gated:
         # the alternative rounds the sum to bf16 in front of the gate: every few-row product keeps the fusion, but for
-        # more columns than the 128 x 256 tiles of the persistent kernel need to fill the chip
-        return M <= 128 or (M <= 256 and N <= 8192)
+        # more columns than the 128 x 256 tiles of the persistent kernel need to fill the chip.  Up to 640 rows where two CTAs
+        # may share the sums of 64-row chunks: 400 x 1024 x 4096 20.5 -> 12.6 us with the norm behind it against the persistent
+        # kernel and a gated residual of its own, 640 x 1280 x 2048 14.8 -> 12.4; without the room 600 x 2048 x 2048 16.3 -> 17.3
+        return M <= 128 or (M <= 256 and N <= 8192) or (M <= 640 and N <= 2048 and -(-N // 128) * -(-M // 64) <= 148)
     # measured inside a replayed graph: up to 64 rows the split-K kernel always wins (50 x 8192 x 1024 6.4 us against
     # 9.1, 50 x 1024 x 4096 6.0 against 16.2); at 65..256 rows only where the persistent kernel has too few tiles for the
     # chip and a long sum (200 x 1024 x 4096 12.8 us against 16.3, but 200 x 1024 x 2048 11.5 against 9.8 and 256 x 768 x 768
@@ -270,9 +272,7 @@ def rows_linear(x: Tensor, w: Tensor, bias: Tensor | None = None, *, norm: RowNo
         if bias.numel() != N or bias.dtype not in (torch.bfloat16, torch.float32):
             raise ValueError("bad bias for rows_linear")
         bias = bias.contiguous()
-    # gated products of a few hundred rows keep the gate in the epilogue as well (chunks of 64 rows: 400 rows 22.4 -> 21.5 ms a request)
-    wide = SKINNY and gate is not None and R <= 640 and N <= 2048
-    if not wide and not use_skinny("nt", R, N, False, 0, K, gate is not None):
+    if not use_skinny("nt", R, N, False, 0, K, gate is not None):
         if gate is not None:
             y = gemm(x, w, "nt", bias=bias)
             out = torch.empty_like(y)

@@ -257,7 +257,7 @@ def test_adamw_and_clip_kernels(dev):
 @pytest.mark.parametrize("offset,grad_dtype,with_p16", [(0, torch.bfloat16, True), (1, torch.bfloat16, True),
                                                           (0, torch.float32, False), (4, torch.float32, True)])
 def test_adamw_vector_and_scalar_paths_agree_with_reference(dev, offset, grad_dtype, with_p16):
-    """Aligned buffers take the 8-wide kernel plus a scalar tail; views that start off a 16-byte boundary take the
+    """Aligned buffers take the 4-wide kernel plus a scalar tail; views that start off a 16-byte boundary take the
     scalar kernel for everything.  Both must give the fp32 reference."""
     from opentau_b200.ops import cuda_ops
     from opentau_b200.ops import reference as ref
@@ -585,11 +585,14 @@ def test_gated_mlp_at_65_to_256_rows_gates_the_fp32_sum(rows, cols, mlp, dev):
 
 
 @pytest.mark.parametrize("R,N,K", [(65, 1024, 2048), (129, 1280, 1088), (200, 1024, 4096), (256, 1032, 2048), (257, 1024, 2048),
-                                   (400, 1024, 4096), (600, 1280, 5120), (640, 2048, 512), (641, 1024, 2048)])
+                                   (400, 1024, 4096), (600, 1280, 5120), (640, 2048, 512), (576, 2048, 512), (641, 1024, 2048),
+                                   (128, 1280, 5120), (300, 128, 256), (250, 4096, 2048)])
 def test_gated_rows_in_chunks(R, N, K, dev):
-    """More than 64 rows run as chunks of at most 64: ragged last chunks, odd column tiles, sums that several CTAs share.  The
-    gate multiplies the fp32 sum, so only the one rounding to bf16 (2^-9) is left."""
-    from opentau_b200.ops import cuda_ops
+    """Chunks of a few rows whose sums several CTAs share: ragged last chunks, odd column tiles, the edges of what is fused.  The
+    gate multiplies the fp32 sum there, so only the one rounding to bf16 (2^-9) is left."""
+    import ctypes
+
+    from opentau_b200.ops import _lib, cuda_ops
     g = torch.Generator(device="cuda").manual_seed(R + N)
     x, w, res = (torch.randn(*s, device=dev, generator=g).to(torch.bfloat16) for s in ((R, K), (N, K), (R, N)))
     mod = torch.randn(3, 3 * N, device=dev, generator=g).to(torch.bfloat16)
@@ -597,8 +600,17 @@ def test_gated_rows_in_chunks(R, N, K, dev):
     norm = cuda_ops.RowNorm(1e-6, mod=mod, idx=idx)
     before = cuda_ops.launch_count
     got = cuda_ops.rows_linear(x, w, residual=res, gated_by=norm)
-    assert (cuda_ops.launch_count - before == 1) == (R <= 640)
+    fused = R <= 640 and (N, R) != (2048, 640)
+    assert (cuda_ops.launch_count - before == 1) == fused == cuda_ops.use_skinny("nt", R, N, False, 0, K)
+    if fused and N <= 2048:                                    # this device's plan: several chunks, enough CTAs
+        plan = (ctypes.c_int * 5)()
+        assert _lib.load("gemm_skinny_tcgen05").otb_gemm_skinny_plan(R, N, K, 148, None, plan) == 0
+        assert plan[0] > 1 and -(-N // 128) * plan[0] * plan[2] >= 32, list(plan)
     cuda_ops.check_status()
     want = res.double() + mod.double()[idx.long(), 2 * N:] * (x.double() @ w.double().T)
-    assert (got.double() - want).norm() < (2 ** -8 if R <= 640 else 2 ** -7) * want.norm()
+    assert (got.double() - want).norm() < (2 ** -8 if fused else 2 ** -7) * want.norm()
     assert torch.equal(got, cuda_ops.rows_linear(x, w, residual=res, gated_by=norm))
+    if fused:                                                  # the same rule and sum where gates come as rows
+        rows_ = cuda_ops.gemm(x, w, "nt", residual=res, gate=mod[:1, 2 * N:])
+        one = res.double() + mod.double()[:1, 2 * N:] * (x.double() @ w.double().T)
+        assert (rows_.double() - one).norm() < 2 ** -8 * one.norm()

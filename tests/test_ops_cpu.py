@@ -288,3 +288,47 @@ def test_attention_backward_refuses_misaligned_tensors_before_any_launch(which):
     B, S, H, D = 1, 64, 4, 64
     strides = (S * H * D, H * D, D) * 3
     assert fn(*base, 0, 0, 0, 1, 1, 1, *[1 << 20] * 4, B, S, S, H, H, D, *strides, 0.125, 0, 0) == -6
+
+
+@pytest.mark.parametrize("cols", [8, 128, 768, 1032, 1280, 2048, 8192, 32768])
+@pytest.mark.parametrize("inner", [8, 64, 256, 1088, 2048, 5120, 16384])
+def test_few_row_plans_fit_the_chip(cols, inner):
+    """Whatever the size, a plan covers the rows without an empty chunk and stays within shared memory; above 64 rows every CTA of
+    a cluster has k-blocks and the clusters are resident at once (as a B200 holds them, two CTAs to an SM up to 64 tokens) unless
+    one CTA to a sum is already too many."""
+    import ctypes
+
+    from opentau_b200.ops import _lib, build
+    if not build.lib_path("gemm_skinny_tcgen05").exists():
+        pytest.skip("native libraries are not built")
+    fits = (ctypes.c_int * 9)(0, 148, 74, 45, 33, 26, 22, 15, 15)
+    plan = (ctypes.c_int * 5)()
+    for rows in (*range(1, 700), 999, 1024, 4097):
+        assert _lib.load("gemm_skinny_tcgen05").otb_gemm_skinny_plan(rows, cols, inner, 148, fits, plan) == 0
+        chunks, nt, splits, stages, smem = plan
+        assert nt % 16 == 0 and 16 <= nt <= 256 and (chunks - 1) * nt < rows <= chunks * nt, (rows, list(plan))
+        kb = -(-inner // 64)
+        per = -(-kb // splits)
+        assert 1 <= splits <= 8 and 1 <= stages <= min(per, 12), (rows, list(plan))
+        assert smem <= (111 if nt <= 64 else 224) * 1024, (rows, list(plan))
+        units = -(-cols // 128) * chunks
+        if rows > 64:
+            assert (splits - 1) * per < kb, (rows, list(plan))
+            assert units <= fits[splits] * (2 if nt <= 64 else 1) or (splits == 1 and units > 148), (rows, list(plan))
+
+
+def test_few_row_plans_share_sums_where_the_chip_is_empty():
+    """100 - 400 rows of an action expert's output products: at least half the SMs work, and no CTA streams more than half the
+    k-blocks of a sum that several could share."""
+    import ctypes
+
+    from opentau_b200.ops import _lib, build
+    if not build.lib_path("gemm_skinny_tcgen05").exists():
+        pytest.skip("native libraries are not built")
+    fits = (ctypes.c_int * 9)(0, 148, 74, 45, 33, 26, 22, 15, 15)
+    plan = (ctypes.c_int * 5)()
+    for rows in (65, 100, 128, 150, 200, 256, 300, 400):
+        for cols, inner in ((1024, 2048), (1024, 4096), (1280, 2048), (1280, 5120)):
+            assert _lib.load("gemm_skinny_tcgen05").otb_gemm_skinny_plan(rows, cols, inner, 148, fits, plan) == 0
+            chunks, nt, splits, _, _ = plan
+            assert -(-cols // 128) * chunks * splits >= 74 and splits >= 2, (rows, cols, inner, list(plan))
