@@ -19,9 +19,11 @@
 // Results are deterministic: no atomics, fixed accumulation order.
 //
 // Order of a block j in the MMA warp: S of block j + 1 (its columns are free once S of j has been read, so it runs under the
-// elementwise work), the accumulation of j, dP of j + 1 (over the columns that held dS of j).  Measured against 32-wide blocks
-// with all operands in shared memory: 4096 positions, 8 heads on 1, width 256, 1024 of them causal: forward + backward 1145 ->
-// 718 us; a pi0.5 training step 164.4 -> 158.0 ms (all weights, batch 8), 214.7 -> 203.7 ms (expert only, batch 16).
+// elementwise work), the accumulation of j, dP of j + 1 (over the columns that held dS of j, once the accumulation has retired:
+// at width 256 the wait costs 0.06 us a block, and the first k-steps of S of j + 2 put into it cost more).  Measured against
+// 32-wide blocks with all operands in shared memory, backward alone: 4096 positions, 8 heads on 1, width 256, 1024 of them
+// causal: 1041 -> 568 us; 8 x 1227 positions (a pi0.5 training step's layer) 913 -> 583; 32 heads of 128 on 8, 2 x 2048: 1121 -> 737;
+// 16 heads of 72, 24 x 256: 225 -> 202.
 #include "common.cuh"
 #include <limits.h>
 
@@ -730,11 +732,13 @@ constexpr int BWD_MAX_SPLITS = 16;
 constexpr double BWD_MAX_SCRATCH = 256.0 * (1 << 20);   // bytes of one output's parts; past it a tile's share is small anyway
 
 // Into how many parts a tile's streamed blocks are dealt.  One block fills an SM, so the time is rounds x the blocks a part
-// streams, plus what every part does once (fixed tiles, first scores, epilogue: about PER_PART blocks' worth) and the
+// streams, plus what every part does once (fixed tiles, first scores, epilogue: PER_PART blocks' worth) and the
 // sums that are written and read in fp32 (charged to the parts of the whole launch) by one more launch, `extra` blocks' worth:
 // short sequences are bound by what the host issues, so parts must win a twentieth as well.  One sample of 4096 keys under one
-// kv head is 32 dK and 32 dV tiles, which left 116 of 148 SMs idle: forward + backward 2.85 ms without parts, 1.15 ms with
-// (8 heads on 1, width 256, 1024 causal positions); a pi0.5 training step at batch 8 (80 tiles) 172.5 -> 167.6 ms.
+// kv head is 32 dK and 32 dV tiles, which leaves 116 of 148 SMs idle: backward 1.48 ms without parts, 0.57 ms with (8 heads on 1,
+// width 256, 1024 causal positions).  Against the best number of parts for each product, over 615 sizes (1 - 16 samples, 200 -
+// 4096 positions, five head layouts of width 64 - 256, no, a fifth and half of the positions causal), the rule costs 1.9 % in the
+// mean with any PER_PART from 2 to 16, and one part always 5.3 %; what is left are masks, which sizes do not show.
 static int pick_bwd_splits(long long tiles, int blocks, int B, double out_bytes, double sum_cost, double extra) {
   static int sms = 0;
   if (sms == 0) {

@@ -1,5 +1,5 @@
 // Block-causal flash attention forward for sm_100a: TMA-fed, S = Q K^T and O += P V on tcgen05 with
-// both accumulators in tensor memory, online softmax by 128 threads that each own one TMEM lane.
+// both accumulators in tensor memory, online softmax by 256 threads, two to a TMEM lane.
 //
 // Mask rule (same as the dense reference): query i sees key j iff q_valid[i] && k_valid[j] &&
 // k_blk[j] <= q_blk[i].  Cached cross-attention keys carry k_blk = INT_MIN.  Rows that see no key
@@ -9,10 +9,11 @@
 // (query position, query head of the GQA group) pair: 128 rows = (128/g) positions x g heads, so one
 // K/V tile load serves every head of the group (MQA: g = 8 -> K/V traffic / 8).
 //
-// Warps: 0 = TMA producer, 1 = MMA issuer (owns TMEM), 2..5 = softmax / correction / epilogue.
-// Per KV block j:  MMA issues S[j+1] = Q K_{j+1}^T early, softmax turns S[j] into bf16 P in shared
-// memory (128B-swizzled, K-major), MMA issues O += P V_j.  O is rescaled lazily: only when the running
-// row maximum grew by more than 2^8 since the maximum in use, so the common case touches O never.
+// Warps: 0 = TMA producer, 1 = MMA issuer (owns TMEM), 2..9 = softmax / correction / epilogue.
+// Per KV block j:  MMA issues S[j+1] = Q K_{j+1}^T early, softmax turns S[j] into bf16 P, in shared memory
+// (128B-swizzled, K-major) or, with two CTAs to an SM (SPLIT_TWO), over the scores in tensor memory, MMA issues
+// O += P V_j.  O is rescaled lazily: only when the running row maximum grew by more than 2^8 since the maximum
+// in use, so the common case touches O never.
 //
 // Few query tiles against many keys (a denoising step or a decoded token against a cached prefix) share the key blocks of
 // a tile among `nsplit` CTAs.  Where the tiles are few enough (SPLIT_CLUSTER) those CTAs are one cluster and the partials
@@ -43,6 +44,7 @@ struct AttnParams {
   int skip_reach;                   // visit every key block: skip the prologue scan for the last reachable key
   int nsplit;                       // 1: write o / lse directly
   int cl_rows;                      // SPLIT_CLUSTER: rows of a tile (32 or 64)
+  int ahead;                        // SPLIT_CLUSTER: key blocks, at most, that a CTA of the first tile requests into L2
   float* part_o;                    // (nsplit, B, Sq, H, D) fp32, accumulators expressed against part m
   float2* part_ml;                  // (nsplit, B, H, Sq): (running maximum in log2 units, row sum)
   KernelStatus* status;
@@ -172,10 +174,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   const uint32_t tmem_S = tmem_base;            // two buffers of BN columns
   const uint32_t tmem_O = tmem_base + 2 * BN;   // Dmma columns
   pdl_launch_dependents();                      // after the TMEM allocation (see common.cuh)
-  if (CL && threadIdx.x == 0) {
-    // the cached keys and values have left L2 since the last pass: on their way while the preceding kernel finishes
+  if (CL && threadIdx.x == 0 && tile == 0) {
+    // The cached keys and values have left L2 since the last pass: on their way while the preceding kernel finishes, requested
+    // by the first tile of a kv head alone.  us with a norm in front, no requests / by every tile / by the first: 50 queries of 8
+    // heads on 1 of 256 against 1018 keys 10.3 / 10.2 / 10.0, 4096 21.2 / 20.7 / 20.3, 32768 122.9 / 130.7 / 119.5; on 4, 4096 keys
+    // 24.2 / 22.8 / 22.8; one query: within 0.2 of none
     const int all = (p.Sk + BN - 1) / BN, per = (all + p.nsplit - 1) / p.nsplit;
-    for (int j = split * per; j < min(all, (split + 1) * per); ++j)
+    for (int j = split * per; j < min(all, split * per + min(per, p.ahead)); ++j)
       for (int c = 0; c < L::NCHUNK; ++c) {
         l2_prefetch_4d(&tma_k, c * 64, kvh, j * BN, b);
         l2_prefetch_4d(&tma_v, c * 64, kvh, j * BN, b);
@@ -237,7 +242,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one()) {
-      mbar_expect_tx(q_full, L::Q_BYTES * ROWS / ATT_M);        // the rows past a 64-row tile are never looked at
+      mbar_expect_tx(q_full, L::Q_BYTES * ROWS / ATT_M);        // the rows past a smaller tile are never looked at
 #pragma unroll
       for (int c = 0; c < L::NCHUNK; ++c)
         tma_load_4d(sQ + c * (ATT_M * 128), &tma_q, q_full, c * 64, kvh * g, p0, b);
@@ -415,7 +420,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         tmem_wait_st();
       }
       l *= alpha;
-      // ---- probabilities -> bf16 -> swizzled shared memory (A operand of the PV product)
+      // ---- probabilities -> bf16 -> swizzled shared memory or tensor memory (A operand of the PV product)
       uint8_t* prow = sP + slot * L::P_BYTES + row * 128;
       float lsum = 0.f;
       const float m_safe = (m_used == -INFINITY) ? 0.f : m_used;
@@ -779,7 +784,7 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
                          long long k_ss, long long k_sh, long long v_sb, long long v_ss, long long v_sh, float scale,
                          int nsplit, float* part_o, float* part_ml, void* status, cudaStream_t stream) {
   if (nsplit < 1 || nsplit > 8) return -7;
-  // split without scratch: one cluster per tile of 64 rows merges on chip
+  // split without scratch: one cluster per tile of 64 or 32 rows merges on chip
   const bool cluster = nsplit > 1 && part_o == nullptr;
   if (nsplit > 1 && !cluster && (part_ml == nullptr || D % 4)) return -7;
   if (B <= 0 || Sq <= 0 || Sk <= 0 || H <= 0 || Hkv <= 0 || H % Hkv) return -2;
@@ -812,10 +817,15 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
   const bool two = dpad <= 128 && nsplit == 1 && (long long)((Sq + ATT_M / g - 1) / (ATT_M / g)) * Hkv * B > sm_count();
   const int bn = dpad == 256 || two ? 64 : 128;
   CUtensorMap tq, tk, tv;
-  // 32-row tiles halve what a cluster's CTAs send one another, where twice the clusters are still resident at once (50 queries of
-  // 8 heads on 1, 1018 keys: 13 clusters, 10.2 -> 9.2 us; 16 queries, 400 keys: 8.9 -> 7.3)
+  // 32-row tiles halve what a cluster's CTAs send one another, where twice the clusters are still resident at once.  Every tile
+  // streams all keys, so the gain fades with their number: us with a norm in front, 64 / 32 rows, 50 queries of 8 heads on 1 of 256
+  // (13 clusters): 384 keys 10.7 / 9.1, 1018 11.7 / 10.0, 4096 21.8 / 20.3, 16384 62.3 / 62.6, 32768 123.2 / 119.5; 20 of 4 heads on
+  // 1 of 64, 4096 keys 12.0 / 11.9.  Clusters in two rounds lose: 50 queries of 8 heads on 4, 1074 keys 13.8 / 18.8
   p.cl_rows = CL_ROWS;
   if (cluster && g <= 32 && cluster_fits(D, nsplit, ((long long)Sq * g + 31) / 32 * Hkv * B)) p.cl_rows = 32;
+  // what a launch requests ahead stays a quarter of L2
+  const long long block_bytes = 4LL * bn * dpad * Hkv * B * nsplit;
+  p.ahead = (int)((32LL << 20) / block_bytes);
   int r = make_map4(&tq, q, D, H, Sq, B, q_sh, q_ss, q_sb, g, (cluster ? p.cl_rows : ATT_M) / g);
   if (r) return 1000 + r;
   r = make_map4(&tk, k, D, Hkv, Sk, B, k_sh, k_ss, k_sb, 1, bn);
@@ -853,7 +863,7 @@ extern "C" int otb_attn_fwd_splitkv(const void* q, const void* k, const void* v,
                        k_ss, k_sh, v_sb, v_ss, v_sh, scale, nsplit, part_o, part_ml, status, stream);
 }
 
-// CTAs per cluster for `tiles` tiles of 64 rows: the most (up to 8) whose clusters are all resident at once, since a second
+// CTAs per cluster for `tiles` tiles of 64 rows (the launch may then halve the tiles): the most (up to 8) whose clusters are all resident at once, since a second
 // round costs more than anything a larger cluster saves; 1 if that leaves fewer than 3.  Measured at 50 queries of 8 heads
 // on 1, width 256, against the merge through global memory: 10.5 us against 17.2 (7 tiles, 1018 keys, 8 CTAs), 12.5 against
 // 17.0 (28 tiles, 639 keys, 4), 16.9 against 19.7 (42 tiles, 900 keys, 3); pairs gain nothing (56 tiles: 20.4 against 20.2)

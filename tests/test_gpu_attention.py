@@ -418,6 +418,32 @@ def test_backward_with_fixed_tiles_in_tensor_memory(D, H, Hkv, S):
         assert _rel(x, w) < 2 ** -8, (name, _rel(x, w))
 
 
+@pytest.mark.parametrize("D,H,Hkv,S", [(64, 4, 1, 900), (72, 16, 16, 260), (128, 8, 2, 641), (200, 4, 4, 449), (256, 8, 1, 1027)])
+def test_backward_of_strided_views_and_repeats(D, H, Hkv, S):
+    """q, k and v as views of one q/k/v buffer (the fixed tiles are addressed by hand), a second sample and a gradient that starts
+    off a 16-byte boundary: the same bits as contiguous tensors give, and the same bits again every time (a block's scores go
+    over the columns that the block before has just read, rings wrap many times)."""
+    from opentau_b200.ops import attention_native, cuda_ops
+    B = 2
+    g = torch.Generator(device="cuda").manual_seed(D + S)
+    qkv = torch.randn(B, S, (H + 2 * Hkv) * D, device="cuda", generator=g).to(torch.bfloat16)
+    q = qkv[..., :H * D].unflatten(-1, (H, D))
+    k, v = (t.unflatten(-1, (Hkv, D)) for t in qkv[..., H * D:].chunk(2, -1))
+    blk = (torch.arange(S, device="cuda") - S // 2).clamp_min(0).expand(B, -1).int().contiguous()
+    valid = torch.ones(B, S, dtype=torch.bool, device="cuda")
+    valid[1, S - 7:] = False
+    raw = torch.randn(B * S * H * D + 1, device="cuda", generator=g).to(torch.bfloat16)
+    do = raw[1:].view(B, S, H * D)
+    assert not q.is_contiguous() and not v.is_contiguous() and do.data_ptr() % 16
+    o, lse = attention_native.attn_fwd(q, k, v, blk, blk, valid, valid, D ** -0.5)
+    args = (o, lse, blk, blk, valid, valid, D ** -0.5)
+    want = attention_native.attn_bwd(do.clone(), q.contiguous(), k.contiguous(), v.contiguous(), *args)
+    for _ in range(4):
+        got = attention_native.attn_bwd(do, q, k, v, *args)
+        assert all(torch.equal(x, y) for x, y in zip(got, want))
+    cuda_ops.check_status()
+
+
 @pytest.mark.parametrize("D,H,Hkv", [(256, 8, 1), (128, 8, 2), (64, 4, 4), (72, 16, 16)])
 @pytest.mark.parametrize("splits", [(2, 3, 2), (4, 16, 7)])
 def test_split_backward_matches_the_unsplit_one(D, H, Hkv, splits):
