@@ -398,10 +398,11 @@ static bool layout_plan(int M, int K, int chunks, int splits, SkinnyPlan* p) {
 // More rows: of the token tiles from 32 to 256 and 1 to 8 CTAs to a sum, the cheapest that is resident at once.  A CTA
 // pays for its k-blocks, for every round of the ring behind the first, for the partials it sends, for its own tokens' epilogue,
 // and the launch for its CTAs: microseconds fitted to 3400 resident plans at 65 - 640 rows, 128 - 2048 columns, K 256 - 8192 inside a
-// replayed graph with cold weights (rms error 6 %; the plan taken costs 1.5 % more than the best one in the mean, 13 % at most).
+// replayed graph with cold weights (rms error 6 %; the plan taken costs 1.5 % more than the best one in the mean, 10 % at most; where
+// rows of K are no multiple of 128 bytes, reading the weights once per chunk costs up to a tenth that this does not charge).
 // The weights are read once per chunk, from L2.  With the norm behind them, us, against one tile of up to 256 rows and
-// against chunks of 64 that two to four CTAs share (what ran before): 100 x 1024 x 4096 9.3 / 11.2 -> 8.0, 200 x 1024 x 4096 15.1 /
-// 12.2 -> 9.7, 256 x 1280 x 5120 31.8 / 16.4 -> 12.5, 200 x 128 x 256 13.8 / 13.8 -> 4.7.
+// against chunks of 64 that two to four CTAs share (what ran before): 100 x 1024 x 4096 9.4 / 11.2 -> 8.7, 200 x 1024 x 4096 14.8 /
+// 12.2 -> 9.5, 256 x 1280 x 5120 31.8 / 16.5 -> 13.0, 200 x 128 x 256 13.8 / 13.8 -> 4.7.
 template <typename F>
 static bool choose_plan(int M, int N, int K, int sms, F clusters, SkinnyPlan* best) {
   const int n_tiles = (N + SK_BW - 1) / SK_BW, num_kb = (K + SK_BK - 1) / SK_BK;

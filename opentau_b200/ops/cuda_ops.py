@@ -73,13 +73,14 @@ def use_skinny(layout: str, M: int, N: int, accumulate: bool, bn: int, K: int = 
     if gated:
         # the alternative rounds the sum to bf16 in front of the gate: every few-row product keeps the fusion, but for
         # more columns than the 128 x 256 tiles of the persistent kernel need to fill the chip.  Up to 640 rows where two CTAs
-        # may share the sums of 64-row chunks: 400 x 1024 x 4096 20.5 -> 12.6 us with the norm behind it against the persistent
-        # kernel and a gated residual of its own, 640 x 1280 x 2048 14.8 -> 12.4; without the room 600 x 2048 x 2048 16.3 -> 17.3
+        # may share the sums of 64-row chunks: 400 x 1024 x 4096 20.6 -> 12.4 us with the norm behind it against the persistent
+        # kernel and a gated residual of its own, 640 x 1280 x 2048 15.0 -> 12.0; without the room 600 x 2048 x 2048 16.3 -> 17.3
         return M <= 128 or (M <= 256 and N <= 8192) or (M <= 640 and N <= 2048 and -(-N // 128) * -(-M // 64) <= 148)
     # measured inside a replayed graph: up to 64 rows the split-K kernel always wins (50 x 8192 x 1024 6.4 us against
-    # 9.1, 50 x 1024 x 4096 6.0 against 16.2); at 65..256 rows only where the persistent kernel has too few tiles for the
-    # chip and a long sum (200 x 1024 x 4096 12.8 us against 16.3, but 200 x 1024 x 2048 11.5 against 9.8 and 256 x 768 x 768
-    # 11.1 against 6.0)
+    # 9.1, 50 x 1024 x 4096 6.0 against 16.2); at 65..256 rows it is taken where the persistent kernel has too few tiles for
+    # the chip and a long sum (with a norm behind it 200 x 1024 x 4096 9.1 us against 18.1).  That line was drawn for one wide
+    # tile of all rows; with the plans as they are shorter sums would gain a little as well (200 x 1024 x 2048 7.6 against 11.7,
+    # 256 x 768 x 768 6.2 against 7.8, 200 x 2560 x 1024 8.1 against 9.7), many columns would not (200 x 8192 x 1024 14.0 against 13.7)
     return M <= 64 or (M <= 256 and N <= 2048 and K >= 3072)
 
 
