@@ -4,7 +4,7 @@ from __future__ import annotations
 
 import os
 from functools import lru_cache
-from ctypes import byref, c_float, c_int, c_longlong, c_void_p
+from ctypes import Structure, byref, c_float, c_int, c_longlong, c_void_p
 
 import torch
 from torch import Tensor
@@ -137,10 +137,79 @@ def bwd_splits(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int) -> tuple[int,
     return tuple(x.value for x in n)
 
 
+class _StoredBwdArgs(Structure):
+    """``OtbAttnBwdStored`` of ``csrc/attention_bwd_stored_tcgen05.cu``."""
+
+    _fields_ = [(n, c_void_p) for n in ("q", "k", "v", "o", "do", "lse", "dq", "dk", "dv", "p", "ds", "cover", "dk_parts", "dv_parts",
+                                        "q_blk", "k_blk", "q_valid", "k_valid", "status")] + \
+        [("strides", c_longlong * 9)] + \
+        [(n, c_int) for n in ("B", "Sq", "Sk", "H", "Hkv", "D", "kv_splits")] + [("scale", c_float)]
+
+
+#: bytes of P and dS together that the backward keeps at most; calls with more go a few samples at a time
+BWD_STORED_LIMIT = 2 << 30
+
+
+@lru_cache(maxsize=1024)
+def bwd_stored_plan(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int) -> tuple[int, int, int]:
+    """``(bytes of P, ints of cover, parts of dK and dV)`` of the stored backward, from the sizes alone."""
+    size, cover, parts = c_longlong(), c_int(), c_int()
+    _lib.load("attention_bwd_stored_tcgen05").otb_attn_bwd_stored_plan(
+        c_int(B), c_int(Sq), c_int(Sk), c_int(H), c_int(Hkv), c_int(D), byref(size), byref(cover), byref(parts))
+    return size.value, cover.value, parts.value
+
+
+def stored_bwd_samples(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int) -> int:
+    """Samples that a launch of the stored backward takes; 0 where one alone has more P and dS than is kept (8 heads of 8192
+    positions): the recomputing kernels."""
+    return min(B, BWD_STORED_LIMIT // (2 * bwd_stored_plan(1, Sq, Sk, H, Hkv, D)[0]))
+
+
+def _attn_bwd_stored(samples: int, do, q, k, v, o, lse, qb, kb, qv, kv, dq, dk, dv, scale: float,
+                     parts: int | None = None) -> bool:
+    """dq, dk, dv through stored P and dS, ``samples`` at a time; False where there is no room for them."""
+    from . import cuda_ops
+    B, Sq, H, D = q.shape
+    Sk, Hkv = k.shape[1], k.shape[2]
+    size, n_cover, _ = bwd_stored_plan(samples, Sq, Sk, H, Hkv, D)
+    try:
+        scratch = torch.empty(2 * size + 4 * n_cover, dtype=torch.uint8, device=q.device)
+    except torch.cuda.OutOfMemoryError:
+        return False
+    s0 = scratch.data_ptr()
+    fn = _entry_args("attention_bwd_stored_tcgen05", "otb_attn_bwd_stored")
+    tensors = (q, k, v, o, do, lse, dq, dk, dv, qb, kb, qv, kv)
+    step = [samples * t.stride(0) * t.element_size() for t in tensors]
+    at = [t.data_ptr() for t in tensors]
+    strides = (c_longlong * 9)(*q.stride()[:3], *k.stride()[:3], *v.stride()[:3])
+    for b0 in range(0, B, samples):
+        n = min(samples, B - b0)
+        m = parts or bwd_stored_plan(n, Sq, Sk, H, Hkv, D)[2]
+        sums = torch.empty(2, m, n * Sk * Hkv * D, dtype=torch.float32, device=q.device) if m > 1 else None
+        sums_at = (sums.data_ptr(), sums.data_ptr() + 4 * sums.stride(0)) if m > 1 else (0, 0)
+        args = _StoredBwdArgs(*at[:9], s0, s0 + size, s0 + 2 * size, *sums_at, *at[9:], cuda_ops.status_pointer(), strides,
+                              n, Sq, Sk, H, Hkv, D, m, scale)
+        rc = fn(byref(args), cuda_ops._stream())
+        if rc != 0:
+            raise RuntimeError(f"native attn_bwd failed with code {rc} (B={B} Sq={Sq} Sk={Sk} H={H} Hkv={Hkv} D={D})")
+        cuda_ops.launch_count += 3 + (m > 1)
+        at = [x + d for x, d in zip(at, step)]
+    return True
+
+
+@lru_cache(maxsize=None)
+def _entry_args(lib: str, name: str):
+    fn = getattr(_lib.load(lib), name)
+    fn.argtypes = [c_void_p, c_void_p]
+    return fn
+
+
 def attn_bwd(do: Tensor, q: Tensor, k: Tensor, v: Tensor, o: Tensor, lse: Tensor, q_blk: Tensor, k_blk: Tensor,
-             q_valid: Tensor, k_valid: Tensor, scale: float, splits: tuple[int, int, int] | None = None):
-    """Returns ``(dq, dk, dv)``; scratch and outputs are allocated here.  ``splits`` forces the parts that the streamed
-    blocks of dQ, dK and dV are dealt to."""
+             q_valid: Tensor, k_valid: Tensor, scale: float, splits: tuple[int, int, int] | None = None,
+             samples: int | None = None, parts: int | None = None):
+    """Returns ``(dq, dk, dv)``; scratch and outputs are allocated here.  ``samples`` forces how many samples at a time go through
+    stored P and dS (0: none, the recomputing kernels) and ``parts`` the parts of a tile of dK and dV there; ``splits`` forces
+    the recomputing kernels and the parts that the streamed blocks of dQ, dK and dV are dealt to."""
     from . import cuda_ops
     B, Sq, H, D = q.shape
     Sk, Hkv = k.shape[1], k.shape[2]
@@ -153,18 +222,22 @@ def attn_bwd(do: Tensor, q: Tensor, k: Tensor, v: Tensor, o: Tensor, lse: Tensor
     dq = torch.empty(B, Sq, H, D, dtype=q.dtype, device=q.device)
     dk = torch.empty(B, Sk, Hkv, D, dtype=q.dtype, device=q.device)
     dv = torch.empty(B, Sk, Hkv, D, dtype=q.dtype, device=q.device)
-    delta = torch.empty(B, H, Sq, dtype=torch.float32, device=q.device)
     qb = q_blk.to(torch.int32).contiguous()
     kb = k_blk.to(torch.int32).contiguous()
     qv = _u8(q_valid)
     kv = _u8(k_valid)
+    if samples is None:
+        samples = stored_bwd_samples(B, Sq, Sk, H, Hkv, D) if splits is None else 0
+    if samples and _attn_bwd_stored(samples, do, q, k, v, o, lse, qb, kb, qv, kv, dq, dk, dv, scale, parts):
+        return dq, dk, dv
+    delta = torch.empty(B, H, Sq, dtype=torch.float32, device=q.device)
     if splits is None:
         splits = bwd_splits(B, Sq, Sk, H, Hkv, D)
-    parts = [torch.empty(m, *t.shape, dtype=torch.float32, device=q.device) if m > 1 else None
-             for m, t in zip(splits, (dq, dk, dv))]
+    sums = [torch.empty(m, *t.shape, dtype=torch.float32, device=q.device) if m > 1 else None
+            for m, t in zip(splits, (dq, dk, dv))]
     rc = _entry("attention_bwd_tcgen05", "otb_attn_bwd", 13 * "p" + 3 * "i" + 4 * "p" + 6 * "i" + 9 * "l" + "fpp")(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(), delta.data_ptr(),
-        dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), *(_ptr(t) for t in parts), *splits, qb.data_ptr(), kb.data_ptr(),
+        dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), *(_ptr(t) for t in sums), *splits, qb.data_ptr(), kb.data_ptr(),
         qv.data_ptr(), kv.data_ptr(), B, Sq, Sk, H, Hkv, D, *q.stride()[:3], *k.stride()[:3], *v.stride()[:3], scale,
         cuda_ops.status_pointer(), cuda_ops._stream())
     if rc != 0:

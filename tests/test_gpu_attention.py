@@ -444,6 +444,74 @@ def test_backward_of_strided_views_and_repeats(D, H, Hkv, S):
     cuda_ops.check_status()
 
 
+@pytest.mark.parametrize("D,H,Hkv", [(256, 8, 1), (256, 8, 4), (200, 2, 2), (128, 32, 1), (72, 4, 4), (64, 8, 2)])
+@pytest.mark.parametrize("Sq,Sk", [(1, 1), (17, 63), (16, 64), (33, 65), (130, 257), (257, 130), (300, 513)])
+@pytest.mark.parametrize("samples,parts", [(1, None), (3, None), (2, 3)])
+def test_stored_backward_matches_the_recomputing_one(D, H, Hkv, Sq, Sk, samples, parts):
+    """Query tiles, stored blocks of 64 and key tiles of 256 with one row more or less; block ids in no order, a tile that sees
+    nothing, keys that nobody sees, queries without a key; several launches for a batch; parts of dK and dV, empty ones among them.
+    Both paths round P and dS to bf16 and sum in fp32: what differs is delta's order of summation and the result's rounding (2^-8).
+    A query that sees one key has dS = 0 but for what dP and delta, fp32 sums of D products of unit normals, lose where they
+    cancel: D 2^-24 of sum |o dO| = 0.64 D, times the scale D^-1/2, below 2^-12 at D = 256, whatever the size of the result."""
+    from opentau_b200.ops import attention_native, cuda_ops
+    B = 3
+    g = torch.Generator(device="cuda").manual_seed(D + 7 * Sq + Sk)
+    q, k, v, do = (torch.randn(*shape, device="cuda", generator=g).to(torch.bfloat16)
+                   for shape in ((B, Sq, H, D), (B, Sk, Hkv, D), (B, Sk, Hkv, D), (B, Sq, H * D)))
+    qb = torch.randint(0, 6, (B, Sq), device="cuda", generator=g, dtype=torch.int32)
+    kb = torch.randint(0, 8, (B, Sk), device="cuda", generator=g, dtype=torch.int32)
+    kb[1, Sk // 2:] = 9                                                # hidden from every query
+    kb[2] = -2147483648                                                # cached keys
+    qv = torch.rand(B, Sq, device="cuda", generator=g) > 0.1
+    kv = torch.rand(B, Sk, device="cuda", generator=g) > 0.1
+    qv[0, Sq // 2:] = False
+    qb[1, :Sq // 3] = -1                                               # sees nothing
+    o, lse = attention_native.attn_fwd(q, k, v, qb, kb, qv, kv, D ** -0.5)
+    args = (do, q, k, v, o, lse, qb, kb, qv, kv, D ** -0.5)
+    want = attention_native.attn_bwd(*args, samples=0)
+    got = attention_native.attn_bwd(*args, samples=samples, parts=parts)
+    again = attention_native.attn_bwd(*args, samples=samples, parts=parts)
+    cuda_ops.check_status()
+    for name, x, y, w in zip(("dq", "dk", "dv"), got, again, want):
+        assert torch.equal(x, y), name
+        diff = (x.double() - w.double()).norm().item()
+        assert bool(torch.isfinite(x).all()) and diff <= 2 ** -8 * w.double().norm().item() + 2 ** -12 * x.numel() ** 0.5, (name, diff)
+    assert float(got[1][1, Sk // 2:].abs().sum()) == 0.0 and float(got[0][0, Sq // 2:].abs().sum()) == 0.0
+
+
+def test_backward_recomputes_where_there_is_no_room_for_p_and_ds(monkeypatch):
+    """A call whose P and dS are more than is kept goes a sample at a time, then without them; so does one that finds no memory."""
+    from opentau_b200.ops import attention_native, cuda_ops
+    B, S, H, Hkv, D = 2, 200, 8, 1, 64
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v, do = (torch.randn(*shape, device="cuda", generator=g).to(torch.bfloat16)
+                   for shape in ((B, S, H, D), (B, S, Hkv, D), (B, S, Hkv, D), (B, S, H * D)))
+    blk, valid = torch.zeros(B, S, dtype=torch.int32, device="cuda"), torch.ones(B, S, dtype=torch.bool, device="cuda")
+    o, lse = attention_native.attn_fwd(q, k, v, blk, blk, valid, valid, D ** -0.5)
+    args = (do, q, k, v, o, lse, blk, blk, valid, valid, D ** -0.5)
+    want = attention_native.attn_bwd(*args, samples=0)
+    both = attention_native.bwd_stored_plan(1, S, S, H, Hkv, D)[0] * 2
+    for limit, launches in ((2 * both, 3), (both, 6), (both - 1, 4)):
+        monkeypatch.setattr(attention_native, "BWD_STORED_LIMIT", limit)
+        before = cuda_ops.launch_count
+        got = attention_native.attn_bwd(*args)
+        cuda_ops.check_status()
+        assert launches <= cuda_ops.launch_count - before <= launches * 3 // 2 + 1
+        assert all(_rel(x, w.double()) < 2 ** -8 for x, w in zip(got, want))
+    monkeypatch.undo()
+    real = torch.empty
+
+    def empty(*a, **kw):
+        if kw.get("dtype") is torch.uint8:
+            raise torch.cuda.OutOfMemoryError
+        return real(*a, **kw)
+
+    monkeypatch.setattr(torch, "empty", empty)
+    got = attention_native.attn_bwd(*args)
+    monkeypatch.undo()
+    assert all(torch.equal(x, w) for x, w in zip(got, want))
+
+
 @pytest.mark.parametrize("D,H,Hkv", [(256, 8, 1), (128, 8, 2), (64, 4, 4), (72, 16, 16)])
 @pytest.mark.parametrize("splits", [(2, 3, 2), (4, 16, 7)])
 def test_split_backward_matches_the_unsplit_one(D, H, Hkv, splits):

@@ -290,6 +290,23 @@ def test_attention_backward_refuses_misaligned_tensors_before_any_launch(which):
     assert fn(*base, 0, 0, 0, 1, 1, 1, *[1 << 20] * 4, B, S, S, H, H, D, *strides, 0.125, 0, 0) == -6
 
 
+@pytest.mark.parametrize("which", ["q", "k", "v", "o", "do", "dq", "dk", "dv", "p", "ds"])
+def test_stored_attention_backward_refuses_misaligned_tensors_before_any_launch(which):
+    """As above for the backward that keeps P and dS, whose blocks move in bulk copies."""
+    from ctypes import byref, c_longlong
+
+    from opentau_b200.ops import attention_native, build
+    if not build.lib_path("attention_bwd_stored_tcgen05").exists():
+        pytest.skip("native libraries are not built")
+    fn = attention_native._entry_args("attention_bwd_stored_tcgen05", "otb_attn_bwd_stored")
+    names = [n for n, _ in attention_native._StoredBwdArgs._fields_][:19]
+    base = {n: 1 << 20 for n in names}
+    base[which] += 8
+    B, S, H, D = 1, 64, 4, 64
+    args = attention_native._StoredBwdArgs(*base.values(), (c_longlong * 9)(*(S * H * D, H * D, D) * 3), B, S, S, H, H, D, 1, 0.125)
+    assert fn(byref(args), 0) == -6
+
+
 @pytest.mark.parametrize("cols", [8, 128, 768, 1032, 1280, 2048, 8192, 32768])
 @pytest.mark.parametrize("inner", [8, 64, 256, 1088, 2048, 5120, 16384])
 def test_few_row_plans_fit_the_chip(cols, inner):
