@@ -74,10 +74,9 @@ def split_kv(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int) -> int:
     nblk = -(-Sk // (64 if D > 128 else 128))
     if ctas * 4 > NUM_SMS:
         # half the chip idle and a long stream: two halves and a merge.  One pass against two halves, inside a replayed graph:
-        # 8 heads on 1 of 256, 40 - 61 tiles: 24.2 / 23.9 us with 11 blocks, 25.6 / 24.4 with 12, 28.8 / 26.3 with 14, 30.6 / 28.0
-        # with 15, 32.1 / 28.0 with 16; 16 heads of 72, 64 tiles: 21.2 / 19.0 with 8, 35.0 / 26.6 with 15.  The line stands where
-        # every width gains about a tenth; with tiles for more than half the SMs it loses (21.3 / 31.9)
-        return 2 if ctas * 2 <= NUM_SMS and nblk >= 15 else 1
+        # 16 heads of 72, 64 tiles: 21.2 / 19.0 us with 8 blocks, 35.0 / 26.6 with 15; with tiles for more than half the SMs it
+        # loses.  Above a width of 128 one pass wins: 8 heads on 1 of 256, 61 tiles of 968 keys 23.6 / 28.4, 64 of 1277 27.0 / 31.6
+        return 2 if D <= 128 and ctas * 2 <= NUM_SMS and nblk >= 15 else 1
     return max(1, min(8, NUM_SMS // ctas, nblk // 2))
 
 

@@ -645,6 +645,393 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   }
 }
 
+// ------------------------------------------------------------------------------------------ head widths above 128, keys unsplit
+// At width 256 the kernel above keeps one tile of scores ahead, but all its softmax warps work on one block: 64 keys took 2970 clocks
+// for 1024 of arithmetic (4096 positions, 8 heads on 1: 200 us).  Here the query tile lies in tensor memory (128 columns) beside
+// two tiles of scores (64 each) and O (256), so a score product reads only keys from shared memory, and two groups of four warps take
+// the blocks in turn, a thread a whole row.  What one group needs of the other is the row's maximum in use, which it publishes
+// before its exponentials; the sums stay each group's own, in terms of the maximum it saw last, and meet at the end.  P goes over the
+// scores it was made from; scores of block j + 2 wait for the commit of the product that reads P of j.
+// us, before / now: 4096 positions, 8 heads on 1, 1024 of them causal 186 / 110; 16 x 1227 (259 causal) 335 / 212; 2 x 1500, 8 on 4 79 /
+// 55; 4 x 589 24 / 19; 5000, 4 heads of 160 125 / 75.  At 4096 a block takes 1700 clocks: the chain from scores to P and the products
+// of two blocks that take turns.
+template <int DPAD>
+struct WideSmem {
+  static constexpr int BN = 64, NCHUNK = DPAD / 64;
+  static constexpr int Y_BYTES = BN * DPAD * 2;        // an item of the ring: 64 rows of Q, K or V
+  static constexpr int NY = 7;
+  static constexpr int OFF_M = NY * Y_BYTES;           // float [2 groups][128]: maxima in use; at the end the row sums
+  static constexpr int OFF_BAR = OFF_M + 2 * ATT_M * 4;
+  static constexpr int NBAR = 1 + 2 * NY + 6 + 8;
+  static constexpr int USED = OFF_BAR + NBAR * 8 + 16;
+  static constexpr int TOTAL = USED + 1024 <= 232448 ? USED + 1024 : 232448;
+  static_assert(USED <= 232448, "shared memory budget");
+  static constexpr int TM_Q = 0, TM_S = DPAD / 2, TM_O = DPAD / 2 + 2 * BN;
+  static_assert(TM_O + DPAD <= 512, "tensor memory budget");
+};
+
+template <int DPAD>
+__global__ void __launch_bounds__(320, 1)
+attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
+                     const __grid_constant__ CUtensorMap tma_v, AttnParams p) {
+  using L = WideSmem<DPAD>;
+  constexpr int BN = L::BN;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  float* m_pub = reinterpret_cast<float*>(smem + L::OFF_M);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
+  uint64_t* q_full = bars;                       // the query tile is in tensor memory
+  uint64_t* y_full = bars + 1;                   // [NY]
+  uint64_t* y_empty = y_full + L::NY;            // [NY]
+  uint64_t* s_full = y_empty + L::NY;            // [2]
+  uint64_t* p_full = s_full + 2;                 // [2] P is in tensor memory
+  uint64_t* pv_done = s_full + 4;                // [2] the product that reads it has retired
+  uint64_t* m_ready = s_full + 6;                // [2][4 quadrants] a group's maxima are published
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NBAR);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int* reach = reinterpret_cast<int*>(tmem_slot + 2);
+  if ((int)(smem - smem_raw) + L::USED > L::TOTAL) {   // base less aligned than assumed: refuse instead of overrunning
+    if (threadIdx.x == 0) report_timeout(p.status, KID_ATTN, 99, (unsigned)(smem - smem_raw));
+    return;
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // late tiles see the most keys where the text behind a prefix is causal: they go first
+  const int tile = gridDim.x - 1 - blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  const int g = p.g, pos_per_tile = ATT_M / g, p0 = tile * pos_per_tile;
+
+  if (threadIdx.x == 0) {
+    mbar_init(q_full, 256);
+    for (int i = 0; i < L::NY; ++i) {
+      mbar_init(&y_full[i], 1);
+      mbar_init(&y_empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&s_full[i], 1);
+      mbar_init(&p_full[i], 128);
+      mbar_init(&pv_done[i], 1);
+    }
+    for (int i = 0; i < 8; ++i) mbar_init(&m_ready[i], 32);
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tma_q);
+    tma_prefetch_desc(&tma_k);
+    tma_prefetch_desc(&tma_v);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();                       // after the TMEM allocation (see common.cuh)
+  pdl_wait();
+
+  // ---- 1 + the last valid key with k_blk <= the tile's largest valid q_blk (no order assumed), searched from the end; the loads
+  // of Q and of the first keys are on their way meanwhile (a tile that sees nothing runs one block)
+  if (warp == 1) {
+    int qmax = INT_MIN, any = 0;
+    for (int i = lane; i < pos_per_tile; i += 32) {
+      const int ps = p0 + i;
+      if (ps < p.Sq && p.q_valid[(long long)b * p.Sq + ps]) {
+        qmax = max(qmax, p.q_blk[(long long)b * p.Sq + ps]);
+        any = 1;
+      }
+    }
+    qmax = __reduce_max_sync(0xffffffffu, qmax);
+    any = __any_sync(0xffffffffu, any);
+    int last = -1;
+    for (int end = p.Sk; any && end > 0 && last < 0; end -= 512) {
+      int kb[16], kv[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int j = end - 512 + i * 32 + lane;
+        kb[i] = j >= 0 ? p.k_blk[(long long)b * p.Sk + j] : 0;
+        kv[i] = j >= 0 ? p.k_valid[(long long)b * p.Sk + j] : 0;
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (kv[i] && kb[i] <= qmax) last = max(last, end - 512 + i * 32 + lane);
+      last = __reduce_max_sync(0xffffffffu, last);
+    }
+    if (lane == 0) *reach = last + 1;
+  }
+  auto load_item = [&](int s, const CUtensorMap* m, int head, int row) {
+    mbar_expect_tx(&y_full[s], L::Y_BYTES);
+#pragma unroll
+    for (int c = 0; c < L::NCHUNK; ++c) tma_load_4d(smem + s * L::Y_BYTES + c * (BN * 128), m, &y_full[s], c * 64, head, row, b);
+  };
+  if (threadIdx.x == 0) {
+    load_item(0, &tma_q, kvh * g, p0);
+    load_item(1, &tma_q, kvh * g, p0 + 64 / g);
+    load_item(2, &tma_k, kvh, 0);
+  }
+  __syncthreads();
+  const int nblk = max(1, (*reach + BN - 1) / BN);
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer, in the order of use: K0 K1 V0 K2 V1 K3 ...
+    if (elect_one()) {
+      int s = 3;
+      uint32_t ph = 1;                           // the ring's first round does not wait
+      for (int i = 1; i < 2 * nblk; ++i) {
+        // items: K0, then K_(i+1)/2 for odd i, V_(i/2 - 1) for even i; the last item is the last V
+        const bool key = (i & 1) && (i + 1) / 2 < nblk;
+        const int j = key ? (i + 1) / 2 : ((i & 1) ? nblk - 1 : i / 2 - 1);
+        mbar_wait(&y_empty[s], ph, abort_flag, p.status, KID_ATTN, 1, i);
+        load_item(s, key ? &tma_k : &tma_v, kvh, j * BN);
+        if (++s == L::NY) { s = 0; ph ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (elect_one()) {
+      const uint32_t idesc_qk = make_idesc_bf16(ATT_M, BN, 0, 0), idesc_pv = make_idesc_bf16(ATT_M, p.Dmma, 0, 1);
+      const int ksteps = p.Dmma / 16;
+      int s = 2;
+      uint32_t ph = 0;
+      auto next = [&]() {
+        if (++s == L::NY) { s = 0; ph ^= 1; }
+      };
+      auto scores = [&](int j) {
+        mbar_wait(&y_full[s], ph, abort_flag, p.status, KID_ATTN, 2, j);
+        tc_fence_after();
+        // 16-byte units: a chunk of 64 columns is 8 KB, a step in it 32 bytes
+        const uint64_t bd = make_smem_desc(smem_u32(smem + s * L::Y_BYTES), 16, 1024);
+        const uint32_t d = tmem_base + L::TM_S + (j & 1) * BN, a = tmem_base + L::TM_Q;
+#pragma unroll
+        for (int kk = 0; kk < DPAD / 16; ++kk)
+          if (kk < ksteps) umma_ts(d, a + kk * 8, bd + (kk >> 2) * 512 + (kk & 3) * 2, idesc_qk, kk != 0 ? 1u : 0u);
+        umma_commit(&y_empty[s]);
+        umma_commit(&s_full[j & 1]);
+        next();
+      };
+      mbar_wait(q_full, 0, abort_flag, p.status, KID_ATTN, 4, 0);
+      tc_fence_after();
+      mbar_arrive(&y_empty[0]);                  // the query tile has been copied out of the ring
+      mbar_arrive(&y_empty[1]);
+      scores(0);
+      if (nblk > 1) scores(1);
+      for (int j = 0; j < nblk; ++j) {
+        const int buf = j & 1;
+        mbar_wait(&p_full[buf], (j >> 1) & 1, abort_flag, p.status, KID_ATTN, 5, j);
+        mbar_wait(&y_full[s], ph, abort_flag, p.status, KID_ATTN, 3, j);
+        tc_fence_after();
+        const uint64_t bd = make_smem_desc(smem_u32(smem + s * L::Y_BYTES), BN * 128, 1024);
+#pragma unroll
+        for (int kk = 0; kk < BN / 16; ++kk)
+          umma_ts(tmem_base + L::TM_O, tmem_base + L::TM_S + buf * BN + kk * 8, bd + kk * 128, idesc_pv, (j | kk) != 0 ? 1u : 0u);
+        umma_commit(&y_empty[s]);
+        umma_commit(&pv_done[buf]);
+        next();
+        if (j + 2 < nblk) {
+          mbar_wait(&pv_done[buf], (j >> 1) & 1, abort_flag, p.status, KID_ATTN, 11, j);
+          scores(j + 2);
+        }
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ softmax: group `grp` takes every second block, a thread a row
+    const int quad = warp & 3, grp = (warp - 2) >> 2, row = quad * 32 + lane;
+    const int pos = p0 + row / g, head = kvh * g + row % g;
+    const bool row_in = pos < p.Sq;
+    const bool q_ok = row_in && p.q_valid[(long long)b * p.Sq + pos] != 0;
+    const int qb = q_ok ? p.q_blk[(long long)b * p.Sq + pos] : INT_MIN;
+    const uint32_t lane_off = uint32_t(quad * 32) << 16;
+    const float scale = p.scale_log2;
+    {
+      // ---- the query tile into tensor memory: this thread's row, half of it
+      const uint8_t* y = smem + (row >> 6) * L::Y_BYTES + (row & 63) * 128;
+      mbar_wait(&y_full[row >> 6], 0, abort_flag, p.status, KID_ATTN, 12, 0);
+#pragma unroll
+      for (int c = 0; c < DPAD / 4; c += 32) {
+        uint32_t r[32];
+#pragma unroll
+        for (int e = 0; e < 32; e += 4) {
+          const int u8 = (grp * (DPAD / 4) + c + e) / 4;
+          const uint4 v = *reinterpret_cast<const uint4*>(y + (u8 >> 3) * (BN * 128) + ((u8 & 7) ^ (row & 7)) * 16);
+          r[e] = v.x; r[e + 1] = v.y; r[e + 2] = v.z; r[e + 3] = v.w;
+        }
+        __syncwarp();
+        tmem_st_x32(tmem_base + L::TM_Q + lane_off + grp * (DPAD / 4) + c, r);
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(q_full);
+    }
+    float m_used = -INFINITY;                    // maximum that O, and this thread's sum, are expressed against
+    float l = 0.f;
+    auto key_id = [&](int j, int h) {            // of this lane's key of the block's half h
+      const int key = j * BN + h * 32 + lane;
+      if (j >= nblk || key >= p.Sk) return INT_MAX;
+      const int kbv = p.k_blk[(long long)b * p.Sk + key];
+      const int kvv = p.k_valid[(long long)b * p.Sk + key];
+      return kvv ? kbv : INT_MAX;
+    };
+    // the maximum in use after block j, from the group that had it
+    auto follow = [&](int j) {
+      const int from = j & 1;
+      mbar_wait(&m_ready[from * 4 + quad], (j >> 1) & 1, abort_flag, p.status, KID_ATTN, 13, j);
+      const float m = m_pub[from * ATT_M + row];
+      if (m != m_used) {
+        l *= (m_used == -INFINITY) ? 0.f : fast_exp2(m_used - m);
+        m_used = m;
+      }
+    };
+    int nx0 = key_id(grp, 0), nx1 = key_id(grp, 1);
+    for (int j = grp; j < nblk; j += 2) {
+      const int kid[2] = {nx0, nx1};
+      // visibility of 32 keys: to every row, to no row, or a test each; `hidden` has a bit for each key this row does not see
+      bool all[2];
+      unsigned hidden[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int gmax = __reduce_max_sync(0xffffffffu, kid[h]);
+        all[h] = __all_sync(0xffffffffu, q_ok && gmax <= qb);
+        hidden[h] = 0;
+        if (!all[h]) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) hidden[h] |= (__shfl_sync(0xffffffffu, kid[h], e) <= qb ? 0u : 1u) << e;
+          if (!q_ok) hidden[h] = ~0u;
+        }
+      }
+      nx0 = key_id(j + 2, 0);
+      nx1 = key_id(j + 2, 1);
+      mbar_wait(&s_full[grp], (j >> 1) & 1, abort_flag, p.status, KID_ATTN, 6, j);
+      tc_fence_after();
+      const uint32_t s_addr = tmem_base + L::TM_S + grp * BN + lane_off;
+      uint32_t r[BN];
+      __syncwarp();
+      tmem_ld_x32(s_addr, r);
+      tmem_ld_x32(s_addr + 32, r + 32);
+      tmem_wait_ld();
+      float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};          // four chains instead of one
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (all[h]) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) m4[e & 3] = fmaxf(m4[e & 3], __uint_as_float(r[h * 32 + e]));
+        } else if (hidden[h] != ~0u) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (!(hidden[h] >> e & 1)) m4[e & 3] = fmaxf(m4[e & 3], __uint_as_float(r[h * 32 + e]));
+        }
+      }
+      const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * scale;      // scale > 0: max commutes with it
+      if (j > 0) follow(j - 1);
+      // lazy rescale: only where the maximum grew by more than 2^8 (warp-uniform: tensor memory is accessed by whole warps)
+      const float m_new = fmaxf(m_used, mx);
+      const bool want = (m_new > m_used + 8.0f) || (m_used == -INFINITY && m_new != -INFINITY);
+      float alpha = 1.f;
+      if (want) {
+        alpha = (m_used == -INFINITY) ? 0.f : fast_exp2(m_used - m_new);
+        m_used = m_new;
+      }
+      m_pub[grp * ATT_M + row] = m_used;
+      mbar_arrive(&m_ready[grp * 4 + quad]);
+      if (__any_sync(0xffffffffu, want) && j > 0) {
+        // O may only be touched once PV(j-1) has retired; PV(j) waits for this thread's P
+        mbar_wait(&pv_done[grp ^ 1], ((j - 1) >> 1) & 1, abort_flag, p.status, KID_ATTN, 8, j);
+        tc_fence_after();
+        const uint32_t o_addr = tmem_base + L::TM_O + lane_off;
+#pragma unroll 1
+        for (int c = 0; c < p.Dmma; c += 16) {
+          uint32_t ro[16];
+          __syncwarp();
+          tmem_ld_x16(o_addr + c, ro);
+          tmem_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) ro[e] = __float_as_uint(__uint_as_float(ro[e]) * alpha);
+          tmem_st_x16(o_addr + c, ro);
+        }
+        tmem_wait_st();
+      }
+      l *= alpha;
+      const float m_safe = (m_used == -INFINITY) ? 0.f : m_used;
+      float lsum[2] = {0.f, 0.f};
+      uint32_t packed[BN / 2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int e = 0; e < 32; e += 2) {
+          float a = fast_exp2(fmaf(__uint_as_float(r[h * 32 + e]), scale, -m_safe));
+          float z = fast_exp2(fmaf(__uint_as_float(r[h * 32 + e + 1]), scale, -m_safe));
+          if (!all[h]) {
+            if (hidden[h] >> e & 1) a = 0.f;
+            if (hidden[h] >> (e + 1) & 1) z = 0.f;
+          }
+          lsum[0] += a;
+          lsum[1] += z;
+          packed[h * 16 + (e >> 1)] = pack_bf16(a, z);
+        }
+      }
+      l += lsum[0] + lsum[1];
+      __syncwarp();
+      tmem_st_x32(s_addr, packed);               // over the scores of my own row, which are all in registers
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(&p_full[grp]);
+    }
+
+    // ---- epilogue: O / l -> bf16 -> global, LSE.  The two groups' sums meet in terms of the last maximum.
+    const int lastj = nblk - 1;
+    if ((lastj & 1) != grp) follow(lastj);
+    asm volatile("bar.sync 1, 256;" ::: "memory");       // nobody reads a maximum any more
+    m_pub[grp * ATT_M + row] = l;
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    l = m_pub[row] + m_pub[ATT_M + row];
+    mbar_wait(&pv_done[lastj & 1], (lastj >> 1) & 1, abort_flag, p.status, KID_ATTN, 9, 0);
+    tc_fence_after();
+    const float inv_l = l > 0.f ? 1.f / l : 0.f;
+    // a warp's 32 rows x half the width go through the ring, which nothing uses any more, and leave in whole pieces of a row:
+    // a thread's own row in 16-byte pieces takes twice the time of the rest of the epilogue
+    constexpr int LD = DPAD * 2 + 16;                    // bytes; the pad spreads the banks
+    uint8_t* orow = smem + row * LD + grp * DPAD;
+    const int cols = min(p.Dmma - grp * (DPAD / 2), DPAD / 2);
+#pragma unroll 1
+    for (int c = 0; c < cols; c += 16) {
+      uint32_t ro[16];
+      __syncwarp();
+      tmem_ld_x16(tmem_base + L::TM_O + lane_off + grp * (DPAD / 2) + c, ro);
+      tmem_wait_ld();
+#pragma unroll
+      for (int h8 = 0; h8 < 2; ++h8) {
+        uint4 o;
+        o.x = pack_bf16(__uint_as_float(ro[h8 * 8 + 0]) * inv_l, __uint_as_float(ro[h8 * 8 + 1]) * inv_l);
+        o.y = pack_bf16(__uint_as_float(ro[h8 * 8 + 2]) * inv_l, __uint_as_float(ro[h8 * 8 + 3]) * inv_l);
+        o.z = pack_bf16(__uint_as_float(ro[h8 * 8 + 4]) * inv_l, __uint_as_float(ro[h8 * 8 + 5]) * inv_l);
+        o.w = pack_bf16(__uint_as_float(ro[h8 * 8 + 6]) * inv_l, __uint_as_float(ro[h8 * 8 + 7]) * inv_l);
+        *reinterpret_cast<uint4*>(orow + c * 2 + h8 * 16) = o;
+      }
+    }
+    __syncwarp();
+    constexpr int LANES = DPAD / 16;                     // that write half a row
+    const int col = grp * (DPAD / 2) + lane % LANES * 8;
+#pragma unroll 4
+    for (int i = lane / LANES; i < 32; i += 32 / LANES) {
+      const int r = quad * 32 + i, rpos = p0 + r / g;
+      if (rpos < p.Sq && col < p.D)
+        *reinterpret_cast<uint4*>(p.o + (((long long)b * p.Sq + rpos) * p.H + kvh * g + r % g) * p.D + col) =
+            *reinterpret_cast<const uint4*>(smem + r * LD + col * 2);
+    }
+    if (row_in && grp == 0)
+      p.lse[((long long)b * p.H + head) * p.Sq + pos] = l > 0.f ? (m_used + log2f(l)) * 0.6931471805599453f : 0.f;
+    tc_fence_before();
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    if (*abort_flag) {
+      for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+    }
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
 // Merge of the split-KV partials: one warp per (batch, position, head) row.
 //   M = max_s m_s over splits with l_s > 0,  L = sum_s l_s 2^(m_s - M),  O = sum_s O_s 2^(m_s - M) / L
 __global__ void attn_combine_kernel(const float* __restrict__ part_o, const float2* __restrict__ part_ml,
@@ -727,6 +1114,21 @@ static int launch_attn(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
   e = launch_pdl(attn_combine_kernel, dim3((unsigned)((rows * 32 + 255) / 256)), dim3(256), 0, stream, 0u,
                  (const float*)p.part_o, (const float2*)p.part_ml, p.o, p.lse, p.nsplit, p.B, p.Sq, p.H, p.D);
   return (int)e;
+}
+
+template <int DPAD>
+static int launch_wide(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p, cudaStream_t stream) {
+  using L = WideSmem<DPAD>;
+  static bool configured = false;
+  auto kern = attn_fwd_wide_kernel<DPAD>;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  const int pos_per_tile = ATT_M / p.g;
+  return (int)launch_pdl(kern, dim3((p.Sq + pos_per_tile - 1) / pos_per_tile, p.Hkv, p.B), dim3(320), (size_t)L::TOTAL, stream, 0u,
+                         tq, tk, tv, p);
 }
 
 }  // namespace otb
@@ -826,7 +1228,9 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
   // what a launch requests ahead stays a quarter of L2
   const long long block_bytes = 4LL * bn * dpad * Hkv * B * nsplit;
   p.ahead = (int)((32LL << 20) / block_bytes);
-  int r = make_map4(&tq, q, D, H, Sq, B, q_sh, q_ss, q_sb, g, (cluster ? p.cl_rows : ATT_M) / g);
+  // unsplit, head width above 128 (64 rows of a query tile at a time: groups up to 64)
+  const bool wide = dpad == 256 && nsplit == 1 && g <= 64;
+  int r = make_map4(&tq, q, D, H, Sq, B, q_sh, q_ss, q_sb, g, (cluster ? p.cl_rows : (wide ? 64 : ATT_M)) / g);
   if (r) return 1000 + r;
   r = make_map4(&tk, k, D, Hkv, Sk, B, k_sh, k_ss, k_sb, 1, bn);
   if (r) return 2000 + r;
@@ -837,7 +1241,7 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
   switch (dpad) {
     case 64: return two ? launch_attn<64, 64, SPLIT_TWO>(tq, tk, tv, p, stream) : RUN(64, 128);
     case 128: return two ? launch_attn<128, 64, SPLIT_TWO>(tq, tk, tv, p, stream) : RUN(128, 128);
-    default: return RUN(256, 64);
+    default: return wide ? launch_wide<256>(tq, tk, tv, p, stream) : RUN(256, 64);
   }
 #undef RUN
 }

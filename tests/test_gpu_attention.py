@@ -391,6 +391,37 @@ def test_cluster_tiles_of_32_and_64_rows(B, Sq, Sk, H, Hkv, D):
     assert (lse.double() - torch.where(ref.isinf(), torch.zeros_like(ref), ref)).abs().max() < 1e-3
 
 
+@pytest.mark.parametrize("D,H,Hkv", [(256, 8, 1), (256, 8, 4), (200, 2, 2), (136, 64, 1)])
+@pytest.mark.parametrize("Sq,Sk", [(1, 1), (15, 64), (17, 65), (33, 128), (130, 129), (65, 300), (200, 513)])
+@pytest.mark.parametrize("big", [1.0, 12.0])
+def test_unsplit_forward_above_width_128(D, H, Hkv, Sq, Sk, big):
+    """Blocks that two groups of warps take in turn: one block, two, an odd and an even number; tiles with a row more or less; block ids
+    in no order, rows that see nothing, rows whose first visible key comes late; scores that make either group rescale.  Against
+    64 bits: P and the result are rounded to bf16 (2^-9 each)."""
+    from opentau_b200.ops import attention_native, cuda_ops
+    B = 2
+    g = torch.Generator(device="cuda").manual_seed(D + 7 * Sq + Sk)
+    q, k, v = (torch.randn(*shape, device="cuda", generator=g) for shape in ((B, Sq, H, D), (B, Sk, Hkv, D), (B, Sk, Hkv, D)))
+    k *= torch.linspace(0.1, big, Sk, device="cuda")[None, :, None, None]     # the maximum keeps growing
+    q, k, v = (t.to(torch.bfloat16) for t in (q, k, v))
+    qb = torch.randint(0, 6, (B, Sq), device="cuda", generator=g, dtype=torch.int32)
+    kb = torch.randint(0, 8, (B, Sk), device="cuda", generator=g, dtype=torch.int32)
+    kb[1, :Sk // 2] = 9
+    qv = torch.rand(B, Sq, device="cuda", generator=g) > 0.1
+    kv = torch.rand(B, Sk, device="cuda", generator=g) > 0.1
+    qb[0, :Sq // 3] = -1                                               # sees nothing
+    o, lse = attention_native.attn_fwd(q, k, v, qb, kb, qv, kv, D ** -0.5, nsplit=1)
+    cuda_ops.check_status()
+    see = qv[:, None, :, None] & kv[:, None, None, :] & (kb[:, None, None, :] <= qb[:, None, :, None])
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double().repeat_interleave(H // Hkv, 2)) * D ** -0.5
+    s = s.masked_fill(~see, -torch.inf)
+    want_lse = s.logsumexp(-1).nan_to_num(neginf=0.0)
+    p = (s - want_lse[..., None]).exp().masked_fill(~see, 0.0)
+    want = torch.einsum("bhqk,bkhd->bqhd", p, v.double().repeat_interleave(H // Hkv, 2)).reshape(B, Sq, H * D)
+    assert _rel(o, want) < 2 ** -8
+    assert float((lse.double() - want_lse).abs().max()) < 1e-4 * big ** 2 + 1e-5      # fp32 sums of scores up to about 5 big
+
+
 @pytest.mark.parametrize("D,H,Hkv,S", [(256, 8, 1, 513), (256, 2, 2, 1000), (200, 4, 4, 449), (136, 8, 4, 65), (128, 4, 2, 1025),
                                        (96, 2, 2, 129), (64, 8, 1, 900), (24, 4, 4, 1000), (16, 32, 1, 130)])
 def test_backward_with_fixed_tiles_in_tensor_memory(D, H, Hkv, S):
