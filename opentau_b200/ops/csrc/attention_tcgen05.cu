@@ -71,12 +71,15 @@ struct AttnSmem {
   static constexpr int OFF_RED = OFF_META + 2 * BN * 4;  // float red[2][128]: row max / row sum exchange
   static constexpr int OFF_KMM = OFF_RED + 2 * ATT_M * 4;  // int kmm[2][BN/32][2]: min / max block id per 32 keys
   static constexpr int OFF_BAR = OFF_KMM + 2 * (BN / 32) * 2 * 4;
-  static constexpr int NBAR = 16;
-  // a cluster's partials lie over the operand tiles: [row][DPAD + 4] floats (the pad spreads the banks and carries the
-  // row's maximum and sum), mine of all rows, then the peers' of the rows I own
+  static constexpr int NBAR = 17;
+  // a cluster's partials: [row][DPAD + 4] floats (the pad spreads the banks and carries the row's maximum and sum).  Mine of all
+  // rows and the peers' of the rows I own lie over the operand tiles; in a tile of DIRECT_ROWS the latter fit behind its query rows
+  static constexpr int DIRECT_ROWS = 32;
   static constexpr int PART_LD = DPAD + 4;
   static constexpr int OFF_PEER = CL_ROWS * PART_LD * 4;
   static_assert(SPLIT != SPLIT_CLUSTER || OFF_PEER + (CL_ROWS + 8) * PART_LD * 4 <= OFF_META, "the partials must fit over the operand tiles");
+  static_assert(SPLIT != SPLIT_CLUSTER || DIRECT_ROWS * DPAD * 2 + (DIRECT_ROWS + 8) * PART_LD * 4 <= OFF_KV, "and behind the query rows");
+  static_assert(SPLIT != SPLIT_CLUSTER || DIRECT_ROWS * PART_LD * 4 <= 2 * STAGE_BYTES, "mine over the keys and values");
   static constexpr int USED = OFF_BAR + NBAR * 8 + 32;
   // room for rounding the base up to 1024 bytes (the kernel has no static shared memory, so the base normally is
   // aligned already); capped at the 227 KB a CTA may own, and checked at run time
@@ -96,6 +99,64 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
+// The rows a CTA of a cluster owns, from the partials of all (mine and the peers', rows of DPAD + 4 floats): M = max m_s,
+// O = sum O_s 2^(m_s - M) / sum l_s 2^(m_s - M).  A warp to a row; every lane weighs the splits by itself and their loads are independent
+// of one another.  (Walking through it once ahead of the dependency wait, against its cold instruction cache, loses where a launch is
+// not resident before its predecessor ends: 8.9 -> 9.8 us in a row of these kernels.)
+template <int DPAD, int N>
+__device__ __forceinline__ void merge_rows(const AttnParams& p, const float* mine, const float* peers, int split, int rpr, int own, int t0,
+                                           int p0, int kvh, int b, int w, int lane) {
+  constexpr int LD = DPAD + 4, NV = DPAD / 128 < 1 ? 1 : DPAD / 128;       // four columns a lane, NV times
+#pragma unroll 1
+  for (int t = w; t < own; t += 8) {
+    float m_s[N], l_s[N], M = -INFINITY;
+    float4 v[N][NV];
+#pragma unroll
+    for (int sp = 0; sp < N; ++sp) {
+      m_s[sp] = -INFINITY;
+      l_s[sp] = 0.f;
+#pragma unroll
+      for (int c = 0; c < NV; ++c) v[sp][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (sp < p.nsplit) {
+        const float* src = sp == split ? mine + t * LD : peers + ((sp < split ? sp : sp - 1) * rpr + t) * LD;
+        const float2 ml = *reinterpret_cast<const float2*>(src + DPAD);
+        if (DPAD >= 128 || lane < DPAD / 4) {
+#pragma unroll
+          for (int c = 0; c < NV; ++c) v[sp][c] = *reinterpret_cast<const float4*>(src + c * 128 + lane * 4);
+        }
+        l_s[sp] = ml.y;
+        if (ml.y > 0.f) m_s[sp] = ml.x;
+      }
+      M = fmaxf(M, m_s[sp]);
+    }
+    float sum = 0.f;
+#pragma unroll
+    for (int sp = 0; sp < N; ++sp) {
+      m_s[sp] = m_s[sp] == -INFINITY ? 0.f : fast_exp2(m_s[sp] - M);       // its weight
+      sum += l_s[sp] * m_s[sp];
+    }
+    const float inv = sum > 0.f ? 1.f / sum : 0.f;
+    const int r = t0 + t, g = p.g, rpos = p0 + r / g, rhead = kvh * g + r % g;
+    __nv_bfloat16* orow = p.o + (((long long)b * p.Sq + rpos) * p.H + rhead) * p.D;
+#pragma unroll
+    for (int c = 0; c < NV; ++c) {
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int sp = 0; sp < N; ++sp) {
+        const float wt = m_s[sp] * inv;              // 0 where nothing is visible; a NaN there stays one
+        acc.x += v[sp][c].x * wt;
+        acc.y += v[sp][c].y * wt;
+        acc.z += v[sp][c].z * wt;
+        acc.w += v[sp][c].w * wt;
+      }
+      const int col = c * 128 + lane * 4;
+      if (col < p.D)
+        *reinterpret_cast<uint2*>(orow + col) = make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));
+    }
+    if (lane == 0)
+      p.lse[((long long)b * p.H + rhead) * p.Sq + rpos] = sum > 0.f ? (M + log2f(sum)) * 0.6931471805599453f : 0.f;
+  }
+}
 template <int DPAD, int BN, int SPLIT>
 __global__ void __launch_bounds__(320, attn_tsp(SPLIT) ? 2 : 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
@@ -112,7 +173,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   int* kmm = reinterpret_cast<int*>(smem + L::OFF_KMM);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
   uint64_t* q_full = bars + 0;
-  uint64_t* kv_full = bars + 1;    // [2]
+  uint64_t* k_full = bars + 1;     // [2]
   uint64_t* kv_empty = bars + 3;   // [2]
   uint64_t* s_full = bars + 5;     // [2]
   uint64_t* s_free = bars + 7;     // [2]
@@ -120,6 +181,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   uint64_t* p_free = bars + 11;    // [2]
   uint64_t* o_full = bars + 13;
   uint64_t* recv_bar = bars + 14;  // the peers' partials of my rows have landed (SPLIT_CLUSTER)
+  uint64_t* v_full = bars + 15;    // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NBAR);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* kv_end_smem = reinterpret_cast<int*>(tmem_slot + 2);
@@ -136,6 +198,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   const int kvh = CL ? blockIdx.y / p.nsplit : blockIdx.y, b = blockIdx.z;
   const int g = p.g;
   const int ROWS = CL ? p.cl_rows : ATT_M;
+  const int q_chunk = ROWS * 128;                    // bytes of the query tile's 64-column chunks
+  const bool direct = CL && ROWS == L::DIRECT_ROWS;  // peers send into room that no operand lies in
   const int pos_per_tile = ROWS / g;
   const int p0 = tile * pos_per_tile;
   // SPLIT_CLUSTER: the tile's valid rows, dealt to the CTAs in order; mine are [t0, t0 + own)
@@ -146,7 +210,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&kv_full[i], 1);
+      mbar_init(&k_full[i], 1);
+      mbar_init(&v_full[i], 1);
       mbar_init(&kv_empty[i], 1);
       mbar_init(&s_full[i], 1);
       mbar_init(&s_free[i], 256);
@@ -174,6 +239,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   const uint32_t tmem_S = tmem_base;            // two buffers of BN columns
   const uint32_t tmem_O = tmem_base + 2 * BN;   // Dmma columns
   pdl_launch_dependents();                      // after the TMEM allocation (see common.cuh)
+  if (direct) cluster_arrive();                 // waited for in front of the first copy to a peer: all have started
   if (CL && threadIdx.x == 0 && tile == 0) {
     // The cached keys and values have left L2 since the last pass: on their way while the preceding kernel finishes, requested
     // by the first tile of a kv head alone.  us with a norm in front, no requests / by every tile / by the first: 50 queries of 8
@@ -245,18 +311,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       mbar_expect_tx(q_full, L::Q_BYTES * ROWS / ATT_M);        // the rows past a smaller tile are never looked at
 #pragma unroll
       for (int c = 0; c < L::NCHUNK; ++c)
-        tma_load_4d(sQ + c * (ATT_M * 128), &tma_q, q_full, c * 64, kvh * g, p0, b);
+        tma_load_4d(sQ + c * q_chunk, &tma_q, q_full, c * 64, kvh * g, p0, b);
       for (int j = 0; j < nblk; ++j) {
         const int slot = j & 1, u = j >> 1;
         mbar_wait(&kv_empty[slot], (u & 1) ^ 1, abort_flag, p.status, KID_ATTN, 1, j);
         uint8_t* sk = sKV + slot * L::STAGE_BYTES;
         uint8_t* sv = sk + L::KV_TILE;
-        mbar_expect_tx(&kv_full[slot], L::STAGE_BYTES);
+        mbar_expect_tx(&k_full[slot], L::KV_TILE);
 #pragma unroll
-        for (int c = 0; c < L::NCHUNK; ++c) {
-          tma_load_4d(sk + c * (BN * 128), &tma_k, &kv_full[slot], c * 64, kvh, (jb0 + j) * BN, b);
-          tma_load_4d(sv + c * (BN * 128), &tma_v, &kv_full[slot], c * 64, kvh, (jb0 + j) * BN, b);
-        }
+        for (int c = 0; c < L::NCHUNK; ++c) tma_load_4d(sk + c * (BN * 128), &tma_k, &k_full[slot], c * 64, kvh, (jb0 + j) * BN, b);
+        mbar_expect_tx(&v_full[slot], L::KV_TILE);
+#pragma unroll
+        for (int c = 0; c < L::NCHUNK; ++c) tma_load_4d(sv + c * (BN * 128), &tma_v, &v_full[slot], c * 64, kvh, (jb0 + j) * BN, b);
       }
     }
   } else if (warp == 1) {
@@ -268,15 +334,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       const uint32_t q_addr = smem_u32(sQ);
       auto issue_qk = [&](int j) {
         const int slot = j & 1, u = j >> 1;
-        mbar_wait(&kv_full[slot], u & 1, abort_flag, p.status, KID_ATTN, 2, j);
+        mbar_wait(&k_full[slot], u & 1, abort_flag, p.status, KID_ATTN, 2, j);
         // TSP: the scores of block j - 2 gave way to their P.  Block j's keys are in the slot of block j - 2, which the
-        // producer filled behind the commit of the PV product that read that P: kv_full stands for both
+        // producer filled behind the commit of the PV product that read that P: k_full stands for both
         if (!TSP) mbar_wait(&s_free[slot], (u & 1) ^ 1, abort_flag, p.status, KID_ATTN, 3, j);
         tc_fence_after();
         const uint32_t k_addr = smem_u32(sKV + slot * L::STAGE_BYTES);
         for (int kk = 0; kk < ksteps_qk; ++kk) {
           const int c = kk >> 2, w = kk & 3;
-          uint64_t ad = make_smem_desc(q_addr + c * (ATT_M * 128) + w * 32, 16, 1024);
+          uint64_t ad = make_smem_desc(q_addr + c * q_chunk + w * 32, 16, 1024);
           uint64_t bd = make_smem_desc(k_addr + c * (BN * 128) + w * 32, 16, 1024);
           umma_ss(tmem_S + slot * BN, ad, bd, idesc_qk, kk != 0 ? 1u : 0u);
         }
@@ -288,6 +354,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         const int slot = j & 1, u = j >> 1;
         if (j + 1 < nblk) issue_qk(j + 1);
         mbar_wait(&p_full[slot], u & 1, abort_flag, p.status, KID_ATTN, 5, j);
+        mbar_wait(&v_full[slot], u & 1, abort_flag, p.status, KID_ATTN, 11, j);
         tc_fence_after();
         const uint32_t p_addr = smem_u32(sP + slot * L::P_BYTES);
         const uint32_t v_addr = smem_u32(sKV + slot * L::STAGE_BYTES + L::KV_TILE);
@@ -487,7 +554,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     tc_fence_after();
     const uint32_t o_addr = tmem_O + lane_off;
     if constexpr (CL) {
-      float* part = reinterpret_cast<float*>(smem);
+      // mine of all rows over operand tiles, which my own MMAs have left; the peers' of my rows in room of their own (32 rows), or
+      // over operand tiles as well once all have left them
+      float* part = reinterpret_cast<float*>(smem + (direct ? L::OFF_KV : 0));
+      float* peers = reinterpret_cast<float*>(smem + (direct ? L::NCHUNK * q_chunk : L::OFF_PEER));
       if (quad * 32 < rows_valid) {                  // warp-uniform; every MMA of mine has retired: the tiles are free
         float* dst = part + row * L::PART_LD;
 #pragma unroll 1
@@ -507,75 +577,25 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         if (half == 0) *reinterpret_cast<float2*>(dst + DPAD) = make_float2(m_used, l);
       }
       fence_async_smem();                            // the bulk copies read what was just written
-      cluster_arrive();                              // after my last MMA: peers may write over my tiles
+      if (!direct) cluster_arrive();                 // after my last MMA: peers may write over my tiles
       cluster_wait();
       asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (st < p.nsplit && st != split) {
-        const int cnt = min(rpr, rows_valid - st * rpr);
-        if (cnt > 0)
-          bulk_to_peer(map_rank(smem_u32(smem + L::OFF_PEER) + (uint32_t)((split < st ? split : split - 1) * rpr) * (L::PART_LD * 4u),
-                                (uint32_t)st),
-                       smem_u32(part + st * rpr * L::PART_LD), (uint32_t)cnt * (L::PART_LD * 4u),
-                       map_rank(smem_u32(recv_bar), (uint32_t)st));
+      {
+        const int owner = warp - 2;                  // a warp sends to one peer: lanes of one would go one after the other
+        const int cnt = owner < p.nsplit ? min(rpr, rows_valid - owner * rpr) : 0;
+        if (lane == 0 && owner != split && cnt > 0)
+          bulk_to_peer(map_rank(smem_u32(peers) + (uint32_t)((split < owner ? split : split - 1) * rpr) * (L::PART_LD * 4u),
+                                (uint32_t)owner),
+                       smem_u32(part + owner * rpr * L::PART_LD), (uint32_t)cnt * (L::PART_LD * 4u),
+                       map_rank(smem_u32(recv_bar), (uint32_t)owner));
+        __syncwarp();
       }
       if (own > 0) mbar_wait(recv_bar, 0, abort_flag, p.status, KID_ATTN, 10, 0);
       __syncwarp();
       cluster_arrive();                              // my rows have all arrived; waited for before leaving
-      const float* peers = reinterpret_cast<const float*>(smem + L::OFF_PEER);
-#pragma unroll 1
-      for (int t = warp - 2; t < own && !*abort_flag; t += 8) {
-        const auto slot_row = [&](int sp) {
-          return sp == split ? part + (t0 + t) * L::PART_LD : peers + ((sp < split ? sp : sp - 1) * rpr + t) * L::PART_LD;
-        };
-        // lane s < nsplit holds split s: (maximum, row sum); M = max m_s, O = sum O_s 2^(m_s - M) / sum l_s 2^(m_s - M)
-        float m_s = -INFINITY, l_s = 0.f;
-        if (lane < p.nsplit) {
-          const float2 ml = *reinterpret_cast<const float2*>(slot_row(lane) + DPAD);
-          l_s = ml.y;
-          m_s = ml.y > 0.f ? ml.x : -INFINITY;
-        }
-        float M = m_s;
-#pragma unroll
-        for (int off = 4; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));   // nsplit <= 8
-        const float w_s = (m_s == -INFINITY) ? 0.f : fast_exp2(m_s - M);
-        float sum = l_s * w_s;
-#pragma unroll
-        for (int off = 4; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-        M = __shfl_sync(0xffffffffu, M, 0);
-        sum = __shfl_sync(0xffffffffu, sum, 0);
-        const float inv = sum > 0.f ? 1.f / sum : 0.f;
-        float acc[DPAD / 32];
-#pragma unroll
-        for (int e = 0; e < DPAD / 32; ++e) acc[e] = 0.f;
-        constexpr int V = DPAD >= 128 ? 4 : 2;       // floats per lane and piece
-        for (int sp = 0; sp < p.nsplit; ++sp) {
-          const float w = __shfl_sync(0xffffffffu, w_s, sp) * inv;   // 0 where nothing is visible; a NaN there stays one
-          const float* src = slot_row(sp) + lane * V;
-#pragma unroll
-          for (int c = 0; c < DPAD / (32 * V); ++c) {
-            float v[V];
-            if (V == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(src + c * 32 * V);
-            else *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(src + c * 32 * V);
-#pragma unroll
-            for (int e = 0; e < V; ++e) acc[c * V + e] += v[e] * w;
-          }
-        }
-        const int r = t0 + t, rpos = p0 + r / g, rhead = kvh * g + r % g;
-        __nv_bfloat16* orow = p.o + (((long long)b * p.Sq + rpos) * p.H + rhead) * p.D;
-#pragma unroll
-        for (int c = 0; c < DPAD / (32 * V); ++c) {
-          const int colo = c * 32 * V + lane * V;
-          if (colo < p.D) {
-            if (V == 4)
-              *reinterpret_cast<uint2*>(orow + colo) =
-                  make_uint2(pack_bf16(acc[c * V], acc[c * V + 1]), pack_bf16(acc[c * V + V - 2], acc[c * V + V - 1]));
-            else
-              *reinterpret_cast<uint32_t*>(orow + colo) = pack_bf16(acc[c * V], acc[c * V + 1]);
-          }
-        }
-        if (lane == 0)
-          p.lse[((long long)b * p.H + rhead) * p.Sq + rpos] = sum > 0.f ? (M + log2f(sum)) * 0.6931471805599453f : 0.f;
-      }
+      const int rows = *abort_flag ? 0 : own;
+      if (p.nsplit <= 4) merge_rows<DPAD, 4>(p, part + t0 * L::PART_LD, peers, split, rpr, rows, t0, p0, kvh, b, warp - 2, lane);
+      else merge_rows<DPAD, 8>(p, part + t0 * L::PART_LD, peers, split, rpr, rows, t0, p0, kvh, b, warp - 2, lane);
     } else {
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
       __nv_bfloat16* orow = p.o + (((long long)b * p.Sq + pos) * p.H + head) * p.D;
@@ -626,7 +646,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
 
   if (CL && warp < 2) {
     __syncwarp();
-    cluster_arrive();
+    if (!direct) cluster_arrive();
     cluster_wait();
     cluster_arrive();
   }
