@@ -193,9 +193,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
       cluster_arrive();
     }
   } else {
-    const int wt = threadIdx.x - 64, ww = warp - 2;
-    pdl_wait();                                       // X, residual, gates and outputs belong to the predecessor
-    // ------------------------------------------------------------------ epilogue operands of my first token
+    const int ww = warp - 2;
     const int flags = EPI >= 0 ? EPI : p.flags;
     const bool glu = (flags & (SK_GLU_GELU | SK_GLU_SILU)) != 0;
     const int n = n0 + lane * 4;
@@ -209,70 +207,99 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
         res_v = *reinterpret_cast<const uint2*>(p.residual + (long long)m * p.ldr + n);
       }
     };
-    fetch_epi(ww);
     float bias_v[4] = {0.f, 0.f, 0.f, 0.f};
-    if ((flags & SK_BIAS) && n < p.N) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        bias_v[e] = (flags & SK_BIAS_F32) ? __ldg(static_cast<const float*>(p.bias) + n + e)
-                                          : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[n + e]);
-    }
-    // ------------------------------------------------------------------ TMEM -> my partial tile -> the tokens' owners
     const int quad = warp & 3;                        // TMEM lane quadrant this warp may read
-    const bool ok = mbar_wait(tfull_bar, 0, abort_flag, p.status, KID_SKINNY, 3, 0);
-    tc_fence_after();
-    {
-      const uint32_t taddr = tmem_base + (uint32_t(quad * 32) << 16);
-      float* col = own_part + quad * 32 + lane;       // weight row inside the tile
-      constexpr int CHUNK = MAXT > 64 ? 32 : 16;      // a chunk's tail past the last token is never looked at
-      const bool have = nkb > 0 && ok;                // a split without k-blocks (or one that gave up) sends zeros
+    bool ok = true;
+    // Everything from the accumulator to the output runs twice: a launch meets its code in a cold instruction cache (about nine
+    // cycles an instruction), so a first pass walks through it in front of the dependency wait, where these warps are idle. It
+    // reads tensor and shared memory whatever they hold, nothing of the predecessor's, and stores nothing.
 #pragma unroll 1
-      for (int c0 = (ww >> 2) * CHUNK; c0 < m_valid; c0 += 2 * CHUNK) {
-        uint32_t r[32];
-        __syncwarp();
-        if (CHUNK == 32) tmem_ld_x32(taddr + c0, r); else tmem_ld_x16(taddr + c0, r);
-        tmem_wait_ld();
-        if (!have) {
+    for (int pass = 0; pass < 2; ++pass) {
+      asm volatile("" : "+r"(pass));                  // one body for both passes
+      const bool live = pass != 0;
+      if (live) {
+        pdl_wait();                                   // X, residual, gates and outputs belong to the predecessor
+        // ---------------------------------------------------------------- epilogue operands of my first token
+        fetch_epi(ww);
+        if ((flags & SK_BIAS) && n < p.N) {
 #pragma unroll
-          for (int j = 0; j < CHUNK; ++j) r[j] = 0u;
+          for (int e = 0; e < 4; ++e)
+            bias_v[e] = (flags & SK_BIAS_F32) ? __ldg(static_cast<const float*>(p.bias) + n + e)
+                                              : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[n + e]);
         }
-        float* dst = col + c0 * SK_BW;
-#pragma unroll
-        for (int j = 0; j < CHUNK; ++j) dst[j * SK_BW] = __uint_as_float(r[j]);
+        if (S > 1) cluster_wait();                    // all have started: their buffers are there before the first copy
+        ok = mbar_wait(tfull_bar, 0, abort_flag, p.status, KID_SKINNY, 3, 0);
+        tc_fence_after();
       }
-    }
-    tc_fence_before();
-    if (S > 1) fence_async_smem();                    // the bulk copies read what the workers have just written
-    workers_sync();
-    if (S > 1) {
-      cluster_wait();
-      if (wt < S && wt != split) {
-        const int owner = wt, cnt = min(tpr, m_valid - owner * tpr);
-        if (cnt > 0)
-          bulk_to_peer(map_rank(smem_u32(peer_part) + (uint32_t)(split < owner ? split : split - 1) * (uint32_t)tpr * (SK_BW * 4u),
-                                (uint32_t)owner),
-                       smem_u32(own_part) + (uint32_t)(owner * tpr) * (SK_BW * 4u), (uint32_t)cnt * (SK_BW * 4u),
-                       map_rank(smem_u32(recv_bar), (uint32_t)owner));
-      }
-      if (own > 0) mbar_wait(recv_bar, 0, abort_flag, p.status, KID_SKINNY, 5, 0);
-      __syncwarp();
-      cluster_arrive();                               // my tokens have all arrived; waited for before leaving
-    }
-    // ------------------------------------------------------------------ reduction + epilogue of my tokens
-    if (!*abort_flag) {
+      // ------------------------------------------------------------------ TMEM -> my partial tile -> the tokens' owners
+      {
+        const uint32_t taddr = tmem_base + (uint32_t(quad * 32) << 16);
+        float* col = own_part + quad * 32 + lane;     // weight row inside the tile
+        constexpr int CHUNK = MAXT > 64 ? 32 : 16;    // a chunk's tail past the last token is never looked at
+        const bool have = nkb > 0 && ok;              // a split without k-blocks (or one that gave up) sends zeros
+        const int c_end = live ? m_valid : 1;
 #pragma unroll 1
-      for (int t = ww; t < own; t += SK_WORKERS / 32) {
+        for (int c0 = live ? (ww >> 2) * CHUNK : 0; c0 < c_end; c0 += 2 * CHUNK) {
+          uint32_t r[32];
+          __syncwarp();
+          if (CHUNK == 32) tmem_ld_x32(taddr + c0, r); else tmem_ld_x16(taddr + c0, r);
+          tmem_wait_ld();
+          if (!have) {
+#pragma unroll
+            for (int j = 0; j < CHUNK; ++j) r[j] = 0u;
+          }
+          float* dst = col + c0 * SK_BW;
+#pragma unroll
+          for (int j = 0; j < CHUNK; ++j)
+            if (live) dst[j * SK_BW] = __uint_as_float(r[j]);
+        }
+      }
+      if (live) {
+        tc_fence_before();
+        if (S > 1) fence_async_smem();                // the bulk copies read what the workers have just written
+        workers_sync();
+        if (S > 1) {
+          const int owner = ww;                       // a warp sends to one peer: a lane after the other would take 0.3 us
+          if (lane == 0 && owner < S && owner != split) {
+            const int cnt = min(tpr, m_valid - owner * tpr);
+            if (cnt > 0)
+              bulk_to_peer(map_rank(smem_u32(peer_part) + (uint32_t)(split < owner ? split : split - 1) * (uint32_t)tpr * (SK_BW * 4u),
+                                    (uint32_t)owner),
+                           smem_u32(own_part) + (uint32_t)(owner * tpr) * (SK_BW * 4u), (uint32_t)cnt * (SK_BW * 4u),
+                           map_rank(smem_u32(recv_bar), (uint32_t)owner));
+          }
+          __syncwarp();
+          if (own > 0) mbar_wait(recv_bar, 0, abort_flag, p.status, KID_SKINNY, 5, 0);
+          __syncwarp();
+          cluster_arrive();                           // my tokens have all arrived; waited for before leaving
+        }
+      }
+      // ------------------------------------------------------------------ reduction + epilogue of my tokens
+      const int t_end = live ? (*abort_flag ? 0 : own) : 1;
+#pragma unroll 1
+      for (int t = live ? ww : 0; t < t_end; t += SK_WORKERS / 32) {
         const int m = m_base + t0 + t;
         const uint2 rv = res_v, gv = gate_v;
-        fetch_epi(t + SK_WORKERS / 32);
+        if (live) fetch_epi(t + SK_WORKERS / 32);
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int s = 0; s < S; ++s) {
-          const float* part = s == split ? own_part + t0 * SK_BW : peer_part + (s < split ? s : s - 1) * tpr * SK_BW;
-          const float4 u = reinterpret_cast<const float4*>(part + t * SK_BW)[lane];
-          v.x += u.x;
-          v.y += u.y;
-          v.z += u.z;
-          v.w += u.w;
+#pragma unroll 1
+        for (int s0 = 0; s0 < S; s0 += 4) {           // four partials in flight, added in rank order
+          float4 u[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int s = s0 + i;
+            const float* part = s == split ? own_part + t0 * SK_BW : peer_part + (s < split ? s : s - 1) * tpr * SK_BW;
+            if (s < S) u[i] = reinterpret_cast<const float4*>(part + t * SK_BW)[lane];
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (s0 + i < S) {
+              v.x += u[i].x;
+              v.y += u[i].y;
+              v.z += u[i].z;
+              v.w += u[i].w;
+            }
+          }
         }
         const float f[4] = {v.x, v.y, v.z, v.w};
         if (!(flags & SK_NO_OUT)) {
@@ -293,11 +320,13 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
               o[0] += q0.x; o[1] += q0.y; o[2] += q1.x; o[3] += q1.y;
             }
             if (flags & SK_OUT_F32) {
-              *reinterpret_cast<float4*>(static_cast<float*>(p.out) + (long long)m * p.ldo + n) =
-                  make_float4(o[0], o[1], o[2], o[3]);
+              if (live)
+                *reinterpret_cast<float4*>(static_cast<float*>(p.out) + (long long)m * p.ldo + n) =
+                    make_float4(o[0], o[1], o[2], o[3]);
             } else {
-              *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.out) + (long long)m * p.ldo + n) =
-                  make_uint2(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]));
+              if (live)
+                *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.out) + (long long)m * p.ldo + n) =
+                    make_uint2(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]));
             }
           }
         }
@@ -311,7 +340,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
             const float g = __bfloat162float(__float2bfloat16(f[e]));
             o[e] = ((flags & SK_GLU_GELU) ? gelu_tanh_f(g) : silu_f(g)) * up;
           }
-          if (!(lane & 8) && n < p.N)
+          if (live && !(lane & 8) && n < p.N)
             *reinterpret_cast<uint2*>(p.out2 + (long long)m * p.ldo2 + (n0 >> 1) + (lane >> 4) * 32 + (lane & 7) * 4) =
                 make_uint2(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]));
         }
