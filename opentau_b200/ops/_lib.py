@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes
 import os
 import threading
+from functools import lru_cache
 from pathlib import Path
 
 from . import build as _build
@@ -32,6 +33,19 @@ def load(name: str) -> ctypes.CDLL:
         lib = ctypes.CDLL(str(path))
         _libs[name] = lib
         return lib
+
+
+_KINDS = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_longlong, "u": ctypes.c_ulonglong, "f": ctypes.c_float}
+
+
+@lru_cache(maxsize=None)
+def entry(lib: str, name: str, kinds: str):
+    """Entry point whose argument types (p pointer, i int, l long long, u unsigned long long, f float) are set once, so that calls
+    hand over plain numbers: boxing the twenty of a product takes 5.0 us against 3.3, forty of an attention 8.6 against 4.7, and steps
+    of a few hundred short launches are host time."""
+    fn = getattr(load(lib), name)
+    fn.argtypes = [_KINDS[k] for k in kinds]
+    return fn
 
 
 def loaded_libraries() -> list[str]:

@@ -44,17 +44,7 @@ def _prep(t: Tensor) -> Tensor:
     return t
 
 
-_KINDS = {"p": c_void_p, "i": c_int, "l": c_longlong, "f": c_float}
-
-
-@lru_cache(maxsize=None)
-def _entry(lib: str, name: str, kinds: str):
-    """Entry point whose argument types (p pointer, i int, l long long, f float) are set once, so that calls hand over plain
-    numbers: half the host time of boxing forty of them (8.6 -> 4.7 us), and calls of a few hundred positions are host
-    time."""
-    fn = getattr(_lib.load(lib), name)
-    fn.argtypes = [_KINDS[k] for k in kinds]
-    return fn
+_entry = _lib.entry
 
 
 def _ptr(t: Tensor | None) -> int:
@@ -176,7 +166,7 @@ def _attn_bwd_stored(samples: int, do, q, k, v, o, lse, qb, kb, qv, kv, dq, dk, 
     except torch.cuda.OutOfMemoryError:
         return False
     s0 = scratch.data_ptr()
-    fn = _entry_args("attention_bwd_stored_tcgen05", "otb_attn_bwd_stored")
+    fn = _entry("attention_bwd_stored_tcgen05", "otb_attn_bwd_stored", "pp")
     tensors = (q, k, v, o, do, lse, dq, dk, dv, qb, kb, qv, kv)
     step = [samples * t.stride(0) * t.element_size() for t in tensors]
     at = [t.data_ptr() for t in tensors]
@@ -194,13 +184,6 @@ def _attn_bwd_stored(samples: int, do, q, k, v, o, lse, qb, kb, qv, kv, dq, dk, 
         cuda_ops.launch_count += 3 + (m > 1)
         at = [x + d for x, d in zip(at, step)]
     return True
-
-
-@lru_cache(maxsize=None)
-def _entry_args(lib: str, name: str):
-    fn = getattr(_lib.load(lib), name)
-    fn.argtypes = [c_void_p, c_void_p]
-    return fn
 
 
 def attn_bwd(do: Tensor, q: Tensor, k: Tensor, v: Tensor, o: Tensor, lse: Tensor, q_blk: Tensor, k_blk: Tensor,

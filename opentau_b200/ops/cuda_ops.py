@@ -10,7 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import os
-from ctypes import c_float, c_int, c_longlong, c_void_p
+from ctypes import c_int, c_longlong, c_void_p
 
 import torch
 from torch import Tensor
@@ -25,13 +25,20 @@ EPI_GLU_GELU, EPI_GLU_SILU, EPI_BIAS_F32, EPI_NO_OUT, EPI_ACT_GELU, EPI_GATE = 1
 _status_ptr: dict[int, int] = {}
 
 
-def _stream() -> c_void_p:
+_call = _lib.entry
+
+
+def _raw_stream() -> int:
     # the handle alone: building a Stream object for every launch took a sixth of a small training step's host time
-    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def _p(t: Tensor | None) -> c_void_p:
-    return c_void_p(t.data_ptr()) if t is not None else c_void_p(0)
+def _stream() -> c_void_p:
+    return c_void_p(_raw_stream())
+
+
+def _ptr(t: Tensor | None) -> int | None:
+    return t.data_ptr() if t is not None else None
 
 
 def _check(rc: int, what: str) -> None:
@@ -92,10 +99,6 @@ class _SkinnyArgs(ctypes.Structure):
                 + [(n, c_int) for n in ("M", "N", "K", "rows_per_gate", "flags", "splits")])
 
 
-def _ptr(t: Tensor | None) -> int | None:
-    return t.data_ptr() if t is not None else None
-
-
 def _skinny_launch(x: Tensor, w: Tensor, out: Tensor | None, M: int, N: int, K: int, flags: int, *, bias=None,
                    residual=None, ldr: int = 0, out2=None, ldo2: int = 0, gate=None, gate_stride: int = 0,
                    rows_per_gate: int = 1, mod_idx=None, splits: int = 0) -> None:
@@ -103,7 +106,7 @@ def _skinny_launch(x: Tensor, w: Tensor, out: Tensor | None, M: int, N: int, K: 
     args = _SkinnyArgs(_ptr(x), _ptr(w), _ptr(out), _ptr(bias), _ptr(residual), _ptr(out2), _ptr(gate), _ptr(mod_idx),
                        status_pointer(), x.stride(0), w.stride(0), out.stride(0) if out is not None else N, ldr, ldo2,
                        gate_stride, M, N, K, rows_per_gate, flags, splits)
-    _check(_lib.load("gemm_skinny_tcgen05").otb_gemm_skinny_bf16(ctypes.byref(args), _stream()),
+    _check(_call("gemm_skinny_tcgen05", "otb_gemm_skinny_bf16", "pp")(ctypes.byref(args), _raw_stream()),
            f"gemm_skinny[{M}x{N}x{K}]")
     launch_count += 1
 
@@ -203,11 +206,9 @@ def gemm(a: Tensor, b: Tensor, layout: str, bias: Tensor | None = None, residual
         if glu is not None:
             return glu_out if not store_out else (out, glu_out)
         return out
-    rc = _lib.load("gemm_tcgen05").otb_gemm_bf16(
-        _p(a), _p(b), _p(out), c_int(M), c_int(N), c_int(K), c_longlong(a.stride(0)), c_longlong(b.stride(0)),
-        c_longlong(out.stride(0) if out is not None else N), c_int(a_mn), c_int(b_mn), _p(bias), _p(residual),
-        c_longlong(ldr), _p(glu_out), c_longlong(ldo2), c_int(flags), c_int(bn), c_void_p(status_pointer()),
-        _stream())
+    rc = _call("gemm_tcgen05", "otb_gemm_bf16", "pppiiillliipplpliipp")(
+        _ptr(a), _ptr(b), _ptr(out), M, N, K, a.stride(0), b.stride(0), out.stride(0) if out is not None else N,
+        a_mn, b_mn, _ptr(bias), _ptr(residual), ldr, _ptr(glu_out), ldo2, flags, bn, status_pointer(), _raw_stream())
     _check(rc, f"gemm[{layout} {M}x{N}x{K}]")
     launch_count += 1
     if glu is not None:
@@ -236,10 +237,9 @@ class RowNorm:
         y = torch.empty(R, H, dtype=x2.dtype, device=x2.device)
         wt = self.weight.to(torch.bfloat16).contiguous() if self.weight is not None else None
         mode = 0 if wt is None else (1 if self.unit_offset else 2)
-        _check(_lib.load("elementwise").otb_rms_fwd(
-            _p(x2), c_longlong(x2.stride(0)), _p(wt), _p(self.mod),
-            c_longlong(self.mod.stride(0) if self.mod is not None else 0), c_int(1), _p(self.idx), _p(y), c_void_p(0),
-            c_longlong(R), c_int(H), c_float(self.eps), c_int(mode), _stream()), "rms_fwd")
+        _check(_call("elementwise", "otb_rms_fwd", "plpplippplifip")(
+            _ptr(x2), x2.stride(0), _ptr(wt), _ptr(self.mod), self.mod.stride(0) if self.mod is not None else 0, 1,
+            _ptr(self.idx), _ptr(y), 0, R, H, self.eps, mode, _raw_stream()), "rms_fwd")
         launch_count += 1
         return y
 
@@ -277,9 +277,9 @@ def rows_linear(x: Tensor, w: Tensor, bias: Tensor | None = None, *, norm: RowNo
         if gate is not None:
             y = gemm(x, w, "nt", bias=bias)
             out = torch.empty_like(y)
-            _check(_lib.load("elementwise").otb_gated_residual(
-                _p(residual), _p(y), _p(gate), c_longlong(gate.stride(0)), c_int(1), _p(gated_by.idx), _p(out),
-                c_longlong(R), c_int(N), _stream()), "gated_residual")
+            _check(_call("elementwise", "otb_gated_residual", "ppplipplip")(
+                _ptr(residual), _ptr(y), _ptr(gate), gate.stride(0), 1, _ptr(gated_by.idx), _ptr(out), R, N,
+                _raw_stream()), "gated_residual")
             launch_count += 1
             return out
         if glu is not None:
@@ -320,9 +320,8 @@ def rms_fwd(x: Tensor, w: Tensor | None, eps: float, unit_offset: bool):
     rstd = torch.empty(R, dtype=torch.float32, device=x.device)
     mode = 0 if w is None else (1 if unit_offset else 2)
     wt = w.to(torch.bfloat16).contiguous() if w is not None else None
-    _check(_lib.load("elementwise").otb_rms_fwd(_p(x2), c_longlong(x2.stride(0)), _p(wt), c_void_p(0), c_longlong(0),
-                                                c_int(1), c_void_p(0), _p(y), _p(rstd), c_longlong(R), c_int(H), c_float(eps),
-                                                c_int(mode), _stream()), "rms_fwd")
+    _check(_call("elementwise", "otb_rms_fwd", "plpplippplifip")(
+        _ptr(x2), x2.stride(0), _ptr(wt), 0, 0, 1, 0, _ptr(y), _ptr(rstd), R, H, eps, mode, _raw_stream()), "rms_fwd")
     launch_count += 1
     return y.view(x.shape), rstd
 
@@ -351,16 +350,16 @@ def rms_bwd(dy: Tensor, x: Tensor, w: Tensor | None, rstd: Tensor, unit_offset: 
     rpb, nb = _bwd_blocks(R)
     partial = torch.empty(nb, H, dtype=torch.float32, device=x.device) if w is not None else None
     wt = w.to(torch.bfloat16).contiguous() if w is not None else None
-    lib = _lib.load("elementwise")
     dr = _dres_rows(dres, R, H)
-    _check(lib.otb_rms_bwd(_p(dy2), _p(x2), c_longlong(x2.stride(0)), _p(wt), c_void_p(0), c_longlong(0), c_int(1),
-                           _p(rstd), _p(dx), _p(partial), c_void_p(0), c_void_p(0), _p(dr), c_longlong(R), c_int(H),
-                           c_int(mode), c_int(rpb), _stream()), "rms_bwd")
+    _check(_call("elementwise", "otb_rms_bwd", "pplpplippppppliiip")(
+        _ptr(dy2), _ptr(x2), x2.stride(0), _ptr(wt), 0, 0, 1, _ptr(rstd), _ptr(dx), _ptr(partial), 0, 0, _ptr(dr), R,
+        H, mode, rpb, _raw_stream()), "rms_bwd")
     launch_count += 1
     dw = None
     if w is not None:
         dw = torch.empty(H, dtype=torch.bfloat16, device=x.device)
-        _check(lib.otb_colsum_partials(_p(partial), c_int(nb), c_int(H), _p(dw), c_int(0), _stream()), "colsum")
+        _check(_call("elementwise", "otb_colsum_partials", "piipip")(
+            _ptr(partial), nb, H, _ptr(dw), 0, _raw_stream()), "colsum")
         launch_count += 1
         dw = dw.to(w.dtype)
     return dx.view(x.shape), dw
@@ -376,9 +375,9 @@ def ada_rms_fwd(x: Tensor, mod: Tensor, eps: float):
     rows_per_mod = S if mod.dim() == 2 else 1
     y = torch.empty(R, H, dtype=x.dtype, device=x.device)
     rstd = torch.empty(R, dtype=torch.float32, device=x.device)
-    _check(_lib.load("elementwise").otb_rms_fwd(_p(x2), c_longlong(x2.stride(0)), c_void_p(0), _p(mod2),
-                                                c_longlong(mod2.stride(0)), c_int(rows_per_mod), c_void_p(0), _p(y), _p(rstd),
-                                                c_longlong(R), c_int(H), c_float(eps), c_int(0), _stream()),
+    _check(_call("elementwise", "otb_rms_fwd", "plpplippplifip")(
+        _ptr(x2), x2.stride(0), 0, _ptr(mod2), mod2.stride(0), rows_per_mod, 0, _ptr(y), _ptr(rstd), R, H, eps, 0,
+        _raw_stream()),
            "ada_rms_fwd")
     launch_count += 1
     return y.view(x.shape), rstd
@@ -396,10 +395,9 @@ def ada_rms_bwd(dy: Tensor, x: Tensor, mod: Tensor, rstd: Tensor, dres: Tensor |
     dx = torch.empty(R, H, dtype=x.dtype, device=x.device)
     dscale = torch.empty(R, H, dtype=x.dtype, device=x.device)
     dshift = torch.empty(R, H, dtype=x.dtype, device=x.device)
-    _check(_lib.load("elementwise").otb_rms_bwd(_p(dy2), _p(x2), c_longlong(x2.stride(0)), c_void_p(0), _p(mod2),
-                                                c_longlong(mod2.stride(0)), c_int(rows_per_mod), _p(rstd), _p(dx),
-                                                c_void_p(0), _p(dscale), _p(dshift), _p(_dres_rows(dres, R, H)),
-                                                c_longlong(R), c_int(H), c_int(0), c_int(1), _stream()), "ada_rms_bwd")
+    _check(_call("elementwise", "otb_rms_bwd", "pplpplippppppliiip")(
+        _ptr(dy2), _ptr(x2), x2.stride(0), 0, _ptr(mod2), mod2.stride(0), rows_per_mod, _ptr(rstd), _ptr(dx), 0,
+        _ptr(dscale), _ptr(dshift), _ptr(_dres_rows(dres, R, H)), R, H, 0, 1, _raw_stream()), "ada_rms_bwd")
     launch_count += 1
     dscale, dshift = dscale.view(B, S, H), dshift.view(B, S, H)
     if mod.dim() == 2:
@@ -415,9 +413,9 @@ def ln_fwd(x: Tensor, w: Tensor, b: Tensor, eps: float):
     y = torch.empty(R, H, dtype=x.dtype, device=x.device)
     mean = torch.empty(R, dtype=torch.float32, device=x.device)
     rstd = torch.empty(R, dtype=torch.float32, device=x.device)
-    _check(_lib.load("elementwise").otb_ln_fwd(_p(x2), _p(w.to(torch.bfloat16).contiguous()),
-                                               _p(b.to(torch.bfloat16).contiguous()), _p(y), _p(mean), _p(rstd),
-                                               c_longlong(R), c_int(H), c_float(eps), _stream()), "ln_fwd")
+    _check(_call("elementwise", "otb_ln_fwd", "pppppplifp")(
+        _ptr(x2), _ptr(w.to(torch.bfloat16).contiguous()), _ptr(b.to(torch.bfloat16).contiguous()), _ptr(y),
+        _ptr(mean), _ptr(rstd), R, H, eps, _raw_stream()), "ln_fwd")
     launch_count += 1
     return y.view(x.shape), mean, rstd
 
@@ -435,12 +433,13 @@ def ln_bwd(dy: Tensor, x: Tensor, w: Tensor, mean: Tensor, rstd: Tensor):
     dx = torch.empty(R, H, dtype=x.dtype, device=x.device)
     rpb, nb = _bwd_blocks(R)
     partial = torch.empty(2, nb, H, dtype=torch.float32, device=x.device)
-    lib = _lib.load("elementwise")
-    _check(lib.otb_ln_bwd(_p(dy2), _p(x2), _p(w.to(torch.bfloat16).contiguous()), _p(mean), _p(rstd), _p(dx),
-                          _p(partial[0]), _p(partial[1]), c_longlong(R), c_int(H), c_int(rpb), _stream()), "ln_bwd")
+    _check(_call("elementwise", "otb_ln_bwd", "ppppppppliip")(
+        _ptr(dy2), _ptr(x2), _ptr(w.to(torch.bfloat16).contiguous()), _ptr(mean), _ptr(rstd), _ptr(dx),
+        _ptr(partial[0]), _ptr(partial[1]), R, H, rpb, _raw_stream()), "ln_bwd")
     out = torch.empty(2, H, dtype=torch.bfloat16, device=x.device)
     for k in range(2):
-        _check(lib.otb_colsum_partials(_p(partial[k]), c_int(nb), c_int(H), _p(out[k]), c_int(0), _stream()), "colsum")
+        _check(_call("elementwise", "otb_colsum_partials", "piipip")(
+            _ptr(partial[k]), nb, H, _ptr(out[k]), 0, _raw_stream()), "colsum")
     launch_count += 3
     return dx.view(x.shape), out[0].to(w.dtype), out[1].to(w.dtype)
 
@@ -455,8 +454,8 @@ def glu_fwd(gu: Tensor, act: str) -> Tensor:
     if gu2.stride(0) != I2:
         gu2 = gu2.contiguous()
     h = torch.empty(M, I2 // 2, dtype=gu.dtype, device=gu.device)
-    _check(_lib.load("elementwise").otb_glu_fwd(_p(gu2), _p(h), c_longlong(M), c_int(I2 // 2), c_int(_ACT[act]),
-                                                _stream()), "glu_fwd")
+    _check(_call("elementwise", "otb_glu_fwd", "ppliip")(
+        _ptr(gu2), _ptr(h), M, I2 // 2, _ACT[act], _raw_stream()), "glu_fwd")
     launch_count += 1
     return h.view(*gu.shape[:-1], I2 // 2)
 
@@ -468,8 +467,8 @@ def glu_bwd(gu: Tensor, dh: Tensor, act: str, inplace: bool = False) -> Tensor:
         gu2 = gu2.contiguous()
     dh2 = dh.reshape(M, I2 // 2).contiguous()
     dgu = gu2 if inplace else torch.empty_like(gu2)
-    _check(_lib.load("elementwise").otb_glu_bwd(_p(gu2), _p(dh2), _p(dgu), c_longlong(M), c_int(I2 // 2),
-                                                c_int(_ACT[act]), _stream()), "glu_bwd")
+    _check(_call("elementwise", "otb_glu_bwd", "pppliip")(
+        _ptr(gu2), _ptr(dh2), _ptr(dgu), M, I2 // 2, _ACT[act], _raw_stream()), "glu_bwd")
     launch_count += 1
     return dgu.view(gu.shape)
 
@@ -485,9 +484,9 @@ def rope_fwd(x: Tensor, cos: Tensor, sin: Tensor, inverse: bool = False) -> Tens
         cos = cos.expand(B, S, D // 2).contiguous()
         sin = sin.expand(B, S, D // 2).contiguous()
     y = torch.empty(B, S, H, D, dtype=x.dtype, device=x.device)
-    _check(_lib.load("elementwise").otb_rope(_p(x), c_longlong(x.stride(0)), c_longlong(x.stride(1)),
-                                             c_longlong(x.stride(2)), _p(cos), _p(sin), _p(y), c_int(B), c_int(S),
-                                             c_int(H), c_int(D), c_int(int(inverse)), _stream()), "rope")
+    _check(_call("elementwise", "otb_rope", "plllpppiiiiip")(
+        _ptr(x), x.stride(0), x.stride(1), x.stride(2), _ptr(cos), _ptr(sin), _ptr(y), B, S, H, D, int(inverse),
+        _raw_stream()), "rope")
     launch_count += 1
     return y
 
@@ -507,22 +506,21 @@ def linear_ce_fwd(h: Tensor, w: Tensor, bias: Tensor | None, labels: Tensor):
     global launch_count
     R, V = h.shape[0], w.shape[0]
     labels = labels.contiguous()
-    lib = _lib.load("elementwise")
     if V <= CE_VOCAB_TILE:
         logits = gemm(h, w, "nt", bias=bias, out_dtype=torch.float32)
         loss = torch.empty(R, dtype=torch.float32, device=h.device)
         lse = torch.empty(R, dtype=torch.float32, device=h.device)
-        _check(lib.otb_ce_fwd(_p(logits), _p(labels), _p(loss), _p(lse), c_longlong(R), c_int(V), _stream()), "ce_fwd")
+        _check(_call("elementwise", "otb_ce_fwd", "pppplip")(
+            _ptr(logits), _ptr(labels), _ptr(loss), _ptr(lse), R, V, _raw_stream()), "ce_fwd")
         launch_count += 1
         return loss, lse
     m = torch.full((R,), float("-inf"), dtype=torch.float32, device=h.device)
     s = torch.zeros(R, dtype=torch.float32, device=h.device)
     tgt = torch.zeros(R, dtype=torch.float32, device=h.device)
-    tile_lib = _lib.load("train_elementwise")
     for c0, c1 in _ce_tiles(V):
         logits = gemm(h, w[c0:c1], "nt", bias=bias[c0:c1] if bias is not None else None, out_dtype=torch.float32)
-        _check(tile_lib.otb_ce_tile_fwd(_p(logits), _p(labels), c_longlong(c0), c_longlong(R), c_int(c1 - c0), _p(m),
-                                        _p(s), _p(tgt), _stream()), "ce_tile_fwd")
+        _check(_call("train_elementwise", "otb_ce_tile_fwd", "ppllipppp")(
+            _ptr(logits), _ptr(labels), c0, R, c1 - c0, _ptr(m), _ptr(s), _ptr(tgt), _raw_stream()), "ce_tile_fwd")
         launch_count += 1
         del logits
     lse = m + torch.log(s)
@@ -536,7 +534,6 @@ def linear_ce_bwd(dloss: Tensor, h: Tensor, w: Tensor, bias: Tensor | None, labe
     ``dw_into``: a ``(V, H)`` gradient buffer the weight gradient is ACCUMULATED into (then ``dw`` is None)."""
     global launch_count
     R, V = h.shape[0], w.shape[0]
-    lib = _lib.load("elementwise")
     labels = labels.contiguous()
     dl32 = dloss.float().contiguous()
     tiles = _ce_tiles(V)
@@ -548,8 +545,8 @@ def linear_ce_bwd(dloss: Tensor, h: Tensor, w: Tensor, bias: Tensor | None, labe
         logits = gemm(h, wc, "nt", bias=bias[c0:c1] if bias is not None else None, out_dtype=torch.float32)
         dlogits = torch.empty(R, c1 - c0, dtype=torch.bfloat16, device=h.device)
         lab = labels if c0 == 0 else labels - c0          # a label outside the tile matches no column
-        _check(lib.otb_ce_bwd(_p(logits), _p(lab), _p(lse), _p(dl32), _p(dlogits), c_longlong(R), c_int(c1 - c0),
-                              _stream()), "ce_bwd")
+        _check(_call("elementwise", "otb_ce_bwd", "ppppplip")(
+            _ptr(logits), _ptr(lab), _ptr(lse), _ptr(dl32), _ptr(dlogits), R, c1 - c0, _raw_stream()), "ce_bwd")
         launch_count += 1
         del logits
         if len(tiles) == 1:
@@ -574,11 +571,11 @@ def col_sum(a: Tensor) -> Tensor:
     rpb = max(1, (R + 255) // 256)
     nb = (R + rpb - 1) // rpb
     partial = torch.empty(nb, H, dtype=torch.float32, device=a.device)
-    lib = _lib.load("elementwise")
-    _check(lib.otb_colsum_bf16(_p(a2), c_longlong(R), c_int(H), c_longlong(a2.stride(0)), _p(partial), c_int(rpb),
-                               _stream()), "colsum_bf16")
+    _check(_call("elementwise", "otb_colsum_bf16", "plilpip")(
+        _ptr(a2), R, H, a2.stride(0), _ptr(partial), rpb, _raw_stream()), "colsum_bf16")
     out = torch.empty(H, dtype=torch.bfloat16, device=a.device)
-    _check(lib.otb_colsum_partials(_p(partial), c_int(nb), c_int(H), _p(out), c_int(0), _stream()), "colsum")
+    _check(_call("elementwise", "otb_colsum_partials", "piipip")(
+        _ptr(partial), nb, H, _ptr(out), 0, _raw_stream()), "colsum")
     launch_count += 2
     return out
 
@@ -586,15 +583,15 @@ def col_sum(a: Tensor) -> Tensor:
 # --------------------------------------------------------------------------------------------- optimizer
 def sumsq_partials(g: Tensor, partial: Tensor) -> None:
     global launch_count
-    _check(_lib.load("elementwise").otb_sumsq(_p(g), c_longlong(g.numel()), c_int(int(g.dtype == torch.bfloat16)),
-                                              _p(partial), c_int(partial.numel()), _stream()), "sumsq")
+    _check(_call("elementwise", "otb_sumsq", "plipip")(
+        _ptr(g), g.numel(), int(g.dtype == torch.bfloat16), _ptr(partial), partial.numel(), _raw_stream()), "sumsq")
     launch_count += 1
 
 
 def clip_coef(partial: Tensor, grad_scale: float, max_norm: float, out: Tensor) -> None:
     global launch_count
-    _check(_lib.load("elementwise").otb_clip_coef(_p(partial), c_int(partial.numel()), c_float(grad_scale),
-                                                  c_float(max_norm), _p(out), _stream()), "clip_coef")
+    _check(_call("elementwise", "otb_clip_coef", "piffpp")(
+        _ptr(partial), partial.numel(), grad_scale, max_norm, _ptr(out), _raw_stream()), "clip_coef")
     launch_count += 1
 
 
@@ -603,10 +600,9 @@ def adamw(p32: Tensor, g: Tensor, m: Tensor, v: Tensor, p16: Tensor | None, *, l
     global launch_count
     n = p32.numel()
     assert g.numel() == n and m.numel() == n and v.numel() == n
-    _check(_lib.load("elementwise").otb_adamw(_p(p32), _p(g), c_int(int(g.dtype == torch.bfloat16)), _p(m), _p(v),
-                                              _p(p16), c_longlong(n), c_float(lr), c_float(beta1), c_float(beta2),
-                                              c_float(eps), c_float(weight_decay), c_float(1.0 - beta1 ** step),
-                                              c_float(1.0 - beta2 ** step), _p(scale), _stream()), "adamw")
+    _check(_call("elementwise", "otb_adamw", "ppippplfffffffpp")(
+        _ptr(p32), _ptr(g), int(g.dtype == torch.bfloat16), _ptr(m), _ptr(v), _ptr(p16), n, lr, beta1, beta2, eps,
+        weight_decay, 1.0 - beta1 ** step, 1.0 - beta2 ** step, _ptr(scale), _raw_stream()), "adamw")
     launch_count += 1
 
 
@@ -618,8 +614,8 @@ def resize_with_pad(img: Tensor, width: int, height: int, pad_value: float = -1.
     rh, rw = int(Hin / ratio), int(Win / ratio)
     x = img.float().contiguous()
     out = torch.empty(N, C, height, width, dtype=torch.float32, device=img.device)
-    _check(_lib.load("elementwise").otb_resize_pad(_p(x), _p(out), c_int(N * C), c_int(Hin), c_int(Win), c_int(height),
-                                                   c_int(width), c_int(rh), c_int(rw), c_float(pad_value), _stream()),
+    _check(_call("elementwise", "otb_resize_pad", "ppiiiiiiifp")(
+        _ptr(x), _ptr(out), N * C, Hin, Win, height, width, rh, rw, pad_value, _raw_stream()),
            "resize_pad")
     launch_count += 1
     return out
@@ -634,9 +630,8 @@ def gated_residual(x: Tensor, y: Tensor, gate: Tensor) -> Tensor:
         g2 = g2.contiguous()
     rows_per_gate = (B * S) // g2.shape[0]
     out = torch.empty_like(x2)
-    _check(_lib.load("elementwise").otb_gated_residual(_p(x2), _p(y2), _p(g2), c_longlong(g2.stride(0)),
-                                                       c_int(rows_per_gate), c_void_p(0), _p(out), c_longlong(B * S), c_int(H),
-                                                       _stream()), "gated_residual")
+    _check(_call("elementwise", "otb_gated_residual", "ppplipplip")(
+        _ptr(x2), _ptr(y2), _ptr(g2), g2.stride(0), rows_per_gate, 0, _ptr(out), B * S, H, _raw_stream()), "gated_residual")
     launch_count += 1
     return out.view(x.shape)
 
@@ -663,11 +658,10 @@ def qkv_post(qkv: Tensor, H: int, Hkv: int, D: int, q_norm, k_norm, cos: Tensor,
     norm = q_norm is not None
     qw = q_norm.weight.to(qkv.dtype) if norm else None
     kw = k_norm.weight.to(qkv.dtype) if norm else None
-    _check(_lib.load("elementwise").otb_qkv_post(
-        _p(qkv), c_longlong(qkv.stride(1)), _p(qw), _p(kw), c_float(q_norm.eps if norm else 0.0),
-        c_int(int(q_norm.unit_offset) if norm else 0), _p(cos), _p(sin), _p(q), _p(k_dst), c_longlong(k_dst.stride(0)),
-        c_longlong(k_dst.stride(1)), _p(v_dst), c_longlong(v_dst.stride(0)), c_longlong(v_dst.stride(1)), c_int(B),
-        c_int(T), c_int(H), c_int(Hkv), c_int(D), _stream()), "qkv_post")
+    _check(_call("elementwise", "otb_qkv_post", "plppfippppllplliiiiip")(
+        _ptr(qkv), qkv.stride(1), _ptr(qw), _ptr(kw), q_norm.eps if norm else 0.0,
+        int(q_norm.unit_offset) if norm else 0, _ptr(cos), _ptr(sin), _ptr(q), _ptr(k_dst), k_dst.stride(0),
+        k_dst.stride(1), _ptr(v_dst), v_dst.stride(0), v_dst.stride(1), B, T, H, Hkv, D, _raw_stream()), "qkv_post")
     launch_count += 1
     return q, k_dst, v_dst
 
@@ -683,10 +677,9 @@ def patch_embed(pixels: Tensor, weight: Tensor, bias: Tensor, pos: Tensor, patch
     pixels = pixels.contiguous()
     weight, bias, pos = weight.float().contiguous(), bias.float().contiguous(), pos.float().contiguous()
     out = torch.empty(B, (H // patch) * (W // patch), N, dtype=out_dtype, device=pixels.device)
-    _check(_lib.load("elementwise").otb_patch_embed(
-        _p(pixels), c_int(int(pixels.dtype == torch.bfloat16)), _p(weight), _p(bias), _p(pos), _p(out),
-        c_int(int(out_dtype == torch.bfloat16)), c_int(B), c_int(C), c_int(H), c_int(W), c_int(patch), c_int(N),
-        _stream()), "patch_embed")
+    _check(_call("elementwise", "otb_patch_embed", "pippppiiiiiiip")(
+        _ptr(pixels), int(pixels.dtype == torch.bfloat16), _ptr(weight), _ptr(bias), _ptr(pos), _ptr(out),
+        int(out_dtype == torch.bfloat16), B, C, H, W, patch, N, _raw_stream()), "patch_embed")
     launch_count += 1
     return out
 
@@ -695,9 +688,8 @@ def time_embed(time: Tensor, dim: int, min_period: float, max_period: float, out
     global launch_count
     t = time.float().contiguous()
     out = torch.empty(*t.shape, dim, dtype=out_dtype, device=t.device)
-    _check(_lib.load("elementwise").otb_time_embed(_p(t), _p(out), c_longlong(t.numel()), c_int(dim),
-                                                   c_float(min_period), c_float(max_period),
-                                                   c_int(int(out_dtype == torch.bfloat16)), _stream()), "time_embed")
+    _check(_call("elementwise", "otb_time_embed", "ppliffip")(
+        _ptr(t), _ptr(out), t.numel(), dim, min_period, max_period, int(out_dtype == torch.bfloat16), _raw_stream()), "time_embed")
     launch_count += 1
     return out
 
@@ -715,9 +707,9 @@ def euler_step_(x: Tensor, v: Tensor, dt: float, frozen: Tensor | None = None, p
         fz = fz.view(torch.uint8) if fz.dtype == torch.bool else fz.to(torch.uint8)
         pf = prefix.float().contiguous()
     D = x.shape[-1]
-    _check(_lib.load("elementwise").otb_euler_step(_p(x), _p(v), c_int(int(v.dtype == torch.bfloat16)), c_float(dt),
-                                                   _p(fz), _p(pf), _p(x16), c_longlong(x.numel() // D), c_int(D),
-                                                   _stream()),
+    _check(_call("elementwise", "otb_euler_step", "ppifppplip")(
+        _ptr(x), _ptr(v), int(v.dtype == torch.bfloat16), dt, _ptr(fz), _ptr(pf), _ptr(x16), x.numel() // D, D,
+        _raw_stream()),
            "euler_step")
     launch_count += 1
     return x
@@ -728,8 +720,8 @@ def flow_interpolate(actions: Tensor, noise: Tensor, time: Tensor) -> tuple[Tens
     a, n, t = actions.float().contiguous(), noise.float().contiguous(), time.float().contiguous()
     x_t, u_t = torch.empty_like(a), torch.empty_like(a)
     D = a.shape[-1]
-    _check(_lib.load("elementwise").otb_flow_interpolate(_p(a), _p(n), _p(t), _p(x_t), _p(u_t),
-                                                         c_longlong(a.numel() // D), c_int(D), _stream()),
+    _check(_call("elementwise", "otb_flow_interpolate", "ppppplip")(
+        _ptr(a), _ptr(n), _ptr(t), _ptr(x_t), _ptr(u_t), a.numel() // D, D, _raw_stream()),
            "flow_interpolate")
     launch_count += 1
     return x_t, u_t
@@ -763,9 +755,8 @@ def dropout_residual_fwd(x: Tensor, y: Tensor, gate: Tensor | None, p: float, se
             g2 = g2.contiguous()
         stride, rpg = g2.stride(0), rows // g2.shape[0]
     out = torch.empty_like(x2)
-    _check(_lib.load("train_elementwise").otb_drop_res_fwd(
-        _p(x2), _p(y2), _p(g2), c_longlong(stride), c_int(rpg), _p(out), c_longlong(rows), c_int(H), c_float(p),
-        ctypes.c_ulonglong(seed), _stream()), "drop_res_fwd")
+    _check(_call("train_elementwise", "otb_drop_res_fwd", "pppliplifup")(
+        _ptr(x2), _ptr(y2), _ptr(g2), stride, rpg, _ptr(out), rows, H, p, seed, _raw_stream()), "drop_res_fwd")
     launch_count += 1
     return out.view(x.shape)
 
@@ -787,9 +778,8 @@ def dropout_residual_bwd(dout: Tensor, y: Tensor | None, gate: Tensor | None, p:
         y2 = y.reshape(-1, H)
         y2 = y2 if y2.is_contiguous() else y2.contiguous()
     dy = torch.empty_like(d2)
-    _check(_lib.load("train_elementwise").otb_drop_res_bwd(
-        _p(d2), _p(y2), _p(g2), c_longlong(stride), c_int(rpg), _p(dy), _p(dgate), c_longlong(rows), c_int(H),
-        c_float(p), ctypes.c_ulonglong(seed), _stream()), "drop_res_bwd")
+    _check(_call("train_elementwise", "otb_drop_res_bwd", "ppplipplifup")(
+        _ptr(d2), _ptr(y2), _ptr(g2), stride, rpg, _ptr(dy), _ptr(dgate), rows, H, p, seed, _raw_stream()), "drop_res_bwd")
     launch_count += 1
     return dy.view(dout.shape), dgate
 
@@ -800,8 +790,8 @@ def masked_mse_fwd(u: Tensor, v: Tensor, frozen: Tensor | None, pad: Tensor | No
     B, T, D = u.shape
     sums = torch.empty(B, dtype=torch.float32, device=u.device)
     counts = torch.empty(B, dtype=torch.float32, device=u.device)
-    _check(_lib.load("train_elementwise").otb_masked_mse_fwd(_p(u), _p(v), _p(frozen), _p(pad), _p(real_dim), c_int(B),
-                                                             c_int(T), c_int(D), _p(sums), _p(counts), _stream()),
+    _check(_call("train_elementwise", "otb_masked_mse_fwd", "pppppiiippp")(
+        _ptr(u), _ptr(v), _ptr(frozen), _ptr(pad), _ptr(real_dim), B, T, D, _ptr(sums), _ptr(counts), _raw_stream()),
            "masked_mse_fwd")
     launch_count += 1
     return sums, counts
@@ -812,8 +802,8 @@ def masked_mse_bwd(u: Tensor, v: Tensor, frozen: Tensor | None, pad: Tensor | No
     global launch_count
     B, T, D = u.shape
     dv = torch.empty_like(v)
-    _check(_lib.load("train_elementwise").otb_masked_mse_bwd(_p(u), _p(v), _p(frozen), _p(pad), _p(real_dim), c_int(B),
-                                                             c_int(T), c_int(D), _p(coef), _p(dv), _stream()),
+    _check(_call("train_elementwise", "otb_masked_mse_bwd", "pppppiiippp")(
+        _ptr(u), _ptr(v), _ptr(frozen), _ptr(pad), _ptr(real_dim), B, T, D, _ptr(coef), _ptr(dv), _raw_stream()),
            "masked_mse_bwd")
     launch_count += 1
     return dv
@@ -824,8 +814,8 @@ def embed_fwd(table: Tensor, ids: Tensor, scale: float) -> Tensor:
     H = table.shape[1]
     flat = ids.reshape(-1).to(torch.int64).contiguous()
     out = torch.empty(flat.numel(), H, dtype=table.dtype, device=table.device)
-    _check(_lib.load("train_elementwise").otb_embed_fwd(_p(table), _p(flat), _p(out), c_longlong(flat.numel()), c_int(H),
-                                                        c_longlong(table.shape[0]), c_float(scale), _stream()),
+    _check(_call("train_elementwise", "otb_embed_fwd", "ppplilfp")(
+        _ptr(table), _ptr(flat), _ptr(out), flat.numel(), H, table.shape[0], scale, _raw_stream()),
            "embed_fwd")
     launch_count += 1
     return out.view(*ids.shape, H)
@@ -843,9 +833,9 @@ def embed_bwd(dout: Tensor, ids: Tensor, grad: Tensor, scale: float, padding_idx
         return
     d2 = dout.reshape(-1, H)
     d2 = d2 if d2.is_contiguous() else d2.contiguous()
-    _check(_lib.load("train_elementwise").otb_embed_bwd(
-        _p(d2), _p(sorted_ids), _p(order), c_longlong(n), _p(grad), c_int(int(grad.dtype == torch.float32)), c_int(H),
-        c_longlong(grad.shape[0]), c_longlong(-1 if padding_idx is None else padding_idx), c_float(scale), _stream()),
+    _check(_call("train_elementwise", "otb_embed_bwd", "ppplpiillfp")(
+        _ptr(d2), _ptr(sorted_ids), _ptr(order), n, _ptr(grad), int(grad.dtype == torch.float32), H, grad.shape[0],
+        -1 if padding_idx is None else padding_idx, scale, _raw_stream()),
         "embed_bwd")
     launch_count += 1
 
@@ -857,8 +847,8 @@ def pos_resample(table: Tensor, gh: int, gw: int) -> Tensor:
     g = int(math.isqrt(table.shape[0]))
     tab = table.detach().float().contiguous()
     out = torch.empty(gh * gw, tab.shape[1], dtype=torch.float32, device=tab.device)
-    _check(_lib.load("train_elementwise").otb_pos_resample(_p(tab), c_int(g), c_int(tab.shape[1]), _p(out), c_int(gh),
-                                                           c_int(gw), _stream()), "pos_resample")
+    _check(_call("train_elementwise", "otb_pos_resample", "piipiip")(
+        _ptr(tab), g, tab.shape[1], _ptr(out), gh, gw, _raw_stream()), "pos_resample")
     launch_count += 1
     return out
 
@@ -870,9 +860,8 @@ def seq_concat(a: Tensor, c: Tensor) -> Tensor:
     B, S1, S2 = a.shape[0], a.shape[1], c.shape[1]
     E = a[0, 0].numel() if S1 else c[0, 0].numel()
     out = torch.empty(B, S1 + S2, *a.shape[2:], dtype=a.dtype, device=a.device)
-    _check(_lib.load("train_elementwise").otb_seq_concat(
-        _p(a), c_longlong(a.stride(0)), c_longlong(a.stride(1)), _p(c), c_longlong(c.stride(0)), c_longlong(c.stride(1)),
-        _p(out), c_longlong(B), c_int(S1), c_int(S2), c_int(E), _stream()), "seq_concat")
+    _check(_call("train_elementwise", "otb_seq_concat", "pllpllpliiip")(
+        _ptr(a), a.stride(0), a.stride(1), _ptr(c), c.stride(0), c.stride(1), _ptr(out), B, S1, S2, E, _raw_stream()), "seq_concat")
     launch_count += 1
     return out
 
@@ -884,7 +873,7 @@ def zero_(t: Tensor) -> Tensor:
     if not (t.is_cuda and t.is_contiguous() and t.numel() > 0):
         return t.zero_()
     from ctypes import c_ulonglong
-    _check(_lib.load("train_elementwise").otb_zero_bytes(_p(t), c_ulonglong(t.numel() * t.element_size()), _stream()),
+    _check(_call("train_elementwise", "otb_zero_bytes", "pup")(_ptr(t), t.numel() * t.element_size(), _raw_stream()),
            "zero_bytes")
     launch_count += 1
     return t

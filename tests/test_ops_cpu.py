@@ -298,7 +298,7 @@ def test_stored_attention_backward_refuses_misaligned_tensors_before_any_launch(
     from opentau_b200.ops import attention_native, build
     if not build.lib_path("attention_bwd_stored_tcgen05").exists():
         pytest.skip("native libraries are not built")
-    fn = attention_native._entry_args("attention_bwd_stored_tcgen05", "otb_attn_bwd_stored")
+    fn = attention_native._entry("attention_bwd_stored_tcgen05", "otb_attn_bwd_stored", "pp")
     names = [n for n, _ in attention_native._StoredBwdArgs._fields_][:19]
     base = {n: 1 << 20 for n in names}
     base[which] += 8
