@@ -74,9 +74,14 @@ def split_kv(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int) -> int:
 def split_cluster(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int) -> int:
     """CTAs of the cluster that shares the keys of a 64-row query tile and merges on chip (1: not this path)."""
     g = H // Hkv
-    if g > 64 or 64 % g or -(-Sk // (64 if D > 128 else 128)) < 3:
+    nblk = -(-Sk // (64 if D > 128 else 128))
+    if g > 64 or 64 % g or nblk < 3:
         return 1
-    return _lib.load("attention_tcgen05").otb_attn_cluster_fit(c_int(D), c_longlong(-(-Sq // (64 // g)) * Hkv * B))
+    n = _lib.load("attention_tcgen05").otb_attn_cluster_fit(c_int(D), c_longlong(-(-Sq // (64 // g)) * Hkv * B))
+    # pairs win where their streams are short: 56 tiles of 8 heads on 1 of 256 against 200, 400, 640 and 1018 keys 9.8, 13.2, 14.9 and
+    # 19.8 us (best of one pass and a merge through global memory: 11.1, 14.1, 17.2, 20.5), 1500 and 3000 keys 25.1 / 22.6 and 45.1 / 33.5;
+    # up to a width of 128 they lose on both ends (64 tiles of 64 against 300 9.6 / 8.0, of 128 against 2000 20.5 / 17.1)
+    return 1 if n == 2 and (D <= 128 or nblk > 16) else n
 
 
 def attn_fwd(q: Tensor, k: Tensor, v: Tensor, q_blk: Tensor, k_blk: Tensor, q_valid: Tensor, k_valid: Tensor,

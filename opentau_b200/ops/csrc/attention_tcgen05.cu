@@ -1287,13 +1287,13 @@ extern "C" int otb_attn_fwd_splitkv(const void* q, const void* k, const void* v,
                        k_ss, k_sh, v_sb, v_ss, v_sh, scale, nsplit, part_o, part_ml, status, stream);
 }
 
-// CTAs per cluster for `tiles` tiles of 64 rows (the launch may then halve the tiles): the most (up to 8) whose clusters are all resident at once, since a second
-// round costs more than anything a larger cluster saves; 1 if that leaves fewer than 3.  Measured at 50 queries of 8 heads
-// on 1, width 256, against the merge through global memory: 10.5 us against 17.2 (7 tiles, 1018 keys, 8 CTAs), 12.5 against
-// 17.0 (28 tiles, 639 keys, 4), 16.9 against 19.7 (42 tiles, 900 keys, 3); pairs gain nothing (56 tiles: 20.4 against 20.2)
-// and clusters that do not fit lose (28 tiles with 8: 20.5).  One query: 7.6 against 11.4 us.
+// CTAs per cluster for `tiles` tiles of 64 rows (the launch may then halve the tiles): the most (up to 8) whose clusters are all
+// resident at once, since a second round costs more than anything a larger cluster saves; 1 if not even pairs are.  Measured at 50
+// queries of 8 heads on 1, width 256, against the best of one pass and a merge through global memory, us: 7 tiles, 1018 keys, 8 CTAs
+// 8.1 / 17; 28 tiles, 639 keys, 4 11.7 / 17.1; 42 tiles, 900 keys, 3 15.6 / 20.1; pairs, 70 tiles of 560 and 1018 keys 15.2 / 16.3 and
+// 20.1 / 23.2 (the caller says where pairs lose).  Clusters that do not fit lose (28 tiles with 8: 20.5).
 extern "C" int otb_attn_cluster_fit(int D, long long tiles) {
-  for (int n = 8; n >= 3; --n)
+  for (int n = 8; n >= 2; --n)
     if (cluster_fits(D, n, tiles)) return n;
   return 1;
 }
