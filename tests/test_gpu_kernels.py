@@ -194,6 +194,24 @@ def test_layer_norm_kernel(dev):
     torch.testing.assert_close(mean.cpu(), mr, rtol=1e-3, atol=1e-4)
 
 
+@pytest.mark.parametrize("rows,H", [(1, 8), (5, 256), (7, 264), (2047, 1152), (2048, 1152), (2049, 1160), (2050, 2048), (2048, 2056),
+                                    (4097, 1024), (2051, 520)])
+def test_layer_norm_forward_at_the_edges_of_its_forms(dev, rows, H):
+    """A warp or a block to a row, the last block's rows, widths with a partial piece, against 64 bits: sums in fp32 (1e-5) and one
+    rounding to bf16 (2^-9)."""
+    from opentau_b200.ops import cuda_ops
+    g = torch.Generator(device=dev).manual_seed(rows + H)
+    x, w, b = (torch.randn(*s, device=dev, generator=g).to(torch.bfloat16) for s in ((rows, H), (H,), (H,)))
+    x += 3.0
+    y, mean, rstd = cuda_ops.ln_fwd(x, w, b, 1e-6)
+    xd = x.double()
+    want_mean, var = xd.mean(-1), xd.var(-1, unbiased=False)
+    want = (xd - want_mean[:, None]) * (var + 1e-6).rsqrt()[:, None] * w.double() + b.double()
+    torch.testing.assert_close(mean.double().view(-1), want_mean, rtol=1e-5, atol=1e-5)
+    torch.testing.assert_close(rstd.double().view(-1), (var + 1e-6).rsqrt(), rtol=1e-4, atol=0)
+    assert float((y.double() - want).norm() / want.norm()) < 2 ** -8
+
+
 @pytest.mark.parametrize("D", [64, 72])     # 72: Qwen3-VL vision heads (8-byte accesses)
 def test_rope_kernel_strided(dev, D):
     from opentau_b200 import ops
