@@ -72,9 +72,11 @@ def check_status(reset: bool = True) -> None:
 SKINNY = os.environ.get("OPENTAU_B200_SKINNY_GEMM", "1") != "0"
 
 
-def use_skinny(layout: str, M: int, N: int, accumulate: bool, bn: int, K: int = 0, gated: bool = True) -> bool:
+def use_skinny(layout: str, M: int, N: int, accumulate: bool, bn: int, K: int = 0, gated: bool = True,
+               end: str = "") -> bool:
     """``x @ W^T`` with few rows goes to the weight-streaming split-K kernel.  ``gated``: the product ends in a gated
-    residual, which only that kernel fuses (the gate then multiplies the fp32 sum)."""
+    residual, which only that kernel fuses (the gate then multiplies the fp32 sum); ``end``: "act" or "glu" where it ends in an
+    activation or a gated MLP's product."""
     if not SKINNY or layout != "nt" or accumulate or bn:
         return False
     if gated:
@@ -83,12 +85,16 @@ def use_skinny(layout: str, M: int, N: int, accumulate: bool, bn: int, K: int = 
         # may share the sums of 64-row chunks: 400 x 1024 x 4096 20.6 -> 12.4 us with the norm behind it against the persistent
         # kernel and a gated residual of its own, 640 x 1280 x 2048 15.0 -> 12.0; without the room 600 x 2048 x 2048 16.3 -> 17.3
         return M <= 128 or (M <= 256 and N <= 8192) or (M <= 640 and N <= 2048 and -(-N // 128) * -(-M // 64) <= 148)
-    # measured inside a replayed graph: up to 64 rows the split-K kernel always wins (50 x 8192 x 1024 6.4 us against
-    # 9.1, 50 x 1024 x 4096 6.0 against 16.2); at 65..256 rows it is taken where the persistent kernel has too few tiles for
-    # the chip and a long sum (with a norm behind it 200 x 1024 x 4096 9.1 us against 18.1).  That line was drawn for one wide
-    # tile of all rows; with the plans as they are shorter sums would gain a little as well (200 x 1024 x 2048 7.6 against 11.7,
-    # 256 x 768 x 768 6.2 against 7.8, 200 x 2560 x 1024 8.1 against 9.7), many columns would not (200 x 8192 x 1024 14.0 against 13.7)
-    return M <= 64 or (M <= 256 and N <= 2048 and K >= 3072)
+    if M <= 64 or (M <= 256 and N <= 2048 and K >= 3072):
+        return True
+    # Up to one CTA of 128 columns x 64 rows to an SM: us in a replayed graph with a norm in front and cold weights, few-row /
+    # persistent kernel: 100 x 1024 x 1024 5.7 / 8.1, 200 x 2560 x 1024 7.5 / 8.8, 256 x 4096 x 2048 12.5 / 12.8, 400 x 2560 x 1024 9.2 / 10.3, 400 x
+    # 1152 x 4096 13.4 / 19.6, 512 x 2048 x 2048 12.7 / 12.9, 768 x 1152 x 4096 14.5 / 20.2, 768 x 768 x 256 6.3 / 6.7; of 570 sizes of 65 - 768 rows, 256 -
+    # 6144 columns, K 128 - 4096 within this line it loses more than a hundredth at eight (4 % at most).  Beyond it: 512 x 3456 x 1024 11.6 /
+    # 11.1, 640 x 2560 x 2048 15.5 / 14.6, 768 x 4096 x 1024 14.7 / 12.9, 200 x 6144 x 1024 11.1 / 10.8; more columns lose from 65 rows on
+    # (100 x 8192 x 1024 9.8 / 8.9).  With an activation at the end it wins on half as many tiles (256 x 1024 x 1024 7.2 / 9.4, 128 x 4304 x 1152
+    # 8.7 / 10.1, 256 x 4304 x 1152 11.4 / 10.6), with a gated MLP's product on narrow ones alone (200 x 4096 x 1024 10.2 / 9.8)
+    return end != "glu" and M <= 768 and N <= 6144 and -(-N // 128) * -(-M // 64) <= (74 if end else 148)
 
 
 class _SkinnyArgs(ctypes.Structure):
@@ -185,7 +191,8 @@ def gemm(a: Tensor, b: Tensor, layout: str, bias: Tensor | None = None, residual
         ldo2 = glu_out.stride(0)
     if splits and (layout != "nt" or accumulate):
         raise ValueError("the split-K kernel computes a @ b^T without accumulation")
-    skinny = bool(splits) or use_skinny(layout, M, N, accumulate, bn, K, gate is not None)
+    skinny = bool(splits) or use_skinny(layout, M, N, accumulate, bn, K, gate is not None,
+                                       "glu" if glu is not None else "act" if act is not None else "")
     g_stride, g_rows = 0, 1
     if gate is not None:
         # out = residual + gate * (a @ b^T): rows of N gates, one per `M / gate rows` consecutive output rows
@@ -273,7 +280,7 @@ def rows_linear(x: Tensor, w: Tensor, bias: Tensor | None = None, *, norm: RowNo
         if bias.numel() != N or bias.dtype not in (torch.bfloat16, torch.float32):
             raise ValueError("bad bias for rows_linear")
         bias = bias.contiguous()
-    if not use_skinny("nt", R, N, False, 0, K, gate is not None):
+    if not use_skinny("nt", R, N, False, 0, K, gate is not None, "glu" if glu is not None else ""):
         if gate is not None:
             y = gemm(x, w, "nt", bias=bias)
             out = torch.empty_like(y)

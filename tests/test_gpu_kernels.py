@@ -194,6 +194,28 @@ def test_layer_norm_kernel(dev):
     torch.testing.assert_close(mean.cpu(), mr, rtol=1e-3, atol=1e-4)
 
 
+@pytest.mark.parametrize("M,N,K", [(65, 6144, 128), (192, 6144, 72), (193, 6144, 72), (256, 4096, 264), (257, 4096, 136), (320, 3456, 1152),
+                                   (321, 3456, 128), (577, 2048, 200), (576, 2048, 200), (768, 1152, 264), (769, 1152, 264), (768, 8, 8)])
+@pytest.mark.parametrize("end", ["plain", "bias_res", "f32", "gelu"])
+def test_products_at_the_line_between_the_two_kernels(dev, M, N, K, end):
+    """Rows and columns on either side of the line, against 64 bits: operands are bf16, sums fp32, one rounding (2^-9; fp32 out: 1e-5)."""
+    from opentau_b200.ops import cuda_ops
+    g = torch.Generator(device=dev).manual_seed(M + N + K)
+    x, w, res, bias = (torch.randn(*s, device=dev, generator=g).to(torch.bfloat16) for s in ((M, K), (N, K), (M, N), (N,)))
+    kw = {"plain": {}, "bias_res": dict(bias=bias, residual=res), "f32": dict(out_dtype=torch.float32),
+          "gelu": dict(bias=bias, act="gelu_tanh")}[end]
+    got = cuda_ops.gemm(x, w, "nt", **kw)
+    cuda_ops.check_status()
+    want = x.double() @ w.double().t()
+    if end != "plain" and end != "f32":
+        want = want + bias.double()
+    if end == "bias_res":
+        want = want + res.double()
+    if end == "gelu":
+        want = torch.nn.functional.gelu(want, approximate="tanh")
+    assert float((got.double() - want).norm() / want.norm()) < (1e-5 if end == "f32" else 2 ** -8)
+
+
 @pytest.mark.parametrize("rows,H", [(1, 8), (5, 256), (7, 264), (2047, 1152), (2048, 1152), (2049, 1160), (2050, 2048), (2048, 2056),
                                     (4097, 1024), (2051, 520)])
 def test_layer_norm_forward_at_the_edges_of_its_forms(dev, rows, H):
