@@ -670,19 +670,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
 // for 1024 of arithmetic (4096 positions, 8 heads on 1: 200 us).  Here the query tile lies in tensor memory (128 columns) beside
 // two tiles of scores (64 each) and O (256), so a score product reads only keys from shared memory, and two groups of four warps take
 // the blocks in turn, a thread a whole row.  What one group needs of the other is the row's maximum in use, which it publishes
-// before its exponentials; the sums stay each group's own, in terms of the maximum it saw last, and meet at the end.  P goes over the
-// scores it was made from; scores of block j + 2 wait for the commit of the product that reads P of j.
-// us, before / now: 4096 positions, 8 heads on 1, 1024 of them causal 186 / 110; 16 x 1227 (259 causal) 335 / 212; 2 x 1500, 8 on 4 79 /
-// 55; 4 x 589 24 / 19; 5000, 4 heads of 160 125 / 75.  At 4096 a block takes 1700 clocks: the chain from scores to P and the products
+// before its exponentials, and behind them the row's sums, which are so added in the order of the kernel above, to the same bits.
+// P goes over the scores it was made from; scores of block j + 2 wait for the commit of the product that reads P of j.
+// us, before / now: 4096 positions, 8 heads on 1, 1024 of them causal 191 / 112; 16 x 1227 (259 causal) 337 / 212; 2 x 1500, 8 on 4 80 /
+// 57; 4 x 589 23 / 18; 5000, 4 heads of 160 236 / 137.  At 4096 a block takes 1700 clocks: the chain from scores to P and the products
 // of two blocks that take turns.
 template <int DPAD>
 struct WideSmem {
   static constexpr int BN = 64, NCHUNK = DPAD / 64;
   static constexpr int Y_BYTES = BN * DPAD * 2;        // an item of the ring: 64 rows of Q, K or V
   static constexpr int NY = 7;
-  static constexpr int OFF_M = NY * Y_BYTES;           // float [2 groups][128]: maxima in use; at the end the row sums
-  static constexpr int OFF_BAR = OFF_M + 2 * ATT_M * 4;
-  static constexpr int NBAR = 1 + 2 * NY + 6 + 8;
+  static constexpr int OFF_M = NY * Y_BYTES;           // float [2 groups][128]: maxima in use
+  static constexpr int OFF_L = OFF_M + 2 * ATT_M * 4;  // float2 [128]: row sums, handed from group to group
+  static constexpr int OFF_BAR = OFF_L + ATT_M * 8;
+  static constexpr int NBAR = 1 + 2 * NY + 6 + 16;
   static constexpr int USED = OFF_BAR + NBAR * 8 + 16;
   static constexpr int TOTAL = USED + 1024 <= 232448 ? USED + 1024 : 232448;
   static_assert(USED <= 232448, "shared memory budget");
@@ -699,6 +700,7 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* m_pub = reinterpret_cast<float*>(smem + L::OFF_M);
+  float2* l_pub = reinterpret_cast<float2*>(smem + L::OFF_L);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
   uint64_t* q_full = bars;                       // the query tile is in tensor memory
   uint64_t* y_full = bars + 1;                   // [NY]
@@ -707,6 +709,7 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
   uint64_t* p_full = s_full + 2;                 // [2] P is in tensor memory
   uint64_t* pv_done = s_full + 4;                // [2] the product that reads it has retired
   uint64_t* m_ready = s_full + 6;                // [2][4 quadrants] a group's maxima are published
+  uint64_t* l_ready = s_full + 14;               // [2][4 quadrants] and its row sums
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NBAR);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* reach = reinterpret_cast<int*>(tmem_slot + 2);
@@ -730,7 +733,7 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       mbar_init(&p_full[i], 128);
       mbar_init(&pv_done[i], 1);
     }
-    for (int i = 0; i < 8; ++i) mbar_init(&m_ready[i], 32);
+    for (int i = 0; i < 16; ++i) mbar_init(&m_ready[i], 32);               // and l_ready behind them
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tma_q);
@@ -880,8 +883,7 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       tc_fence_before();
       mbar_arrive(q_full);
     }
-    float m_used = -INFINITY;                    // maximum that O, and this thread's sum, are expressed against
-    float l = 0.f;
+    float m_used = -INFINITY;                    // maximum that O and the sums are expressed against
     auto key_id = [&](int j, int h) {            // of this lane's key of the block's half h
       const int key = j * BN + h * 32 + lane;
       if (j >= nblk || key >= p.Sk) return INT_MAX;
@@ -893,11 +895,13 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
     auto follow = [&](int j) {
       const int from = j & 1;
       mbar_wait(&m_ready[from * 4 + quad], (j >> 1) & 1, abort_flag, p.status, KID_ATTN, 13, j);
-      const float m = m_pub[from * ATT_M + row];
-      if (m != m_used) {
-        l *= (m_used == -INFINITY) ? 0.f : fast_exp2(m_used - m);
-        m_used = m;
-      }
+      m_used = m_pub[from * ATT_M + row];
+    };
+    // the row's sums up to block j: of the first and of the second 32 keys of every block, in the order of the blocks
+    auto sums_of = [&](int j) {
+      const int from = j & 1;
+      mbar_wait(&l_ready[from * 4 + quad], (j >> 1) & 1, abort_flag, p.status, KID_ATTN, 14, j);
+      return l_pub[row];
     };
     int nx0 = key_id(grp, 0), nx1 = key_id(grp, 1);
     for (int j = grp; j < nblk; j += 2) {
@@ -967,7 +971,6 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
         }
         tmem_wait_st();
       }
-      l *= alpha;
       const float m_safe = (m_used == -INFINITY) ? 0.f : m_used;
       float lsum[2] = {0.f, 0.f};
       uint32_t packed[BN / 2];
@@ -981,26 +984,25 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
             if (hidden[h] >> e & 1) a = 0.f;
             if (hidden[h] >> (e + 1) & 1) z = 0.f;
           }
-          lsum[0] += a;
-          lsum[1] += z;
+          lsum[h] += a + z;
           packed[h * 16 + (e >> 1)] = pack_bf16(a, z);
         }
       }
-      l += lsum[0] + lsum[1];
       __syncwarp();
       tmem_st_x32(s_addr, packed);               // over the scores of my own row, which are all in registers
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(&p_full[grp]);
+      const float2 before = j > 0 ? sums_of(j - 1) : make_float2(0.f, 0.f);
+      l_pub[row] = make_float2(fmaf(before.x, alpha, lsum[0]), fmaf(before.y, alpha, lsum[1]));
+      mbar_arrive(&l_ready[grp * 4 + quad]);
     }
 
-    // ---- epilogue: O / l -> bf16 -> global, LSE.  The two groups' sums meet in terms of the last maximum.
+    // ---- epilogue: O / l -> bf16 -> global, LSE
     const int lastj = nblk - 1;
     if ((lastj & 1) != grp) follow(lastj);
-    asm volatile("bar.sync 1, 256;" ::: "memory");       // nobody reads a maximum any more
-    m_pub[grp * ATT_M + row] = l;
-    asm volatile("bar.sync 1, 256;" ::: "memory");
-    l = m_pub[row] + m_pub[ATT_M + row];
+    const float2 sums = sums_of(lastj);
+    const float l = sums.x + sums.y;
     mbar_wait(&pv_done[lastj & 1], (lastj >> 1) & 1, abort_flag, p.status, KID_ATTN, 9, 0);
     tc_fence_after();
     const float inv_l = l > 0.f ? 1.f / l : 0.f;
