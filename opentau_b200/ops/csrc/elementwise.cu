@@ -360,10 +360,35 @@ __global__ void ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bf
 }
 
 // A warp to a row: all of a row's loads are in flight together and its two sums need no block barrier.  A block to a row, as above,
-// spends its time on those.  us in a replayed graph, a block / a warp: 12288 rows of 1152 (the vision tower of a training step) 20.3 /
-// 9.8 (57 MB: 8.6 at the copy's rate), 3072 6.3 / 4.7, 4096 of 2048 8.9 / 8.5, 1024 of 128 2.6 / 1.8.  Few rows are one round trip either way, which
-// more threads to a row make shorter: 768 rows of 1152 3.0 / 3.5, 300 of 768 1.9 / 2.3.
+// spends its time on those.  The sums are added in the order of the block (a piece of 256 columns is what one of its warps holds), so
+// the results are the same bits: the lanes trade whole pieces first, which sums NV pieces in few exchanges.
+// us in a replayed graph, a block / a warp: 12288 rows of 1152 (the vision tower of a training step) 20.4 / 10.6 (57 MB: 8.6 at the
+// copy's rate), 3072 6.3 / 5.2, 4096 of 1024 6.3 / 4.8, 1024 of 128 2.7 / 2.0.  Few rows are one round trip either way, which more
+// threads to a row make shorter (2048 rows of 1152 4.7 / 4.9), and wide rows are too many steps for a warp (3000 of 1544 6.7 / 7.4).
 constexpr int LN_WARP_ROWS = 4;      // of a block
+
+// Sum over lanes and pieces: v[p] over all lanes in `warp_sum`'s order, then the pieces in the order of `block_sum`.
+template <int P>
+__device__ __forceinline__ float pieces_sum(float (&v)[P]) {
+  const int lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int half = P / 2; half > 0; half >>= 1, o >>= 1) {      // a lane keeps the pieces whose bit `half` is its bit `o`
+    const bool upper = lane & o;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const float keep = upper ? v[i + half] : v[i], send = upper ? v[i] : v[i + half];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+#pragma unroll
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  o = 16;
+#pragma unroll
+  for (int half = P / 2; half > 0; half >>= 1, o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
+
 template <int NV>
 __global__ void __launch_bounds__(LN_WARP_ROWS * 32)
 ln_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
@@ -386,28 +411,29 @@ ln_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
       for (int e = 0; e < 8; ++e) v[i][e] = 0.f;
     }
   }
-  float s = 0.f;
+  constexpr int P = NV <= 2 ? 2 : NV <= 4 ? 4 : 8;
+  float s[P];
 #pragma unroll
-  for (int i = 0; i < NV; ++i)
+  for (int i = 0; i < P; ++i) {
+    s[i] = 0.f;
+    if (i < NV) {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) s += v[i][e];
+      for (int e = 0; e < 8; ++e) s[i] += v[i < NV ? i : 0][e];
+    }
+  }
+  const float mean = pieces_sum(s) / H;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  const float mean = s / H;
-  float ss = 0.f;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    if (lane + i * 32 < nvec) {
+  for (int i = 0; i < P; ++i) {
+    s[i] = 0.f;
+    if (i < NV && lane + i * 32 < nvec) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        const float d = v[i][e] - mean;
-        ss += d * d;
+        const float d = v[i < NV ? i : 0][e] - mean;
+        s[i] += d * d;
       }
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-  const float rstd = rsqrtf(ss / H + eps);
+  const float rstd = rsqrtf(pieces_sum(s) / H + eps);
   if (lane == 0) {
     if (mean_out) mean_out[row] = mean;
     if (rstd_out) rstd_out[row] = rstd;
@@ -1139,10 +1165,9 @@ extern "C" int otb_ln_fwd(const void* x, const void* w, const void* b, void* y, 
                           long long rows, int H, float eps, cudaStream_t stream) {
   if (H % 8 || rows <= 0) return -1;
   // many rows, or rows that a warp takes in one access
-  if (H <= 2048 && (rows >= 2048 || H <= 256)) {
+  if (H <= 256 || (H <= 1280 && rows >= 3072)) {
     const int nvec = H >> 3;
-    const auto kern = nvec <= 64 ? ln_fwd_warp_kernel<2> : nvec <= 128 ? ln_fwd_warp_kernel<4>
-                    : nvec <= 160 ? ln_fwd_warp_kernel<5> : ln_fwd_warp_kernel<8>;
+    const auto kern = nvec <= 64 ? ln_fwd_warp_kernel<2> : nvec <= 128 ? ln_fwd_warp_kernel<4> : ln_fwd_warp_kernel<5>;
     return (int)launch_pdl(kern, dim3((unsigned)((rows + LN_WARP_ROWS - 1) / LN_WARP_ROWS)), dim3(LN_WARP_ROWS * 32), 0, stream, 0u,
                            (const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, mean, rstd, rows, H, eps);
   }

@@ -216,8 +216,8 @@ def test_products_at_the_line_between_the_two_kernels(dev, M, N, K, end):
     assert float((got.double() - want).norm() / want.norm()) < (1e-5 if end == "f32" else 2 ** -8)
 
 
-@pytest.mark.parametrize("rows,H", [(1, 8), (5, 256), (7, 264), (2047, 1152), (2048, 1152), (2049, 1160), (2050, 2048), (2048, 2056),
-                                    (4097, 1024), (2051, 520)])
+@pytest.mark.parametrize("rows,H", [(1, 8), (5, 256), (7, 264), (3071, 1152), (3072, 1152), (3073, 1160), (3074, 1280), (3072, 1288),
+                                    (4097, 1024), (3075, 520), (3073, 512), (2051, 2056)])
 def test_layer_norm_forward_at_the_edges_of_its_forms(dev, rows, H):
     """A warp or a block to a row, the last block's rows, widths with a partial piece, against 64 bits: sums in fp32 (1e-5) and one
     rounding to bf16 (2^-9)."""
