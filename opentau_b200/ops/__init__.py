@@ -228,7 +228,7 @@ def linear_act(x: Tensor, w: Tensor, bias: Tensor | None, act: str) -> Tensor:
     needs_grad = torch.is_grad_enabled() and (x.requires_grad or w.requires_grad)
     if (not oracle_mode() and not needs_grad and x.is_cuda and x.dtype == torch.bfloat16 and act == "gelu_tanh"):
         from . import cuda_ops
-        y = cuda_ops.gemm(x.reshape(-1, x.shape[-1]), w, "nt", bias=bias, act="gelu_tanh")
+        y = cuda_ops.gemm(x.reshape(-1, x.shape[-1]), w, "nt", bias=bias, act="gelu_tanh", no_grad=True)
         return y.view(*x.shape[:-1], w.shape[0])
     return ref.act_fn(linear(x, w, bias), act)
 

@@ -73,10 +73,10 @@ SKINNY = os.environ.get("OPENTAU_B200_SKINNY_GEMM", "1") != "0"
 
 
 def use_skinny(layout: str, M: int, N: int, accumulate: bool, bn: int, K: int = 0, gated: bool = True,
-               end: str = "") -> bool:
+               end: str = "", no_grad: bool = True) -> bool:
     """``x @ W^T`` with few rows goes to the weight-streaming split-K kernel.  ``gated``: the product ends in a gated
     residual, which only that kernel fuses (the gate then multiplies the fp32 sum); ``end``: "act" or "glu" where it ends in an
-    activation or a gated MLP's product."""
+    activation or a gated MLP's product; ``no_grad``: nothing is differentiated through it."""
     if not SKINNY or layout != "nt" or accumulate or bn:
         return False
     if gated:
@@ -87,6 +87,7 @@ def use_skinny(layout: str, M: int, N: int, accumulate: bool, bn: int, K: int = 
         return M <= 128 or (M <= 256 and N <= 8192) or (M <= 640 and N <= 2048 and -(-N // 128) * -(-M // 64) <= 148)
     if M <= 64 or (M <= 256 and N <= 2048 and K >= 3072):
         return True
+    # A product that is differentiated keeps the persistent kernel and with it the order of its sums: few of a training pass are this small.
     # Up to one CTA of 128 columns x 64 rows to an SM: us in a replayed graph with a norm in front and cold weights, few-row /
     # persistent kernel: 100 x 1024 x 1024 5.7 / 8.1, 200 x 2560 x 1024 7.5 / 8.8, 256 x 4096 x 2048 12.5 / 12.8, 400 x 2560 x 1024 9.2 / 10.3, 400 x
     # 1152 x 4096 13.4 / 19.6, 512 x 2048 x 2048 12.7 / 12.9, 768 x 1152 x 4096 14.5 / 20.2, 768 x 768 x 256 6.3 / 6.7; of 570 sizes of 65 - 768 rows, 256 -
@@ -94,7 +95,7 @@ def use_skinny(layout: str, M: int, N: int, accumulate: bool, bn: int, K: int = 
     # 11.1, 640 x 2560 x 2048 15.5 / 14.6, 768 x 4096 x 1024 14.7 / 12.9, 200 x 6144 x 1024 11.1 / 10.8; more columns lose from 65 rows on
     # (100 x 8192 x 1024 9.8 / 8.9).  With an activation at the end it wins on half as many tiles (256 x 1024 x 1024 7.2 / 9.4, 128 x 4304 x 1152
     # 8.7 / 10.1, 256 x 4304 x 1152 11.4 / 10.6), with a gated MLP's product on narrow ones alone (200 x 4096 x 1024 10.2 / 9.8)
-    return end != "glu" and M <= 768 and N <= 6144 and -(-N // 128) * -(-M // 64) <= (74 if end else 148)
+    return no_grad and end != "glu" and M <= 768 and N <= 6144 and -(-N // 128) * -(-M // 64) <= (74 if end else 148)
 
 
 class _SkinnyArgs(ctypes.Structure):
@@ -126,9 +127,10 @@ def _operand(t: Tensor) -> Tensor:
 def gemm(a: Tensor, b: Tensor, layout: str, bias: Tensor | None = None, residual: Tensor | None = None,
          out: Tensor | None = None, accumulate: bool = False, out_dtype: torch.dtype | None = None,
          glu: str | None = None, glu_out: Tensor | None = None, store_out: bool = True, act: str | None = None,
-         bn: int = 0, splits: int = 0, gate: Tensor | None = None) -> Tensor:
+         bn: int = 0, splits: int = 0, gate: Tensor | None = None, no_grad: bool = False) -> Tensor:
     """tcgen05 GEMM.  layout 'nt': a(M,K) b(N,K); 'nn': a(M,K) b(K,N); 'tn': a(K,M) b(K,N).  ``bn`` forces the column
-    tile of the persistent kernel, ``splits`` (1, 2, 4, 8) forces the weight-streaming split-K kernel."""
+    tile of the persistent kernel, ``splits`` (1, 2, 4, 8) forces the weight-streaming split-K kernel; ``no_grad`` as in
+    ``use_skinny``."""
     global launch_count
     a, b = _operand(a), _operand(b)
     if layout == "nt":
@@ -192,7 +194,7 @@ def gemm(a: Tensor, b: Tensor, layout: str, bias: Tensor | None = None, residual
     if splits and (layout != "nt" or accumulate):
         raise ValueError("the split-K kernel computes a @ b^T without accumulation")
     skinny = bool(splits) or use_skinny(layout, M, N, accumulate, bn, K, gate is not None,
-                                       "glu" if glu is not None else "act" if act is not None else "")
+                                       "glu" if glu is not None else "act" if act is not None else "", no_grad)
     g_stride, g_rows = 0, 1
     if gate is not None:
         # out = residual + gate * (a @ b^T): rows of N gates, one per `M / gate rows` consecutive output rows

@@ -59,10 +59,10 @@ class LinearFn(torch.autograd.Function):
     """``y = x @ w.T (+ bias) (+ residual)``."""
 
     @staticmethod
-    def forward(ctx, x, w, bias, residual):
+    def forward(ctx, x, w, bias, residual, no_grad=False):
         x2 = _flat2d(x)
         r2 = _flat2d(residual) if residual is not None else None
-        y = prims.mm_nt(x2, w, bias=bias, residual=r2)
+        y = prims.mm_nt(x2, w, bias=bias, residual=r2, no_grad=no_grad)
         ctx.save_for_backward(x2, w)
         ctx.wref, ctx.bref = w, bias
         ctx.x_shape = x.shape
@@ -83,11 +83,16 @@ class LinearFn(torch.autograd.Function):
         if ctx.bref is not None and ctx.needs_input_grad[2]:
             db = _sink_vec(ctx.bref, prims.col_sum(dy2))
         dres = dy if ctx.has_res else None
-        return dx, dw, db, dres
+        return dx, dw, db, dres, None
+
+
+def _no_grad(*ts) -> bool:
+    """No gradient is asked for (a function's own ``needs_input_grad`` leaves ``torch.no_grad()`` out)."""
+    return not (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in ts))
 
 
 def linear(x, w, bias=None, residual=None):
-    return LinearFn.apply(x, w, bias, residual)
+    return LinearFn.apply(x, w, bias, residual, _no_grad(x, w, bias, residual))
 
 
 class GatedMLPFn(torch.autograd.Function):
@@ -99,12 +104,12 @@ class GatedMLPFn(torch.autograd.Function):
     """
 
     @staticmethod
-    def forward(ctx, x, w_gu, w_down, residual, act):
+    def forward(ctx, x, w_gu, w_down, residual, act, no_grad=False):
         x2 = _flat2d(x)
         need_bwd = any(ctx.needs_input_grad[:3])
         gu, h = prims.mm_nt_glu(x2, w_gu, act, keep_gu=need_bwd)
         r2 = _flat2d(residual) if residual is not None else None
-        y = prims.mm_nt(h, w_down, residual=r2)
+        y = prims.mm_nt(h, w_down, residual=r2, no_grad=no_grad)
         if need_bwd:
             ctx.save_for_backward(x2, gu, h, w_gu, w_down)
         ctx.wgu, ctx.wdown = w_gu, w_down
@@ -123,11 +128,11 @@ class GatedMLPFn(torch.autograd.Function):
         del dh, h
         dwgu = _sink_wgrad(ctx.wgu, dgu, x2) if ctx.needs_input_grad[1] else None
         dx = prims.mm_nn(dgu, w_gu).view(ctx.x_shape) if ctx.needs_input_grad[0] else None
-        return dx, dwgu, dwd, (dy if ctx.has_res else None), None
+        return dx, dwgu, dwd, (dy if ctx.has_res else None), None, None
 
 
 def gated_mlp(x, w_gu, w_down, act, residual=None):
-    return GatedMLPFn.apply(x, w_gu, w_down, residual, act)
+    return GatedMLPFn.apply(x, w_gu, w_down, residual, act, _no_grad(x, w_gu, w_down, residual))
 
 
 class RMSNormFn(torch.autograd.Function):

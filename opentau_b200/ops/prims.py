@@ -24,12 +24,13 @@ def _cuda(x: Tensor) -> bool:
 
 # ----------------------------------------------------------------------------- GEMMs
 def mm_nt(a: Tensor, b: Tensor, bias: Tensor | None = None, residual: Tensor | None = None,
-          out: Tensor | None = None, accumulate: bool = False, out_dtype: torch.dtype | None = None) -> Tensor:
-    """``a (M,K) @ b (N,K).T`` (+bias over N) (+residual (M,N)); fp32 accumulate."""
+          out: Tensor | None = None, accumulate: bool = False, out_dtype: torch.dtype | None = None,
+          no_grad: bool = False) -> Tensor:
+    """``a (M,K) @ b (N,K).T`` (+bias over N) (+residual (M,N)); fp32 accumulate.  ``no_grad``: of an inference pass."""
     if _cuda(a):
         from . import cuda_ops
         return cuda_ops.gemm(a, b, "nt", bias=bias, residual=residual, out=out, accumulate=accumulate,
-                             out_dtype=out_dtype)
+                             out_dtype=out_dtype, no_grad=no_grad)
     y = a @ b.t()
     if bias is not None:
         y = y + bias

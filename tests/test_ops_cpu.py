@@ -349,3 +349,19 @@ def test_few_row_plans_share_sums_where_the_chip_is_empty():
             assert _lib.load("gemm_skinny_tcgen05").otb_gemm_skinny_plan(rows, cols, inner, 148, fits, plan) == 0
             chunks, nt, splits, _, _ = plan
             assert -(-cols // 128) * chunks * splits >= 74 and splits >= 2, (rows, cols, inner, list(plan))
+
+
+@pytest.mark.parametrize("grad_mode,frozen,want", [(True, False, False), (False, False, True), (True, True, True)])
+def test_products_know_whether_they_are_differentiated(monkeypatch, grad_mode, frozen, want):
+    """A product that is differentiated keeps the persistent kernel's order of sums; parameters under ``no_grad`` do not count."""
+    from opentau_b200.ops import cuda_ops
+    seen, mm_nt = [], prims.mm_nt
+    monkeypatch.setattr(prims, "mm_nt", lambda *a, no_grad=False, **kw: (seen.append(no_grad), mm_nt(*a, **kw))[1])
+    w = torch.nn.Parameter(torch.randn(8, 16), requires_grad=not frozen)
+    with torch.set_grad_enabled(grad_mode):
+        y = fused.linear(torch.randn(3, 16), w)
+    if not want:
+        y.sum().backward()
+        assert w.grad is not None
+    assert seen == [want]
+    assert cuda_ops.use_skinny("nt", 400, 1152, False, 0, 4096, False, "", want) is (want and cuda_ops.SKINNY)
