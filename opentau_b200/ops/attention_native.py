@@ -112,10 +112,10 @@ def attn_fwd(q: Tensor, k: Tensor, v: Tensor, q_blk: Tensor, k_blk: Tensor, q_va
             part_ml = torch.empty(nsplit, B, H, Sq, 2, dtype=torch.float32, device=q.device)
             cuda_ops.launch_count += 1
         rc = _entry("attention_tcgen05", "otb_attn_fwd_splitkv", kinds + "ipppp")(
-            *args, nsplit, _ptr(part_o), _ptr(part_ml), cuda_ops.status_pointer(), cuda_ops._stream())
+            *args, nsplit, _ptr(part_o), _ptr(part_ml), cuda_ops.status_pointer(), cuda_ops._raw_stream())
     else:
         rc = _entry("attention_tcgen05", "otb_attn_fwd", kinds + "pp")(*args, cuda_ops.status_pointer(),
-                                                                       cuda_ops._stream())
+                                                                       cuda_ops._raw_stream())
     if rc != 0:
         raise RuntimeError(f"native attn_fwd failed with code {rc} (B={B} Sq={Sq} Sk={Sk} H={H} Hkv={Hkv} D={D})")
     cuda_ops.launch_count += 1
@@ -165,7 +165,7 @@ def _attn_bwd_stored(samples: int, do, q, k, v, o, lse, qb, kb, qv, kv, dq, dk, 
     from . import cuda_ops
     B, Sq, H, D = q.shape
     Sk, Hkv = k.shape[1], k.shape[2]
-    size, n_cover, _ = bwd_stored_plan(samples, Sq, Sk, H, Hkv, D)
+    size, n_cover, planned = bwd_stored_plan(samples, Sq, Sk, H, Hkv, D)
     try:
         scratch = torch.empty(2 * size + 4 * n_cover, dtype=torch.uint8, device=q.device)
     except torch.cuda.OutOfMemoryError:
@@ -173,21 +173,21 @@ def _attn_bwd_stored(samples: int, do, q, k, v, o, lse, qb, kb, qv, kv, dq, dk, 
     s0 = scratch.data_ptr()
     fn = _entry("attention_bwd_stored_tcgen05", "otb_attn_bwd_stored", "pp")
     tensors = (q, k, v, o, do, lse, dq, dk, dv, qb, kb, qv, kv)
-    step = [samples * t.stride(0) * t.element_size() for t in tensors]
     at = [t.data_ptr() for t in tensors]
     strides = (c_longlong * 9)(*q.stride()[:3], *k.stride()[:3], *v.stride()[:3])
     for b0 in range(0, B, samples):
         n = min(samples, B - b0)
-        m = parts or bwd_stored_plan(n, Sq, Sk, H, Hkv, D)[2]
+        m = parts or (planned if n == samples else bwd_stored_plan(n, Sq, Sk, H, Hkv, D)[2])
         sums = torch.empty(2, m, n * Sk * Hkv * D, dtype=torch.float32, device=q.device) if m > 1 else None
         sums_at = (sums.data_ptr(), sums.data_ptr() + 4 * sums.stride(0)) if m > 1 else (0, 0)
         args = _StoredBwdArgs(*at[:9], s0, s0 + size, s0 + 2 * size, *sums_at, *at[9:], cuda_ops.status_pointer(), strides,
                               n, Sq, Sk, H, Hkv, D, m, scale)
-        rc = fn(byref(args), cuda_ops._stream())
+        rc = fn(byref(args), cuda_ops._raw_stream())
         if rc != 0:
             raise RuntimeError(f"native attn_bwd failed with code {rc} (B={B} Sq={Sq} Sk={Sk} H={H} Hkv={Hkv} D={D})")
         cuda_ops.launch_count += 3 + (m > 1)
-        at = [x + d for x, d in zip(at, step)]
+        if b0 + samples < B:
+            at = [x + samples * t.stride(0) * t.element_size() for x, t in zip(at, tensors)]
     return True
 
 
