@@ -422,9 +422,10 @@ def ln_fwd(x: Tensor, w: Tensor, b: Tensor, eps: float):
     y = torch.empty(R, H, dtype=x.dtype, device=x.device)
     mean = torch.empty(R, dtype=torch.float32, device=x.device)
     rstd = torch.empty(R, dtype=torch.float32, device=x.device)
+    # held until the launch is issued: a converted weight that died with its pointer would lend the bias its memory
+    wt, bt = w.to(torch.bfloat16).contiguous(), b.to(torch.bfloat16).contiguous()
     _check(_call("elementwise", "otb_ln_fwd", "pppppplifp")(
-        _ptr(x2), _ptr(w.to(torch.bfloat16).contiguous()), _ptr(b.to(torch.bfloat16).contiguous()), _ptr(y),
-        _ptr(mean), _ptr(rstd), R, H, eps, _raw_stream()), "ln_fwd")
+        _ptr(x2), _ptr(wt), _ptr(bt), _ptr(y), _ptr(mean), _ptr(rstd), R, H, eps, _raw_stream()), "ln_fwd")
     launch_count += 1
     return y.view(x.shape), mean, rstd
 
@@ -442,9 +443,10 @@ def ln_bwd(dy: Tensor, x: Tensor, w: Tensor, mean: Tensor, rstd: Tensor):
     dx = torch.empty(R, H, dtype=x.dtype, device=x.device)
     rpb, nb = _bwd_blocks(R)
     partial = torch.empty(2, nb, H, dtype=torch.float32, device=x.device)
+    wt = w.to(torch.bfloat16).contiguous()
     _check(_call("elementwise", "otb_ln_bwd", "ppppppppliip")(
-        _ptr(dy2), _ptr(x2), _ptr(w.to(torch.bfloat16).contiguous()), _ptr(mean), _ptr(rstd), _ptr(dx),
-        _ptr(partial[0]), _ptr(partial[1]), R, H, rpb, _raw_stream()), "ln_bwd")
+        _ptr(dy2), _ptr(x2), _ptr(wt), _ptr(mean), _ptr(rstd), _ptr(dx), _ptr(partial[0]), _ptr(partial[1]), R, H, rpb,
+        _raw_stream()), "ln_bwd")
     out = torch.empty(2, H, dtype=torch.bfloat16, device=x.device)
     for k in range(2):
         _check(_call("elementwise", "otb_colsum_partials", "piipip")(

@@ -234,6 +234,22 @@ def test_layer_norm_forward_at_the_edges_of_its_forms(dev, rows, H):
     assert float((y.double() - want).norm() / want.norm()) < 2 ** -8
 
 
+@pytest.mark.parametrize("rows,H", [(64, 256), (3, 520), (3072, 1152)])
+def test_layer_norm_of_bf16_rows_with_fp32_weights(dev, rows, H):
+    """Weight and bias are converted for the launch and must not share memory while it is made.  Against 64 bits with the weights
+    as the kernel reads them (bf16): one rounding of the result (2^-9)."""
+    from opentau_b200.ops import cuda_ops
+    g = torch.Generator(device=dev).manual_seed(rows + H)
+    x = torch.randn(rows, H, device=dev, generator=g).to(torch.bfloat16)
+    dy = torch.randn(rows, H, device=dev, generator=g).to(torch.bfloat16)
+    w, b = (torch.randn(H, device=dev, generator=g) for _ in range(2))
+    y, mean, rstd = cuda_ops.ln_fwd(x, w, b, 1e-6)
+    want = torch.nn.functional.layer_norm(x.double(), (H,), w.to(torch.bfloat16).double(), b.to(torch.bfloat16).double(), 1e-6)
+    assert float((y.double() - want).norm() / want.norm()) < 2 ** -8
+    for got, ref in zip(cuda_ops.ln_bwd(dy, x, w, mean, rstd), cuda_ops.ln_bwd(dy, x, w.to(torch.bfloat16), mean, rstd)):
+        assert torch.equal(got.to(ref.dtype), ref)
+
+
 @pytest.mark.parametrize("D", [64, 72])     # 72: Qwen3-VL vision heads (8-byte accesses)
 def test_rope_kernel_strided(dev, D):
     from opentau_b200 import ops
