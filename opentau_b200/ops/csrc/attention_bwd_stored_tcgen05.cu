@@ -5,7 +5,7 @@
 // fills half of the tensor memory, so that scores have no second buffer and every block waits for the elementwise work.
 // Here the operands are made once and stored:
 //
-//   attn_bwd_cover_kernel    how many blocks of 64 keys each pair of query tiles has to visit
+//   attn_bwd_cover_kernel    how many blocks of 64 keys each pair of query tiles has to visit, and which 64 rows of it see any
 //   attn_bwd_scores_kernel   tile = 128 query rows (position x head of the group), streams blocks of 64 keys:
 //                              S = Q K_j^T, dP = dO V_j^T -> P, dS = P o (dP - delta) * scale -> bf16 -> global
 //                            No accumulator: both fixed tiles lie in tensor memory beside two pairs of (S, dP), so the products of
@@ -19,8 +19,9 @@
 // it is written by bulk copies of contiguous memory and read without another swizzle.
 //
 // Hidden blocks are neither computed nor stored: the first cover[b][t] key blocks of query tiles 2 t and 2 t + 1 are, in whole tiles
-// of dK and dV (four blocks) or up to the last key, and the products look nowhere else.  Results are deterministic: no
-// atomics, fixed order of accumulation.
+// of dK and dV (four blocks) or up to the last key.  The products multiply P and dS, zeros included, by what stands in K, Q and dO, where
+// padding may hold anything: dQ ends with the pair's last visible block, and dK and dV leave out every 64 rows that see nothing.
+// Results are deterministic: no atomics, fixed order of accumulation.
 //
 // us for the whole backward, recomputing / stored: 4096 positions, 8 heads on 1 of 256, 1024 of them causal 545 / 289; 8 x 1227 and
 // 16 x 1227 (259 causal; a training step's layer) 579 / 270 and 940 / 512; 2 x 700, 8 on 4 117 / 55; 2 x 2048, 32 on 8 of 128 735 / 480;
@@ -54,7 +55,8 @@ struct StoredParams {
   const float* lse;                            // (B, H, Sq), natural log
   const __nv_bfloat16* o;                      // (B, Sq, H, D) contiguous
   __nv_bfloat16 *P, *dS;                       // (B, Hkv, 2 ptiles, kblks, ST_IMAGE)
-  int* cover;                                  // (B, ptiles)
+  int* cover;                                  // (B, ptiles): key blocks of a pair, whole tiles of dK and dV
+  unsigned* reach;                             // (B, ptiles): blocks up to the last visible key; bit 28 + i: rows 64 i .. see any
   __nv_bfloat16 *dq, *dk, *dv;                 // contiguous
   float *dk_parts, *dv_parts;                  // splits > 1: (splits, B, Sk, Hkv, D) fp32
   KernelStatus* status;
@@ -80,31 +82,40 @@ __device__ __forceinline__ float st_exp2(float x) {
 }
 
 // ------------------------------------------------------------------------------------------ cover
-// One block per pair of query tiles: 1 + the last valid key with k_blk <= the pair's largest valid q_blk (no order assumed),
-// searched from the end a thousand keys at a time, rounded up to the key tiles of dK and dV.
+constexpr unsigned REACH_MASK = (1u << 28) - 1;   // blocks; above it the four bits
+// One block per pair of query tiles: 1 + the last valid key with k_blk <= the pair's largest valid q_blk (no order assumed), searched
+// from the end a thousand keys at a time until every 64 rows with a valid one have found a key.
 __global__ void __launch_bounds__(256) attn_bwd_cover_kernel(StoredParams p) {
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x, b = blockIdx.y, pos_per = 2 * ST_M / p.g;
-  __shared__ int s_qmax, s_last;
+  __shared__ int s_qmax[4], s_last;
+  __shared__ unsigned s_any, s_found;
+  if (threadIdx.x < 4) s_qmax[threadIdx.x] = INT_MIN;
   if (threadIdx.x == 0) {
-    s_qmax = INT_MIN;
     s_last = -1;
+    s_any = s_found = 0;
   }
   bool any = false;
-  int qmax = INT_MIN;
-  const int ps = t * pos_per + threadIdx.x;
+  int qblk = INT_MIN;
+  const int ps = t * pos_per + threadIdx.x, quarter = threadIdx.x * p.g / 64;
   if ((int)threadIdx.x < pos_per && ps < p.Sq && p.q_valid[(long long)b * p.Sq + ps]) {      // pos_per <= 256
     any = true;
-    qmax = p.q_blk[(long long)b * p.Sq + ps];
+    qblk = p.q_blk[(long long)b * p.Sq + ps];
   }
   const int some = __syncthreads_or(any);
-  if (any) atomicMax(&s_qmax, qmax);
+  if (any) {
+    atomicMax(&s_qmax[quarter], qblk);
+    atomicOr(&s_any, 1u << quarter);
+  }
   __syncthreads();
-  qmax = s_qmax;
-  int last = -1;
+  int qmax[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) qmax[i] = s_qmax[i];
+  const unsigned asked = s_any;
   for (int end = p.Sk; some && end > 0; end -= 1024) {
-    int kb[4], kv[4];
+    int kb[4], kv[4], last = -1;
+    unsigned found = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int j = end - 1024 + i * 256 + (int)threadIdx.x;
@@ -112,13 +123,27 @@ __global__ void __launch_bounds__(256) attn_bwd_cover_kernel(StoredParams p) {
       kv[i] = j >= 0 ? p.k_valid[(long long)b * p.Sk + j] : 0;
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (kv[i] && kb[i] <= qmax) last = max(last, end - 1024 + i * 256 + (int)threadIdx.x);
-    if (__syncthreads_or(last >= 0)) break;
+    for (int i = 0; i < 4; ++i) {
+      unsigned sees = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) sees |= (kv[i] && kb[i] <= qmax[q] ? 1u : 0u) << q;
+      if (sees & asked) last = max(last, end - 1024 + i * 256 + (int)threadIdx.x);
+      found |= sees & asked;
+    }
+    last = __reduce_max_sync(0xffffffffu, last);
+    found = __reduce_or_sync(0xffffffffu, found);
+    if (found && (threadIdx.x & 31) == 0) {
+      atomicMax(&s_last, last);
+      atomicOr(&s_found, found);
+    }
+    __syncthreads();
+    if (__syncthreads_and(s_found == asked)) break;
   }
-  if (last >= 0) atomicMax(&s_last, last);
-  __syncthreads();
-  if (threadIdx.x == 0) p.cover[(long long)b * p.ptiles + t] = min((s_last + 4 * ST_BN) / (4 * ST_BN) * 4, p.kblks);
+  if (threadIdx.x == 0) {
+    const int blocks = (s_last + ST_BN) / ST_BN;
+    p.reach[(long long)b * p.ptiles + t] = (unsigned)blocks | s_found << 28;
+    p.cover[(long long)b * p.ptiles + t] = min((blocks + 3) / 4 * 4, p.kblks);
+  }
 }
 
 // ------------------------------------------------------------------------------------------ P and dS
@@ -553,16 +578,34 @@ struct JobWalk {
     }
     j.b = sample_head / p.Hkv;
     j.kvh = sample_head - j.b * p.Hkv;
-    const int* cover = p.cover + (long long)j.b * p.ptiles;
+    const unsigned* reach = p.reach + (long long)j.b * p.ptiles;
     j.lo = 0;
     if (j.which == 0) {
-      j.nsteps = cover[j.tile];
-    } else {
-      int n = 0;
-      for (int t0 = 0; t0 < p.ptiles; t0 += 32)
-        n += __popc(__ballot_sync(0xffffffffu, t0 + lane < p.ptiles && cover[t0 + lane] > 4 * j.tile));
-      j.lo = (int)((long long)n * j.split / p.splits);
-      j.nsteps = 4 * ((int)((long long)n * (j.split + 1) / p.splits) - j.lo);
+      j.nsteps = reach[j.tile] & REACH_MASK;
+    } else {                                     // a part takes pairs in equal numbers, of each pair the 64 rows that see any key
+      auto steps_of = [&](int t) {
+        const unsigned r = t < p.ptiles ? reach[t] : 0u;
+        return (r & REACH_MASK) > 4u * j.tile ? __popc(r >> 28) : 0;
+      };
+      int n = 0, steps = 0;
+      for (int t0 = 0; t0 < p.ptiles; t0 += 32) {
+        const int mine = steps_of(t0 + lane);
+        n += __popc(__ballot_sync(0xffffffffu, mine > 0));
+        steps += mine;
+      }
+      if (p.splits > 1) {
+        j.lo = (int)((long long)n * j.split / p.splits);
+        const int hi = (int)((long long)n * (j.split + 1) / p.splits);
+        steps = 0;
+        for (int t0 = 0, seen = 0; t0 < p.ptiles && seen < hi; t0 += 32) {
+          const int mine = steps_of(t0 + lane);
+          const unsigned in = __ballot_sync(0xffffffffu, mine > 0);
+          const int at = seen + __popc(in & ((1u << lane) - 1));
+          if (at >= j.lo && at < hi) steps += mine;
+          seen += __popc(in);
+        }
+      }
+      j.nsteps = __reduce_add_sync(0xffffffffu, steps);
     }
     return true;
   }
@@ -620,7 +663,7 @@ attn_bwd_products_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_
     const int x0 = rank * (n2 >> 1);
     while (walk.next(j)) {
       const long long images = ((long long)j.b * p.Hkv + j.kvh) * (2 * p.ptiles) * p.kblks;
-      const int* cover = p.cover + (long long)j.b * p.ptiles;
+      const unsigned* reach = p.reach + (long long)j.b * p.ptiles;
       int s = s0;                                // the elected lane's position in the ring
       uint32_t ph = ph0;
       auto slot = [&](int what) {
@@ -647,10 +690,12 @@ attn_bwd_products_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_
           const CUtensorMap* ta = j.which == 1 ? &tm_ds : &tm_p;
           const CUtensorMap* tb = j.which == 1 ? &tm_q : &tm_do;
           for (int t = 0, seen = 0, left = j.nsteps; left > 0 && t < p.ptiles; ++t) {
-            if (cover[t] <= 4 * j.tile || seen++ < j.lo) continue;
-            left -= 4;
+            const unsigned r = reach[t];
+            if ((r & REACH_MASK) <= 4u * j.tile || seen++ < j.lo) continue;
 #pragma unroll 1
             for (int q = 0; q < 4; ++q) {        // 64 rows: half a tile of the pair
+              if (!(r >> (28 + q) & 1)) continue;
+              --left;
               const int tq = 2 * t + (q >> 1);
               const int row0 = (int)(images + (long long)tq * p.kblks + 4 * j.tile + 2 * rank) * ST_M + (q & 1) * 64;
               uint8_t* sa = slot(t);
@@ -889,7 +934,7 @@ extern "C" void otb_attn_bwd_stored_plan(int B, int Sq, int Sk, int H, int Hkv, 
   const int g = H / Hkv, pairs = st_sms() / 2;
   const long long pt = (Sq + 2 * ST_M / g - 1) / (2 * ST_M / g), kb = (Sk + ST_BN - 1) / ST_BN, kt = (kb + 3) / 4, kv = (long long)Hkv * B;
   *operand_bytes = kv * 2 * pt * kb * ST_IMAGE * 2;
-  *cover_ints = (int)(B * pt);
+  *cover_ints = (int)(2 * B * pt);               // and, behind it, reach
   // the longest share of a CTA pair, and the parts' sums
   *kv_splits = 1;
   const double dpad = D <= 64 ? 64 : (D <= 128 ? 128 : 256), step_us = 0.3 * (0.4 + 0.6 * dpad / 256);
@@ -953,6 +998,7 @@ extern "C" int otb_attn_bwd_stored(const OtbAttnBwdStored* a, cudaStream_t strea
   p.P = static_cast<__nv_bfloat16*>(a->P);
   p.dS = static_cast<__nv_bfloat16*>(a->dS);
   p.cover = a->cover;
+  p.reach = reinterpret_cast<unsigned*>(a->cover + (long long)B * p.ptiles);
   p.dq = static_cast<__nv_bfloat16*>(a->dq);
   p.dk = static_cast<__nv_bfloat16*>(a->dk);
   p.dv = static_cast<__nv_bfloat16*>(a->dv);

@@ -510,6 +510,32 @@ def test_stored_backward_matches_the_recomputing_one(D, H, Hkv, Sq, Sk, samples,
     assert float(got[1][1, Sk // 2:].abs().sum()) == 0.0 and float(got[0][0, Sq // 2:].abs().sum()) == 0.0
 
 
+@pytest.mark.parametrize("D,H,Hkv", [(256, 8, 1), (256, 8, 4), (200, 2, 2), (128, 32, 1), (72, 4, 4), (64, 8, 2)])
+@pytest.mark.parametrize("seen,asked", [(300, 333), (64, 700), (257, 130), (1, 1), (449, 513)])
+@pytest.mark.parametrize("samples", [1, 2, 0])
+def test_backward_reads_no_key_or_query_behind_the_last_visible_block(D, H, Hkv, seen, asked, samples):
+    """NaN in the keys behind the block that holds the last visible one (64 keys, 128 up to head width 128), and in the query rows behind
+    the last valid one's, leaves every gradient as if zeros stood there, bit for bit."""
+    from opentau_b200.ops import attention_native, cuda_ops
+    B, S, g = 2, 700, H // Hkv
+    gen = torch.Generator(device="cuda").manual_seed(D + seen)
+    q, k, v, do = (torch.randn(*shape, device="cuda", generator=gen).to(torch.bfloat16)
+                   for shape in ((B, S, H, D), (B, S, Hkv, D), (B, S, Hkv, D), (B, S, H, D)))
+    block = 64 if D > 128 else 128
+    keys, rows = -(-seen // block) * block, -(-asked * g // block) * block // g
+    blk = torch.zeros(B, S, dtype=torch.int32, device="cuda")
+    qv, kv = (torch.arange(S, device="cuda").expand(B, -1) < n for n in (asked, seen))
+    out = []
+    for fill in (float("nan"), 0.0):
+        k[:, keys:], v[:, keys:], q[:, rows:], do[:, rows:] = fill, fill, fill, fill
+        o, lse = attention_native.attn_fwd(q, k, v, blk, blk, qv, kv, D ** -0.5, nsplit=1)
+        grads = attention_native.attn_bwd(do.reshape(B, S, H * D), q, k, v, o, lse, blk, blk, qv, kv, D ** -0.5, samples=samples)
+        out.append((o.view(B, S, H, D)[:, :asked], *grads))
+    cuda_ops.check_status()
+    for name, x, want in zip(("o", "dq", "dk", "dv"), *out):
+        assert torch.equal(x, want), name
+
+
 def test_backward_recomputes_where_there_is_no_room_for_p_and_ds(monkeypatch):
     """A call whose P and dS are more than is kept goes a sample at a time, then without them; so does one that finds no memory."""
     from opentau_b200.ops import attention_native, cuda_ops
