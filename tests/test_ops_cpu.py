@@ -307,6 +307,55 @@ def test_stored_attention_backward_refuses_misaligned_tensors_before_any_launch(
     assert fn(byref(args), 0) == -6
 
 
+@pytest.mark.parametrize("B,S,D,room,want", [
+    (4, 700, 256, None, [(0, 4, 1)]), (1, 700, 256, None, [(0, 1, 8)]),
+    (1, 700, 256, "operands", None),               # room for P and dS, none for the parts' sums
+    (4, 700, 256, 2, [(0, 2, 1), (2, 2, 1)]), (4, 700, 256, 1, [(i, 1, 1) for i in range(4)]), (3, 300, 64, 2, [(0, 2, 1), (2, 1, 1)]),
+    (4, 700, 256, 0, None)])
+def test_stored_attention_backward_takes_fewer_samples_where_memory_is_short(monkeypatch, B, S, D, room, want):
+    """Room for all scratch or none is taken: every sample once, in parts that do not depend on the room; the recomputing kernels
+    where not one sample finds it."""
+    from opentau_b200.ops import attention_native, build, cuda_ops
+    if not build.lib_path("attention_bwd_stored_tcgen05").exists():
+        pytest.skip("native libraries are not built")
+    H, Hkv = 8, 1
+    size, cover, parts = attention_native.bwd_stored_plan(B, S, S, H, Hkv, D)
+    operands = 2 * size + 4 * cover
+    limit = {None: 1 << 60, "operands": operands}.get(room) if not isinstance(room, int) else operands * room // B + 64
+    real, calls = torch.empty, []
+
+    def empty(*shape, **kw):
+        scratch = shape[0] if kw.get("dtype") is torch.uint8 else 0
+        sums = 4 * shape[1] * shape[2] if kw.get("dtype") is torch.float32 and shape[0] == 2 else 0
+        if scratch > limit or (sums and operands + sums > limit):
+            raise torch.cuda.OutOfMemoryError
+        return real(*shape, **kw)
+
+    def launch(*a):
+        if len(a) == 2:
+            args = a[0]._obj
+            b0 = (args.q - q.data_ptr()) // (2 * q.stride(0))
+            calls.append((b0, args.B, args.kv_splits))
+            assert args.k == k[b0].data_ptr() and args.lse == lse[b0].data_ptr()
+            if args.kv_splits > 1:
+                assert args.dv_parts == args.dk_parts + 4 * args.kv_splits * args.B * S * Hkv * D and args.dk_parts % 16 == 0
+        else:
+            calls.append("recomputed")
+        return 0
+
+    q, o, do = (real(B, S, H, D, dtype=torch.bfloat16) for _ in range(3))
+    k, v = (real(B, S, Hkv, D, dtype=torch.bfloat16) for _ in range(2))
+    lse = torch.zeros(B, H, S)
+    blk, valid = torch.zeros(B, S, dtype=torch.int32), torch.ones(B, S, dtype=torch.bool)
+    monkeypatch.setattr(attention_native, "_entry", lambda *a: launch)
+    monkeypatch.setattr(cuda_ops, "_raw_stream", lambda: 0)
+    monkeypatch.setattr(cuda_ops, "status_pointer", lambda: 0)
+    monkeypatch.setattr(torch, "empty", empty)
+    monkeypatch.setattr(attention_native, "stored_bwd_samples", lambda *a: B)
+    attention_native.attn_bwd(do.view(B, S, H * D), q, k, v, o.view(B, S, H * D), lse, blk, blk, valid, valid, 0.1)
+    assert calls == (want or ["recomputed"])
+
+
 @pytest.mark.parametrize("cols", [8, 128, 768, 1032, 1280, 2048, 8192, 32768])
 @pytest.mark.parametrize("inner", [8, 64, 256, 1088, 2048, 5120, 16384])
 def test_few_row_plans_fit_the_chip(cols, inner):
