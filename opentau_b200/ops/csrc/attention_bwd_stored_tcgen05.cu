@@ -46,7 +46,7 @@ struct StoredParams {
   int B, Sq, Sk, H, Hkv, D, g;
   int ptiles, kblks, key_tiles;                // pairs of query tiles; key blocks of the scratch; tiles of 256 keys
   int splits;                                  // parts of a dK / dV tile's query rows
-  int dq_few;                                  // dQ jobs of a CTA pair that has one dK / dV job more than others
+  int dq_more;                                 // dQ jobs of the CTA pairs that have one dK / dV job more than others, all together
   float scale, scale_log2;
   const int* q_blk;
   const int* k_blk;
@@ -538,8 +538,8 @@ constexpr int PR_THREADS = 192;                  // warp 0 copies, warp 1 MMA, w
 struct Job {
   int which, b, kvh, tile, split, lo, nsteps;
 };
-// Pair i takes the dK / dV jobs i, i + pairs, ...: long ones, all of one length; then a run of dQ jobs, `dq_few` where it has one of
-// the former more than others, an equal share of the rest where it has not.  Every role walks through the jobs by itself.
+// Pair i takes the dK / dV jobs i, i + pairs, ...: long ones, all of one length; then a run of dQ jobs: an equal share of the first
+// `dq_more` where it has one of the former more than others, of the rest where it has not.  Every role walks through the jobs by itself.
 struct JobWalk {
   const StoredParams& p;
   int lane, pair, pairs, kv, next_kv, n_kv, next_q, end_q;
@@ -548,14 +548,11 @@ struct JobWalk {
     n_kv = kv * 2 * p.key_tiles * p.splits;
     next_kv = pair;
     const int n_q = kv * p.ptiles, more = n_kv % pairs;
-    if (pair < more) {
-      next_q = pair * p.dq_few;
-      end_q = next_q + p.dq_few;
-    } else {
-      const int first = more * p.dq_few;
-      next_q = first + (int)((long long)(n_q - first) * (pair - more) / (pairs - more));
-      end_q = first + (int)((long long)(n_q - first) * (pair - more + 1) / (pairs - more));
-    }
+    const bool has_more = pair < more;
+    const int first = has_more ? 0 : p.dq_more, jobs = has_more ? p.dq_more : n_q - p.dq_more;
+    const int i = has_more ? pair : pair - more, of = has_more ? more : pairs - more;
+    next_q = first + (int)((long long)jobs * i / of);
+    end_q = first + (int)((long long)jobs * (i + 1) / of);
   }
   __device__ bool next(Job& j) {                 // by whole warps
     int sample_head;
@@ -866,19 +863,29 @@ static int image_map(CUtensorMap* m, const void* base, long long rows) {
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 }
 
-// How the jobs of dQ, dK and dV are dealt to CTA pairs: those with one dK / dV job more than others get `few` dQ jobs, so that all
-// end together; returns the steps of the longest share (an end of a job counts as four).
-static double deal_jobs(long long kv, long long pt, long long kb, long long kt, int splits, int pairs, int* few) {
+// How the jobs of dQ, dK and dV are dealt to CTA pairs: the pairs with one dK / dV job more than others take `more_q` dQ jobs together,
+// the others the rest, so that the longest share is shortest; returns its steps (an end of a job counts as four).  With 36 (sample, kv
+// head)s of one tile each 72 of 74 pairs have a dK / dV job: left to the other two, the 36 dQ jobs take 54 us (one query of 32 heads,
+// width 256), one to every second of the 72 25.
+static double deal_jobs(long long kv, long long pt, long long kb, long long kt, int splits, int pairs, int* more_q) {
   const long long n_kv = kv * 2 * kt * splits, n_q = kv * pt, base = n_kv / pairs, more = n_kv % pairs;
   const double len_kv = 4.0 * ((pt + splits - 1) / splits) + 4.0, len_q = kb + 4.0;
   const double mean = (n_kv * len_kv + n_q * len_q) / pairs;
-  long long q = more ? (long long)((mean - (base + 1) * len_kv) / len_q + 0.5) : 0;
+  // as many to each pair of `more` as end by the mean, or one more
+  long long q = more ? (long long)((mean - (base + 1) * len_kv) / len_q) : 0;
   if (q < 0) q = 0;
-  if (more && q * more > n_q) q = n_q / more;
-  *few = (int)q;
-  const long long rest = (n_q - q * more + pairs - more - 1) / (pairs - more);
-  const double first = more ? (base + 1) * len_kv + q * len_q : 0.0, second = base * len_kv + rest * len_q;
-  return first > second ? first : second;
+  double best = 0.0;
+  for (int i = 0; i < (more ? 2 : 1); ++i, ++q) {
+    const long long jobs = q * more < n_q ? q * more : n_q, rest = n_q - jobs;
+    const double first = more ? (base + 1) * len_kv + (jobs + more - 1) / more * len_q : 0.0;
+    const double second = base * len_kv + (rest + pairs - more - 1) / (pairs - more) * len_q;
+    const double longest = first > second ? first : second;
+    if (i == 0 || longest < best) {
+      best = longest;
+      *more_q = (int)jobs;
+    }
+  }
+  return best;
 }
 
 static int st_sms() {
@@ -941,13 +948,20 @@ extern "C" void otb_attn_bwd_stored_plan(int B, int Sq, int Sk, int H, int Hkv, 
   const double out_bytes = 4.0 * B * Sk * Hkv * D;
   double best = 0;
   for (int s = 1; s <= ST_MAX_SPLITS && s <= pt && (s == 1 || s * out_bytes <= 256.0 * (1 << 20)); ++s) {
-    int few;
-    const double cost = deal_jobs(kv, pt, kb, kt, s, pairs, &few) * step_us + (s > 1 ? 5.0 + 2 * out_bytes * (2 * s + 0.5) / 5e6 : 0.0);
+    int more_q;
+    const double cost = deal_jobs(kv, pt, kb, kt, s, pairs, &more_q) * step_us + (s > 1 ? 5.0 + 2 * out_bytes * (2 * s + 0.5) / 5e6 : 0.0);
     if (s == 1 || cost < best) {
       best = cost;
       *kv_splits = s;
     }
   }
+}
+
+// dQ jobs that the pairs with one dK / dV job more than others take together (deal_jobs), for tests on the host.
+extern "C" int otb_attn_bwd_stored_deal(int kv, int ptiles, int kblks, int key_tiles, int splits, int pairs) {
+  int more_q = 0;
+  deal_jobs(kv, ptiles, kblks, key_tiles, splits, pairs, &more_q);
+  return more_q;
 }
 
 // Arguments of one call (mirrored field by field by the ctypes structure of the Python launcher).  q (B,Sq,H,D), k / v (B,Sk,Hkv,D)
@@ -1008,7 +1022,7 @@ extern "C" int otb_attn_bwd_stored(const OtbAttnBwdStored* a, cudaStream_t strea
   if (rows > INT_MAX) return -8;
   const long long jobs = (long long)Hkv * B * (p.ptiles + 2 * p.key_tiles * p.splits);
   const int pairs = (int)(jobs < st_sms() / 2 ? jobs : st_sms() / 2);
-  deal_jobs((long long)Hkv * B, p.ptiles, p.kblks, p.key_tiles, p.splits, pairs, &p.dq_few);
+  deal_jobs((long long)Hkv * B, p.ptiles, p.kblks, p.key_tiles, p.splits, pairs, &p.dq_more);
   StoredMaps m;
   const long long* t = a->strides;
   int r = st_map(&m.q, a->q, D, H, Sq, B, t[2], t[1], t[0], g, 64 / g);

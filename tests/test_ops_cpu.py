@@ -356,6 +356,32 @@ def test_stored_attention_backward_takes_fewer_samples_where_memory_is_short(mon
     assert calls == (want or ["recomputed"])
 
 
+@pytest.mark.parametrize("kv", [1, 8, 35, 36, 37, 46, 74, 110, 184, 900])
+@pytest.mark.parametrize("Sq_rows,Sk", [(2, 2), (256, 64), (300, 903), (900, 113), (5000, 5000), (256, 4000)])
+def test_stored_attention_backward_deals_its_jobs_evenly(kv, Sq_rows, Sk):
+    """Every dQ job goes to one CTA pair, and no pair's share is above the mean by more than the job of each kind that a share of
+    whole jobs cannot avoid (and one for the rounding of equal runs)."""
+    from opentau_b200.ops import _lib, build
+    if not build.lib_path("attention_bwd_stored_tcgen05").exists():
+        pytest.skip("native libraries are not built")
+    pt, kb = -(-Sq_rows // 256), -(-Sk // 64)
+    kt = -(-kb // 4)
+    for splits in (1, 3):
+        if splits > pt:
+            continue
+        n_q, n_kv = kv * pt, kv * 2 * kt * splits
+        pairs = min(74, n_q + n_kv)
+        more = n_kv % pairs
+        more_q = _lib.load("attention_bwd_stored_tcgen05").otb_attn_bwd_stored_deal(kv, pt, kb, kt, splits, pairs)
+        assert 0 <= more_q <= (n_q if more else 0)
+        len_kv, len_q = 4 * -(-pt // splits) + 4, kb + 4
+        run = [(more_q * (i + 1) // more - more_q * i // more) for i in range(more)]
+        run += [((n_q - more_q) * (i + 1) // (pairs - more) - (n_q - more_q) * i // (pairs - more)) for i in range(pairs - more)]
+        assert sum(run) == n_q
+        shares = [(n_kv // pairs + (i < more)) * len_kv + r * len_q for i, r in enumerate(run)]
+        assert max(shares) <= sum(shares) / pairs + len_kv + 2 * len_q, (splits, max(shares), sum(shares) / pairs)
+
+
 @pytest.mark.parametrize("cols", [8, 128, 768, 1032, 1280, 2048, 8192, 32768])
 @pytest.mark.parametrize("inner", [8, 64, 256, 1088, 2048, 5120, 16384])
 def test_few_row_plans_fit_the_chip(cols, inner):
