@@ -154,8 +154,15 @@ def bwd_stored_plan(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int) -> tuple
 
 
 def stored_bwd_samples(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int) -> int:
-    """Samples that a launch of the stored backward takes; 0 where one alone has more P and dS than is kept (8 heads of 8192
-    positions): the recomputing kernels."""
+    """Samples that a launch of the stored backward takes; 0, the recomputing kernels, where one alone has more P and dS than is kept
+    (8 heads of more than 8192 positions) and for many short samples."""
+    # A sample of up to 128 query rows and 128 keys is one tile of each recomputing kernel, with nothing to recompute, and a quarter
+    # of a stored pair of 256 rows times a tile of 256 keys.  Stored / recomputing, geometric mean over 1297 such sizes of fourteen head
+    # layouts by their tiles to an SM: 0.79 up to 0.3, where the chip is empty either way, 1.07 to 0.5, 1.39 to 0.7, 1.43 (0.78 - 1.85)
+    # above; 2048 sequences of 6, 16 heads of 72, 5786 us and 2.2 GB of scratch against 3524 us and none.  Padding in one
+    # direction or of a last tile does not turn it: with at least twice the area 0.72 (679 sizes, 0.32 - 1.22)
+    if Sq * (H // Hkv) <= 128 and Sk <= 128 and B * Hkv > 0.3 * NUM_SMS:
+        return 0
     return min(B, BWD_STORED_LIMIT // (2 * bwd_stored_plan(1, Sq, Sk, H, Hkv, D)[0]))
 
 

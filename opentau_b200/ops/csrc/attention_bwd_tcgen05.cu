@@ -1,5 +1,6 @@
-// Block-causal flash attention backward for sm_100a (tcgen05 + TMEM + TMA) without scratch memory for P and dS: for calls of which
-// not even one sample's P and dS find room (attention_bwd_stored_tcgen05.cu keeps them and takes about half the time).
+// Block-causal flash attention backward for sm_100a (tcgen05 + TMEM + TMA) without scratch memory for P and dS: for many samples of one
+// tile each, where nothing is recomputed, and for calls of which not even one sample's P and dS find room
+// (attention_bwd_stored_tcgen05.cu keeps them and elsewhere takes about half the time).
 //
 // Three launches of one templated kernel, each an "inner products -> elementwise -> accumulate" pipeline
 // with the same warp roles as the forward kernel (warp 0 TMA, warp 1 MMA, warps 2..9 elementwise: two warps per

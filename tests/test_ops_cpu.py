@@ -382,6 +382,18 @@ def test_stored_attention_backward_deals_its_jobs_evenly(kv, Sq_rows, Sk):
         assert max(shares) <= sum(shares) / pairs + len_kv + 2 * len_q, (splits, max(shares), sum(shares) / pairs)
 
 
+@pytest.mark.parametrize("size,want", [
+    ((2048, 6, 6, 16, 16, 72), 0), ((45, 128, 128, 8, 8, 64), 0), ((44, 128, 128, 8, 1, 64), 44), ((45, 16, 128, 8, 1, 256), 0),
+    ((45, 17, 128, 8, 1, 256), 45), ((45, 16, 129, 8, 1, 256), 45), ((1, 8192, 8192, 8, 1, 256), 1), ((1, 8193, 8193, 8, 1, 256), 0),
+    ((4, 4096, 4096, 8, 1, 256), 4), ((8, 4097, 4097, 8, 1, 256), 3), ((16, 1227, 1227, 8, 1, 256), 16)])
+def test_attention_backward_keeps_p_and_ds_where_they_are_worth_it(size, want):
+    """One tile of 128 rows and 128 keys to a sample and many samples: nothing is recomputed, and nothing is stored."""
+    from opentau_b200.ops import attention_native, build
+    if not build.lib_path("attention_bwd_stored_tcgen05").exists():
+        pytest.skip("native libraries are not built")
+    assert attention_native.stored_bwd_samples(*size) == want
+
+
 @pytest.mark.parametrize("cols", [8, 128, 768, 1032, 1280, 2048, 8192, 32768])
 @pytest.mark.parametrize("inner", [8, 64, 256, 1088, 2048, 5120, 16384])
 def test_few_row_plans_fit_the_chip(cols, inner):
