@@ -752,27 +752,38 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
   pdl_wait();
 
   // ---- 1 + the last valid key with k_blk <= the tile's largest valid q_blk (no order assumed), searched from the end; the loads
-  // of Q and of the first keys are on their way meanwhile (a tile that sees nothing runs one block)
+  // of Q and of the first keys are on their way meanwhile (a tile that sees nothing runs one block).  All reads that the last 512 keys
+  // take are in flight together, those of the queries beside them
   if (warp == 1) {
-    int qmax = INT_MIN, any = 0;
-    for (int i = lane; i < pos_per_tile; i += 32) {
-      const int ps = p0 + i;
-      if (ps < p.Sq && p.q_valid[(long long)b * p.Sq + ps]) {
-        qmax = max(qmax, p.q_blk[(long long)b * p.Sq + ps]);
-        any = 1;
-      }
-    }
-    qmax = __reduce_max_sync(0xffffffffu, qmax);
-    any = __any_sync(0xffffffffu, any);
-    int last = -1;
-    for (int end = p.Sk; any && end > 0 && last < 0; end -= 512) {
-      int kb[16], kv[16];
+    int kb[16], kv[16];
+    auto fetch_keys = [&](int end) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const int j = end - 512 + i * 32 + lane;
         kb[i] = j >= 0 ? p.k_blk[(long long)b * p.Sk + j] : 0;
         kv[i] = j >= 0 ? p.k_valid[(long long)b * p.Sk + j] : 0;
       }
+    };
+    fetch_keys(p.Sk);
+    int qb[4], qv[4];                            // pos_per_tile <= 128
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int ps = p0 + i * 32 + lane;
+      const bool in = i * 32 + lane < pos_per_tile && ps < p.Sq;
+      qb[i] = in ? p.q_blk[(long long)b * p.Sq + ps] : 0;
+      qv[i] = in ? p.q_valid[(long long)b * p.Sq + ps] : 0;
+    }
+    int qmax = INT_MIN, any = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (qv[i]) qmax = max(qmax, qb[i]);
+      any |= qv[i];
+    }
+    qmax = __reduce_max_sync(0xffffffffu, qmax);
+    any = __any_sync(0xffffffffu, any);
+    int last = -1;
+    for (int end = p.Sk; any && end > 0 && last < 0; end -= 512) {
+      if (end < p.Sk) fetch_keys(end);
 #pragma unroll
       for (int i = 0; i < 16; ++i)
         if (kv[i] && kb[i] <= qmax) last = max(last, end - 512 + i * 32 + lane);
@@ -1250,8 +1261,13 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
   // what a launch requests ahead stays a quarter of L2
   const long long block_bytes = 4LL * bn * dpad * Hkv * B * nsplit;
   p.ahead = (int)((32LL << 20) / block_bytes);
-  // unsplit, head width above 128 (64 rows of a query tile at a time: groups up to 64)
-  const bool wide = dpad == 256 && nsplit == 1 && g <= 64;
+  // unsplit, head width above 128 (64 rows of a query tile at a time: groups up to 64).  Where a kv head has one query tile the other
+  // kernel does not look for the last visible key, and of a few blocks that and the query tile's way into tensor memory are the larger
+  // part: us, 8 heads on 1 of 256, wide / other, 148 tiles of 96 rows against 20, 100, 192 and 256 keys 8.9 / 7.2, 9.5 / 8.8, 10.9 / 10.3 and
+  // 11.9 / 11.6; 600 tiles 36.6 / 31.5, 42.9 / 42.0, 48.5 / 55.0 and 53.1 / 64.6.  With more tiles to a kv head both look, and wide wins
+  // (tiles of 248 rows against 20 and 128 keys 8.2 / 9.0 and 8.7 / 10.1)
+  const bool brief = p.skip_reach && (Sk <= 64 || (Sk <= 192 && (long long)Hkv * B <= 2 * sm_count()));
+  const bool wide = dpad == 256 && nsplit == 1 && g <= 64 && !brief;
   int r = make_map4(&tq, q, D, H, Sq, B, q_sh, q_ss, q_sb, g, (cluster ? p.cl_rows : (wide ? 64 : ATT_M)) / g);
   if (r) return 1000 + r;
   r = make_map4(&tk, k, D, Hkv, Sk, B, k_sh, k_ss, k_sb, 1, bn);

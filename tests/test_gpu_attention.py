@@ -422,6 +422,25 @@ def test_unsplit_forward_above_width_128(D, H, Hkv, Sq, Sk, big):
     assert float((lse.double() - want_lse).abs().max()) < 1e-4 * big ** 2 + 1e-5      # fp32 sums of scores up to about 5 big
 
 
+@pytest.mark.parametrize("D,H,Hkv", [(256, 8, 1), (256, 2, 2), (160, 4, 4), (136, 64, 1)])
+@pytest.mark.parametrize("Sk", [1, 20, 64, 65, 128, 192, 193, 256, 300])
+def test_forward_of_one_query_tile_gives_the_bits_of_several(D, H, Hkv, Sk):
+    """A tile to a kv head and a few blocks of keys take another kernel than several tiles, where both sum in one order."""
+    from opentau_b200.ops import attention_native, cuda_ops
+    B, one = 3, 128 * Hkv // H
+    gen = torch.Generator(device="cuda").manual_seed(D + Sk)
+    q, k, v = (torch.randn(*s, device="cuda", generator=gen).to(torch.bfloat16)
+               for s in ((B, 2 * one + 1, H, D), (B, Sk, Hkv, D), (B, Sk, Hkv, D)))
+    qb = torch.randint(0, 6, q.shape[:2], device="cuda", generator=gen, dtype=torch.int32)
+    kb = torch.randint(0, 7, (B, Sk), device="cuda", generator=gen, dtype=torch.int32)
+    qv, kv = torch.rand(q.shape[:2], device="cuda", generator=gen) > 0.1, torch.rand(B, Sk, device="cuda", generator=gen) > 0.1
+    all_o, all_lse = attention_native.attn_fwd(q, k, v, qb, kb, qv, kv, D ** -0.5, nsplit=1)
+    for n in (1, one):
+        o, lse = attention_native.attn_fwd(q[:, :n].contiguous(), k, v, qb[:, :n], kb, qv[:, :n], kv, D ** -0.5, nsplit=1)
+        assert torch.equal(o, all_o[:, :n]) and torch.equal(lse, all_lse[:, :, :n])
+    cuda_ops.check_status()
+
+
 @pytest.mark.parametrize("D,H,Hkv,S", [(256, 8, 1, 513), (256, 2, 2, 1000), (200, 4, 4, 449), (136, 8, 4, 65), (128, 4, 2, 1025),
                                        (96, 2, 2, 129), (64, 8, 1, 900), (24, 4, 4, 1000), (16, 32, 1, 130)])
 def test_backward_with_fixed_tiles_in_tensor_memory(D, H, Hkv, S):
