@@ -65,8 +65,9 @@ def split_kv(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int) -> int:
     if ctas * 4 > NUM_SMS:
         # half the chip idle and a long stream: two halves and a merge.  One pass against two halves, inside a replayed graph:
         # 16 heads of 72, 64 tiles: 21.2 / 19.0 us with 8 blocks, 35.0 / 26.6 with 15; with tiles for more than half the SMs it
-        # loses.  Above a width of 128 one pass wins: 8 heads on 1 of 256, 61 tiles of 968 keys 23.6 / 28.4, 64 of 1277 27.0 / 31.6
-        return 2 if D <= 128 and ctas * 2 <= NUM_SMS and nblk >= 15 else 1
+        # loses.  Above a width of 128 one pass is a kernel of its own, and its blocks are half as large: 8 heads on 1 of 256, 38 - 74
+        # tiles of 24 blocks 30.5 / 33.8, 47 52.4 / 53.2, 64 66.8 / 64.9, 128 126.4 / 115.5, 256 242.2 / 212.0
+        return 2 if ctas * 2 <= NUM_SMS and nblk >= (64 if D > 128 else 15) else 1
     return max(1, min(8, NUM_SMS // ctas, nblk // 2))
 
 

@@ -394,6 +394,15 @@ def test_attention_backward_keeps_p_and_ds_where_they_are_worth_it(size, want):
     assert attention_native.stored_bwd_samples(*size) == want
 
 
+@pytest.mark.parametrize("size,want", [
+    ((1, 8192, 8192, 1, 1, 256), 2), ((1, 4737, 4096, 1, 1, 256), 2), ((1, 9472, 8192, 1, 1, 256), 2), ((1, 9473, 8192, 1, 1, 256), 1), ((1, 968, 968, 8, 1, 256), 1),
+    ((1, 8192, 4032, 1, 1, 256), 1), ((1, 4096, 4096, 1, 1, 256), 4), ((1, 1024, 1920, 8, 8, 72), 2), ((1, 1024, 1792, 8, 8, 72), 1)])
+def test_attention_forward_splits_long_streams_of_few_tiles(size, want):
+    """Tiles for a quarter to half of the SMs: two halves from where the stream is long enough to pay for the merge."""
+    from opentau_b200.ops import attention_native
+    assert attention_native.split_kv(*size) == want
+
+
 @pytest.mark.parametrize("cols", [8, 128, 768, 1032, 1280, 2048, 8192, 32768])
 @pytest.mark.parametrize("inner", [8, 64, 256, 1088, 2048, 5120, 16384])
 def test_few_row_plans_fit_the_chip(cols, inner):
