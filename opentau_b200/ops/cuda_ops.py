@@ -87,15 +87,27 @@ def use_skinny(layout: str, M: int, N: int, accumulate: bool, bn: int, K: int = 
         return M <= 128 or (M <= 256 and N <= 8192) or (M <= 640 and N <= 2048 and -(-N // 128) * -(-M // 64) <= 148)
     if M <= 64 or (M <= 256 and N <= 2048 and K >= 3072):
         return True
-    # A product that is differentiated keeps the persistent kernel and with it the order of its sums: few of a training pass are this small.
-    # Up to one CTA of 128 columns x 64 rows to an SM: us in a replayed graph with a norm in front and cold weights, few-row /
-    # persistent kernel: 100 x 1024 x 1024 5.7 / 8.1, 200 x 2560 x 1024 7.5 / 8.8, 256 x 4096 x 2048 12.5 / 12.8, 400 x 2560 x 1024 9.2 / 10.3, 400 x
-    # 1152 x 4096 13.4 / 19.6, 512 x 2048 x 2048 12.7 / 12.9, 768 x 1152 x 4096 14.5 / 20.2, 768 x 768 x 256 6.3 / 6.7; of 570 sizes of 65 - 768 rows, 256 -
-    # 6144 columns, K 128 - 4096 within this line it loses more than a hundredth at eight (4 % at most).  Beyond it: 512 x 3456 x 1024 11.6 /
-    # 11.1, 640 x 2560 x 2048 15.5 / 14.6, 768 x 4096 x 1024 14.7 / 12.9, 200 x 6144 x 1024 11.1 / 10.8; more columns lose from 65 rows on
-    # (100 x 8192 x 1024 9.8 / 8.9).  With an activation at the end it wins on half as many tiles (256 x 1024 x 1024 7.2 / 9.4, 128 x 4304 x 1152
-    # 8.7 / 10.1, 256 x 4304 x 1152 11.4 / 10.6), with a gated MLP's product on narrow ones alone (200 x 4096 x 1024 10.2 / 9.8)
-    return no_grad and end != "glu" and M <= 768 and N <= 6144 and -(-N // 128) * -(-M // 64) <= (74 if end else 148)
+    # a product that is differentiated keeps the persistent kernel and with it the order of its sums: few of a training pass are this small
+    return no_grad and end != "glu" and M <= 768 and N <= 6144 and _few_row_wins(M, N, K, end)
+
+
+def _few_row_wins(M: int, N: int, K: int, end: str) -> bool:
+    """Products of 65 - 768 rows of an inference pass: up to one CTA of 128 columns x 64 rows to an SM, fewer where the sum is short."""
+    tiles = -(-N // 128) * -(-M // 64)
+    if end:
+        # with an activation it wins on half as many tiles: 256 x 1024 x 1024 7.2 / 9.4 us (few-row / persistent kernel), 128 x 4304 x 1152
+        # 8.7 / 10.1, 256 x 4304 x 1152 11.4 / 10.6; with a gated MLP's product on narrow ones alone (200 x 4096 x 1024 10.2 / 9.8)
+        return tiles <= 74
+    if tiles > 148 or K < 128:
+        return False
+    # The persistent kernel's cost is one round of tiles whatever their number; the few-row kernel's grows with the area, the less the
+    # longer the sum that it splits.  us in a replayed graph with a norm in front and cold weights, few-row / persistent kernel: 100 x 1024 x
+    # 1024 5.7 / 8.1, 333 x 2560 x 1024 8.8 / 9.8, 400 x 1024 x 4096 13.3 / 19.9, 450 x 2048 x 8192 28.5 / 34.8; beyond the line 512 x 2048 x
+    # 1152 11.1 / 10.0, 256 x 3456 x 1152 10.5 / 10.2.  More than one round of 64-column tiles turns it again: 400 x 2560 x 1024 9.5 /
+    # 10.4, 550 x 2048 x 2048 14.5 / 15.4.  Of 7437 random sizes up to 148 tiles, K 64 - 8192, the line takes 5874 at 0.74 in the mean and loses more than
+    # a twentieth at 69 (outputs of 16 columns, up to 13 %); what it leaves is 1.02 in the mean, sums below 128 1.00
+    line = 48 if K < 256 else 60 if K < 512 else 82 if K < 1024 else 105 if K < 2048 else 112 if K < 4096 else 148
+    return M * N <= line * 64 * 128 or (K >= 256 and -(-M // 128) * -(-N // 64) > 148)
 
 
 class _SkinnyArgs(ctypes.Structure):

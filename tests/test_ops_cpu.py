@@ -403,6 +403,19 @@ def test_attention_forward_splits_long_streams_of_few_tiles(size, want):
     assert attention_native.split_kv(*size) == want
 
 
+@pytest.mark.parametrize("M,N,K,end,want", [
+    (100, 1024, 1024, "", True), (333, 2560, 1024, "", True), (400, 2560, 1024, "", True), (768, 1152, 4304, "", True), (512, 2048, 1152, "", False),
+    (256, 3456, 1152, "", False), (450, 2048, 2048, "", False), (550, 2048, 2048, "", True), (450, 2048, 8192, "", True), (400, 1024, 32, "", False),
+    (400, 1024, 128, "", False), (384, 1024, 128, "", True), (247, 4736, 512, "", False), (800, 256, 1024, "", False), (64, 256, 32, "", True),
+    (256, 4304, 1152, "act", False), (128, 4304, 1152, "act", True), (200, 1024, 1024, "glu", False)])
+def test_line_between_the_few_row_and_the_persistent_kernel(M, N, K, end, want):
+    """Products of 65 - 768 rows of an inference pass: the few-row kernel where the sum is long enough for the area."""
+    from opentau_b200.ops import cuda_ops
+    if not cuda_ops.SKINNY:
+        pytest.skip("the few-row kernel is switched off")
+    assert cuda_ops.use_skinny("nt", M, N, False, 0, K, False, end, True) is want
+
+
 @pytest.mark.parametrize("cols", [8, 128, 768, 1032, 1280, 2048, 8192, 32768])
 @pytest.mark.parametrize("inner", [8, 64, 256, 1088, 2048, 5120, 16384])
 def test_few_row_plans_fit_the_chip(cols, inner):
