@@ -167,44 +167,53 @@ def stored_bwd_samples(B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int) -> in
     return min(B, BWD_STORED_LIMIT // (2 * bwd_stored_plan(1, Sq, Sk, H, Hkv, D)[0]))
 
 
+@lru_cache(maxsize=1024)
+def _stored_layout(samples: int, at_once: int, B: int, Sq: int, Sk: int, H: int, Hkv: int, D: int, parts: int | None):
+    """Scratch of the stored backward, ``at_once`` samples at a time: bytes of P, offset of the parts' sums and of all, bytes of a
+    sample's share of a part; and the launches ``(first sample, samples, parts)``.  The parts of dK and dV, and with them the order of
+    the sums, are those of ``samples`` at a time."""
+    size, n_cover, _ = bwd_stored_plan(at_once, Sq, Sk, H, Hkv, D)
+    sums_off, one = -(-(2 * size + 4 * n_cover) // 16) * 16, 4 * Sk * Hkv * D
+    launches = []
+    for g0 in range(0, B, samples):
+        g1 = min(g0 + samples, B)
+        m = parts or bwd_stored_plan(g1 - g0, Sq, Sk, H, Hkv, D)[2]
+        launches += [(b0, min(at_once, g1 - b0), m) for b0 in range(g0, g1, at_once)]
+    return size, sums_off, sums_off + max((2 * m * n * one for _, n, m in launches if m > 1), default=0), one, launches
+
+
 def _attn_bwd_stored(samples: int, do, q, k, v, o, lse, qb, kb, qv, kv, dq, dk, dv, scale: float,
                      parts: int | None = None) -> bool:
     """dq, dk, dv through stored P and dS, ``samples`` at a time, or fewer where there is no room for as many; False where one
-    sample finds none.  The parts of dK and dV, and with them the order of the sums, are those of ``samples`` either way."""
+    sample finds none."""
     from . import cuda_ops
     B, Sq, H, D = q.shape
     Sk, Hkv = k.shape[1], k.shape[2]
-    groups = [(b0, n, parts or bwd_stored_plan(n, Sq, Sk, H, Hkv, D)[2])
-              for b0 in range(0, B, samples) for n in (min(samples, B - b0),)]
+    at_once = samples
     while True:                                  # one allocation: P, dS, cover, and the parts' fp32 dK and dV
-        size, n_cover, _ = bwd_stored_plan(samples, Sq, Sk, H, Hkv, D)
-        sums_off = -(-(2 * size + 4 * n_cover) // 16) * 16
-        one = 4 * Sk * Hkv * D                   # bytes of a sample's share of a part
-        room = max((2 * m * min(n, samples) * one for _, n, m in groups if m > 1), default=0)
+        size, sums_off, total, one, launches = _stored_layout(samples, at_once, B, Sq, Sk, H, Hkv, D, parts)
         try:
-            scratch = torch.empty(sums_off + room, dtype=torch.uint8, device=q.device)
+            scratch = torch.empty(total, dtype=torch.uint8, device=q.device)
             break
         except torch.cuda.OutOfMemoryError:
-            if samples == 1:
+            if at_once == 1:
                 return False
-            samples = (samples + 1) // 2
+            at_once = (at_once + 1) // 2
     s0 = scratch.data_ptr()
     fn = _entry("attention_bwd_stored_tcgen05", "otb_attn_bwd_stored", "pp")
     tensors = (q, k, v, o, do, lse, dq, dk, dv, qb, kb, qv, kv)
     at = [t.data_ptr() for t in tensors]
     strides = (c_longlong * 9)(*q.stride()[:3], *k.stride()[:3], *v.stride()[:3])
-    for g0, g_n, m in groups:
-        for b0 in range(g0, g0 + g_n, samples):
-            n = min(samples, g0 + g_n - b0)
-            sums_at = (s0 + sums_off, s0 + sums_off + m * n * one) if m > 1 else (0, 0)
-            args = _StoredBwdArgs(*at[:9], s0, s0 + size, s0 + 2 * size, *sums_at, *at[9:], cuda_ops.status_pointer(), strides,
-                                  n, Sq, Sk, H, Hkv, D, m, scale)
-            rc = fn(byref(args), cuda_ops._raw_stream())
-            if rc != 0:
-                raise RuntimeError(f"native attn_bwd failed with code {rc} (B={B} Sq={Sq} Sk={Sk} H={H} Hkv={Hkv} D={D})")
-            cuda_ops.launch_count += 3 + (m > 1)
-            if b0 + n < B:
-                at = [x + n * t.stride(0) * t.element_size() for x, t in zip(at, tensors)]
+    for b0, n, m in launches:
+        sums_at = (s0 + sums_off, s0 + sums_off + m * n * one) if m > 1 else (0, 0)
+        args = _StoredBwdArgs(*at[:9], s0, s0 + size, s0 + 2 * size, *sums_at, *at[9:], cuda_ops.status_pointer(), strides,
+                              n, Sq, Sk, H, Hkv, D, m, scale)
+        rc = fn(byref(args), cuda_ops._raw_stream())
+        if rc != 0:
+            raise RuntimeError(f"native attn_bwd failed with code {rc} (B={B} Sq={Sq} Sk={Sk} H={H} Hkv={Hkv} D={D})")
+        cuda_ops.launch_count += 3 + (m > 1)
+        if b0 + n < B:
+            at = [x + n * t.stride(0) * t.element_size() for x, t in zip(at, tensors)]
     return True
 
 
