@@ -115,7 +115,8 @@ def test_attention_autograd_on_gpu_matches_cpu():
 @pytest.mark.parametrize("D", [64, 72, 128, 256])
 @pytest.mark.parametrize("H,Hkv", [(8, 1), (8, 4), (4, 4)])
 @pytest.mark.parametrize("Sq,cross", [(50, 0), (131, 0), (50, 203), (300, 0)])
-def test_attn_bwd_matches_dense(D, H, Hkv, Sq, cross):
+@pytest.mark.parametrize("samples", [2, 0])                # through stored P and dS, and recomputed
+def test_attn_bwd_matches_dense(D, H, Hkv, Sq, cross, samples):
     from opentau_b200 import ops
     from opentau_b200.ops import attention_native, cuda_ops
     dev = torch.device("cuda:0")
@@ -126,7 +127,7 @@ def test_attn_bwd_matches_dense(D, H, Hkv, Sq, cross):
     o, lse = attention_native.attn_fwd(q, k, v, qb, kb, qv, kv, scale)
     g = torch.Generator().manual_seed(5)
     do = (torch.randn(B, Sq, H * D, generator=g) * qv.cpu()[:, :, None]).to(torch.bfloat16).to(dev)
-    dq, dk, dv = attention_native.attn_bwd(do, q, k, v, o, lse, qb, kb, qv, kv, scale)
+    dq, dk, dv = attention_native.attn_bwd(do, q, k, v, o, lse, qb, kb, qv, kv, scale, samples=samples)
     cuda_ops.check_status()
     qc, kc, vc = q.cpu().float(), k.cpu().float(), v.cpu().float()
     o_ref, lse_ref = ops.prims.attn_fwd(qc, kc, vc, qb.cpu(), kb.cpu(), qv.cpu(), kv.cpu(), scale)
@@ -443,7 +444,8 @@ def test_forward_of_one_query_tile_gives_the_bits_of_several(D, H, Hkv, Sk):
 
 @pytest.mark.parametrize("D,H,Hkv,S", [(256, 8, 1, 513), (256, 2, 2, 1000), (200, 4, 4, 449), (136, 8, 4, 65), (128, 4, 2, 1025),
                                        (96, 2, 2, 129), (64, 8, 1, 900), (24, 4, 4, 1000), (16, 32, 1, 130)])
-def test_backward_with_fixed_tiles_in_tensor_memory(D, H, Hkv, S):
+@pytest.mark.parametrize("samples", [2, 0])
+def test_backward_with_fixed_tiles_in_tensor_memory(D, H, Hkv, S, samples):
     """Rings that wrap twice, last blocks and tiles of one column or row, head widths off the 64-column pieces, against 64 bits.
     P, dS and the results are rounded to bf16 (2^-9 each): the sums' relative error stays below two of them."""
     from opentau_b200.ops import attention_native, cuda_ops
@@ -456,7 +458,7 @@ def test_backward_with_fixed_tiles_in_tensor_memory(D, H, Hkv, S):
     valid[1, S - 7:] = False
     o, lse = attention_native.attn_fwd(q, k, v, blk, blk, valid, valid, D ** -0.5)
     do[~valid] = 0
-    got = attention_native.attn_bwd(do.view(B, S, -1), q, k, v, o, lse, blk, blk, valid, valid, D ** -0.5)
+    got = attention_native.attn_bwd(do.view(B, S, -1), q, k, v, o, lse, blk, blk, valid, valid, D ** -0.5, samples=samples)
     cuda_ops.check_status()
     qd, kd, vd = (t.double().requires_grad_() for t in (q, k, v))
     see = valid[:, None, :, None] & valid[:, None, None, :] & (blk[:, None, None, :] <= blk[:, None, :, None])
@@ -469,7 +471,8 @@ def test_backward_with_fixed_tiles_in_tensor_memory(D, H, Hkv, S):
 
 
 @pytest.mark.parametrize("D,H,Hkv,S", [(64, 4, 1, 900), (72, 16, 16, 260), (128, 8, 2, 641), (200, 4, 4, 449), (256, 8, 1, 1027)])
-def test_backward_of_strided_views_and_repeats(D, H, Hkv, S):
+@pytest.mark.parametrize("samples", [2, 1, 0])
+def test_backward_of_strided_views_and_repeats(D, H, Hkv, S, samples):
     """q, k and v as views of one q/k/v buffer (the fixed tiles are addressed by hand), a second sample and a gradient that starts
     off a 16-byte boundary: the same bits as contiguous tensors give, and the same bits again every time (a block's scores go
     over the columns that the block before has just read, rings wrap many times)."""
@@ -487,9 +490,9 @@ def test_backward_of_strided_views_and_repeats(D, H, Hkv, S):
     assert not q.is_contiguous() and not v.is_contiguous() and do.data_ptr() % 16
     o, lse = attention_native.attn_fwd(q, k, v, blk, blk, valid, valid, D ** -0.5)
     args = (o, lse, blk, blk, valid, valid, D ** -0.5)
-    want = attention_native.attn_bwd(do.clone(), q.contiguous(), k.contiguous(), v.contiguous(), *args)
+    want = attention_native.attn_bwd(do.clone(), q.contiguous(), k.contiguous(), v.contiguous(), *args, samples=samples)
     for _ in range(4):
-        got = attention_native.attn_bwd(do, q, k, v, *args)
+        got = attention_native.attn_bwd(do, q, k, v, *args, samples=samples)
         assert all(torch.equal(x, y) for x, y in zip(got, want))
     cuda_ops.check_status()
 
@@ -565,15 +568,19 @@ def test_backward_recomputes_where_there_is_no_room_for_p_and_ds(monkeypatch):
     blk, valid = torch.zeros(B, S, dtype=torch.int32, device="cuda"), torch.ones(B, S, dtype=torch.bool, device="cuda")
     o, lse = attention_native.attn_fwd(q, k, v, blk, blk, valid, valid, D ** -0.5)
     args = (do, q, k, v, o, lse, blk, blk, valid, valid, D ** -0.5)
-    want = attention_native.attn_bwd(*args, samples=0)
+    want = {n: attention_native.attn_bwd(*args, samples=n) for n in (2, 1, 0)}
+    assert all(_rel(x, w.double()) < 2 ** -8 for n in (2, 1) for x, w in zip(want[n], want[0]))
     both = attention_native.bwd_stored_plan(1, S, S, H, Hkv, D)[0] * 2
-    for limit, launches in ((2 * both, 3), (both, 6), (both - 1, 4)):
+    entry, taken = attention_native._entry, []
+    monkeypatch.setattr(attention_native, "_entry", lambda lib, *a: (taken.append(lib), entry(lib, *a))[1])
+    for limit, samples in ((2 * both, 2), (both, 1), (both - 1, 0)):
         monkeypatch.setattr(attention_native, "BWD_STORED_LIMIT", limit)
-        before = cuda_ops.launch_count
+        assert attention_native.stored_bwd_samples(B, S, S, H, Hkv, D) == samples
+        taken.clear()
         got = attention_native.attn_bwd(*args)
         cuda_ops.check_status()
-        assert launches <= cuda_ops.launch_count - before <= launches * 3 // 2 + 1
-        assert all(_rel(x, w.double()) < 2 ** -8 for x, w in zip(got, want))
+        assert taken == ["attention_bwd_stored_tcgen05" if samples else "attention_bwd_tcgen05"]
+        assert all(torch.equal(x, w) for x, w in zip(got, want[samples]))
     monkeypatch.undo()
     real = torch.empty
 
@@ -585,7 +592,26 @@ def test_backward_recomputes_where_there_is_no_room_for_p_and_ds(monkeypatch):
     monkeypatch.setattr(torch, "empty", empty)
     got = attention_native.attn_bwd(*args)
     monkeypatch.undo()
-    assert all(torch.equal(x, w) for x, w in zip(got, want))
+    assert all(torch.equal(x, w) for x, w in zip(got, want[0]))
+
+
+@pytest.mark.parametrize("B,Sq,Sk,H,Hkv,D", [(36, 2, 2, 32, 1, 256), (9, 113, 113, 8, 4, 256), (23, 34, 903, 2, 2, 256), (3, 106, 106, 12, 12, 64),
+                                             (110, 244, 7, 1, 1, 128), (37, 300, 70, 1, 1, 72), (74, 20, 300, 1, 1, 64)])
+def test_stored_backward_of_many_kv_heads(B, Sq, Sk, H, Hkv, D):
+    """(sample, kv head)s whose jobs are no multiple of the CTA pairs, dealt in every way; against the recomputing kernels as above."""
+    from opentau_b200.ops import attention_native, cuda_ops
+    g = torch.Generator(device="cuda").manual_seed(B + Sq)
+    q, k, v, do = (torch.randn(*shape, device="cuda", generator=g).to(torch.bfloat16)
+                   for shape in ((B, Sq, H, D), (B, Sk, Hkv, D), (B, Sk, Hkv, D), (B, Sq, H * D)))
+    qb, kb = (torch.randint(0, n, (B, s), device="cuda", generator=g, dtype=torch.int32) for n, s in ((6, Sq), (8, Sk)))
+    qv, kv = (torch.rand(B, s, device="cuda", generator=g) > 0.1 for s in (Sq, Sk))
+    o, lse = attention_native.attn_fwd(q, k, v, qb, kb, qv, kv, D ** -0.5)
+    args = (do, q, k, v, o, lse, qb, kb, qv, kv, D ** -0.5)
+    got, want = attention_native.attn_bwd(*args, samples=B), attention_native.attn_bwd(*args, samples=0)
+    cuda_ops.check_status()
+    for name, x, w in zip(("dq", "dk", "dv"), got, want):
+        diff = (x.double() - w.double()).norm().item()
+        assert bool(torch.isfinite(x).all()) and diff <= 2 ** -8 * w.double().norm().item() + 2 ** -12 * x.numel() ** 0.5, (name, diff)
 
 
 @pytest.mark.parametrize("D,H,Hkv", [(256, 8, 1), (128, 8, 2), (64, 4, 4), (72, 16, 16)])

@@ -195,7 +195,9 @@ def test_layer_norm_kernel(dev):
 
 
 @pytest.mark.parametrize("M,N,K", [(65, 6144, 128), (192, 6144, 72), (193, 6144, 72), (256, 4096, 264), (257, 4096, 136), (320, 3456, 1152),
-                                   (321, 3456, 128), (577, 2048, 200), (576, 2048, 200), (768, 1152, 264), (769, 1152, 264), (768, 8, 8)])
+                                   (321, 3456, 128), (577, 2048, 200), (576, 2048, 200), (768, 1152, 264), (769, 1152, 264), (768, 8, 8),
+                                   (384, 1024, 128), (385, 1024, 128), (480, 1024, 264), (481, 1024, 264), (420, 2048, 1152), (421, 2048, 1152),
+                                   (512, 2304, 520), (513, 2304, 520)])
 @pytest.mark.parametrize("end", ["plain", "bias_res", "f32", "gelu"])
 def test_products_at_the_line_between_the_two_kernels(dev, M, N, K, end):
     """Rows and columns on either side of the line, against 64 bits: operands are bf16, sums fp32, one rounding (2^-9; fp32 out: 1e-5)."""
@@ -232,6 +234,19 @@ def test_layer_norm_forward_at_the_edges_of_its_forms(dev, rows, H):
     torch.testing.assert_close(mean.double().view(-1), want_mean, rtol=1e-5, atol=1e-5)
     torch.testing.assert_close(rstd.double().view(-1), (var + 1e-6).rsqrt(), rtol=1e-4, atol=0)
     assert float((y.double() - want).norm() / want.norm()) < 2 ** -8
+
+
+@pytest.mark.parametrize("H", [264, 512, 520, 768, 1152, 1280])
+def test_layer_norm_by_warps_gives_the_bits_of_the_block_form(dev, H):
+    """3072 rows take a warp each, the same rows in slices of fewer a block each; rows don't depend on one another."""
+    from opentau_b200.ops import cuda_ops
+    g = torch.Generator(device=dev).manual_seed(H)
+    x, w, b = (torch.randn(*s, device=dev, generator=g).to(torch.bfloat16) for s in ((3075, H), (H,), (H,)))
+    x = x * 3 + 1
+    whole = cuda_ops.ln_fwd(x, w, b, 1e-6)
+    for lo, hi in ((0, 1), (0, 1024), (1024, 3075)):
+        part = cuda_ops.ln_fwd(x[lo:hi].contiguous(), w, b, 1e-6)
+        assert all(torch.equal(p.view(hi - lo, -1), t.view(3075, -1)[lo:hi]) for p, t in zip(part, whole))
 
 
 @pytest.mark.parametrize("rows,H", [(64, 256), (3, 520), (3072, 1152)])
