@@ -103,9 +103,10 @@ def _few_row_wins(M: int, N: int, K: int, end: str) -> bool:
     # The persistent kernel's cost is one round of tiles whatever their number; the few-row kernel's grows with the area, the less the
     # longer the sum that it splits.  us in a replayed graph with a norm in front and cold weights, few-row / persistent kernel: 100 x 1024 x
     # 1024 5.7 / 8.1, 333 x 2560 x 1024 8.8 / 9.8, 400 x 1024 x 4096 13.3 / 19.9, 450 x 2048 x 8192 28.5 / 34.8; on the line 256 x 3456 x
-    # 1152 10.5 / 10.2 and 768 x 1152 x 1152 even, beyond it 512 x 2048 x 1152 11.1 / 10.0.  More than one round of 64-column tiles turns it again: 400 x 2560 x 1024 9.5 /
-    # 10.4, 550 x 2048 x 2048 14.5 / 15.4.  Of 7437 random sizes up to 148 tiles, K 64 - 8192, the line takes 5875 at 0.74 in the mean and loses more than
-    # a twentieth at 69 (outputs of 16 columns, up to 13 %); what it leaves is 1.02 in the mean, sums below 128 1.00
+    # 1152 10.5 / 10.2 and 768 x 1152 x 1152 even, beyond it 512 x 2048 x 1152 11.1 / 10.0.  More than one round of 64-column tiles turns it
+    # again: 400 x 2560 x 1024 9.5 / 10.4, 550 x 2048 x 2048 14.5 / 15.4.  Of 7437 random sizes up to 148 tiles, K 64 - 8192, the line takes
+    # 5875 at 0.74 in the mean and loses more than a twentieth at 69 (outputs of 16 columns, up to 13 %); what it leaves is 1.02 in the
+    # mean, sums below 128 1.00
     line = 48 if K < 256 else 60 if K < 512 else 82 if K < 1024 else 108 if K < 2048 else 112 if K < 4096 else 148
     return M * N <= line * 64 * 128 or (K >= 256 and -(-M // 128) * -(-N // 64) > 148)
 

@@ -405,7 +405,7 @@ def test_attention_forward_splits_long_streams_of_few_tiles(size, want):
 
 @pytest.mark.parametrize("M,N,K,end,want", [
     (100, 1024, 1024, "", True), (333, 2560, 1024, "", True), (400, 2560, 1024, "", True), (768, 1152, 4304, "", True), (512, 2048, 1152, "", False),
-    (256, 3456, 1152, "", True), (768, 1152, 1152, "", True), (257, 3456, 1152, "", False), (450, 2048, 2048, "", False), (550, 2048, 2048, "", True), (450, 2048, 8192, "", True), (400, 1024, 32, "", False),
+    (256, 3456, 1152, "", True), (768, 1152, 1152, "", True), (250, 3600, 1152, "", False), (257, 3456, 1152, "", True), (450, 2048, 2048, "", False), (550, 2048, 2048, "", True), (450, 2048, 8192, "", True), (400, 1024, 32, "", False),
     (400, 1024, 128, "", False), (384, 1024, 128, "", True), (247, 4736, 512, "", False), (800, 256, 1024, "", False), (64, 256, 32, "", True),
     (256, 4304, 1152, "act", False), (128, 4304, 1152, "act", True), (200, 1024, 1024, "glu", False)])
 def test_line_between_the_few_row_and_the_persistent_kernel(M, N, K, end, want):
