@@ -96,13 +96,21 @@ __global__ void __launch_bounds__(256) attn_bwd_cover_kernel(StoredParams p) {
     s_last = -1;
     s_any = s_found = 0;
   }
-  bool any = false;
-  int qblk = INT_MIN;
+  // the queries and the last thousand keys in one round trip
+  int kb[4], kv[4];
+  auto fetch_keys = [&](int end) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int j = end - 1024 + i * 256 + (int)threadIdx.x;
+      kb[i] = j >= 0 ? p.k_blk[(long long)b * p.Sk + j] : 0;
+      kv[i] = j >= 0 ? p.k_valid[(long long)b * p.Sk + j] : 0;
+    }
+  };
+  fetch_keys(p.Sk);
   const int ps = t * pos_per + threadIdx.x, quarter = threadIdx.x * p.g / 64;
-  if ((int)threadIdx.x < pos_per && ps < p.Sq && p.q_valid[(long long)b * p.Sq + ps]) {      // pos_per <= 256
-    any = true;
-    qblk = p.q_blk[(long long)b * p.Sq + ps];
-  }
+  const bool in = (int)threadIdx.x < pos_per && ps < p.Sq;                                   // pos_per <= 256
+  const int qblk = in ? p.q_blk[(long long)b * p.Sq + ps] : INT_MIN;
+  const bool any = in && p.q_valid[(long long)b * p.Sq + ps] != 0;
   const int some = __syncthreads_or(any);
   if (any) {
     atomicMax(&s_qmax[quarter], qblk);
@@ -114,14 +122,9 @@ __global__ void __launch_bounds__(256) attn_bwd_cover_kernel(StoredParams p) {
   for (int i = 0; i < 4; ++i) qmax[i] = s_qmax[i];
   const unsigned asked = s_any;
   for (int end = p.Sk; some && end > 0; end -= 1024) {
-    int kb[4], kv[4], last = -1;
+    if (end < p.Sk) fetch_keys(end);
+    int last = -1;
     unsigned found = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int j = end - 1024 + i * 256 + (int)threadIdx.x;
-      kb[i] = j >= 0 ? p.k_blk[(long long)b * p.Sk + j] : 0;
-      kv[i] = j >= 0 ? p.k_valid[(long long)b * p.Sk + j] : 0;
-    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       unsigned sees = 0;
@@ -590,9 +593,14 @@ struct JobWalk {
         n += __popc(__ballot_sync(0xffffffffu, mine > 0));
         steps += mine;
       }
+      steps = __reduce_add_sync(0xffffffffu, steps);
       if (p.splits > 1) {
         j.lo = (int)((long long)n * j.split / p.splits);
         const int hi = (int)((long long)n * (j.split + 1) / p.splits);
+        if (steps == 4 * n) {                    // all rows of all pairs
+          j.nsteps = 4 * (hi - j.lo);
+          return true;
+        }
         steps = 0;
         for (int t0 = 0, seen = 0; t0 < p.ptiles && seen < hi; t0 += 32) {
           const int mine = steps_of(t0 + lane);
@@ -601,8 +609,9 @@ struct JobWalk {
           if (at >= j.lo && at < hi) steps += mine;
           seen += __popc(in);
         }
+        steps = __reduce_add_sync(0xffffffffu, steps);
       }
-      j.nsteps = __reduce_add_sync(0xffffffffu, steps);
+      j.nsteps = steps;
     }
     return true;
   }
@@ -690,8 +699,8 @@ attn_bwd_products_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_
             const unsigned r = reach[t];
             if ((r & REACH_MASK) <= 4u * j.tile || seen++ < j.lo) continue;
 #pragma unroll 1
-            for (int q = 0; q < 4; ++q) {        // 64 rows: half a tile of the pair
-              if (!(r >> (28 + q) & 1)) continue;
+            for (unsigned rows = r >> 28; rows != 0; rows &= rows - 1) {        // 64 rows: half a tile of the pair
+              const int q = __ffs(rows) - 1;
               --left;
               const int tq = 2 * t + (q >> 1);
               const int row0 = (int)(images + (long long)tq * p.kblks + 4 * j.tile + 2 * rank) * ST_M + (q & 1) * 64;
