@@ -23,11 +23,16 @@
 // padding may hold anything: dQ ends with the pair's last visible block, and dK and dV leave out every 64 rows that see nothing.
 // Results are deterministic: no atomics, fixed order of accumulation.
 //
-// us for the whole backward, recomputing / stored: 4096 positions, 8 heads on 1 of 256, 1024 of them causal 545 / 289; 8 x 1227 and
-// 16 x 1227 (259 causal; a training step's layer) 579 / 270 and 940 / 512; 2 x 700, 8 on 4 117 / 55; 2 x 2048, 32 on 8 of 128 735 / 480;
-// 24 x 256 and 3 x 1024, 16 of 72 211 / 125 and 205 / 146; 2 x 3000, 16 of 64 668 / 533; below 300 positions the host's time, alike.
-// What bounds it: P and dS are written once and read three times.  At 16 x 1227 the scores take 248 us for 0.8 GB written (memory
-// takes about 4.8 TB/s of pure writes), the products 240 us for 1.2 GB read; with their A operands in L2 they would take 183.  Tried
+// us for the whole backward, recomputing / stored: 4096 positions, 8 heads on 1 of 256, 1024 of them causal 556 / 306; 8 x 1227 and
+// 16 x 1227 (259 causal; a training step's layer) 577 / 274 and 938 / 508; 2 x 700, 8 on 4 115 / 45; 2 x 2048, 32 on 8 of 128 744 / 488;
+// 24 x 256 and 3 x 1024, 16 of 72 211 / 124 and 196 / 146; 2 x 3000, 16 of 64 783 / 558; 2 x 566, 16 of 72 94 / 60, 200 of 256 76 / 27; up to
+// about 300 positions of few samples a call is the host's time either way (33 us of launches, 37 recomputing).  Many samples of
+// one tile lose (2048 x 6 3534 / 5337) and stay with the recomputing kernels (stored_bwd_samples).
+// What bounds it: at 16 x 1227 the scores take 248 us, 1.5 us a block of 128 x 64, with DRAM at 48 % of its peak (0.63 GB written, 0.37 read
+// of q, o, dO and what other tiles' writes push out of L2), the tensor pipe at 34 % and issue slots at 47 %: the chain of a block from its
+// products through tensor memory and the elementwise warps to the staged images, and the start of every query tile (fixed tiles, delta)
+// that nothing runs under.  4096 positions, longer runs of one tile, 1.2 us a block.  The products read P and dS three times, 240 us for 1.2 GB;
+// with their A operands in L2 they would take 183.  Tried
 // and slower: S and dP of 128 keys without a second buffer (scores 117 -> 138 us at 4096 positions), eight elementwise warps (160),
 // all scores of a thread in registers at once (168: spills), storing warps of their own (127), products cut into runs
 // of equal length with fp32 sums at the cuts (289 -> 315 us in all: the streams of the pairs drift apart in memory).

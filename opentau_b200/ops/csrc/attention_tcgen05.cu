@@ -672,8 +672,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
 // the blocks in turn, a thread a whole row.  What one group needs of the other is the row's maximum in use, which it publishes
 // before its exponentials, and behind them the row's sums, which are so added in the order of the kernel above, to the same bits.
 // P goes over the scores it was made from; scores of block j + 2 wait for the commit of the product that reads P of j.
-// us, before / now: 4096 positions, 8 heads on 1, 1024 of them causal 191 / 112; 16 x 1227 (259 causal) 337 / 212; 2 x 1500, 8 on 4 80 /
-// 57; 4 x 589 23 / 18; 5000, 4 heads of 160 236 / 137.  At 4096 a block takes 1700 clocks: the chain from scores to P and the products
+// us, before / now: 4096 positions, 8 heads on 1, 1024 of them causal 191 / 104; 16 x 1227 (259 causal) 337 / 193; 2 x 1500, 8 on 4 80 /
+// 55; 4 x 589 23 / 18; 5000, 4 heads of 160 236 / 135.  At 4096 a block takes 1700 clocks: the chain from scores to P and the products
 // of two blocks that take turns.
 template <int DPAD>
 struct WideSmem {
