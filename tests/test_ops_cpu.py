@@ -395,8 +395,9 @@ def test_attention_backward_keeps_p_and_ds_where_they_are_worth_it(size, want):
 
 
 @pytest.mark.parametrize("size,want", [
-    ((1, 8192, 8192, 1, 1, 256), 2), ((1, 4737, 4096, 1, 1, 256), 2), ((1, 9472, 8192, 1, 1, 256), 2), ((1, 9473, 8192, 1, 1, 256), 1), ((1, 968, 968, 8, 1, 256), 1),
-    ((1, 8192, 4032, 1, 1, 256), 1), ((1, 4096, 4096, 1, 1, 256), 4), ((1, 1024, 1920, 8, 8, 72), 2), ((1, 1024, 1792, 8, 8, 72), 1)])
+    ((1, 8192, 8192, 1, 1, 256), 2), ((1, 4737, 4096, 1, 1, 256), 2), ((1, 9472, 8192, 1, 1, 256), 2), ((1, 9473, 8192, 1, 1, 256), 1),
+    ((1, 968, 968, 8, 1, 256), 1), ((1, 8192, 4032, 1, 1, 256), 1), ((1, 4096, 4096, 1, 1, 256), 4), ((1, 1024, 1920, 8, 8, 72), 2),
+    ((1, 1024, 1792, 8, 8, 72), 1)])
 def test_attention_forward_splits_long_streams_of_few_tiles(size, want):
     """Tiles for a quarter to half of the SMs: two halves from where the stream is long enough to pay for the merge."""
     from opentau_b200.ops import attention_native
@@ -404,10 +405,12 @@ def test_attention_forward_splits_long_streams_of_few_tiles(size, want):
 
 
 @pytest.mark.parametrize("M,N,K,end,want", [
-    (100, 1024, 1024, "", True), (333, 2560, 1024, "", True), (400, 2560, 1024, "", True), (768, 1152, 4304, "", True), (512, 2048, 1152, "", False),
-    (256, 3456, 1152, "", True), (768, 1152, 1152, "", True), (250, 3600, 1152, "", False), (257, 3456, 1152, "", True), (450, 2048, 2048, "", False), (550, 2048, 2048, "", True), (450, 2048, 8192, "", True), (400, 1024, 32, "", False),
-    (400, 1024, 128, "", False), (384, 1024, 128, "", True), (247, 4736, 512, "", False), (800, 256, 1024, "", False), (64, 256, 32, "", True),
-    (256, 4304, 1152, "act", False), (128, 4304, 1152, "act", True), (200, 1024, 1024, "glu", False)])
+    (100, 1024, 1024, "", True), (333, 2560, 1024, "", True), (400, 2560, 1024, "", True), (768, 1152, 4304, "", True),
+    (512, 2048, 1152, "", False), (256, 3456, 1152, "", True), (768, 1152, 1152, "", True), (250, 3600, 1152, "", False),
+    (257, 3456, 1152, "", True), (450, 2048, 2048, "", False), (550, 2048, 2048, "", True), (450, 2048, 8192, "", True),
+    (400, 1024, 32, "", False), (400, 1024, 128, "", False), (384, 1024, 128, "", True), (247, 4736, 512, "", False),
+    (800, 256, 1024, "", False), (64, 256, 32, "", True), (256, 4304, 1152, "act", False), (128, 4304, 1152, "act", True),
+    (200, 1024, 1024, "glu", False)])
 def test_line_between_the_few_row_and_the_persistent_kernel(M, N, K, end, want):
     """Products of 65 - 768 rows of an inference pass: the few-row kernel where the sum is long enough for the area."""
     from opentau_b200.ops import cuda_ops
